@@ -267,6 +267,7 @@ __device__ __forceinline__ void gemm_i8_device(const CUtensorMap& tmW, const CUt
       }
       tc_fence_before_sync();
       mbar_arrive(&tm_empty[b]);
+      fence_proxy_async_smem();                // the next scale rows arrive through the async proxy: not before the reads above
       mbar_arrive(&empty_bar[s]);
     }
     float* P = reinterpret_cast<float*>(smem);

@@ -1,0 +1,31 @@
+"""8-bit-activation GEMMs whose k loop comes round to a stage again: repeated launches give the same bits, and every row is scaled by its
+own block factors."""
+import pytest
+import torch
+
+from fastllm_b200.ops import quant_gemm as QG
+from fastllm_b200.ops.quant import LinearWeight
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["fp8", "int8", "int4g128"])
+@pytest.mark.parametrize("rows", [9, 32, 64, 128])
+def test_stages_are_not_refilled_under_their_readers(kind, rows):
+    if kind == "int4g128" and rows > 64:
+        rows = 61
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    n, k = 28672, 4096                       # one CTA per output tile: 32 k blocks through at most 8 stages
+    w = LinearWeight.from_dense((torch.randn(n, k, device="cuda", generator=g) * 0.02).bfloat16(), kind)
+    # blocks of very different sizes: a factor of another block is off by orders of magnitude
+    x = (torch.randn(rows, k, device="cuda", generator=g) * torch.exp2(torch.randint(-6, 7, (rows, k // 128, 1), device="cuda", generator=g).float())
+         .expand(-1, -1, 128).reshape(rows, k)).bfloat16()
+    first = w(x)
+    for _ in range(20):
+        assert torch.equal(w(x), first)
+    # both grids are symmetric around what the kernel read; 2^-8: the result's rounding, and fp32 sums of 4096 products
+    want = QG.round_act(x, 1 if kind == "fp8" else 0).double()
+    # the rounded activations are stored in bf16 for this statement: 2^-9 per factor on top
+    want = want @ w.dequant(torch.bfloat16).double().t()
+    err = (first.double() - want).norm(dim=1) / want.norm(dim=1)
+    assert err.max() < 3 * 2.0 ** -8, err
