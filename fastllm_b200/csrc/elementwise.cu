@@ -50,42 +50,52 @@ struct NormQuantOut {
   int ld_a;
 };
 
-template <bool BF16, int QMODE = 0>
-__global__ void rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ y,
+// A row's vectors stay in registers, NV of 16 bytes a thread (up to NV * 8 * blockDim columns).  Few rows (decode): a vector a thread, the latency
+// of one load, one reduction and one store; many rows: four vectors a thread, so that 16 rows of 8 KB are in flight on an SM (bound by the
+// row's two passes over DRAM: 8190 x 4096 in 25 us, 58 us with the row staged as fp32 in shared memory behind 512 threads).
+template <bool BF16, int QMODE, int NV>
+__global__ void __launch_bounds__(1024) rmsnorm_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, uint16_t* __restrict__ y,
                                uint16_t* residual, int H, int ldx, int ldy, float eps, float unit_offset, NormQuantOut qo = {}) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float sh[32];
-  extern __shared__ float rowbuf[];   // H floats
-  const int row = blockIdx.x;
+  const int row = blockIdx.x, vecs = H / 8;
   const uint4* xp = reinterpret_cast<const uint4*>(x + (size_t)row * ldx);
   uint4* rp = residual ? reinterpret_cast<uint4*>(residual + (size_t)row * H) : nullptr;
+  uint4 val[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    val[k] = i < vecs ? xp[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
   float ss = 0.f;
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-    uint4 v = xp[i];
-    float2 a = unpack_16<BF16>(v.x), b = unpack_16<BF16>(v.y), c = unpack_16<BF16>(v.z), d = unpack_16<BF16>(v.w);
-    if (rp) {
-      uint4 r = rp[i];
-      float2 ra = unpack_16<BF16>(r.x), rb = unpack_16<BF16>(r.y), rc = unpack_16<BF16>(r.z), rd = unpack_16<BF16>(r.w);
-      a.x += ra.x; a.y += ra.y; b.x += rb.x; b.y += rb.y; c.x += rc.x; c.y += rc.y; d.x += rd.x; d.y += rd.y;
-      uint4 o;
-      o.x = pack_16<BF16>(a.x, a.y); o.y = pack_16<BF16>(b.x, b.y); o.z = pack_16<BF16>(c.x, c.y); o.w = pack_16<BF16>(d.x, d.y);
-      rp[i] = o;
-      // keep the rounded value so that the norm sees exactly what later layers will read
-      a = unpack_16<BF16>(o.x); b = unpack_16<BF16>(o.y); c = unpack_16<BF16>(o.z); d = unpack_16<BF16>(o.w);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    float2 a = unpack_16<BF16>(val[k].x), b = unpack_16<BF16>(val[k].y), c = unpack_16<BF16>(val[k].z), d = unpack_16<BF16>(val[k].w);
+    if (rp && i < vecs) {
+      const uint4 r = rp[i];
+      const float2 ra = unpack_16<BF16>(r.x), rb = unpack_16<BF16>(r.y), rc = unpack_16<BF16>(r.z), rd = unpack_16<BF16>(r.w);
+      // the rounded sum: the norm sees exactly what later layers will read
+      val[k] = make_uint4(pack_16<BF16>(a.x + ra.x, a.y + ra.y), pack_16<BF16>(b.x + rb.x, b.y + rb.y), pack_16<BF16>(c.x + rc.x, c.y + rc.y),
+                          pack_16<BF16>(d.x + rd.x, d.y + rd.y));
+      rp[i] = val[k];
+      a = unpack_16<BF16>(val[k].x); b = unpack_16<BF16>(val[k].y); c = unpack_16<BF16>(val[k].z); d = unpack_16<BF16>(val[k].w);
     }
-    float* rb_ = rowbuf + i * 8;
-    rb_[0] = a.x; rb_[1] = a.y; rb_[2] = b.x; rb_[3] = b.y; rb_[4] = c.x; rb_[5] = c.y; rb_[6] = d.x; rb_[7] = d.y;
     ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
   }
   ss = block_sum(ss, sh);
   const float inv = rsqrtf(ss / (float)H + eps);
   const uint4* wp = reinterpret_cast<const uint4*>(w);
   uint4* yp = reinterpret_cast<uint4*>(y + (size_t)row * ldy);
-  for (int i = threadIdx.x; i < H / 8; i += blockDim.x) {
-    uint4 wv = wp[i];
-    float2 wa = unpack_16<BF16>(wv.x), wb = unpack_16<BF16>(wv.y), wc = unpack_16<BF16>(wv.z), wd = unpack_16<BF16>(wv.w);
-    const float* r = rowbuf + i * 8;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i >= vecs) break;
+    const uint4 wv = wp[i];
+    const float2 wa = unpack_16<BF16>(wv.x), wb = unpack_16<BF16>(wv.y), wc = unpack_16<BF16>(wv.z), wd = unpack_16<BF16>(wv.w);
+    const float2 r0 = unpack_16<BF16>(val[k].x), r1 = unpack_16<BF16>(val[k].y), r2 = unpack_16<BF16>(val[k].z), r3 = unpack_16<BF16>(val[k].w);
+    const float r[8] = {r0.x, r0.y, r1.x, r1.y, r2.x, r2.y, r3.x, r3.y};
     uint4 o;
     o.x = pack_16<BF16>(r[0] * inv * (wa.x + unit_offset), r[1] * inv * (wa.y + unit_offset));
     o.y = pack_16<BF16>(r[2] * inv * (wb.x + unit_offset), r[3] * inv * (wb.y + unit_offset));
@@ -311,6 +321,107 @@ __global__ void qkv_post_kernel(const QkvPostParams p) {
       *reinterpret_cast<unsigned short*>(da + 2 * i) = a8;
       *reinterpret_cast<unsigned short*>(db + 2 * i) = e4m3x2_of((r.x - af.x) * 16.0f, (r.y - af.y) * 16.0f);
     }
+  }
+}
+
+// The same with 16-byte accesses, where the widths allow it: a thread owns the two vectors of eight elements that a rotation pairs (a head of 128
+// takes 8 threads, so a warp has four heads under way) and walks IT heads, whose loads are requested together and which share the
+// token's angles in registers.  Bound by reading and writing the rows once: 8190 tokens x 48 heads x 128 in 38 us (182 us a warp per head).
+template <bool BF16, int IT>
+__global__ void __launch_bounds__(256) qkv_rows_kernel(const QkvPostParams p, int warps_per_tok) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int gw = (int)((blockIdx.x * 256 + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const int tok = gw / warps_per_tok, part = gw - tok * warps_per_tok;
+  if (tok >= p.M) return;
+  const int D = p.D, units = D >> 4, per = 32 / units;                     // threads of a head, heads of a warp
+  const int u = lane % units, sub = lane / units, heads = p.Hq + 2 * p.Hkv;
+  const int half = p.rot >> 1;
+  const bool neox = p.rope_mode == 1;
+  const bool turns = p.rope_mode != 0 && (neox ? 8 * u < half : 16 * u < p.rot);
+  // elements of this thread's two vectors
+  const int rest = p.rope_mode == 1 ? u - (half >> 3) : u;
+  const int e0 = neox ? (turns ? 8 * u : p.rot + 16 * rest) : 16 * u, e1 = neox && turns ? half + 8 * u : e0 + 8;
+  const uint16_t* row = p.qkv + (size_t)tok * p.ld_qkv;
+  uint4 va[IT], vb[IT];
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int head = (part * IT + it) * per + sub;
+    if (head < heads) {
+      va[it] = *reinterpret_cast<const uint4*>(row + (size_t)head * D + e0);
+      vb[it] = *reinterpret_cast<const uint4*>(row + (size_t)head * D + e1);
+    } else {
+      va[it] = vb[it] = make_uint4(0u, 0u, 0u, 0u);
+    }
+  }
+  const int slot = p.slots[tok];
+  float cs[8], sn[8];
+  if (turns) {
+    const size_t at = (size_t)p.positions[tok] * half + 8 * u;
+    const float4 c0 = *reinterpret_cast<const float4*>(p.cos_tab + at), c1 = *reinterpret_cast<const float4*>(p.cos_tab + at + 4);
+    const float4 s0 = *reinterpret_cast<const float4*>(p.sin_tab + at), s1 = *reinterpret_cast<const float4*>(p.sin_tab + at + 4);
+    cs[0] = c0.x; cs[1] = c0.y; cs[2] = c0.z; cs[3] = c0.w; cs[4] = c1.x; cs[5] = c1.y; cs[6] = c1.z; cs[7] = c1.w;
+    sn[0] = s0.x; sn[1] = s0.y; sn[2] = s0.z; sn[3] = s0.w; sn[4] = s1.x; sn[5] = s1.y; sn[6] = s1.z; sn[7] = s1.w;
+  }
+#pragma unroll
+  for (int it = 0; it < IT; ++it) {
+    const int head = (part * IT + it) * per + sub;
+    const bool is_q = head < p.Hq, is_k = !is_q && head < p.Hq + p.Hkv;
+    float a[8], b[8];
+    const uint32_t au[4] = {va[it].x, va[it].y, va[it].z, va[it].w}, bu[4] = {vb[it].x, vb[it].y, vb[it].z, vb[it].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = unpack_16<BF16>(au[j]), g = unpack_16<BF16>(bu[j]);
+      a[2 * j] = f.x; a[2 * j + 1] = f.y; b[2 * j] = g.x; b[2 * j + 1] = g.y;
+    }
+    if (p.q_norm_w != nullptr || p.k_norm_w != nullptr) {
+      float ss = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += a[j] * a[j] + b[j] * b[j];
+      for (int o = units >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const uint16_t* nw = is_q ? p.q_norm_w : is_k ? p.k_norm_w : nullptr;
+      if (nw != nullptr) {
+        const float inv = rsqrtf(ss / (float)D + p.eps);
+        const uint4 wa = *reinterpret_cast<const uint4*>(nw + e0), wb = *reinterpret_cast<const uint4*>(nw + e1);
+        const uint32_t wu[4] = {wa.x, wa.y, wa.z, wa.w}, xu[4] = {wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {          // rounded to the storage type after the norm, as a separate norm would
+          const float2 f = unpack_16<BF16>(wu[j]), g = unpack_16<BF16>(xu[j]);
+          const float2 r = unpack_16<BF16>(pack_16<BF16>(a[2 * j] * inv * (f.x + p.norm_unit_offset), a[2 * j + 1] * inv * (f.y + p.norm_unit_offset)));
+          const float2 t = unpack_16<BF16>(pack_16<BF16>(b[2 * j] * inv * (g.x + p.norm_unit_offset), b[2 * j + 1] * inv * (g.y + p.norm_unit_offset)));
+          a[2 * j] = r.x; a[2 * j + 1] = r.y; b[2 * j] = t.x; b[2 * j + 1] = t.y;
+        }
+      }
+    }
+    if (head >= heads) continue;
+    if (turns && (is_q || is_k)) {
+      if (neox) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float x = a[j], y = b[j];
+          a[j] = x * cs[j] - y * sn[j];
+          b[j] = y * cs[j] + x * sn[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float x = a[2 * j], y = a[2 * j + 1], z = b[2 * j], t = b[2 * j + 1];
+          a[2 * j] = x * cs[j] - y * sn[j];
+          a[2 * j + 1] = x * sn[j] + y * cs[j];
+          b[2 * j] = z * cs[4 + j] - t * sn[4 + j];
+          b[2 * j + 1] = z * sn[4 + j] + t * cs[4 + j];
+        }
+      }
+    }
+    uint16_t* dst;
+    if (is_q) {
+      dst = p.q_out + (size_t)tok * p.ld_q + (size_t)head * D;
+    } else {
+      if (slot < 0) continue;
+      dst = (is_k ? p.k_pool : p.v_pool) + ((size_t)slot * p.Hkv + (is_k ? head - p.Hq : head - p.Hq - p.Hkv)) * D;
+    }
+    *reinterpret_cast<uint4*>(dst + e0) = make_uint4(pack_16<BF16>(a[0], a[1]), pack_16<BF16>(a[2], a[3]), pack_16<BF16>(a[4], a[5]), pack_16<BF16>(a[6], a[7]));
+    *reinterpret_cast<uint4*>(dst + e1) = make_uint4(pack_16<BF16>(b[0], b[1]), pack_16<BF16>(b[2], b[3]), pack_16<BF16>(b[4], b[5]), pack_16<BF16>(b[6], b[7]));
   }
 }
 
@@ -724,6 +835,20 @@ __global__ void route_topk_kernel(const RouteParams p) {
 
 using namespace fb;
 
+// Two waves of one CTA an SM or fewer: a vector a thread; more rows: four a thread, two where that leaves no full warp group.
+template <bool BF16, int QMODE>
+static void launch_rmsnorm(const void* x, const void* w, void* y, void* residual, int M, int H, int ldx, int ldy, float eps, float unit_offset, const NormQuantOut& qo,
+                           cudaStream_t s) {
+  const int vecs = H / 8;
+  const int nv = vecs > 1024 ? 4 : M <= 296 ? 1 : vecs > 256 ? 4 : vecs > 128 ? 2 : 1;
+  const int threads = ((vecs + nv - 1) / nv + 31) / 32 * 32;
+#define FB_NORM(NV)                                                                                                                             \
+  launch_k(rmsnorm_kernel<BF16, QMODE, NV>, dim3(M), dim3(threads), 0, s, 0, (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, (uint16_t*)residual, H, ldx, ldy, \
+           eps, unit_offset, qo);
+  if (nv == 1) { FB_NORM(1) } else if (nv == 2) { FB_NORM(2) } else { FB_NORM(4) }
+#undef FB_NORM
+}
+
 // RMSNorm that also emits the row quantised for an 8-bit-activation GEMM (mode 1: int8 + scales + block sums, mode 2: e4m3 +
 // scales; scale tables [H / 128, ld_a]), or writes y rounded to the int8 (mode 3) / e4m3 (mode 4) grid.  H % 128 == 0.
 extern "C" int fb_rmsnorm_quant(const void* x, const void* w, void* y, void* residual, int M, int H, int ldx, int ldy, float eps,
@@ -731,19 +856,10 @@ extern "C" int fb_rmsnorm_quant(const void* x, const void* w, void* y, void* res
                                 void* stream) {
   if (M <= 0) return 0;
   if (H % 128 != 0 || H > 32768 || mode < 1 || mode > 4 || (mode <= 2 && ldq % 8 != 0)) return -1;
-  int threads = H / 8;
-  threads = threads > 1024 ? 1024 : ((threads + 31) / 32) * 32;
-  const size_t smem = (size_t)H * sizeof(float);
   auto s = reinterpret_cast<cudaStream_t>(stream);
   NormQuantOut qo;
   qo.xq = (uint8_t*)xq; qo.ldq = ldq; qo.scales = scales; qo.sums = sums; qo.ld_a = ld_a;
-#define FB_NQ(BF, QM)                                                                                                          \
-  {                                                                                                                            \
-    static DeviceOnce cfg;                                                                                                     \
-    if (cfg.need()) { cudaFuncSetAttribute(rmsnorm_kernel<BF, QM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4); }  \
-    launch_k(rmsnorm_kernel<BF, QM>, dim3(M), dim3(threads), smem, s, 0, (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, \
-             (uint16_t*)residual, H, ldx, ldy, eps, unit_offset, qo);                                                          \
-  }
+#define FB_NQ(BF, QM) launch_rmsnorm<BF, QM>(x, w, y, residual, M, H, ldx, ldy, eps, unit_offset, qo, s);
   if (dtype == 1) { if (mode == 1) FB_NQ(true, 1) else if (mode == 2) FB_NQ(true, 2) else if (mode == 3) FB_NQ(true, 3) else FB_NQ(true, 4) }
   else { if (mode == 1) FB_NQ(false, 1) else if (mode == 2) FB_NQ(false, 2) else if (mode == 3) FB_NQ(false, 3) else FB_NQ(false, 4) }
 #undef FB_NQ
@@ -754,19 +870,9 @@ extern "C" int fb_rmsnorm(const void* x, const void* w, void* y, void* residual,
                           float unit_offset, int dtype, void* stream) {
   if (M <= 0) return 0;
   if (H % 8 != 0 || H > 32768) return -1;
-  int threads = H / 8;
-  threads = threads > 1024 ? 1024 : ((threads + 31) / 32) * 32;
-  const size_t smem = (size_t)H * sizeof(float);
   auto s = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == 1) {
-    static DeviceOnce cfg;
-    if (cfg.need()) { cudaFuncSetAttribute(rmsnorm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4); }
-    launch_k(rmsnorm_kernel<true>, dim3(M), dim3(threads), smem, s, 0, (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, (uint16_t*)residual, H, ldx, ldy, eps, unit_offset, NormQuantOut{});
-  } else {
-    static DeviceOnce cfg;
-    if (cfg.need()) { cudaFuncSetAttribute(rmsnorm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 32768 * 4); }
-    launch_k(rmsnorm_kernel<false>, dim3(M), dim3(threads), smem, s, 0, (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, (uint16_t*)residual, H, ldx, ldy, eps, unit_offset, NormQuantOut{});
-  }
+  if (dtype == 1) launch_rmsnorm<true, 0>(x, w, y, residual, M, H, ldx, ldy, eps, unit_offset, NormQuantOut{}, s);
+  else launch_rmsnorm<false, 0>(x, w, y, residual, M, H, ldx, ldy, eps, unit_offset, NormQuantOut{}, s);
   return (int)cudaGetLastError();
 }
 
@@ -782,10 +888,27 @@ extern "C" int fb_qkv_post(const void* qkv, int ld_qkv, void* q_out, int ld_q, v
   p.q_norm_w = (const uint16_t*)q_norm_w; p.k_norm_w = (const uint16_t*)k_norm_w; p.cos_tab = cos_tab; p.sin_tab = sin_tab;
   p.M = M; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.rot = rot; p.rope_mode = rope_mode; p.eps = eps; p.norm_unit_offset = norm_unit_offset;
   p.kv8 = 0; p.q8a = nullptr; p.q8b = nullptr;
+  auto s = reinterpret_cast<cudaStream_t>(stream);
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  // whole pairs of vectors: the rotated part (its halves, where they pair) and what lies behind it in multiples of 16 elements, a power of two of
+  // threads a head, 16-byte rows
+  if ((D == 32 || D == 64 || D == 128 || D == 256 || D == 512) && (rope_mode == 0 || rot % 16 == 0) && ld_qkv % 8 == 0 && ld_q % 8 == 0 && aligned(qkv) &&
+      aligned(q_out) && aligned(k_pool) && aligned(v_pool) && aligned(cos_tab) && aligned(sin_tab) && aligned(q_norm_w) && aligned(k_norm_w)) {
+    if (rope_mode == 0) p.rot = 0;
+    const int per = 512 / D;                             // heads of a warp at a time
+    const int steps = (Hq + 2 * Hkv + per - 1) / per;
+    const int it = M >= 256 ? (steps >= 4 ? 4 : steps >= 2 ? 2 : 1) : 1;       // few tokens: as many warps as there are
+    const int wpt = (steps + it - 1) / it;
+    const dim3 grid((unsigned)(((long long)M * wpt + 7) / 8));
+#define FB_QR(BF, IT) launch_k(qkv_rows_kernel<BF, IT>, grid, dim3(256), 0, s, 0, p, wpt);
+    if (dtype == 1) { if (it == 4) FB_QR(true, 4) else if (it == 2) FB_QR(true, 2) else FB_QR(true, 1) }
+    else { if (it == 4) FB_QR(false, 4) else if (it == 2) FB_QR(false, 2) else FB_QR(false, 1) }
+#undef FB_QR
+    return (int)cudaGetLastError();
+  }
   const long long warps = (long long)M * (Hq + 2 * Hkv);
   const int wpb = 8;
   const int blocks = (int)((warps + wpb - 1) / wpb);
-  auto s = reinterpret_cast<cudaStream_t>(stream);
   if (dtype == 1) launch_k(qkv_post_kernel<true>, dim3(blocks), dim3(wpb * 32), 0, s, 0, p);
   else launch_k(qkv_post_kernel<false>, dim3(blocks), dim3(wpb * 32), 0, s, 0, p);
   return (int)cudaGetLastError();
