@@ -4,9 +4,9 @@
 //                pair its row in the expert-sorted buffer (-1 if the expert lives on another rank).  Deterministic:
 //                rows inside a segment follow (token, k) order.
 //   moe_gather   copies each routed token row into its sorted position
-//   grouped GEMM the swap-AB tcgen05 decode GEMM run once per (expert, 128/256-token chunk) through blockIdx.z; the
-//                weight tile coordinate is offset into the stacked expert matrix, the activation tile into the sorted
-//                buffer; experts without tokens exit at once.  gate/up uses the SwiGLU epilogue.
+//   grouped GEMM swap-AB tcgen05 products of all experts in one persistent launch (moe_stream_kernel): a tile list over the
+//                experts that got rows, weights from the stacked matrix, activations from the sorted buffer.  gate/up uses
+//                the SwiGLU epilogue.
 //   moe_combine  out[t] = sum_k w[t,k] * y_sorted[pos[t,k]]   in fixed k order (deterministic)
 //
 // Role of the reference's MergeMOE / FusedMOE (src/devices/cuda/cudadevice.cpp:8279-8562) and of its routed-row
@@ -22,68 +22,11 @@ namespace fb {
 
 constexpr int KID_MOE_GROUPED = 40;
 
-struct MoeGroupInfo {
-  const int* counts;       // [E_local] routed rows per expert
-  const int* offsets;      // [E_local] first row of the expert's segment in the sorted buffer
-  int rows_per_chunk;      // MPAD
-  int chunks;              // blockIdx.z = expert * chunks + chunk
-  int n_rows_w;            // weight rows per expert in the stacked matrix
-  long long out_stride_e;  // unused (outputs follow the sorted rows)
-  int ld_bias_e;           // bias elements per expert (0: no per-expert stride)
-  int n_local, compact;    // compact: grid.z enumerates existing (expert, chunk) pairs (moe_find_item)
-};
-
-// counts / offsets / pos of the experts in [first, first + n_local).
-// Small problems (pairs <= 4096): one thread per (token, k) pair; rank inside the expert segment = number of earlier pairs
-// routed to the same expert, so the order is deterministic without any sorting pass.
-__global__ void moe_plan_small_kernel(const int* __restrict__ idx, int pairs, int first, int n_local, int* __restrict__ counts,
-                                      int* __restrict__ offsets, int* __restrict__ pos, int* __restrict__ total_rows, int pad) {
-  __shared__ int s_idx[4096];
-  __shared__ int s_cnt[1024];
-  __shared__ int s_off[1024];
-  pdl_launch_dependents();
-  pdl_wait();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = idx[i] - first;
-    s_idx[i] = (e >= 0 && e < n_local) ? e : -1;
-  }
-  for (int e = threadIdx.x; e < n_local; e += blockDim.x) s_cnt[e] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x)
-    if (s_idx[i] >= 0) atomicAdd(&s_cnt[s_idx[i]], 1);
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    // warp-level exclusive scan of the padded counts, 32 experts at a time
-    int carry = 0;
-    for (int base = 0; base < n_local; base += 32) {
-      const int e = base + threadIdx.x;
-      const int c = e < n_local ? (s_cnt[e] + pad - 1) / pad * pad : 0;
-      int incl = c;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)threadIdx.x >= o) incl += v;
-      }
-      if (e < n_local) s_off[e] = carry + incl - c;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (threadIdx.x == 0) *total_rows = carry;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < n_local; e += blockDim.x) { counts[e] = s_cnt[e]; offsets[e] = s_off[e]; }
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-    const int e = s_idx[i];
-    if (e < 0) { pos[i] = -1; continue; }
-    int rank = 0;
-    for (int j = 0; j < i; ++j) rank += (s_idx[j] == e);
-    pos[i] = s_off[e] + rank;
-  }
-}
-
-// The same plan with warp votes: pairs are taken in chunks of 32; a chunk's lanes learn by `match.any` how many earlier lanes
+// counts / offsets / pos of the experts in [first, first + n_local); rows of a segment follow (token, k) order.
+// One CTA, warp votes: pairs are taken in chunks of 32; a chunk's lanes learn by `match.any` how many earlier lanes
 // go to the same expert, one lane per (chunk, expert) records the chunk's count, a scan over the chunks per expert turns the
-// counts into bases, and rank = base of the chunk + earlier lanes of the chunk.  Same (deterministic) order as above at
-// O(chunks) instead of O(pairs) work per thread.  Needs chunks * n_local <= 8192 (16-bit counts in shared memory).
+// counts into bases, and rank = base of the chunk + earlier lanes of the chunk.  Needs chunks * n_local <= 8192 (16-bit counts in
+// shared memory).
 __global__ void __launch_bounds__(1024)
 moe_plan_warp_kernel(const int* __restrict__ idx, int pairs, int first, int n_local, int* __restrict__ counts,
                      int* __restrict__ offsets, int* __restrict__ pos, int* __restrict__ total_rows, int pad) {
@@ -145,64 +88,63 @@ moe_plan_warp_kernel(const int* __restrict__ idx, int pairs, int first, int n_lo
   }
 }
 
-// Large problems, the same order: every warp owns a contiguous run of pairs.  It counts its experts chunk by chunk (`match.any`, the first
-// lane of an expert adds), a scan over the warps turns the counts into first rows, and a second walk hands the rows out.
-// Shared memory: [32 warps][n_local] counters.
+// Larger problems, the same order: a CTA per 1024 pairs.  It counts the experts of all pairs itself, those before its own apart (the ids are a few
+// hundred KB in L2; no scratch, no second launch, nothing to wait for), then ranks its own pairs like the kernel above, a chunk of 32 a warp.
+// 32760 pairs, 128 experts: 8 us (71 us when one CTA walked all pairs twice).  Shared memory: [2][n_local] counters, [32][n_local] 16-bit ones.
 __global__ void __launch_bounds__(1024)
-moe_plan_large_kernel(const int* __restrict__ idx, int pairs, int first, int n_local, int* __restrict__ counts, int* __restrict__ offsets,
-                      int* __restrict__ pos, int* __restrict__ total_rows, int pad) {
-  extern __shared__ int s_run[];
-  __shared__ int s_cnt[1024];
+moe_plan_blocks_kernel(const int* __restrict__ idx, int pairs, int first, int n_local, int* __restrict__ counts, int* __restrict__ offsets,
+                       int* __restrict__ pos, int* __restrict__ total_rows, int pad) {
+  extern __shared__ int s_dyn[];
+  int* before = s_dyn;                                         // pairs ahead of this CTA's, then their expert's row for its first one
+  int* rest = before + n_local;
+  uint16_t* s_w = reinterpret_cast<uint16_t*>(rest + n_local);
   pdl_launch_dependents();
   pdl_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, start = blockIdx.x * 1024;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  int* run = s_run + warp * n_local;
-  for (int e = lane; e < n_local; e += 32) run[e] = 0;
-  __syncwarp();
-  const int per = ((pairs + 1023) / 1024) * 32;                // pairs of a warp, whole chunks
-  const int i0 = warp * per, i1 = min(pairs, i0 + per);
-  auto expert = [&](int i) {
-    const int e = i < i1 ? idx[i] - first : -1;
-    return e >= 0 && e < n_local ? e : -1;
-  };
-  for (int c = i0; c < i1; c += 32) {
-    const int e = expert(c + lane);
-    const uint32_t same = __match_any_sync(0xffffffffu, e);
-    if (e >= 0 && (same & lt_mask) == 0) run[e] += __popc(same);
-    __syncwarp();
-  }
+  for (int e = tid; e < 2 * n_local; e += 1024) s_dyn[e] = 0;
+  for (int i = tid; i < 16 * n_local; i += 1024) reinterpret_cast<uint32_t*>(s_w)[i] = 0u;
   __syncthreads();
-  for (int e = threadIdx.x; e < n_local; e += blockDim.x) {
-    int n = 0;
-    for (int w = 0; w < 32; ++w) { const int v = s_run[w * n_local + e]; s_run[w * n_local + e] = n; n += v; }
-    s_cnt[e] = n;
+  int own = -1;
+#pragma unroll 4
+  for (int i = tid; i < pairs; i += 1024) {
+    const int e = idx[i] - first;
+    const bool ok = e >= 0 && e < n_local;
+    if (ok) atomicAdd(i < start ? before + e : rest + e, 1);
+    if (i - tid == start) own = ok ? e : -1;
   }
+  const uint32_t same = __match_any_sync(0xffffffffu, own);
+  const int rank = __popc(same & lt_mask);
+  if (own >= 0 && rank == 0) s_w[warp * n_local + own] = (uint16_t)__popc(same);
   __syncthreads();
-  if (warp == 0) {
+  for (int e = tid; e < n_local; e += 1024) {
+    int run = 0;
+    for (int w = 0; w < 32; ++w) {
+      const int v = s_w[w * n_local + e];
+      s_w[w * n_local + e] = (uint16_t)run;
+      run += v;
+    }
+  }
+  if (warp == 31) {
     int carry = 0;
     for (int base = 0; base < n_local; base += 32) {
-      const int e = base + lane, n = e < n_local ? s_cnt[e] : 0, c = (n + pad - 1) / pad * pad;
+      const int e = base + lane, b = e < n_local ? before[e] : 0, n = e < n_local ? b + rest[e] : 0, c = (n + pad - 1) / pad * pad;
       int incl = c;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += v;
       }
-      if (e < n_local) { counts[e] = n; offsets[e] = s_cnt[e] = carry + incl - c; }
+      if (e < n_local) {
+        before[e] = carry + incl - c + b;
+        if (blockIdx.x == 0) { counts[e] = n; offsets[e] = carry + incl - c; }
+      }
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) *total_rows = carry;
+    if (lane == 0 && blockIdx.x == 0) *total_rows = carry;
   }
   __syncthreads();
-  for (int c = i0; c < i1; c += 32) {
-    const int e = expert(c + lane);
-    const uint32_t same = __match_any_sync(0xffffffffu, e);
-    if (c + lane < i1) pos[c + lane] = e < 0 ? -1 : s_cnt[e] + run[e] + __popc(same & lt_mask);
-    __syncwarp();
-    if (e >= 0 && (same & lt_mask) == 0) run[e] += __popc(same);
-    __syncwarp();
-  }
+  if (start + tid < pairs) pos[start + tid] = own < 0 ? -1 : before[own] + (int)s_w[warp * n_local + own] + rank;
 }
 
 __global__ void moe_gather_kernel(const uint16_t* __restrict__ x, const int* __restrict__ pos, uint16_t* __restrict__ xs, int T,
@@ -299,39 +241,224 @@ moe_plan_table_kernel(const long long* __restrict__ meta, const int* __restrict_
   }
 }
 
-// grouped dense GEMM: one (expert, chunk) per blockIdx.z
-template <int MPAD, bool BF16, class Epi>
+// Grouped dense GEMM: one CTA per SM walks (expert, row chunk, 128 weight rows) tiles, swap-AB as in the decode GEMM (weight rows x tokens).
+//
+// Bound: the weight stream while an expert gets few rows (every touched expert is read once), the tensor core from a few hundred rows on.
+// The tile list is made on the device from the routed counts; the ring of operand stages runs on across tiles, so the short k of
+// an expert's projections (512 to 2048: 8 to 32 stages) does not pay a pipeline fill, a TMEM set-up and a drain per tile, and two
+// accumulators let the epilogue of a tile run under the products of the next.  Chunks of one expert are neighbours in the list: the
+// second reads the weights from L2.  The product is as wide as the chunk has rows (multiples of 16), whatever the tile is laid out for.
+// Per layer of width 2048 (gate/up + down; us; one CTA per tile before): 128 experts x 768 at 4095 x 8 rows 948 -> 600, 512 x 512 at 4001 x 10
+// rows 1597 -> 640, at 32 x 10 rows 657 -> 263, 128 x 768 at 32 x 8 rows 237 -> 179.
+struct MoeStreamInfo {
+  const int* counts;       // [n_local] routed rows per expert
+  const int* offsets;      // [n_local] first row of the expert's segment in the sorted buffer
+  int n_local, n_tiles;    // weight tiles per expert
+};
+
+constexpr int MS_MAX_EXPERTS = 1024;
+template <int MPAD>
+struct MoeStreamCfg {
+  static constexpr int A_BYTES = 128 * 128;
+  static constexpr int BOX = MPAD < 64 ? MPAD : 64;                 // token rows per load
+  static constexpr int STAGE_BYTES = A_BYTES + MPAD * 128;
+  static constexpr int X_BYTES = 2 * 32 * 64 * 4;                   // up sums on their way to the gate's warps, two buffers of 32 tokens
+  static constexpr int TAIL_BYTES = X_BYTES + (MS_MAX_EXPERTS + 1) * 4 + 28 + 512;
+  static constexpr int MAX_STAGES = (226 * 1024 - TAIL_BYTES) / STAGE_BYTES;
+  static constexpr int STAGES = MAX_STAGES > 12 ? 12 : MAX_STAGES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES + 1024;
+  static constexpr int TMEM_COLS = 2 * MPAD < 32 ? 32 : 2 * MPAD;
+};
+
+struct MoeTile { int e, n_tile, row0, rows; };
+// tile t of the list; first[e] = chunks of the experts before e
+template <int MPAD>
+__device__ __forceinline__ MoeTile moe_tile(const MoeStreamInfo& gi, const int* first, int t) {
+  int lo = 0, hi = gi.n_local - 1;                     // the last expert whose first tile is at or before t
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (first[mid] * gi.n_tiles <= t) lo = mid; else hi = mid - 1;
+  }
+  MoeTile r;
+  const int ch = first[lo + 1] - first[lo], at = t - first[lo] * gi.n_tiles, cnt = gi.counts[lo];
+  const int per = ((cnt + ch - 1) / ch + 15) & ~15;    // rows of a chunk: equal shares, at most MPAD
+  const int chunk = at % ch;
+  r.e = lo;
+  r.n_tile = at / ch;
+  r.row0 = chunk * per;
+  r.rows = min(per, cnt - r.row0);
+  return r;
+}
+
+template <int MPAD, bool BF16, bool EXTRA>
 __global__ void __launch_bounds__(192, 1)
-moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmParams base,
-                        const MoeGroupInfo gi) {
-  int e = blockIdx.z / gi.chunks, chunk = blockIdx.z - e * gi.chunks;
+moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmParams p, const MoeStreamInfo gi) {
+  using Cfg = MoeStreamCfg<MPAD>;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ int wsum[6];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  float* X = reinterpret_cast<float*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
+  int* first = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(X) + Cfg::X_BYTES);              // [n_local + 1]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(first + MS_MAX_EXPERTS + 8);
+  uint64_t* empty_bar = full_bar + Cfg::STAGES;
+  uint64_t* acc_full = empty_bar + Cfg::STAGES;        // [2]
+  uint64_t* acc_empty = acc_full + 2;                  // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  bool dead = false;
   pdl_launch_dependents();
-  pdl_wait();   // counts / offsets come from the plan kernel
-  if (gi.compact && !moe_find_item(gi.counts, gi.n_local, gi.rows_per_chunk, (int)blockIdx.z, e, chunk)) return;
-  const int cnt = gi.counts[e];
-  const int row0 = chunk * gi.rows_per_chunk;
-  if (row0 >= cnt) return;                          // uniform over the cluster (same blockIdx.z)
-  GemmParams p = base;
-  const int seg = gi.offsets[e] + row0;
-  p.M = cnt - row0 < gi.rows_per_chunk ? cnt - row0 : gi.rows_per_chunk;
-  p.x_row0 = seg;
-  p.w_row0 = e * gi.n_rows_w;
-  const int out_cols = (p.flags & GEMM_SWIGLU) ? (p.N >> 1) : p.N;
-  (void)out_cols;
-  p.out = reinterpret_cast<uint16_t*>(base.out) + (size_t)seg * base.ld_out;
-  if (base.bias != nullptr) p.bias = reinterpret_cast<const uint16_t*>(base.bias) + (size_t)e * gi.ld_bias_e;
-  uint32_t tmem_base;
-  gemm_smallm_device<MPAD, BF16, 1, Epi>(tmW, tmX, p, tmem_base, KID_MOE_GROUPED, Epi());
-  if ((threadIdx.x >> 5) == 1) tmem_dealloc(tmem_base, SmallMCfg<MPAD, 1>::TMEM_COLS);
+  if (tid == 0) {
+    for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+    mbar_init_fence();
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
+  pdl_wait();                                          // counts and offsets come from the plan kernel
+  {
+    const int each = (gi.n_local + 191) / 192, e0 = tid * each;
+    int sum = 0;
+    for (int i = 0; i < each; ++i) sum += e0 + i < gi.n_local ? (gi.counts[e0 + i] + MPAD - 1) / MPAD : 0;
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    int run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += wsum[w];
+    for (int i = 0; i < each; ++i) {
+      if (e0 + i >= gi.n_local) break;
+      first[e0 + i] = run;
+      run += (gi.counts[e0 + i] + MPAD - 1) / MPAD;
+      if (e0 + i == gi.n_local - 1) first[gi.n_local] = run;
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const int total = first[gi.n_local] * gi.n_tiles, kb_cnt = p.kb_total;
+
+  if (warp == 0) {
+    if (elect_one()) {
+      const uint64_t pol_w = l2_policy_evict_first();
+      const uint64_t pol_x = l2_policy_evict_last();
+      int it = 0;
+      for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
+        const MoeTile m = moe_tile<MPAD>(gi, first, t);
+        if (m.rows <= 0) continue;
+        const int w_row = (m.e * gi.n_tiles + m.n_tile) * 128, x_row = gi.offsets[m.e] + m.row0, boxes = (m.rows + Cfg::BOX - 1) / Cfg::BOX;
+        for (int i = 0; i < kb_cnt; ++i, ++it) {
+          const int s = it % Cfg::STAGES;
+          if (!mbar_wait(&empty_bar[s], ((uint32_t)(it / Cfg::STAGES) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 1)) break;
+          uint8_t* a = smem + s * Cfg::STAGE_BYTES;
+          mbar_expect_tx(&full_bar[s], Cfg::A_BYTES + boxes * Cfg::BOX * 128);
+          if (MPAD <= 64) tma_load_2d_hint(a, &tmW, &full_bar[s], i * 64, w_row, pol_w);
+          else tma_load_2d(a, &tmW, &full_bar[s], i * 64, w_row);                 // (the expert's next chunk reads them again)
+          for (int b = 0; b < boxes; ++b) tma_load_2d_hint(a + Cfg::A_BYTES + b * Cfg::BOX * 128, &tmX, &full_bar[s], i * 64, x_row + b * Cfg::BOX, pol_x);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (elect_one()) {
+      int it = 0, u = 0;
+      for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
+        const MoeTile m = moe_tile<MPAD>(gi, first, t);
+        if (m.rows <= 0) continue;
+        const int buf = u & 1;
+        if (!mbar_wait(&acc_empty[buf], ((uint32_t)(u >> 1) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 4)) break;
+        tc_fence_after_sync();
+        const uint32_t acc = tmem_base + (uint32_t)(buf * MPAD), idesc = p.idesc | ((uint32_t)((m.rows + 15) >> 4) << 18);      // N = rows in multiples of 16
+        for (int i = 0; i < kb_cnt; ++i, ++it) {
+          const int s = it % Cfg::STAGES;
+          if (!mbar_wait(&full_bar[s], (uint32_t)(it / Cfg::STAGES) & 1u, dead, KID_MOE_GROUPED, 2)) break;
+          tc_fence_after_sync();
+          const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
+          const uint64_t da = make_smem_desc(a_addr, 16, 1024, SWZ_128B), db = make_smem_desc(a_addr + Cfg::A_BYTES, 16, 1024, SWZ_128B);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f16(acc, da + 2 * k, db + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+          umma_commit(&empty_bar[s]);
+        }
+        if (dead) break;
+        umma_commit(&acc_full[buf]);
+        ++u;
+      }
+    }
+    __syncwarp();
+  } else {
+    // a thread whose wait ran out still walks the tiles: it meets the named barriers below
+    const int q = warp & 3, n_local = q * 32 + lane;
+    const bool swiglu = (p.flags & GEMM_SWIGLU) != 0;
+    uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
+    int u = 0, ci = 0;                                 // tiles and 32-token pieces done
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      const MoeTile m = moe_tile<MPAD>(gi, first, t);
+      if (m.rows <= 0) continue;
+      const int buf = u & 1;
+      mbar_wait(&acc_full[buf], (uint32_t)(u >> 1) & 1u, dead, KID_MOE_GROUPED, 3);
+      ++u;
+      __syncwarp();
+      tc_fence_after_sync();
+      const uint32_t acc = tmem_base + (uint32_t)(buf * MPAD) + ((uint32_t)(q * 32) << 16);
+      uint16_t* orow = outp + (size_t)(gi.offsets[m.e] + m.row0) * p.ld_out;
+      constexpr int CH = MPAD < 32 ? MPAD : 32;
+      for (int c0 = 0; c0 < m.rows; c0 += CH, ++ci) {
+        uint32_t r[32];
+        __syncwarp();
+        if (CH == 32) tmem_ld_32x32b_x32(acc + c0, r); else tmem_ld_32x32b_x16(acc + c0, r);
+        tmem_ld_wait();
+        const int cnt = min(CH, m.rows - c0);
+        if (swiglu) {
+          // rows 0..63 of a tile are gate rows, 64..127 the up rows of the same columns: barrier 1 + b "buffer b holds up sums", 3 + b "buffer b has been read"
+          const int b = ci & 1;
+          float* xb = X + b * 32 * 64;
+          if (q >= 2) {
+            if (ci >= 2) asm volatile("bar.sync %0, 128;\n" ::"r"(3 + b) : "memory");
+#pragma unroll
+            for (int j = 0; j < CH; ++j) xb[j * 64 + n_local - 64] = __uint_as_float(r[j]);
+            asm volatile("bar.arrive %0, 128;\n" ::"r"(1 + b) : "memory");
+          } else {
+            asm volatile("bar.sync %0, 128;\n" ::"r"(1 + b) : "memory");
+            const int n = m.n_tile * 64 + n_local;
+            const bool live = !dead && n < (p.N >> 1);
+#pragma unroll
+            for (int j = 0; j < CH; ++j) {
+              const float g = __uint_as_float(r[j]), up = xb[j * 64 + n_local];
+              const float v = (p.flags & GEMM_GLU_CLAMP) ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : silu_f(g) * up;
+              if (live && j < cnt) orow[(size_t)(c0 + j) * p.ld_out + n] = (uint16_t)(pack_16<BF16>(v, 0.f) & 0xFFFFu);
+            }
+            asm volatile("bar.arrive %0, 128;\n" ::"r"(3 + b) : "memory");
+          }
+        } else {
+          const int n = m.n_tile * 128 + n_local;
+          const bool live = !dead && n < p.N;
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            float v = __uint_as_float(r[j]);
+            if (EXTRA && (p.flags & GEMM_GELU)) v = gelu_erf_f(v);
+            if (live && j < cnt) orow[(size_t)(c0 + j) * p.ld_out + n] = (uint16_t)(pack_16<BF16>(v, 0.f) & 0xFFFFu);
+          }
+        }
+      }
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+    }
+    if (swiglu && q >= 2)                              // the last two buffers' arrivals are taken, too
+      for (int k = ci > 2 ? ci - 2 : 0; k < ci; ++k) asm volatile("bar.sync %0, 128;\n" ::"r"(3 + (k & 1)) : "memory");
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
 }
 
 template <int MPAD, bool BF16>
-static cudaError_t launch_grouped(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, const MoeGroupInfo& gi,
-                                  int nsplit, int n_tiles, int nz, cudaStream_t stream) {
-  using Cfg = SmallMCfg<MPAD, 1>;
-  auto plain = moe_grouped_gemm_kernel<MPAD, BF16, StoreEpilogue<BF16>>;
-  auto extra = moe_grouped_gemm_kernel<MPAD, BF16, ExtraEpilogue<BF16>>;
-  auto kern = (p.flags & GEMM_EXTRA_FLAGS) ? extra : plain;
+static cudaError_t launch_stream(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, const MoeStreamInfo& gi, int grid, cudaStream_t stream) {
+  using Cfg = MoeStreamCfg<MPAD>;
+  auto plain = moe_stream_kernel<MPAD, BF16, false>;
+  auto extra = moe_stream_kernel<MPAD, BF16, true>;
   static DeviceOnce configured;
   if (configured.need()) {
     cudaError_t e = cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
@@ -339,15 +466,13 @@ static cudaError_t launch_grouped(const CUtensorMap& tmW, const CUtensorMap& tmX
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nsplit, n_tiles, nz);
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = nsplit; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, 1);
-  return cudaLaunchKernelEx(&cfg, kern, tmW, tmX, p, gi);
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, 0);
+  return cudaLaunchKernelEx(&cfg, (p.flags & GEMM_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
 }
 
 }  // namespace fb
@@ -357,19 +482,15 @@ using namespace fb;
 extern "C" int fb_moe_plan(const int* idx, int T, int topk, int first, int n_local, int* counts, int* offsets, int* pos,
                            int* total_rows, int pad, void* stream) {
   if (n_local <= 0 || n_local > 1024 || T <= 0) return -1;
-  static const bool warp_plan = [] { const char* e = getenv("FB_MOE_PLAN_WARP"); return !(e && e[0] == '0'); }();
-  if (warp_plan && T * topk <= 4096 && ((T * topk + 31) / 32) * n_local <= 8192) {
-    launch_k(moe_plan_warp_kernel, dim3(1), dim3(1024), 0, reinterpret_cast<cudaStream_t>(stream), 0, idx, T * topk, first, n_local, counts, offsets, pos, total_rows, pad);
+  auto s = reinterpret_cast<cudaStream_t>(stream);
+  const int pairs = T * topk;
+  if (pairs <= 4096 && ((pairs + 31) / 32) * n_local <= 8192) {
+    launch_k(moe_plan_warp_kernel, dim3(1), dim3(1024), 0, s, 0, idx, pairs, first, n_local, counts, offsets, pos, total_rows, pad);
     return (int)cudaGetLastError();
   }
-  if (T * topk <= 4096) {
-    launch_k(moe_plan_small_kernel, dim3(1), dim3(1024), 0, reinterpret_cast<cudaStream_t>(stream), 0, idx, T * topk, first, n_local, counts, offsets, pos, total_rows, pad);
-    return (int)cudaGetLastError();
-  }
-  const size_t smem = (size_t)32 * n_local * 4;
   static DeviceOnce cfg;
-  if (cfg.need()) cudaFuncSetAttribute(moe_plan_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024 * 4);
-  launch_k(moe_plan_large_kernel, dim3(1), dim3(1024), smem, reinterpret_cast<cudaStream_t>(stream), 0, idx, T * topk, first, n_local, counts, offsets, pos, total_rows, pad);
+  if (cfg.need()) cudaFuncSetAttribute(moe_plan_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 72 * 1024);
+  launch_k(moe_plan_blocks_kernel, dim3((pairs + 1023) / 1024), dim3(1024), (size_t)72 * n_local, s, 0, idx, pairs, first, n_local, counts, offsets, pos, total_rows, pad);
   return (int)cudaGetLastError();
 }
 
@@ -419,49 +540,39 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
                                        int total_rows, float act_limit, float act_alpha, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (E_local <= 0 || rows_cap <= 0) return 0;
-  if (K % 8 != 0 || N % 8 != 0 || ((flags & GEMM_SWIGLU) && N % 128 != 0) || (dtype != 0 && dtype != 1)) return -1;
-  const int n_rows_w = (N + 127) / 128 * 128;
+  if (K % 8 != 0 || N % 8 != 0 || ((flags & GEMM_SWIGLU) && N % 128 != 0) || (dtype != 0 && dtype != 1) || bias != nullptr || E_local > MS_MAX_EXPERTS) return -1;
+  const int n_tiles = (N + 127) / 128;
   const bool bf16 = dtype == 1;
-  // rows per chunk: low 16 bits of max_rows_per_expert = most rows an expert can get, high 16 bits = chunk size hint (0: auto)
-  const int hint = max_rows_per_expert >> 16;
-  max_rows_per_expert &= 0xFFFF;
-  int mpad = max_rows_per_expert <= 16 ? 16 : max_rows_per_expert <= 32 ? 32 : max_rows_per_expert <= 64 ? 64 : 128;
-  if (hint == 16 || hint == 32 || hint == 64 || hint == 128) mpad = hint < mpad ? hint : mpad;
-  const int chunks = (max_rows_per_expert + mpad - 1) / mpad;
-  GemmParams p;
-  p.out = out; p.bias = bias; p.residual = nullptr;
-  p.M = 0; p.N = N; p.K = K; p.ld_out = ld_out; p.ld_res = 0;
-  p.kb_total = (K + 63) / 64; p.flags = flags;
+  // rows the tile is laid out for: low 16 bits of max_rows_per_expert = most rows an expert can get, the rest = rows of a typical busy expert (0: the most)
+  const int hint = max_rows_per_expert >> 16, most = max_rows_per_expert & 0xFFFF, want = hint > 0 && hint < most ? hint : most;
+  int mpad = 16;
+  while (mpad < want && mpad < 256) mpad <<= 1;
+  GemmParams p = {};
+  p.out = out; p.N = N; p.K = K; p.ld_out = ld_out; p.kb_total = (K + 63) / 64; p.flags = flags;
   p.act_limit = act_limit; p.act_alpha = act_alpha;
-  p.scatter_tp = 0; p.scatter_rows = 1; p.scatter_rank = 0; p.w_row0 = 0; p.x_row0 = 0;
-  for (int i = 0; i < 8; ++i) p.scatter_out[i] = nullptr;
-  const int n_tiles = n_rows_w / 128;
-  // k split: keep clusters small, experts already provide parallelism
-  int nsplit = 1;
-  while (nsplit < 4 && n_tiles * E_local * nsplit < 148 && (p.kb_total / (nsplit * 2)) >= 8) nsplit *= 2;
-  p.kb_per_split = (p.kb_total + nsplit - 1) / nsplit;
-  p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, mpad);
-  MoeGroupInfo gi;
-  gi.counts = counts; gi.offsets = offsets; gi.rows_per_chunk = mpad; gi.chunks = chunks; gi.n_rows_w = n_rows_w; gi.out_stride_e = 0;
-  gi.ld_bias_e = N;
+  p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, 0);
+  MoeStreamInfo gi;
+  gi.counts = counts; gi.offsets = offsets; gi.n_local = E_local; gi.n_tiles = n_tiles;
   CUtensorMap tmW, tmX;
-  if (!make_tmap_2d(&tmW, W, (uint64_t)E_local * n_rows_w, K, K, 128, 64, 2, 3)) return -2;
-  if (!make_tmap_2d(&tmX, Xs, rows_cap, K, K, mpad, 64, 2, 3)) return -2;
-  int nz = E_local * chunks;
-  gi.n_local = E_local; gi.compact = 0;
-  if (total_rows > 0) {               // upper bound of the routed rows: one grid slot per existing row chunk
-    const int bound = E_local + (total_rows + mpad - 1) / mpad;
-    if (bound < nz) { nz = bound; gi.compact = 1; }
+  if (!make_tmap_2d(&tmW, W, (uint64_t)E_local * n_tiles * 128, K, K, 128, 64, 2, 3)) return -2;
+  if (!make_tmap_2d(&tmX, Xs, rows_cap, K, K, mpad < 64 ? mpad : 64, 64, 2, 3)) return -2;
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  if (nz > 65535) return -1;
-#define FB_MG(MP)                                                                                              \
-  return (int)(bf16 ? launch_grouped<MP, true>(tmW, tmX, p, gi, nsplit, n_tiles, nz, stream)                    \
-                    : launch_grouped<MP, false>(tmW, tmX, p, gi, nsplit, n_tiles, nz, stream));
+  // no more CTAs than tiles can exist: every routed row touches an expert, every expert's last chunk may be short
+  long long bound = (long long)E_local * ((most + mpad - 1) / mpad);
+  if (total_rows > 0 && bound > (long long)total_rows) bound = total_rows;
+  const int grid = (int)(bound * n_tiles < sms ? bound * n_tiles : sms);
+#define FB_MG(MP) return (int)(bf16 ? launch_stream<MP, true>(tmW, tmX, p, gi, grid, stream) : launch_stream<MP, false>(tmW, tmX, p, gi, grid, stream));
   switch (mpad) {
     case 16: FB_MG(16)
     case 32: FB_MG(32)
     case 64: FB_MG(64)
-    default: FB_MG(128)
+    case 128: FB_MG(128)
+    default: FB_MG(256)
   }
 #undef FB_MG
 }

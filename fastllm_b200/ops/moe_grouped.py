@@ -199,6 +199,8 @@ def forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, experts, add:
     hint = 16 if mean <= 6 else 32 if mean <= 12 else 64 if mean <= 24 else 128
     if st.kind == "int4g" and QG.INT_A8 and mean <= 12:
         hint = 16          # the 16-row integer kernel has dedicated unpack warps; a second chunk re-reads its weights from L2
+    if st.kind == "dense":
+        hint = min(int(mean + 2.0 * mean ** 0.5), 0x7FFF)          # rows of a busy expert: the kernel lays its tiles out for them
     max_rows = min(T, 0xFFFF) | (hint << 16)
     s = _stream()
     counts, offsets, pos, total = plan if plan is not None else _make_plan(idx, experts)
