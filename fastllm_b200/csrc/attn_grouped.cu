@@ -117,7 +117,9 @@ __device__ __forceinline__ bool ag_item(const AttnGroupedParams& p, int w, int& 
   return ok;
 }
 
-template <bool BF16, int GP, int MODE>
+// TERMS 2: probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder), for models whose decode kept
+// them in fp32; the product is made twice, which the page stream hides.
+template <bool BF16, int GP, int MODE, int TERMS>
 __global__ void __launch_bounds__(192, 3)
 attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                     const AttnGroupedParams p) {
@@ -128,7 +130,7 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint8_t* v_smem = k_smem + dt * AG_TILE;                     // an odd last half block reads one tile past the values: allocated
   uint8_t* q_smem = v_smem + 2 * vblocks * AG_TILE;
   uint8_t* p_smem = q_smem + dt * AG_QTILE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + AG_P_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + TERMS * AG_P_BYTES);
   uint64_t* full_k = bars;
   uint64_t* full_v = bars + 1;
   uint64_t* empty_k = bars + 2;
@@ -204,8 +206,8 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after_sync();
         for (int blk = 0; blk < vblocks; ++blk) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            umma_f16(tmem_o + blk * 16, make_smem_desc(vb + 2 * blk * AG_TILE + k * 2048, AG_TILE, 1024, SWZ_128B),
+          for (int k = 0; k < 8 * TERMS; ++k)              // (the second term's tile lies behind the first one's)
+            umma_f16(tmem_o + blk * 16, make_smem_desc(vb + 2 * blk * AG_TILE + (k & 7) * 2048, AG_TILE, 1024, SWZ_128B),
                      make_smem_desc(pb + k * 512, 256, 128, SWZ_NONE), p.idesc_o, k != 0 ? 1u : 0u);
         }
         umma_commit(o_full);
@@ -263,11 +265,18 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             bits = BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(pv)) : __half_as_ushort(__float2half_rn(pv));
             // the sum of what the tensor core will see
             float pr = BF16 ? __bfloat162float(__ushort_as_bfloat16(bits)) : __half2float(__ushort_as_half(bits));
+            if (TERMS == 2) {
+              const float rest = pv - pr;
+              const uint16_t lo = BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(rest)) : __half_as_ushort(__float2half_rn(rest));
+              *reinterpret_cast<uint16_t*>(pb + AG_P_BYTES + (h >> 3) * 128 + (h & 7) * 16) = lo;
+              pr = pv;
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) pr += __shfl_xor_sync(0xffffffffu, pr, o);
             if (lane == 0) red_sum[q * 16 + h] = pr;
           }
           if (h < GP || it == 0) *reinterpret_cast<uint16_t*>(pb + (h >> 3) * 128 + (h & 7) * 16) = bits;      // unused rows: zeroed once
+          if (TERMS == 2 && h >= GP && it == 0) *reinterpret_cast<uint16_t*>(pb + AG_P_BYTES + (h >> 3) * 128 + (h & 7) * 16) = 0;
         }
       }
       fence_proxy_async_smem();
@@ -392,12 +401,12 @@ extern "C" int fb_grouped_plan(const int* kv_lens, int B, int window, int chunk,
 // keep: first tokens a window keeps; softcap 0: none; sinks [H], head_gate (row stride ld_head_gate, one logit per head): null for none.
 // q: [B, >= H * D] (row stride ld_q), k_pool [num_slots, G, D], v_pool [num_slots, G, V], out / gate [B, >= H * V]; 16-bit (dtype 0 = fp16,
 // 1 = bf16).  splits: most pages one query's keys touch; part_o [B * H * splits * V], part_ml [B * H * splits * 2] floats.
-extern "C" int fb_grouped_decode(const void* q, long long ld_q, const void* k_pool, const void* v_pool, void* out, long long ld_out,
-                                 const void* gate, long long ld_gate, const int* page_table, const int* kv_lens, const int* work,
+static int grouped_decode(const void* q, long long ld_q, const void* k_pool, const void* v_pool, void* out, long long ld_out,
+                          const void* gate, long long ld_gate, const int* page_table, const int* kv_lens, const int* work,
                                  const int* n_work, float* part_o, float* part_ml, int B, int H, int G, int D, int V, long long num_slots,
                                  int max_pages, int splits, int max_items, int window, int chunk, int keep, float scale, float softcap,
                                  const float* sinks, const float* head_gate, long long ld_head_gate, const float* score_bias, const float* cos_v,
-                                 const float* sin_v, int rot_v, int tab_rows, int dtype, void* stream_) {
+                                 const float* sin_v, int rot_v, int tab_rows, int terms, int dtype, void* stream_) {
   if (B <= 0) return 0;
   if (H <= 0 || G <= 0 || H % G != 0 || H > 65535 || D <= 0 || V <= 0 || D > 256 || V > 256 || D % 8 != 0 || V % 8 != 0 || num_slots < AG_PAGE ||
       max_pages <= 0 || splits <= 0 || keep < 0 || softcap < 0.f || (dtype != 0 && dtype != 1) || rot_v < 0 || (rot_v & 1) || rot_v > V || (score_bias != nullptr && sinks != nullptr) ||
@@ -424,27 +433,47 @@ extern "C" int fb_grouped_decode(const void* q, long long ld_q, const void* k_po
   const uint32_t f = dtype == 1 ? 1u : 0u;
   p.idesc_s = make_idesc(f, f, 0, 0, 128, AG_N);
   p.idesc_o = make_idesc(f, f, 1, 0, 128, AG_N);
-  const int smem = (p.dt + 2 * ((p.vt + 1) / 2)) * AG_TILE + p.dt * AG_QTILE + AG_P_BYTES + 1024 + 1024;
+  const int smem = (p.dt + 2 * ((p.vt + 1) / 2)) * AG_TILE + p.dt * AG_QTILE + terms * AG_P_BYTES + 1024 + 1024;
   int occ = (227 * 1024) / (smem + 1024);
   occ = occ < 1 ? 1 : occ > 3 ? 3 : occ;
   const int HG = H / G, gp = HG >= 16 ? 16 : HG;
   const int mode = score_bias != nullptr ? 2 : keep > 0 || softcap > 0.f || sinks != nullptr || head_gate != nullptr || rot_v > 0 ? 1 : 0;
-#define FB_AG(BF, GPV, MODE)                                                                                                         \
+#define FB_AG(BF, GPV, MODE, TERMS)                                                                                                         \
   {                                                                                                                                  \
     static DeviceOnce cfg;                                                                                                           \
-    if (cfg.need()) cudaFuncSetAttribute(attn_grouped_kernel<BF, GPV, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
-    launch_k<PDL_ATTN>(attn_grouped_kernel<BF, GPV, MODE>, dim3(sm_count * occ), dim3(192), smem, stream, 0, tmQ, tmK, tmV, p);        \
+    if (cfg.need()) cudaFuncSetAttribute(attn_grouped_kernel<BF, GPV, MODE, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); \
+    launch_k<PDL_ATTN>(attn_grouped_kernel<BF, GPV, MODE, TERMS>, dim3(sm_count * occ), dim3(192), smem, stream, 0, tmQ, tmK, tmV, p);        \
   }
-#define FB_AG_GP(BF, MODE)                                                                                                           \
+#define FB_AG_GP(BF, MODE, TERMS)                                                                                                           \
   {                                                                                                                                  \
-    if (gp <= 1) FB_AG(BF, 1, MODE) else if (gp <= 2) FB_AG(BF, 2, MODE) else if (gp <= 4) FB_AG(BF, 4, MODE)                            \
-    else if (gp <= 8) FB_AG(BF, 8, MODE) else FB_AG(BF, 16, MODE)                                                                      \
+    if (gp <= 1) FB_AG(BF, 1, MODE, TERMS) else if (gp <= 2) FB_AG(BF, 2, MODE, TERMS) else if (gp <= 4) FB_AG(BF, 4, MODE, TERMS)                            \
+    else if (gp <= 8) FB_AG(BF, 8, MODE, TERMS) else FB_AG(BF, 16, MODE, TERMS)                                                                      \
     launch_k<PDL_COMBINE>(attn_grouped_combine_kernel<BF, MODE>, dim3(B, H), dim3(128), 0, stream, 0, p, (uint16_t*)out, ld_out,       \
                           (const uint16_t*)gate, ld_gate, head_gate, ld_head_gate);                                                  \
   }
-  if (dtype == 1) { if (mode == 2) FB_AG_GP(true, 2) else if (mode == 1) FB_AG_GP(true, 1) else FB_AG_GP(true, 0) }
-  else { if (mode == 2) FB_AG_GP(false, 2) else if (mode == 1) FB_AG_GP(false, 1) else FB_AG_GP(false, 0) }
+  if (terms == 2) { if (dtype == 1) FB_AG_GP(true, 0, 2) else FB_AG_GP(false, 0, 2) }
+  else if (dtype == 1) { if (mode == 2) FB_AG_GP(true, 2, 1) else if (mode == 1) FB_AG_GP(true, 1, 1) else FB_AG_GP(true, 0, 1) }
+  else { if (mode == 2) FB_AG_GP(false, 2, 1) else if (mode == 1) FB_AG_GP(false, 1, 1) else FB_AG_GP(false, 0, 1) }
 #undef FB_AG_GP
 #undef FB_AG
   return (int)cudaGetLastError();
+}
+
+extern "C" int fb_grouped_decode(const void* q, long long ld_q, const void* k_pool, const void* v_pool, void* out, long long ld_out,
+                                 const void* gate, long long ld_gate, const int* page_table, const int* kv_lens, const int* work,
+                                 const int* n_work, float* part_o, float* part_ml, int B, int H, int G, int D, int V, long long num_slots,
+                                 int max_pages, int splits, int max_items, int window, int chunk, int keep, float scale, float softcap,
+                                 const float* sinks, const float* head_gate, long long ld_head_gate, const float* score_bias, const float* cos_v,
+                                 const float* sin_v, int rot_v, int tab_rows, int dtype, void* stream) {
+  return grouped_decode(q, ld_q, k_pool, v_pool, out, ld_out, gate, ld_gate, page_table, kv_lens, work, n_work, part_o, part_ml, B, H, G, D, V, num_slots, max_pages,
+                        splits, max_items, window, chunk, keep, scale, softcap, sinks, head_gate, ld_head_gate, score_bias, cos_v, sin_v, rot_v, tab_rows, 1, dtype,
+                        stream);
+}
+
+// Plain causal decode at any head width, probabilities in two terms; operands as above.
+extern "C" int fb_wide_decode(const void* q, long long ld_q, const void* k_pool, const void* v_pool, void* out, long long ld_out, const void* gate, long long ld_gate,
+                              const int* page_table, const int* kv_lens, const int* work, const int* n_work, float* part_o, float* part_ml, int B, int H, int G,
+                              int D, int V, long long num_slots, int max_pages, int splits, int max_items, float scale, int dtype, void* stream) {
+  return grouped_decode(q, ld_q, k_pool, v_pool, out, ld_out, gate, ld_gate, page_table, kv_lens, work, n_work, part_o, part_ml, B, H, G, D, V, num_slots, max_pages,
+                        splits, max_items, 0, 0, 0, scale, 0.f, nullptr, nullptr, 0, nullptr, nullptr, nullptr, 0, 0, 2, dtype, stream);
 }

@@ -416,7 +416,7 @@ class DecoderModel:
                                   sinks=lw.sinks, q8_ready=q8 is not None)
             else:                # prefill: the tensor-core prefill kernel over a 16-bit scratch copy of the pages it reads
                 a = A.attn_prefill(q, k_pool, v_pool, fb.page_table, fb.kv_lens, fb.cu_q, self.attn_scale, Hq, Hkv, D,
-                                   cu_q_host=fb.cu_q_host)
+                                   cu_q_host=fb.cu_q_host, plans=fb.__dict__.setdefault("_prefill_plans", {}))
             if lw.out_gate is not None:
                 a = (a.float() * torch.sigmoid(lw.out_gate(x).float())).to(a.dtype)
             if lw.head_gate is not None:
@@ -433,6 +433,9 @@ class DecoderModel:
         if q is None:
             q = A.qkv_post(lw.qkv(x), fb.positions, fb.slots, k_pool, v_pool, Hq, Hkv, D, cos, sin, self.rope_mode, rot,
                            lw.q_norm, lw.k_norm, c.rms_eps, c.norm_unit_offset)
+        gate = None                  # head widths other than 128: the output gate is part of the attention's epilogue
+        if lw.out_gate is not None and A.wide_ok(q, k_pool, Hq, Hkv, D):
+            gate = lw.out_gate(x)
         if fb.is_decode:
             qm = 0
             if lw.o.kind != "dense" and lw.post_ln is None:
@@ -442,11 +445,11 @@ class DecoderModel:
                 qm = qm if qm in (1, 2) else 0
             a = A.attn_decode(q, k_pool, v_pool, fb.page_table, fb.kv_lens, self.attn_scale, Hq, Hkv, D, ws=fb.decode_ws,
                               planned=fb.decode_planned, quant_mode=qm, window=int(lw.window or 0), softcap=float(c.attn_softcap or 0.0),
-                              sinks=lw.sinks)
+                              sinks=lw.sinks, gate=gate)
         else:
             a = A.attn_prefill(q, k_pool, v_pool, fb.page_table, fb.kv_lens, fb.cu_q, self.attn_scale, Hq, Hkv, D,
-                               cu_q_host=fb.cu_q_host)
-        if lw.out_gate is not None:
+                               cu_q_host=fb.cu_q_host, gate=gate, plans=fb.__dict__.setdefault("_prefill_plans", {}))
+        if lw.out_gate is not None and gate is None:
             a = (a.float() * torch.sigmoid(lw.out_gate(x).float())).to(a.dtype)
         if lw.head_gate is not None:
             a = self._head_gate(lw, x, a, Hq, D)

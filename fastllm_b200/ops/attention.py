@@ -374,6 +374,18 @@ def kv_append_fp8(k, v, k_pool, v_pool, slots):
     _lib.check(rc, "fb_kv_append_fp8")
 
 
+def wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim) -> bool:
+    """Plain causal attention at a head width other than 128 runs on the kernels for any width (``csrc/attn_wide.cu``,
+    ``csrc/attn_grouped.cu``): 16-bit rows and pages, multiples of 8 up to 256."""
+    return bool(q.is_cuda and head_dim != 128 and head_dim % 8 == 0 and head_dim <= 256 and q.dtype in (torch.float16, torch.bfloat16)
+                and k_pool.dtype == q.dtype and k_pool.shape[1] == PAGE_LEN and num_q_heads % num_kv_heads == 0 and q.stride(-1) == 1
+                and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
+
+
+def _gate_args(gate):
+    return _ptr(gate), gate.stride(0) if gate is not None else 0
+
+
 KV8_KERNEL = True          # e4m3 page pools run the decode kernel's KV8 mode (tests switch it off to compare with the PyTorch path)
 # e4m3 pages straight into the fp8 tensor core (queries and probabilities as two e4m3 terms each) instead of converting every
 # page to an fp16 operand tile in shared memory
@@ -382,8 +394,10 @@ KV8_MMA = os.environ.get("FB_KV8_MMA", "1") != "0"
 
 def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num_kv_heads, head_dim,
                 ws: DecodeWorkspace | None = None, out=None, planned=False, grid_ctas=0, quant_mode: int = 0,
-                window: int = 0, softcap: float = 0.0, sinks=None, q8_ready: bool = False):
+                window: int = 0, softcap: float = 0.0, sinks=None, q8_ready: bool = False, gate=None):
     """One new token per request. q: ``[B, Hq*D]`` -> ``[B, Hq*D]``.
+
+    ``gate`` (head widths of ``wide_ok`` only): 16-bit logits ``[B, Hq*D]``, contiguous rows; the output is multiplied by their sigmoid.
 
     ``window`` > 0: sliding-window attention; ``softcap`` > 0: tanh soft-capping of the logits; ``sinks``: fp32 ``[Hq]`` per-head
     sink logits in the softmax denominator.  All three run inside the same kernels.
@@ -403,6 +417,21 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
     G = num_q_heads // num_kv_heads
     kv8 = (k_pool.dtype == torch.float8_e4m3fn and v_pool.dtype == torch.float8_e4m3fn and KV8_KERNEL
            and q.dtype in (torch.float16, torch.bfloat16))
+    if not variant and wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim):
+        P_ = page_table.shape[1]
+        if ws is None or ws.part_o.numel() < B * num_q_heads * ws.max_pages * head_dim:
+            ws, planned = DecodeWorkspace(B, num_kv_heads, G, P_, q.device, head_dim), False
+        if B > ws.max_batch or P_ > ws.max_pages:
+            raise ValueError("decode workspace too small for this batch / page table")
+        if not planned:
+            ws.plan(seq_lens)
+        out = torch.empty_like(q) if out is None else out
+        rc = _lib.kernels().fb_wide_decode(_ptr(q), q.stride(0), _ptr(k_pool), _ptr(v_pool), _ptr(out), out.stride(0), *_gate_args(gate), _ptr(page_table),
+                                           _ptr(seq_lens), _ptr(ws.work), _ptr(ws.n_work), _ptr(ws.part_o), _ptr(ws.part_ml), B, num_q_heads, num_kv_heads,
+                                           head_dim, head_dim, k_pool.shape[0] * PAGE_LEN, page_table.stride(0), ws.max_pages, ws.work.shape[0], float(scale),
+                                           dtype_code(q.dtype), _stream())
+        _lib.check(rc, "fb_wide_decode")
+        return out
     if head_dim != 128 or G > 16 or k_pool.shape[1] != PAGE_LEN or (k_pool.dtype != q.dtype and not kv8):
         cu = torch.arange(B + 1, dtype=torch.int32, device=q.device)
         if variant or k_pool.dtype != q.dtype:
@@ -483,9 +512,23 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
     return out
 
 
+def _query_blocks(cu_q, cu_q_host, device, plans: dict | None):
+    """(int32 ``[n, 2]`` on the device: request and first row of every block of 128 new tokens; n).  Causal work grows with the block's start:
+    the longest are scheduled first.  Kept in ``plans``."""
+    if plans is not None and "blocks" in plans:
+        return plans["blocks"]
+    cu = cu_q_host if cu_q_host is not None else cu_q.tolist()
+    blocks = sorted(((b, q0) for b in range(len(cu) - 1) for q0 in range(0, cu[b + 1] - cu[b], 128)), key=lambda t: -t[1])
+    got = (torch.tensor(blocks, dtype=torch.int32).to(device, non_blocking=True), len(blocks)) if blocks else (None, 0)
+    if plans is not None:
+        plans["blocks"] = got
+    return got
+
+
 def attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim, out=None,
-                 cu_q_host=None):
-    """Packed causal prefill (also chunked prefill / prefix-cache continuation). q: ``[T, Hq*D]``."""
+                 cu_q_host=None, gate=None, plans: dict | None = None):
+    """Packed causal prefill (also chunked prefill / prefix-cache continuation). q: ``[T, Hq*D]``; ``gate`` as in ``attn_decode``;
+    ``plans``: a dict that lives as long as the batch does, for what the layers of a pass share."""
     if cpu_native(q) and k_pool.dtype == torch.float32:
         return cpu.attention_paged(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim)
     if (q.is_cuda and k_pool.dtype == torch.float8_e4m3fn and head_dim == 128 and k_pool.shape[1] == PAGE_LEN
@@ -501,25 +544,29 @@ def attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_head
         pt[mask] = torch.arange(used.numel(), device=q.device, dtype=page_table.dtype)
         kt = k_pool.index_select(0, used).to(q.dtype)
         vt = v_pool.index_select(0, used).to(q.dtype)
-        return attn_prefill(q, kt, vt, pt, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim, out, cu_q_host)
+        return attn_prefill(q, kt, vt, pt, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim, out, cu_q_host, plans=plans)
+    if wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim):
+        blk, n_blocks = _query_blocks(cu_q, cu_q_host, q.device, plans)
+        out = torch.empty_like(q) if out is None else out
+        if not n_blocks:
+            return out
+        rc = _lib.kernels().fb_attn_wide(_ptr(q), q.stride(0), q.shape[0], _ptr(k_pool), _ptr(v_pool), k_pool.shape[0] * PAGE_LEN, _ptr(page_table),
+                                         page_table.stride(0), _ptr(cu_q), _ptr(kv_lens), _ptr(out), out.stride(0), *_gate_args(gate), _ptr(blk), n_blocks,
+                                         num_q_heads, num_kv_heads, head_dim, head_dim, float(scale), dtype_code(q.dtype), _stream())
+        _lib.check(rc, "fb_attn_wide")
+        return out
     if not q.is_cuda or head_dim != 128 or k_pool.shape[1] != PAGE_LEN:
         o = paged_attention_ref(q, k_pool, v_pool, page_table, kv_lens.cpu(), cu_q.cpu(), scale, num_q_heads, num_kv_heads,
                                 head_dim)
         return o
-    cu = cu_q_host if cu_q_host is not None else cu_q.tolist()
-    blocks = []
-    for b in range(len(cu) - 1):
-        for q0 in range(0, cu[b + 1] - cu[b], 128):
-            blocks.append((b, q0))
-    blocks.sort(key=lambda t: -t[1])        # causal work grows with the block's start: longest blocks are scheduled first
+    blk, n_blocks = _query_blocks(cu_q, cu_q_host, q.device, plans)
     if out is None:
         out = torch.empty_like(q)
-    if not blocks:
+    if not n_blocks:
         return out
-    blk = torch.tensor(blocks, dtype=torch.int32).to(q.device, non_blocking=True)
     num_slots = k_pool.shape[0] * k_pool.shape[1]
     rc = _lib.kernels().fb_attn_prefill(_ptr(q), q.stride(0), q.shape[0], _ptr(k_pool), _ptr(v_pool), _ptr(out), out.stride(0),
-                                        _ptr(blk), len(blocks), _ptr(cu_q), _ptr(kv_lens), _ptr(page_table), num_q_heads,
+                                        _ptr(blk), n_blocks, _ptr(cu_q), _ptr(kv_lens), _ptr(page_table), num_q_heads,
                                         num_kv_heads, head_dim, num_slots, page_table.stride(0), float(scale),
                                         dtype_code(q.dtype), _stream())
     _lib.check(rc, "fb_attn_prefill")
@@ -531,6 +578,12 @@ def attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_head
 # ---------------------------------------------------------------------------------------------------
 _lib.register_sigs({"fb_mla_decode": [ctypes.c_void_p] * 10 + [ctypes.c_int] * 4 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                       ctypes.c_float, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]}, ["attn_mla"])
+_lib.register_sigs({
+    "fb_wide_decode": [ctypes.c_void_p, ctypes.c_longlong] + [ctypes.c_void_p] * 3 + [ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong]
+                      + [ctypes.c_void_p] * 6 + [ctypes.c_int] * 5 + [ctypes.c_longlong] + [ctypes.c_int] * 3 + [ctypes.c_float, ctypes.c_int, ctypes.c_void_p],
+    "fb_attn_wide": [ctypes.c_void_p, ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p, ctypes.c_int]
+                    + [ctypes.c_void_p] * 3 + [ctypes.c_longlong, ctypes.c_void_p, ctypes.c_longlong, ctypes.c_void_p] + [ctypes.c_int] * 5
+                    + [ctypes.c_float, ctypes.c_int, ctypes.c_void_p]}, ["attn_grouped", "attn_wide"])
 _MLA_WS: dict = {}
 
 

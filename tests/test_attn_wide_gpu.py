@@ -1,0 +1,80 @@
+"""Attention at head widths other than 128: the kernels against 64-bit attention, and no further off than the fp32 evaluation."""
+import pytest
+import torch
+
+from fastllm_b200.ops import attention as A
+
+pytestmark = pytest.mark.gpu
+PAGE = A.PAGE_LEN
+
+
+def _setup(dtype, D, Hq, Hkv, lens, news, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    counts = [(n + PAGE - 1) // PAGE for n in lens]
+    order = torch.randperm(sum(counts), generator=g, device="cuda").to(torch.int32)
+    table = torch.zeros(len(lens), max(counts) + 1, dtype=torch.int32, device="cuda")
+    for b, c in enumerate(counts):
+        table[b, :c] = order[sum(counts[:b]):sum(counts[:b]) + c]
+    pools = [rnd(sum(counts), PAGE, Hkv, D).to(dtype) for _ in range(2)]
+    q, gate = (1.5 * rnd(sum(news), Hq * D)).to(dtype), rnd(sum(news), Hq * D).to(dtype)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    return q, gate, *pools, table, i32(lens), i32([sum(news[:i]) for i in range(len(news) + 1)])
+
+
+def _exact(q, gate, k_pool, v_pool, table, lens, cu, scale, Hq, Hkv, D):
+    out = torch.empty(q.shape, dtype=torch.float64, device=q.device)
+    cu = cu.tolist()
+    for b, L in enumerate(lens.tolist()):
+        r0, r1 = cu[b], cu[b + 1]
+        pg = table[b, :(L + PAGE - 1) // PAGE].long()
+        k, v = (p[pg].reshape(-1, Hkv, D)[:L].double().repeat_interleave(Hq // Hkv, dim=1) for p in (k_pool, v_pool))
+        s = torch.einsum("qhd,khd->hqk", q[r0:r1].double().view(-1, Hq, D), k) * scale
+        hidden = torch.arange(L, device=q.device)[None, :] > torch.arange(L - (r1 - r0), L, device=q.device)[:, None]
+        out[r0:r1] = torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hidden, float("-inf")), -1), v).reshape(r1 - r0, -1)
+    return out if gate is None else out * torch.sigmoid(gate.double())
+
+
+rel = lambda x, y: ((x.double() - y).norm() / y.norm()).item()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 2), (72, 3, 3), (192, 2, 1), (256, 8, 1), (256, 20, 1)])
+def test_wide_attention(dtype, D, Hq, Hkv):
+    scale = D ** -0.5
+    # prompts: one token, tile edges, a continuation, several steps
+    lens, news = [1, 128, 129, 300, 700], [1, 128, 129, 57, 700]
+    q, gate, kp, vp, pt, ln, cu = _setup(dtype, D, Hq, Hkv, lens, news, D)
+    assert A.wide_ok(q, kp, Hq, Hkv, D)
+    for gt in (None, gate):
+        got = A.attn_prefill(q, kp, vp, pt, ln, cu, scale, Hq, Hkv, D, gate=gt)
+        want = _exact(q, gt, kp, vp, pt, ln, cu, scale, Hq, Hkv, D)
+        old = A.paged_attention_ref(q, kp, vp, pt, ln.cpu(), cu.cpu(), scale, Hq, Hkv, D)
+        if gt is not None:
+            old = (old.float() * torch.sigmoid(gt.float())).to(old.dtype)
+        # both end in one rounding to 16 bits; 2 %: which of two neighbours a tie goes to
+        assert rel(got, want) <= 1.02 * rel(old, want)
+        assert (got.double() - want).abs().max() <= 1.5 * (old.double() - want).abs().max()
+    # decoded tokens
+    lens = [1, 127, 128, 129, 1000]
+    q, gate, kp, vp, pt, ln, cu = _setup(dtype, D, Hq, Hkv, lens, [1] * 5, D + 1)
+    for gt in (None, gate):
+        got = A.attn_decode(q, kp, vp, pt, ln, scale, Hq, Hkv, D, gate=gt)
+        want = _exact(q, gt, kp, vp, pt, ln, cu, scale, Hq, Hkv, D)
+        old = A.paged_attention_ref(q, kp, vp, pt, ln.cpu(), cu.cpu(), scale, Hq, Hkv, D)
+        if gt is not None:
+            old = (old.float() * torch.sigmoid(gt.float())).to(old.dtype)
+        assert rel(got, want) <= 1.05 * rel(old, want)
+
+
+def test_large_scores_and_empty_rows():
+    """Scores far apart, a row whose request holds nothing (a padded decode row), a batch larger than a workspace made for another one."""
+    D, Hq, Hkv = 256, 4, 2
+    q, gate, kp, vp, pt, ln, cu = _setup(torch.bfloat16, D, Hq, Hkv, [400, 64], [200, 64], 3)
+    q = q * 30
+    want = _exact(q, None, kp, vp, pt, ln, cu, D ** -0.5, Hq, Hkv, D)
+    old = A.paged_attention_ref(q, kp, vp, pt, ln.cpu(), cu.cpu(), D ** -0.5, Hq, Hkv, D)
+    assert rel(A.attn_prefill(q, kp, vp, pt, ln, cu, D ** -0.5, Hq, Hkv, D), want) <= 1.02 * rel(old, want)
+    ln[1] = 0
+    out = A.attn_decode(q[:2].contiguous(), kp, vp, pt, ln, D ** -0.5, Hq, Hkv, D)
+    assert torch.isfinite(out).all() and (out[1] == 0).all()
