@@ -649,15 +649,24 @@ class DecoderModel:
         ckv = lw.kv_a(x)                                   # [T, lora + rope]
         cos, sin = self.rope_tables()
         lat_pool = kv[0]
+        if lw.w_uk_t is None:
+            lw.w_uk_t = lw.w_uk.transpose(1, 2).to(x.dtype).contiguous()      # [H, lora, nope]
+            lw.w_uv_c = lw.w_uv.to(x.dtype).contiguous()                      # [H, vd, lora]
+        if not fb.is_decode and MOE._MLA_KERNEL and lw.idx_wq is None and rope and q.is_cuda:
+            la = lw.__dict__.get("_prompt")
+            if la is None:
+                la = lw._prompt = LA.from_absorbed(H, nope, rope, lora, vd, lw.w_uk, lw.w_uk_t, lw.w_uv_c, self.attn_scale, self.rope_mode == A.ROPE_NEOX)
+            if self.rope_mode != A.ROPE_NONE and LA.prompt_ok(la, q, lat_pool):
+                # prompts: keys and values of all heads expanded from the latents once, attention on plain heads
+                A.mla_post(ckv, q, q, lat_pool, fb.positions, fb.slots, lw.kv_a_norm, cos, sin, 0, nope, rope, lora, self.rope_mode, c.latent_norm_eps or c.rms_eps)
+                o = LA.attention(la, q, lat_pool, fb, q, None, (cos, sin))
+                return self._row_parallel_norm(lw.o, o, residual, next_ln, consumer=consumer)
         # latent norm + rope of the shared key into the cache entry, rope of the heads' rotary query parts: one launch
         q_full = torch.empty((T, H, lora + rope), device=x.device, dtype=x.dtype)
         A.mla_post(ckv, q, q_full, lat_pool, fb.positions, fb.slots, lw.kv_a_norm, cos, sin, H, nope, rope, lora, self.rope_mode,
                    c.latent_norm_eps or c.rms_eps)
         # absorb: q_lat[h] = q_nope[h] @ W_UK[h] -> attention in latent space with a single shared "KV head"; one batched
         # tensor-core launch over the heads, written straight into q_full[..., :lora]
-        if lw.w_uk_t is None:
-            lw.w_uk_t = lw.w_uk.transpose(1, 2).to(x.dtype).contiguous()      # [H, lora, nope]
-            lw.w_uv_c = lw.w_uv.to(x.dtype).contiguous()                      # [H, vd, lora]
         B.linear_batched(q, lw.w_uk_t, H, nope + rope, q_full.view(T, H * (lora + rope)), lora + rope)
         sel = None
         if lw.idx_wq is not None and kv[1] is not None and qr is not None:

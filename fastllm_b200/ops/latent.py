@@ -62,7 +62,8 @@ class LatentWeights:
         self.q_norm = None
         self.q_pad = 0
         self.kv_norm = None
-        self.w_ukv = None        # [heads * (dim + vdim), lv]: keys of all heads, then values (the expanding GEMM)
+        self.w_ukv = None        # [heads * (dim + vdim), lv]: keys of all heads, then values (the expanding GEMM); None: the two below
+        self.w_uk = None         # [heads * dim, lv]
         self.w_uk_t = None       # [heads, lv, dim]   queries -> latent space
         self.w_uv = None         # [heads, vdim, lv]  latent space -> values
         self.gate = "elem"       # "elem": one per element, "head": one per head, "": none
@@ -149,6 +150,22 @@ def build(spec, q, g, dkv, kv_norm, uk, uv, uq=None, q_norm=None, more=()):
     w.w_uk_t = uk.reshape(H, w.dim, w.lv).transpose(1, 2).contiguous()
     w.w_uv = uv.reshape(H, w.vdim, w.lv).contiguous()
     return w, pad_rows(torch.cat([*parts, *more], dim=0), 32), pad_cols(pad_rows(heads(uq), 32), 8).contiguous() if uq is not None else None
+
+
+def from_absorbed(heads: int, nope: int, rope: int, lora: int, vdim: int, w_uk, w_uk_t, w_uv, scale: float, neox: bool) -> LatentWeights:
+    """Multi-head latent attention (DeepSeek layout) as such a layer: queries [own | rotated] a head, cached rows [latent | rotated part], no
+    gate.  ``w_uk`` [heads, nope, lora], ``w_uk_t`` [heads, lora, nope], ``w_uv`` [heads, vdim, lora]."""
+    w = LatentWeights()
+    w.heads, w.dim, w.vdim, w.rank, w.lv, w.rot, w.rd = heads, nope, vdim, lora, lora, rope, rope
+    w.ld, w.scale, w.neox, w.gate = lora + rope, float(scale), neox, ""
+    w.w_uk, w.w_uk_t, w.w_uv = w_uk.reshape(heads * nope, lora), w_uk_t, w_uv
+    return w
+
+
+def prompt_ok(lw: LatentWeights, q, pool) -> bool:
+    """Prompts of an ungated layer over whole latents and rotated parts, without padding between them."""
+    return bool(q.is_cuda and q.dtype in (torch.float16, torch.bfloat16) and pool.dtype == q.dtype and pool.shape[1] == 128 and q.stride(-1) == 1
+                and lw.dim % 8 == 0 and lw.vdim % 8 == 0 and lw.lv % 64 == 0 and lw.rd % 8 == 0 and lw.w_uk.dtype == q.dtype and expand_ok(lw, q.dtype))
 
 
 def pad_out_proj(o, spec):
@@ -278,13 +295,21 @@ def _absorbed(lw, q, gate, head_gate, pool, page_table, kv_lens, out, positions,
     B.linear_batched(o_lat.view(n, H * lw.lv), lw.w_uv, H, lw.lv, out, lw.vdim, gate=gate)
 
 
+def expand(lw, rows):
+    """Latent rows [n, lv] -> (keys [n, >= heads * dim], values [n, >= heads * vdim])"""
+    if lw.w_ukv is None:
+        return B.linear(rows, lw.w_uk), B.linear(rows, lw.w_uv.view(-1, lw.lv))
+    kv = B.linear(rows, lw.w_ukv)
+    return kv[:, :lw.heads * lw.dim], kv[:, lw.heads * lw.dim:]
+
+
 def window_attention(lw, grp, q, gate, kv, out, head_gate=None, shared=None):
-    """Prefill kernel over one group's expanded keys and values ``kv`` [n_keys, >= heads * (dim + vdim)]; ``shared``: [n_keys, rd] rotated key
-    parts."""
+    """Prefill kernel over one group's expanded keys and values ``kv``: [n_keys, >= heads * (dim + vdim)], or a pair of matrices; ``shared``:
+    [n_keys, rd] rotated key parts."""
     H = lw.heads
-    k, v = kv[:, :H * lw.dim], kv[:, H * lw.dim:]
+    k, v = kv if isinstance(kv, tuple) else (kv[:, :H * lw.dim], kv[:, H * lw.dim:])
     st = lambda t: t.stride(0) if t is not None else 0
-    rc = _lib.kernels().fb_attn_window(_ptr(q), q.stride(0), lw.hd, q.shape[0], _ptr(k), kv.stride(0), _ptr(v), kv.stride(0), _ptr(shared), st(shared), kv.shape[0],
+    rc = _lib.kernels().fb_attn_window(_ptr(q), q.stride(0), lw.hd, q.shape[0], _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(shared), st(shared), k.shape[0],
                                        _ptr(out), out.stride(0), _ptr(gate), st(gate), _ptr(head_gate), st(head_gate), _ptr(grp.blocks), grp.n_blocks,
                                        H, lw.dim, lw.rd, lw.vdim, lw.window, lw.scale, dtype_code(q.dtype), _stream())
     _lib.check(rc, "fb_attn_window")
@@ -312,7 +337,7 @@ def attention(lw, proj, pool, fb, q=None, head_gate=None, rope=None):
         S.rope_heads(qr, lw.hd, qr, lw.hd, H, lw.rot, lw.rd, fb.positions, *rope, lw.neox)
     for grp in pl.groups:
         rows = S.gather_rows(pool.view(-1, lw.ld), grp.key_idx)
-        window_attention(lw, grp, q, gate, B.linear(rows[:, :lw.lv], lw.w_ukv), out, head_gate, rows[:, lw.lv:] if lw.rd else None)
+        window_attention(lw, grp, q, gate, expand(lw, rows[:, :lw.lv]), out, head_gate, rows[:, lw.lv:] if lw.rd else None)
     return out
 
 

@@ -1,0 +1,59 @@
+"""Prompts of multi-head latent attention: expanded keys and values against 64-bit attention, and no further off than the absorbed products."""
+import pytest
+import torch
+
+from fastllm_b200.models.decoder import ForwardBatch
+from fastllm_b200.ops import attention as A
+from fastllm_b200.ops import basic as B
+from fastllm_b200.ops import latent as LA
+from fastllm_b200.ops import moe as MOE
+
+pytestmark = pytest.mark.gpu
+PAGE = A.PAGE_LEN
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("mode", [A.ROPE_INTERLEAVED, A.ROPE_NEOX])
+@pytest.mark.parametrize("H,lens,news", [(16, [700, 300, 90], [700, 44, 1]), (5, [17, 256, 16], [17, 255, 16])])
+def test_mla_prompt(dtype, mode, H, lens, news):
+    nope, rope, lora, vd = 128, 64, 512, 128
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    T, counts = sum(news), [(n + PAGE - 1) // PAGE for n in lens]
+    order = torch.randperm(sum(counts), generator=g, device="cuda").to(torch.int32)
+    table = torch.zeros(len(lens), max(counts) + 1, dtype=torch.int32, device="cuda")
+    for b, c in enumerate(counts):
+        table[b, :c] = order[sum(counts[:b]):sum(counts[:b]) + c]
+    pool = rnd(sum(counts) + 1, PAGE, 1, lora + rope).to(dtype)
+    w_uk, w_uv = ((lora ** -0.5 * rnd(H, n, lora)).to(dtype) for n in (nope, vd))
+    q = rnd(T, H * (nope + rope)).to(dtype)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu = [sum(news[:i]) for i in range(len(news) + 1)]
+    pos = [lens[b] - n + j for b, n in enumerate(news) for j in range(n)]
+    fb = ForwardBatch(ids=i32([0] * T), positions=i32(pos), slots=i32([-1] * T), page_table=table, kv_lens=i32(lens), cu_q=i32(cu), cu_q_host=cu, kv_lens_host=lens)
+    cos, sin = A.build_rope_tables(rope, 1024, 1e4, None, "cuda")
+    scale = (nope + rope) ** -0.5
+    la = LA.from_absorbed(H, nope, rope, lora, vd, w_uk, w_uk.transpose(1, 2).contiguous(), w_uv, scale, mode == A.ROPE_NEOX)
+    assert LA.prompt_ok(la, q, pool)
+    # the absorbed products
+    q3 = q.view(T, H, nope + rope)
+    q_full = torch.empty(T, H, lora + rope, device="cuda", dtype=dtype)
+    q_full[..., lora:] = A.apply_rope_ref(q3[..., nope:], fb.positions, cos, sin, mode, rope)
+    B.linear_batched(q, la.w_uk_t, H, nope + rope, q_full.view(T, -1), lora + rope)
+    old = torch.empty(T, H * vd, device="cuda", dtype=dtype)
+    B.linear_batched(MOE.mla_paged_attention(q_full, pool, fb, scale, lora).reshape(T, H * lora), w_uv, H, lora, old, vd)
+    # 64 bits
+    want = torch.empty(T, H, vd, dtype=torch.float64, device="cuda")
+    qr = torch.cat([q3[..., :nope].double(), A.apply_rope_ref(q3[..., nope:].float(), fb.positions, cos, sin, mode, rope).double()], dim=-1)
+    for b, L in enumerate(lens):
+        rows = pool[table[b, :counts[b]].long()].reshape(-1, lora + rope)[:L].double()
+        k = torch.cat([torch.einsum("kr,hdr->khd", rows[:, :lora], w_uk.double()), rows[:, None, lora:].expand(-1, H, -1)], dim=-1)
+        s = torch.einsum("qhd,khd->hqk", qr[cu[b]:cu[b + 1]], k) * scale
+        s = s.masked_fill(torch.arange(L, device="cuda")[None, :] > torch.arange(L - news[b], L, device="cuda")[:, None], float("-inf"))
+        want[cu[b]:cu[b + 1]] = torch.einsum("hqk,khv->qhv", torch.softmax(s, -1), torch.einsum("kr,hvr->khv", rows[:, :lora], w_uv.double()))
+    want = want.view(T, -1)
+    qc = q.clone()
+    got = LA.attention(la, qc, pool, fb, qc, None, (cos, sin))
+    rel = lambda x: ((x.double() - want).norm() / want.norm()).item()
+    # both ways round four times to 16 bits between the projections
+    assert rel(got) <= 1.05 * rel(old), (rel(got), rel(old))
