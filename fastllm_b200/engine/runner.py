@@ -159,60 +159,69 @@ class ModelRunner:
         if self.control is not None and mtp_hidden is None:
             self.control.prefill(chunks, keep_hidden)
         dev = self.device
-        ids, pos, slots, cu, kv_lens, rows = [], [], [], [0], [], []
-        P = self.max_pages
-        pt = np.zeros((len(chunks), P), dtype=np.int32)
-        pl = self.cfg.page_len
-        sslots = []
+        P, pl, n_req = self.max_pages, self.cfg.page_len, len(chunks)
+        lens = [len(ch[0]) for ch in chunks]
+        T = sum(lens)
+        cu, kv_lens, rows, sslots = [0], [], [], []
         mm_rows, mm_vals, pos3 = [], [], []          # image-token rows of the packed batch, their embeddings, 3-D positions
         ex_rows = []                                 # rows that take a model's visual-expert weights
         any_mm = any(len(ch) > 5 and ch[5] is not None for ch in chunks)
         for b, ch in enumerate(chunks):
             toks, start, pages, want = ch[:4]
+            n = lens[b]
             if any_mm:
                 mm = ch[5] if len(ch) > 5 else None
                 if mm is not None:
-                    offs, rws = mm.rows(start, len(toks))
+                    offs, rws = mm.rows(start, n)
                     if offs:
                         mm_rows.extend(cu[-1] + o for o in offs)
                         mm_vals.append(mm.embeds[rws])
-                    pos3.append(mm.positions(start, len(toks)))
-                    ex_rows.extend(cu[-1] + o for o in mm.expert_rows(start, len(toks)))
+                    pos3.append(mm.positions(start, n))
+                    ex_rows.extend(cu[-1] + o for o in mm.expert_rows(start, n))
                 else:
-                    pos3.append(torch.arange(start, start + len(toks))[None].expand(3, -1))
+                    pos3.append(torch.arange(start, start + n)[None].expand(3, -1))
             ss = ch[4] if len(ch) > 4 and ch[4] is not None and ch[4] >= 0 else self.state_slots     # default: the scratch slot
             sslots.append(ss)
             if self.state_slots and start == 0 and mtp_hidden is None:
                 self.kv.reset_state(ss)              # a request starts (or restarts after an eviction) from empty state
-            n = len(toks)
-            ids.extend(toks)
-            pos.extend(range(start, start + n))
-            pg = np.asarray(pages, dtype=np.int64)
-            p_idx = np.arange(start, start + n)
-            slots.extend((pg[p_idx // pl] * pl + p_idx % pl).tolist())
             cu.append(cu[-1] + n)
             kv_lens.append(start + n)
-            pt[b, :len(pages)] = pages
             if isinstance(want, (list, tuple)):
                 rows.extend(cu[-2] + int(w) for w in want)
             elif want:
                 # True: the chunk's last row; an integer n > 1: its last n rows (speculative verification reads them all)
                 nrows = 1 if want is True else max(1, min(int(want), n))
                 rows.extend(range(cu[-1] - nrows, cu[-1]))
-        T = len(ids)
-        meta = torch.tensor(ids + pos + slots, dtype=torch.int32)
-        if dev.type == "cuda":
-            meta = meta.pin_memory().to(dev, non_blocking=True)
-        fb = ForwardBatch(ids=meta[:T], positions=meta[T:2 * T], slots=meta[2 * T:3 * T],
-                          page_table=torch.from_numpy(pt).to(dev), kv_lens=torch.tensor(kv_lens, dtype=torch.int32).to(dev),
-                          cu_q=torch.tensor(cu, dtype=torch.int32).to(dev),
-                          logit_rows=torch.tensor(rows, dtype=torch.long).to(dev) if rows else torch.zeros(0, dtype=torch.long, device=dev),
-                          is_decode=False, cu_q_host=cu,
-                          state_slots=torch.tensor(sslots, dtype=torch.int32).to(dev) if self.state_slots else None,
+        # everything the step reads travels in one pinned buffer -> one copy: [logit rows (64 bit) | ids | positions | slots | page table |
+        # lengths | row offsets | state slots]
+        n_rows = max(1, len(rows))                   # no row asked for: one all the same, to keep shapes valid
+        buf = torch.empty((2 * n_rows + 3 * T + n_req * (P + 3) + 1,), dtype=torch.int32, pin_memory=dev.type == "cuda")
+        m = buf.numpy()
+        at = 2 * n_rows
+        m[:at].view(np.int64)[:] = rows or 0
+        ids, pos, slots = (m[at + k * T:at + (k + 1) * T] for k in range(3))
+        at += 3 * T
+        pt = m[at:at + n_req * P].reshape(n_req, P)
+        pt[:] = 0
+        for b, ch in enumerate(chunks):
+            toks, start, pages = ch[:3]
+            lo, hi = cu[b], cu[b + 1]
+            ids[lo:hi] = toks
+            pt[b, :len(pages)] = pages
+            where = np.arange(start, start + lens[b])
+            pos[lo:hi] = where
+            slots[lo:hi] = np.asarray(pages, dtype=np.int64)[where // pl] * pl + where % pl
+        at += n_req * P
+        m[at:at + n_req] = kv_lens
+        m[at + n_req:at + 2 * n_req + 1] = cu
+        m[at + 2 * n_req + 1:at + 3 * n_req + 1] = sslots
+        d = buf.to(dev, non_blocking=True)
+        d_ids = 2 * n_rows
+        fb = ForwardBatch(ids=d[d_ids:d_ids + T], positions=d[d_ids + T:d_ids + 2 * T], slots=d[d_ids + 2 * T:d_ids + 3 * T],
+                          page_table=d[at - n_req * P:at].view(n_req, P), kv_lens=d[at:at + n_req], cu_q=d[at + n_req:at + 2 * n_req + 1],
+                          logit_rows=d[:d_ids].view(torch.int64), is_decode=False, cu_q_host=cu,
+                          state_slots=d[at + 2 * n_req + 1:at + 3 * n_req + 1] if self.state_slots else None,
                           state_slots_host=sslots if self.state_slots else None)
-        if not rows:
-            # still run the stack to fill the cache; ask for one row to keep shapes valid
-            fb.logit_rows = torch.zeros(1, dtype=torch.long, device=dev)
         if any_mm:
             fb.rope_pos3 = torch.cat(pos3, dim=1)
             if mm_rows and mtp_hidden is None:
