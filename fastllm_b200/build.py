@@ -32,7 +32,7 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "--use_fast_math", "-Xptxas", "-v",
 ]
 # translation units that state fp32 results exactly (32-bit angles, norms, matrix products) are compiled without fast-math
-PRECISE_UNITS = {"stream32", "full32", "gla", "mlstm", "rglru"}
+PRECISE_UNITS = {"stream32", "full32", "gdn_prompt", "gla", "mlstm", "rglru"}
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fopenmp", "-march=x86-64-v3", "-Wall", "-Wno-unused-function"]
 
 

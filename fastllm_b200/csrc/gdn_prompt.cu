@@ -1,0 +1,704 @@
+// Gated DeltaNet prompts for sm_100a: the causal convolution over packed sequences and the chunked gated delta rule with the gated RMSNorm
+// behind it.  Per value head, with q, k normalised to unit length (q also scaled by 128^-1/2), decay g_t <= 0 and write strength beta_t:
+//     S_t = e^(g_t) S_(t-1) + k_t (beta_t (v_t - (e^(g_t) S_(t-1))^T k_t))^T,     o_t = S_t^T q_t.
+//
+// 64 tokens a chunk, G the running sum of g inside it, S the state it starts from:
+//     V' = T (beta v - beta e^G (K S)),   T = (I + A)^-1,   A_ts = beta_t e^(G_t - G_s) (k_t . k_s) for s < t
+//     S <- e^(G_last) S + sum_t e^(G_last - G_t) k_t V'_t^T,     o_t = e^(G_t) q_t S + sum_(s <= t) e^(G_t - G_s) (q_t . k_s) V'_s
+//  * gdn_chunk_inverse_kernel  gates, norms and T of every (chunk, head), in parallel: K K^T on the tensor core, the unit lower-triangular
+//                              inverse by forward substitution, a column per thread in registers.
+//  * gdn_chunk_scan_kernel     the chain over the chunks.  Columns of the state never meet: two warps carry 16 of them through all chunks.
+//                              S^T stays in registers as accumulator fragments, which are operand fragments of the next product as they
+//                              are (the k index of both operands is permuted alike); the chunk's keys and T are fetched a chunk ahead.
+//  * gdn_chunk_out_kernel      outputs of every (chunk, head), in parallel, with the norm over the head and the gate in the epilogue.
+// Products run on tf32 operands with fp32 accumulation.  Queries, keys and values are 16-bit numbers and exact there (their norms are
+// factors of rows, applied in fp32); every fp32 operand enters as two terms, the rounded value and the rounded remainder, so that products
+// carry 22 bits of it.  Decays, norms, gates, T and the state are fp32.
+//
+// 4001 tokens x 32 heads: 0.54 ms a layer (convolution 41 us, T 62, chain 270, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
+#include "ptx.cuh"
+#include "launch.h"
+
+FB_DEFINE_ERROR_API(gdn_prompt)
+
+namespace fb {
+
+constexpr int GP_T = 64;                         // tokens a chunk
+constexpr int GP_D = 128;                        // width of keys and of values
+constexpr int GP_LDK = GP_D + 8;                 // 16-bit rows of keys / queries: 272 bytes, conflict-free ldmatrix
+constexpr int GP_LDT = GP_T + 8;                 // fp32 rows read as pairs: conflict-free
+constexpr int GP_VECS = 9;                       // vectors of 64 a (chunk, head), see below
+// write strengths; beta e^G / |k|; e^(G_last - G) / |k|; e^G / |q|; the running log2-decay and what its rounding left; 1 / |k|; 128^-1/2 / |q|; e^G_last
+enum { GV_BETA, GV_CB, GV_CD, GV_EQ, GV_G, GV_GLO, GV_RK, GV_RQ, GV_LAST };
+
+struct GdnPromptParams {
+  const uint16_t* y; long long ld_y;             // [T, 2 Hk 128 + Hv 128] queries | keys | values behind the convolution
+  const uint16_t* a; const uint16_t* b; long long ld_ab;       // [T, Hv] decay and write-strength logits
+  const uint16_t* z; long long ld_z;             // [T, Hv 128] output gate
+  const float* A_log; const float* dt_bias;      // [Hv]
+  const uint16_t* norm_w;                        // [128]
+  float* state;                                  // [slots, Hv, 128, 128]
+  uint16_t* out;                                 // [T, Hv 128]
+  const int* chunks;                             // [n_chunks][3] = (first row, rows, state slot in a request's first chunk, else -1)
+  const int* reqs;                               // [n_reqs][4] = (first chunk, chunks, state slot, rows)
+  float* inv;                                    // [units][64][64]; unit = chunk * Hn + head - h0
+  float* vecs;                                   // [units][GP_VECS][64]
+  float* vnew;                                   // [units][128 v][64 t]
+  float* s0;                                     // [units][128 v][128 d]
+  int Hk, Hv, h0, Hn;
+  float eps;
+};
+
+template <bool BF16> __device__ __forceinline__ float gp_ld(uint16_t v) { return BF16 ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v)); }
+template <bool BF16> __device__ __forceinline__ uint16_t gp_st(float v) { return BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v)); }
+__device__ __forceinline__ float gp_ex2(float x) { return exp2f(x); }       // (a chunk's decay multiplies the state once a chunk: its error adds up)
+__device__ __forceinline__ float gp_tf32(float x) { uint32_t y; asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(y) : "f"(x)); return __uint_as_float(y); }
+__device__ __forceinline__ void gp_split(float x, float& hi, float& lo) { hi = gp_tf32(x); lo = gp_tf32(x - hi); }
+__device__ __forceinline__ void gp_mma_tf32(float* c, const float* a, float b0, float b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+                 "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+template <bool BF16>
+__device__ __forceinline__ void gp_mma_16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  if (BF16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void gp_ldsm4(uint32_t* r, const uint16_t* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+__device__ __forceinline__ void gp_ldsm4_t(uint32_t* r, const uint16_t* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
+}
+// 16 bytes global -> shared; `ok` false: zeros
+__device__ __forceinline__ void gp_cp16(void* dst, const void* src, bool ok) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void gp_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void gp_cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// ------------------------------------------------------------------------------------------------
+// causal depth-wise convolution of four taps + SiLU.  A thread takes 8 channels of 16 tokens: bound by the rows it reads and writes once
+// (4001 x 8192 channels: 131 MB).  The requests' windows are advanced by the kernel behind it, which this one must not overtake.
+// ------------------------------------------------------------------------------------------------
+constexpr int GP_CT = 16;
+template <bool BF16>
+__global__ void __launch_bounds__(256) gdn_conv_prompt_kernel(const uint16_t* __restrict__ x, long long ldx, const uint16_t* __restrict__ w,
+                                                              const uint16_t* __restrict__ state, const int* __restrict__ chunks, uint16_t* __restrict__ out, int C) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int c8 = blockIdx.x * 256 + threadIdx.x;
+  const int* ch = chunks + 3 * blockIdx.y;
+  const int row0 = ch[0], n = ch[1], slot = ch[2], t0 = blockIdx.z * GP_CT;
+  if (c8 * 8 >= C || t0 >= n) return;
+  float wf[8][4];
+  {
+    const uint4* wp = reinterpret_cast<const uint4*>(w + (size_t)c8 * 32);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint4 v = wp[i];
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { const float2 f = unpack_16<BF16>(u[j]); wf[2 * i + (j >> 1)][2 * (j & 1)] = f.x; wf[2 * i + (j >> 1)][2 * (j & 1) + 1] = f.y; }
+    }
+  }
+  float win[3][8];
+  const bool first = slot >= 0 && t0 == 0;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    if (first) {
+      const uint16_t* sp = state + ((size_t)slot * C + c8 * 8) * 3 + j;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) win[j][e] = gp_ld<BF16>(sp[3 * e]);
+    } else {
+      const uint4 v = *reinterpret_cast<const uint4*>(x + (size_t)(row0 + t0 - 3 + j) * ldx + c8 * 8);
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { const float2 f = unpack_16<BF16>(u[e]); win[j][2 * e] = f.x; win[j][2 * e + 1] = f.y; }
+    }
+  }
+  const int cnt = min(GP_CT, n - t0);
+#pragma unroll 4
+  for (int t = 0; t < cnt; ++t) {
+    const uint4 v = *reinterpret_cast<const uint4*>(x + (size_t)(row0 + t0 + t) * ldx + c8 * 8);
+    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = unpack_16<BF16>(u[e]);
+      const float in[2] = {f.x, f.y};
+      float r[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int c = 2 * e + k;
+        const float s = fmaf(in[k], wf[c][3], fmaf(win[2][c], wf[c][2], fmaf(win[1][c], wf[c][1], win[0][c] * wf[c][0])));
+        win[0][c] = win[1][c]; win[1][c] = win[2][c]; win[2][c] = in[k];
+        r[k] = __fdividef(s, 1.0f + __expf(-s));
+      }
+      o[e] = pack_16<BF16>(r[0], r[1]);
+    }
+    *reinterpret_cast<uint4*>(out + (size_t)(row0 + t0 + t) * C + c8 * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
+// the last three inputs of every request become its window
+__global__ void __launch_bounds__(256) gdn_conv_state_kernel(const uint16_t* __restrict__ x, long long ldx, uint16_t* state, const int* __restrict__ chunks,
+                                                             const int* __restrict__ reqs, int C) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= C) return;
+  const int* rq = reqs + 4 * blockIdx.y;
+  const int row0 = chunks[3 * rq[0]], n = rq[3];
+  uint16_t* sp = state + ((size_t)rq[2] * C + c) * 3;
+  const uint16_t h[3] = {sp[0], sp[1], sp[2]};
+  uint16_t o[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int i = n + j;                          // place in [window | new inputs]
+    o[j] = i < 3 ? h[i] : x[(size_t)(row0 + i - 3) * ldx + c];
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) sp[j] = o[j];
+}
+
+// ------------------------------------------------------------------------------------------------
+// gates, norms and T
+// ------------------------------------------------------------------------------------------------
+template <bool BF16>
+__global__ void __launch_bounds__(128) gdn_chunk_inverse_kernel(const GdnPromptParams p) {
+  __shared__ __align__(16) uint16_t ks[GP_T * GP_LDK];
+  __shared__ __align__(16) float As[GP_T * (GP_T + 4)];
+  __shared__ float sg[GP_T], sl[GP_T], sb[GP_T], rk[GP_T], rq[GP_T];
+  __shared__ double part;
+  constexpr int LDA = GP_T + 4;
+  const int c = blockIdx.x, hl = blockIdx.y, h = p.h0 + hl, hk = h / (p.Hv / p.Hk);
+  const int row0 = p.chunks[3 * c], n = p.chunks[3 * c + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint16_t* q0 = p.y + (size_t)row0 * p.ld_y + hk * GP_D;
+  const uint16_t* k0 = q0 + p.Hk * GP_D;
+  // half a warp a row: its keys into shared memory, squares of keys and queries
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int t = i * 8 + (tid >> 4), col = (tid & 15) * 8;
+    uint4 kv = make_uint4(0u, 0u, 0u, 0u), qv = kv;
+    if (t < n) {
+      kv = *reinterpret_cast<const uint4*>(k0 + (size_t)t * p.ld_y + col);
+      qv = *reinterpret_cast<const uint4*>(q0 + (size_t)t * p.ld_y + col);
+    }
+    *reinterpret_cast<uint4*>(ks + t * GP_LDK + col) = kv;
+    float sk = 0.f, sq = 0.f;
+    const uint32_t ku[4] = {kv.x, kv.y, kv.z, kv.w}, qu[4] = {qv.x, qv.y, qv.z, qv.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 a = unpack_16<BF16>(ku[e]), b = unpack_16<BF16>(qu[e]);
+      sk = fmaf(a.x, a.x, fmaf(a.y, a.y, sk));
+      sq = fmaf(b.x, b.x, fmaf(b.y, b.y, sq));
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) { sk += __shfl_xor_sync(0xffffffffu, sk, o); sq += __shfl_xor_sync(0xffffffffu, sq, o); }
+    if ((tid & 15) == 0) { rk[t] = 1.0f / sqrtf(sk + 1e-6f); rq[t] = 0.08838834764831845f / sqrtf(sq + 1e-6f); }
+  }
+  // running log2-decay, one token a thread; in 64 bits, for decays are exponentials of its differences (after 64 tokens that forget nearly
+  // everything an fp32 sum has units of 2^-15)
+  double G = 0.0;
+  float beta = 0.f;
+  if (tid < GP_T) {
+    if (tid < n) {
+      const size_t at = (size_t)(row0 + tid) * p.ld_ab + h;
+      const float x = gp_ld<BF16>(p.a[at]) + p.dt_bias[h];
+      G = (double)(-expf(p.A_log[h]) * (x > 20.f ? x : log1pf(expf(x)))) * 1.4426950408889634;
+      beta = 1.0f / (1.0f + expf(-gp_ld<BF16>(p.b[at])));
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const double u = __shfl_up_sync(0xffffffffu, G, o); if (lane >= o) G += u; }
+    if (tid == 31) part = G;
+  }
+  __syncthreads();
+  if (tid < GP_T) {
+    if (warp == 1) G += part;
+    sg[tid] = (float)G;
+    sl[tid] = (float)(G - (double)sg[tid]);
+    sb[tid] = beta;
+  }
+  __syncthreads();
+  const size_t unit = (size_t)c * p.Hn + hl;
+  if (tid < GP_T) {
+    float* v = p.vecs + unit * GP_VECS * GP_T + tid;
+    const double last = (double)sg[GP_T - 1] + (double)sl[GP_T - 1];
+    const float eG = gp_ex2((float)G);
+    v[GV_BETA * GP_T] = beta;
+    v[GV_CB * GP_T] = beta * eG * rk[tid];
+    v[GV_CD * GP_T] = rk[tid] * gp_ex2((float)(last - G));
+    v[GV_EQ * GP_T] = rq[tid] * eG;
+    v[GV_G * GP_T] = sg[tid];
+    v[GV_GLO * GP_T] = sl[tid];
+    v[GV_RK * GP_T] = rk[tid];
+    v[GV_RQ * GP_T] = rq[tid];
+    v[GV_LAST * GP_T] = gp_ex2((float)last);
+  }
+  // A, a warp 16 rows of it up to the diagonal
+  {
+    const int m0 = warp * 16, g = lane >> 2, q = lane & 3;
+    uint32_t a[8][4];
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) gp_ldsm4(a[kk], ks + (m0 + (lane & 15)) * GP_LDK + kk * 16 + (lane >> 4) * 8);
+    for (int nt = 0; nt < 8; ++nt) {
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      if (nt <= 2 * warp + 1) {
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 2) {
+          uint32_t b[4];
+          gp_ldsm4(b, ks + (nt * 8 + (lane & 7)) * GP_LDK + kk * 16 + (lane >> 3) * 8);
+          gp_mma_16<BF16>(acc, a[kk], b[0], b[1]);
+          gp_mma_16<BF16>(acc, a[kk + 1], b[2], b[3]);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int i = m0 + g + 8 * (e >> 1), j = nt * 8 + 2 * q + (e & 1);
+        As[i * LDA + j] = j < i ? acc[e] * (sb[i] * rk[i]) * (rk[j] * gp_ex2((sg[i] - sg[j]) + (sl[i] - sl[j]))) : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+  if (tid < GP_T) {
+    float t[GP_T];
+    float* dst = p.inv + unit * GP_T * GP_T + tid;
+#pragma unroll
+    for (int i = 0; i < GP_T; ++i) {
+      float s[4] = {i == tid ? 1.f : 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < i; j += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(As + i * LDA + j);        // (zeros from column i on)
+        s[0] = fmaf(-a.x, t[j], s[0]);
+        if (j + 1 < i) s[1] = fmaf(-a.y, t[j + 1], s[1]);
+        if (j + 2 < i) s[2] = fmaf(-a.z, t[j + 2], s[2]);
+        if (j + 3 < i) s[3] = fmaf(-a.w, t[j + 3], s[3]);
+      }
+      t[i] = (s[0] + s[1]) + (s[2] + s[3]);
+      dst[i * GP_T] = t[i];
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// the chain over a request's chunks: a CTA of four warps takes 32 columns of a head's state, two warps 16 of them: each carries 64 of the 128 key
+// channels.  They add up K S, share out the columns of T's product (equal parts of its triangle) and exchange V', twice a chunk
+// through shared memory.  Bound by the issue of tf32 products (310 a warp and chunk at about 16 cycles; with one warp for all 128
+// channels 620, on half of the tensor cores): 270 us a layer at 4001 tokens x 32 heads, 375 us before.
+// ------------------------------------------------------------------------------------------------
+constexpr int GS_THREADS = 128;
+constexpr int GS_LDV = 40;
+constexpr int GS_K = GP_T * GP_LDK * 2, GS_T = GP_T * GP_LDT * 4, GS_V = GP_T * GS_LDV * 2, GS_VEC = 3 * GP_T * 4;
+constexpr int GS_STAGE = GS_K + GS_T + GS_V + GS_VEC;
+constexpr int GS_STAGES = 2;
+constexpr int GS_PART = 8 * 32 * 16, GS_NEW = 4 * 32 * 16;       // bytes of a warp's partial K S and of its columns of V'
+constexpr int GS_SMEM = GS_STAGES * GS_STAGE + 4 * (GS_PART + GS_NEW);
+
+template <bool BF16>
+__global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPromptParams p) {
+  extern __shared__ __align__(16) uint8_t gs_smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const int pair = warp >> 1, half = warp & 1, d0 = half * 64;
+  const int hl = blockIdx.y, h = p.h0 + hl, hk = h / (p.Hv / p.Hk), v0 = blockIdx.x * 32;
+  float4* part_own = reinterpret_cast<float4*>(gs_smem + GS_STAGES * GS_STAGE + warp * GS_PART) + lane;
+  const float4* part_other = reinterpret_cast<const float4*>(gs_smem + GS_STAGES * GS_STAGE + (warp ^ 1) * GS_PART) + lane;
+  float4* new_own = reinterpret_cast<float4*>(gs_smem + GS_STAGES * GS_STAGE + 4 * GS_PART + warp * GS_NEW) + lane;
+  const float4* new_other = reinterpret_cast<const float4*>(gs_smem + GS_STAGES * GS_STAGE + 4 * GS_PART + (warp ^ 1) * GS_NEW) + lane;
+  auto meet = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(1 + pair) : "memory"); };
+  const int* rq = p.reqs + 4 * blockIdx.z;
+  const int c0 = rq[0], nc = rq[1], slot = rq[2];
+  auto fetch = [&](int i) {
+    uint8_t* st = gs_smem + (i % GS_STAGES) * GS_STAGE;
+    const int c = c0 + i, row0 = p.chunks[3 * c], n = p.chunks[3 * c + 1];
+    const size_t unit = (size_t)c * p.Hn + hl;
+    const uint16_t* kp = p.y + (size_t)row0 * p.ld_y + (p.Hk + hk) * GP_D;
+    const uint16_t* vp = p.y + (size_t)row0 * p.ld_y + (size_t)2 * p.Hk * GP_D + (size_t)h * GP_D + v0;
+    const float* tp = p.inv + unit * GP_T * GP_T;
+    const float* gp = p.vecs + unit * GP_VECS * GP_T;
+#pragma unroll
+    for (int j = tid; j < GP_T * 16; j += GS_THREADS) {
+      const int t = j >> 4, u = j & 15;
+      gp_cp16(st + (t * GP_LDK + u * 8) * 2, kp + (size_t)(t < n ? t : 0) * p.ld_y + u * 8, t < n);
+      gp_cp16(st + GS_K + (t * GP_LDT + u * 4) * 4, tp + t * GP_T + u * 4, true);
+    }
+#pragma unroll
+    for (int j = tid; j < GP_T * 4; j += GS_THREADS) {
+      const int t = j >> 2, u = j & 3;
+      gp_cp16(st + GS_K + GS_T + (t * GS_LDV + u * 8) * 2, vp + (size_t)(t < n ? t : 0) * p.ld_y + u * 8, t < n);
+    }
+    if (tid < 48) gp_cp16(st + GS_K + GS_T + GS_V + tid * 16, gp + tid * 4, true);           // beta, cb, cd
+  };
+  float s[8][4];                                  // S^T: rows v = g, g + 8, columns d = d0 + 8 i + 2 q, + 1
+  float* S = p.state + ((size_t)slot * p.Hv + h) * GP_D * GP_D + (size_t)d0 * GP_D + v0 + pair * 16;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[i][e] = S[(size_t)(8 * i + 2 * q + (e & 1)) * GP_D + g + 8 * (e >> 1)];
+  fetch(0);
+  gp_cp_commit();
+  for (int i = 0; i < nc; ++i) {
+    if (i + 1 < nc) fetch(i + 1);
+    gp_cp_commit();
+    gp_cp_wait<1>();
+    __syncthreads();
+    const uint8_t* st = gs_smem + (i % GS_STAGES) * GS_STAGE;
+    const uint16_t* ks = reinterpret_cast<const uint16_t*>(st) + d0;
+    const float* ts = reinterpret_cast<const float*>(st + GS_K);
+    const uint16_t* vs = reinterpret_cast<const uint16_t*>(st + GS_K + GS_T);
+    const float* vec = reinterpret_cast<const float*>(st + GS_K + GS_T + GS_V);
+    const size_t unit = (size_t)(c0 + i) * p.Hn + hl;
+    const float last = __ldg(p.vecs + (unit * GP_VECS + GV_LAST) * GP_T);
+    const int vr = v0 + pair * 16 + g;
+    float* s0 = p.s0 + (unit * GP_D + vr) * GP_D + d0 + 2 * q;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      *reinterpret_cast<float2*>(s0 + 8 * j) = make_float2(s[j][0], s[j][1]);
+      *reinterpret_cast<float2*>(s0 + 8 * GP_D + 8 * j) = make_float2(s[j][2], s[j][3]);
+    }
+    // (K S)^T [16 v x 64 t] over this warp's channels
+    float r[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) r[j][0] = r[j][1] = r[j][2] = r[j][3] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      float hi[4], lo[4];
+      gp_split(s[kk][0], hi[0], lo[0]); gp_split(s[kk][2], hi[1], lo[1]); gp_split(s[kk][1], hi[2], lo[2]); gp_split(s[kk][3], hi[3], lo[3]);
+      uint32_t b[8];
+      gp_ldsm4(b, ks + lane * GP_LDK + kk * 8);
+      gp_ldsm4(b + 4, ks + (32 + lane) * GP_LDK + kk * 8);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 f = unpack_16<BF16>(b[j]);
+        gp_mma_tf32(r[j], hi, f.x, f.y);
+        gp_mma_tf32(r[j], lo, f.x, f.y);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) part_own[32 * j] = make_float4(r[j][0], r[j][1], r[j][2], r[j][3]);
+    meet();
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int t = 8 * j + 2 * q;
+      const float4 o = part_other[32 * j];
+      const float2 be = *reinterpret_cast<const float2*>(vec + t), cb = *reinterpret_cast<const float2*>(vec + GP_T + t);
+      const uint16_t* vp = vs + t * GS_LDV + pair * 16 + g;
+      r[j][0] = fmaf(-cb.x, r[j][0] + o.x, be.x * gp_ld<BF16>(vp[0]));
+      r[j][1] = fmaf(-cb.y, r[j][1] + o.y, be.y * gp_ld<BF16>(vp[GS_LDV]));
+      r[j][2] = fmaf(-cb.x, r[j][2] + o.z, be.x * gp_ld<BF16>(vp[8]));
+      r[j][3] = fmaf(-cb.y, r[j][3] + o.w, be.y * gp_ld<BF16>(vp[GS_LDV + 8]));
+    }
+    // V'^T = (right-hand side)^T T^T: token tiles 0, 3, 4, 7 or 1, 2, 5, 6, 18 products of the triangle each
+    float w[4][4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) w[x][0] = w[x][1] = w[x][2] = w[x][3] = 0.f;
+    auto tile = [&](int x) { return 2 * x + ((x & 1) ^ half); };
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) {
+      float hi[4], lo[4];
+      gp_split(r[kk][0], hi[0], lo[0]); gp_split(r[kk][2], hi[1], lo[1]); gp_split(r[kk][1], hi[2], lo[2]); gp_split(r[kk][3], hi[3], lo[3]);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        if (tile(x) < kk) continue;
+        const float2 tv = *reinterpret_cast<const float2*>(ts + (8 * tile(x) + g) * GP_LDT + 8 * kk + 2 * q);
+        float bh0, bl0, bh1, bl1;
+        gp_split(tv.x, bh0, bl0);
+        gp_split(tv.y, bh1, bl1);
+        gp_mma_tf32(w[x], hi, bh0, bh1);
+        gp_mma_tf32(w[x], lo, bh0, bh1);
+        gp_mma_tf32(w[x], hi, bl0, bl1);
+      }
+    }
+    float* vn = p.vnew + (unit * GP_D + vr) * GP_T + 2 * q;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      new_own[32 * x] = make_float4(w[x][0], w[x][1], w[x][2], w[x][3]);
+      *reinterpret_cast<float2*>(vn + 8 * tile(x)) = make_float2(w[x][0], w[x][1]);
+      *reinterpret_cast<float2*>(vn + 8 * GP_T + 8 * tile(x)) = make_float2(w[x][2], w[x][3]);
+    }
+    meet();
+    // S^T <- e^(G_last) S^T + (decayed V')^T K.  The chunk's sum is made by itself: the tensor core's sums are cut off, not rounded, which would
+    // add up in a state that forgets slowly
+    float u[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) u[j][0] = u[j][1] = u[j][2] = u[j][3] = 0.f;
+#pragma unroll
+    for (int y = 0; y < 8; ++y) {
+      const bool mine = y < 4;
+      const int x = y & 3, kk = 2 * x + ((x & 1) ^ (mine ? half : half ^ 1));
+      const float4 wv = mine ? make_float4(w[x][0], w[x][1], w[x][2], w[x][3]) : new_other[32 * x];
+      const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 8 * kk + 2 * q);
+      float hi[4], lo[4];
+      gp_split(wv.x * cd.x, hi[0], lo[0]); gp_split(wv.z * cd.x, hi[1], lo[1]);
+      gp_split(wv.y * cd.y, hi[2], lo[2]); gp_split(wv.w * cd.y, hi[3], lo[3]);
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        uint32_t b[4];
+        gp_ldsm4_t(b, ks + (8 * kk + (lane & 7)) * GP_LDK + (j + (lane >> 3)) * 8);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = unpack_16<BF16>(b[e]);
+          gp_mma_tf32(u[j + e], hi, f.x, f.y);
+          gp_mma_tf32(u[j + e], lo, f.x, f.y);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], last, u[j][e]);
+    __syncthreads();                              // the stage is refilled by the next fetch
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) S[(size_t)(8 * i + 2 * q + (e & 1)) * GP_D + g + 8 * (e >> 1)] = s[i][e];
+}
+
+// ------------------------------------------------------------------------------------------------
+// outputs of a chunk: warps 2 x 4 over (32 tokens, 32 columns); state halves and V' pass through one buffer, two CTAs share an SM
+// ------------------------------------------------------------------------------------------------
+constexpr int GO_THREADS = 256;
+constexpr int GO_QK = GP_T * GP_LDK * 2, GO_P = GP_T * GP_LDT * 4, GO_B = GP_D * GP_LDT * 4;
+constexpr int GO_SMEM = 2 * GO_QK + GO_P + GO_B + GP_T * 4 * 4;
+
+template <bool BF16>
+__global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnPromptParams p) {
+  extern __shared__ __align__(16) uint8_t go_smem[];
+  uint16_t* qs = reinterpret_cast<uint16_t*>(go_smem);
+  uint16_t* ks = reinterpret_cast<uint16_t*>(go_smem + GO_QK);
+  float* Ps = reinterpret_cast<float*>(go_smem + 2 * GO_QK);
+  float* Bs = reinterpret_cast<float*>(go_smem + 2 * GO_QK + GO_P);
+  float* red = reinterpret_cast<float*>(go_smem + 2 * GO_QK + GO_P + GO_B);       // [64][4]
+  const int c = blockIdx.x, hl = blockIdx.y, h = p.h0 + hl, hk = h / (p.Hv / p.Hk);
+  const int row0 = p.chunks[3 * c], n = p.chunks[3 * c + 1];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+  const size_t unit = (size_t)c * p.Hn + hl;
+  const float* vec = p.vecs + unit * GP_VECS * GP_T;
+  const uint16_t* qp = p.y + (size_t)row0 * p.ld_y + hk * GP_D;
+  for (int j = tid; j < GP_T * 16; j += GO_THREADS) {
+    const int t = j >> 4, u = j & 15;
+    const uint16_t* src = qp + (size_t)(t < n ? t : 0) * p.ld_y + u * 8;
+    gp_cp16(qs + t * GP_LDK + u * 8, src, t < n);
+    gp_cp16(ks + t * GP_LDK + u * 8, src + p.Hk * GP_D, t < n);
+  }
+  gp_cp_commit();
+  auto fetch = [&](const float* src, int ld) {    // [128 v][64] into the buffer
+#pragma unroll
+    for (int j = tid; j < GP_D * 16; j += GO_THREADS) {
+      const int v = j >> 4, u = j & 15;
+      gp_cp16(Bs + v * GP_LDT + u * 4, src + (size_t)v * ld + u * 4, true);
+    }
+    gp_cp_commit();
+  };
+  const float* s0 = p.s0 + unit * GP_D * GP_D;
+  fetch(s0, GP_D);
+  gp_cp_wait<1>();
+  __syncthreads();
+  {                                               // decayed scores, 16 tokens x 32 keys a warp
+    const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 4;
+    uint32_t a[8][4];
+#pragma unroll
+    for (int kk = 0; kk < 8; ++kk) gp_ldsm4(a[kk], qs + (m0 + (lane & 15)) * GP_LDK + kk * 16 + (lane >> 4) * 8);
+    const float gi[2] = {__ldg(vec + GV_G * GP_T + m0 + g), __ldg(vec + GV_G * GP_T + m0 + g + 8)};
+    const float li[2] = {__ldg(vec + GV_GLO * GP_T + m0 + g), __ldg(vec + GV_GLO * GP_T + m0 + g + 8)};
+    const float ri[2] = {__ldg(vec + GV_RQ * GP_T + m0 + g), __ldg(vec + GV_RQ * GP_T + m0 + g + 8)};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int nt = n0 + x;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      if (nt * 8 < m0 + 16) {
+#pragma unroll
+        for (int kk = 0; kk < 8; kk += 2) {
+          uint32_t b[4];
+          gp_ldsm4(b, ks + (nt * 8 + (lane & 7)) * GP_LDK + kk * 16 + (lane >> 3) * 8);
+          gp_mma_16<BF16>(acc, a[kk], b[0], b[1]);
+          gp_mma_16<BF16>(acc, a[kk + 1], b[2], b[3]);
+        }
+      }
+      const int j = nt * 8 + 2 * q;
+      const float2 lj = __ldg(reinterpret_cast<const float2*>(vec + GV_GLO * GP_T + j));
+      const float2 gj = __ldg(reinterpret_cast<const float2*>(vec + GV_G * GP_T + j)), rj = __ldg(reinterpret_cast<const float2*>(vec + GV_RK * GP_T + j));
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int i = m0 + g + 8 * e;
+        float2 o;
+        o.x = j <= i ? acc[2 * e] * ri[e] * (rj.x * gp_ex2((gi[e] - gj.x) + (li[e] - lj.x))) : 0.f;
+        o.y = j + 1 <= i ? acc[2 * e + 1] * ri[e] * (rj.y * gp_ex2((gi[e] - gj.y) + (li[e] - lj.y))) : 0.f;
+        *reinterpret_cast<float2*>(Ps + i * GP_LDT + j) = o;
+      }
+    }
+  }
+  const int tg = warp >> 2, vg = warp & 3;
+  float acc[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[m][j][0] = acc[m][j][1] = acc[m][j][2] = acc[m][j][3] = 0.f;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    gp_cp_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int kk = 0; kk < 8; kk += 2) {
+      uint32_t a[2][4];                           // rows 0-7 | 8-15 of k step kk, then of kk + 1
+#pragma unroll
+      for (int m = 0; m < 2; ++m) gp_ldsm4(a[m], qs + (tg * 32 + m * 16 + (lane & 15)) * GP_LDK + half * 64 + (kk + (lane >> 4)) * 8);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        float af[2][4];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const float2 f0 = unpack_16<BF16>(a[m][2 * x]), f1 = unpack_16<BF16>(a[m][2 * x + 1]);
+          af[m][0] = f0.x; af[m][1] = f1.x; af[m][2] = f0.y; af[m][3] = f1.y;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 sv = *reinterpret_cast<const float2*>(Bs + (vg * 32 + j * 8 + g) * GP_LDT + (kk + x) * 8 + 2 * q);
+          float h0, l0, h1, l1;
+          gp_split(sv.x, h0, l0);
+          gp_split(sv.y, h1, l1);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            gp_mma_tf32(acc[m][j], af[m], h0, h1);
+            gp_mma_tf32(acc[m][j], af[m], l0, l1);
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (half == 0) fetch(s0 + GP_T, GP_D);
+    else fetch(p.vnew + unit * GP_D * GP_T, GP_T);
+  }
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const float e0 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g), e1 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g + 8);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { acc[m][j][0] *= e0; acc[m][j][1] *= e0; acc[m][j][2] *= e1; acc[m][j][3] *= e1; }
+  }
+  gp_cp_wait<0>();
+  __syncthreads();
+  for (int kk = 0; kk < 4 * (tg + 1); ++kk) {     // (scores behind the diagonal are zeros)
+    float hi[2][4], lo[2][4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const float* pp = Ps + (tg * 32 + m * 16 + g) * GP_LDT + kk * 8 + 2 * q;
+      const float2 f0 = *reinterpret_cast<const float2*>(pp), f1 = *reinterpret_cast<const float2*>(pp + 8 * GP_LDT);
+      gp_split(f0.x, hi[m][0], lo[m][0]); gp_split(f1.x, hi[m][1], lo[m][1]); gp_split(f0.y, hi[m][2], lo[m][2]); gp_split(f1.y, hi[m][3], lo[m][3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 sv = *reinterpret_cast<const float2*>(Bs + (vg * 32 + j * 8 + g) * GP_LDT + kk * 8 + 2 * q);
+      float h0, l0, h1, l1;
+      gp_split(sv.x, h0, l0);
+      gp_split(sv.y, h1, l1);
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        gp_mma_tf32(acc[m][j], hi[m], h0, h1);
+        gp_mma_tf32(acc[m][j], lo[m], h0, h1);
+        gp_mma_tf32(acc[m][j], hi[m], l0, l1);
+      }
+    }
+  }
+  // RMS norm of the head's row and the gate, with the roundings of the separate operators (16-bit row, normalised row, weighted row)
+  float o16[2][4][4];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    float ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float f = gp_ld<BF16>(gp_st<BF16>(acc[m][j][e]));
+        o16[m][j][e] = f;
+        ss[e >> 1] = fmaf(f, f, ss[e >> 1]);
+      }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 1);
+      ss[e] += __shfl_xor_sync(0xffffffffu, ss[e], 2);
+      if (q == 0) red[(tg * 32 + m * 16 + g + 8 * e) * 4 + vg] = ss[e];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = tg * 32 + m * 16 + g + 8 * e;
+      if (t >= n) continue;
+      const float4 r4 = *reinterpret_cast<const float4*>(red + t * 4);
+      const float inv = 1.0f / sqrtf(((r4.x + r4.y) + (r4.z + r4.w)) * (1.0f / 128.0f) + p.eps);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int v = vg * 32 + j * 8 + 2 * q;
+        const float2 nw = unpack_16<BF16>(*reinterpret_cast<const uint32_t*>(p.norm_w + v));
+        const float2 y1 = unpack_16<BF16>(pack_16<BF16>(o16[m][j][2 * e] * inv, o16[m][j][2 * e + 1] * inv));
+        const float2 y2 = unpack_16<BF16>(pack_16<BF16>(nw.x * y1.x, nw.y * y1.y));
+        const uint16_t* zp = p.z + (size_t)(row0 + t) * p.ld_z + (size_t)h * GP_D + v;
+        const float z0 = gp_ld<BF16>(zp[0]), z1 = gp_ld<BF16>(zp[1]);
+        *reinterpret_cast<uint32_t*>(p.out + ((size_t)(row0 + t) * p.Hv + h) * GP_D + v) =
+            pack_16<BF16>(y2.x * (z0 / (1.0f + expf(-z0))), y2.y * (z1 / (1.0f + expf(-z1))));
+      }
+    }
+}
+
+}  // namespace fb
+
+using namespace fb;
+
+// x [T, C] 16-bit rows (stride ldx, a multiple of 8 elements, 16-byte aligned), w [C, 4], state [slots, C, 3]; chunks / reqs as in
+// GdnPromptParams; out [T, C].  C % 8 == 0.
+extern "C" int fb_gdn_conv_prompt(const void* x, long long ldx, const void* w, void* state, const int* chunks, int n_chunks, const int* reqs, int n_reqs, void* out,
+                                  int C, int dtype, void* stream_) {
+  if (n_chunks <= 0 || n_reqs <= 0) return 0;
+  if (C % 8 != 0 || ldx % 8 != 0 || (dtype != 0 && dtype != 1) || n_chunks > 65535 || n_reqs > 65535) return -1;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  const dim3 grid((C / 8 + 255) / 256, n_chunks, GP_T / GP_CT);
+  if (dtype == 1)
+    launch_k(gdn_conv_prompt_kernel<true>, grid, dim3(256), 0, s, 0, (const uint16_t*)x, ldx, (const uint16_t*)w, (const uint16_t*)state, chunks, (uint16_t*)out, C);
+  else
+    launch_k(gdn_conv_prompt_kernel<false>, grid, dim3(256), 0, s, 0, (const uint16_t*)x, ldx, (const uint16_t*)w, (const uint16_t*)state, chunks, (uint16_t*)out, C);
+  gdn_conv_state_kernel<<<dim3((C + 255) / 256, n_reqs), 256, 0, s>>>((const uint16_t*)x, ldx, (uint16_t*)state, chunks, reqs, C);
+  return (int)cudaGetLastError();
+}
+
+// One pass of the chunked rule over the heads [h0, h0 + Hn); see GdnPromptParams for the operands.  Scratch: inv n_chunks * Hn * 4096,
+// vecs * 576, vnew * 8192, s0 * 16384 floats.
+extern "C" int fb_gdn_prompt(const void* y, long long ld_y, const void* a, const void* b, long long ld_ab, const void* z, long long ld_z, const float* A_log,
+                             const float* dt_bias, const void* norm_w, float* state, void* out, const int* chunks, int n_chunks, const int* reqs, int n_reqs,
+                             float* inv, float* vecs, float* vnew, float* s0, int Hk, int Hv, int h0, int Hn, float eps, int dtype, void* stream_) {
+  if (n_chunks <= 0 || n_reqs <= 0 || Hn <= 0) return 0;
+  if (Hk <= 0 || Hv % Hk != 0 || ld_y % 8 != 0 || (dtype != 0 && dtype != 1) || Hn > 65535 || n_reqs > 65535) return -1;
+  GdnPromptParams p = {};
+  p.y = (const uint16_t*)y; p.ld_y = ld_y; p.a = (const uint16_t*)a; p.b = (const uint16_t*)b; p.ld_ab = ld_ab; p.z = (const uint16_t*)z; p.ld_z = ld_z;
+  p.A_log = A_log; p.dt_bias = dt_bias; p.norm_w = (const uint16_t*)norm_w; p.state = state; p.out = (uint16_t*)out; p.chunks = chunks; p.reqs = reqs;
+  p.inv = inv; p.vecs = vecs; p.vnew = vnew; p.s0 = s0; p.Hk = Hk; p.Hv = Hv; p.h0 = h0; p.Hn = Hn; p.eps = eps;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  static DeviceOnce once;
+  if (once.need()) {
+    cudaError_t e = cudaSuccess;
+    const void* scan[2] = {(const void*)gdn_chunk_scan_kernel<true>, (const void*)gdn_chunk_scan_kernel<false>};
+    const void* outk[2] = {(const void*)gdn_chunk_out_kernel<true>, (const void*)gdn_chunk_out_kernel<false>};
+    for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
+      e = cudaFuncSetAttribute(scan[i], cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(outk[i], cudaFuncAttributeMaxDynamicSharedMemorySize, GO_SMEM);
+    }
+    if (e != cudaSuccess) return (int)e;
+  }
+  const dim3 units(n_chunks, Hn), scan(GP_D / 32, Hn, n_reqs);
+  if (dtype == 1) {
+    gdn_chunk_inverse_kernel<true><<<units, 128, 0, s>>>(p);
+    gdn_chunk_scan_kernel<true><<<scan, GS_THREADS, GS_SMEM, s>>>(p);
+    gdn_chunk_out_kernel<true><<<units, GO_THREADS, GO_SMEM, s>>>(p);
+  } else {
+    gdn_chunk_inverse_kernel<false><<<units, 128, 0, s>>>(p);
+    gdn_chunk_scan_kernel<false><<<scan, GS_THREADS, GS_SMEM, s>>>(p);
+    gdn_chunk_out_kernel<false><<<units, GO_THREADS, GO_SMEM, s>>>(p);
+  }
+  return (int)cudaGetLastError();
+}

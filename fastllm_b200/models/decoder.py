@@ -474,6 +474,11 @@ class DecoderModel:
             y = L.causal_conv1d_decode(mixed, lw.conv_w, conv_state, fb.state_slots)
             core = L.gated_delta_decode(y, a, b, z, lw.A_log, lw.dt_bias, lw.norm_w, c.rms_eps, rec_state, fb.state_slots,
                                         lw.Hk, lw.Hv, lw.Dk, lw.Dv)
+        elif L.prompt_kernels_ok(proj, lw.conv_w, conv_state, rec_state, lw.Hk, lw.Hv, lw.Dk, lw.Dv):
+            plan = fb.__dict__.get("_gdn_plan")
+            if plan is None:
+                plan = fb._gdn_plan = L._PromptPlan(fb.cu_q_host, fb.state_slots_host, x.device)
+            core = L.gated_delta_prompt(proj, lw.conv_w, conv_state, lw.A_log, lw.dt_bias, lw.norm_w, c.rms_eps, rec_state, plan, lw.Hk, lw.Hv)
         else:
             y = L.causal_conv1d(mixed, lw.conv_w, conv_state, fb.cu_q_host, fb.state_slots_host)
             q, k, v = y[:, :kd].reshape(T, lw.Hk, lw.Dk), y[:, kd:2 * kd].reshape(T, lw.Hk, lw.Dk), y[:, 2 * kd:].reshape(T, lw.Hv, lw.Dv)

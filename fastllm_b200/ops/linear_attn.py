@@ -15,7 +15,8 @@ With ``q, k`` L2-normalised per head, ``q`` scaled by ``Dk^-1/2``, decay ``g_t <
     S_t = exp(g_t) S_{t-1} + k_t (beta_t (v_t - (exp(g_t) S_{t-1})^T k_t))^T ,      o_t = S_t^T q_t
 
 CUDA tensors of decode steps run ``csrc/linear_attn.cu`` (one CTA per (request, value head), the state column of a
-thread in registers); everything else is the PyTorch definition below, which is also the test oracle.
+thread in registers), prompts ``csrc/gdn_prompt.cu`` (``gated_delta_prompt``); everything else is the PyTorch definition below,
+which is also the test oracle.
 """
 from __future__ import annotations
 
@@ -32,8 +33,14 @@ _lib.register_sigs({
     "fb_gdn_conv_update": [P, P, P, P, P, I, I, I, I, I, P],
     "fb_gdn_recurrent": [P, I, P, I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, FLT, I, P],
 }, ["linear_attn"])
+L64 = ctypes.c_longlong
+_lib.register_sigs({
+    "fb_gdn_conv_prompt": [P, L64, P, P, P, I, P, I, P, I, I, P],
+    "fb_gdn_prompt": [P, L64, P, P, L64, P, L64, P, P, P, P, P, P, I, P, I, P, P, P, P, I, I, I, I, FLT, I, P],
+}, ["gdn_prompt"])
 
 CHUNK = 64
+SCRATCH_BYTES = 1 << 30        # of the chunked kernels: more chunks than fit are taken over fewer heads at a time
 
 
 def l2norm(x: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
@@ -168,6 +175,53 @@ def gated_delta_rule(q, k, v, a, b, A_log, dt_bias, rec_state, cu_q, slots, rep:
         else:
             out[t0:t1] = gated_delta_chunked(qf[t0:t1], kf[t0:t1], vf[t0:t1], g[t0:t1], beta[t0:t1], S)
     return out.to(v.dtype)
+
+
+class _PromptPlan:
+    """Chunks (first row, rows, state slot of a request's first one, else -1) and requests (first chunk, chunks, slot, rows) of a packed batch."""
+
+    def __init__(self, cu, slots, device):
+        chunks, reqs = [], []
+        for i, slot in enumerate(slots):
+            n = cu[i + 1] - cu[i]
+            if n > 0:
+                reqs.append((len(chunks), (n + CHUNK - 1) // CHUNK, slot, n))
+                chunks += [(cu[i] + c, min(CHUNK, n - c), slot if c == 0 else -1) for c in range(0, n, CHUNK)]
+        self.n_chunks, self.n_reqs = len(chunks), len(reqs)
+        meta = torch.tensor([x for t in chunks for x in t] + [x for t in reqs for x in t], dtype=torch.int32).to(device, non_blocking=True)
+        self.chunks, self.reqs = meta[:3 * len(chunks)], meta[3 * len(chunks):]
+
+
+def prompt_kernels_ok(proj, conv_w, conv_state, rec_state, Hk, Hv, Dk, Dv) -> bool:
+    """The prompt kernels cover 16-bit models with 128-wide heads and four taps, whose merged projection has aligned rows."""
+    return bool(proj.is_cuda and proj.dtype in (torch.float16, torch.bfloat16) and conv_w.dtype == proj.dtype and conv_state.dtype == proj.dtype
+                and rec_state.dtype == torch.float32 and Dk == 128 and Dv == 128 and Hv % Hk == 0 and conv_w.shape[1] == 4
+                and proj.stride(1) == 1 and proj.stride(0) % 8 == 0 and proj.data_ptr() % 16 == 0
+                and conv_w.is_contiguous() and conv_state.is_contiguous() and rec_state.is_contiguous())
+
+
+def gated_delta_prompt(proj, conv_w, conv_state, A_log, dt_bias, norm_w, eps, rec_state, plan: _PromptPlan, Hk, Hv):
+    """Everything between the projections for packed prompts: proj ``[T, >= 2 Hk 128 + 2 Hv 128 + 2 Hv]`` with columns ``[q | k | v | z | b | a]``
+    -> gated, normalised heads ``[T, Hv 128]``; advances the requests' windows and states."""
+    T, C, vd = proj.shape[0], (2 * Hk + Hv) * 128, Hv * 128
+    dev, dt, lib = proj.device, dtype_code(proj.dtype), _lib.kernels()
+    y = torch.empty((T, C), device=dev, dtype=proj.dtype)
+    out = torch.empty((T, vd), device=dev, dtype=proj.dtype)
+    if plan.n_chunks == 0:
+        return out
+    rc = lib.fb_gdn_conv_prompt(_ptr(proj), proj.stride(0), _ptr(conv_w), _ptr(conv_state), _ptr(plan.chunks), plan.n_chunks, _ptr(plan.reqs), plan.n_reqs,
+                                _ptr(y), C, dt, _stream())
+    _lib.check(rc, "fb_gdn_conv_prompt")
+    sizes = [plan.n_chunks * k for k in (64 * 64, 9 * 64, 128 * 64, 128 * 128)]        # T, vectors, V', first states
+    step = max(1, min(Hv, SCRATCH_BYTES // (4 * sum(sizes))))
+    scratch = torch.empty((sum(sizes) * step,), device=dev, dtype=torch.float32).split([k * step for k in sizes])
+    b, a = proj[:, C + vd:], proj[:, C + vd + Hv:]
+    for h0 in range(0, Hv, step):
+        rc = lib.fb_gdn_prompt(_ptr(y), C, _ptr(a), _ptr(b), proj.stride(0), _ptr(proj[:, C:]), proj.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(norm_w),
+                               _ptr(rec_state), _ptr(out), _ptr(plan.chunks), plan.n_chunks, _ptr(plan.reqs), plan.n_reqs, *(_ptr(t) for t in scratch),
+                               Hk, Hv, h0, min(step, Hv - h0), float(eps), dt, _stream())
+        _lib.check(rc, "fb_gdn_prompt")
+    return out
 
 
 def gated_delta_decode(mixed, a, b, z, A_log, dt_bias, norm_w, eps, rec_state, slots_dev, Hk, Hv, Dk, Dv):
