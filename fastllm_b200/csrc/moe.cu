@@ -7,7 +7,7 @@
 //   grouped GEMM swap-AB tcgen05 products of all experts in one persistent launch (moe_stream_kernel): a tile list over the
 //                experts that got rows, weights from the stacked matrix, activations from the sorted buffer.  gate/up uses
 //                the SwiGLU epilogue.
-//   moe_combine  out[t] = sum_k w[t,k] * y_sorted[pos[t,k]]   in fixed k order (deterministic)
+//   moe_combine  out[t] = sum_k w[t,k] * y_sorted[pos[t,k]]   in fixed k order (deterministic), plus a shared expert's row, gated
 //
 // Role of the reference's MergeMOE / FusedMOE (src/devices/cuda/cudadevice.cpp:8279-8562) and of its routed-row
 // kernels ("Grouped...Indexed", src/devices/cuda/moe/fastllm-moe-fp8.cu; route count/offset/scatter in
@@ -162,10 +162,12 @@ __global__ void moe_gather_kernel(const uint16_t* __restrict__ x, const int* __r
 
 template <bool BF16>
 __global__ void moe_combine_kernel(const uint16_t* __restrict__ ys, const int* __restrict__ pos, const float* __restrict__ w,
-                                   const uint16_t* __restrict__ add, uint16_t* __restrict__ out, int topk, int H) {
+                                   const uint16_t* __restrict__ add, const float* __restrict__ add_gate, int ld_gate, uint16_t* __restrict__ out, int topk,
+                                   int H) {
   const int t = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
+  const float ga = add_gate != nullptr ? 1.0f / (1.0f + __expf(-add_gate[(size_t)t * ld_gate])) : 1.0f;
   for (int c = threadIdx.x; c < H / 8; c += blockDim.x) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int k = 0; k < topk; ++k) {
@@ -180,7 +182,8 @@ __global__ void moe_combine_kernel(const uint16_t* __restrict__ ys, const int* _
     if (add != nullptr) {
       const uint4 v = *reinterpret_cast<const uint4*>(add + (size_t)t * H + c * 8);
       const float2 a = unpack_16<BF16>(v.x), b = unpack_16<BF16>(v.y), cc = unpack_16<BF16>(v.z), d = unpack_16<BF16>(v.w);
-      acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y; acc[4] += cc.x; acc[5] += cc.y; acc[6] += d.x; acc[7] += d.y;
+      acc[0] += ga * a.x; acc[1] += ga * a.y; acc[2] += ga * b.x; acc[3] += ga * b.y;
+      acc[4] += ga * cc.x; acc[5] += ga * cc.y; acc[6] += ga * d.x; acc[7] += ga * d.y;
     }
     uint4 o;
     o.x = pack_16<BF16>(acc[0], acc[1]); o.y = pack_16<BF16>(acc[2], acc[3]);
@@ -510,14 +513,22 @@ extern "C" int fb_moe_gather(const void* x, const int* pos, void* xs, int T, int
   return (int)cudaGetLastError();
 }
 
-extern "C" int fb_moe_combine(const void* ys, const int* pos, const float* w, const void* add, void* out, int T, int topk, int H,
-                              int dtype, void* stream) {
+// add (optional) [T, H]: a shared expert's rows; add_gate (optional): one fp32 logit per token (ld_gate apart), add counts times its sigmoid.
+extern "C" int fb_moe_combine_gated(const void* ys, const int* pos, const float* w, const void* add, const float* add_gate, int ld_gate, void* out, int T, int topk,
+                                    int H, int dtype, void* stream) {
   if (T <= 0) return 0;
   if (H % 8 != 0) return -1;
   auto s = reinterpret_cast<cudaStream_t>(stream);
-  if (dtype == 1) launch_k(moe_combine_kernel<true>, dim3(T), dim3(256), 0, s, 0, (const uint16_t*)ys, pos, w, (const uint16_t*)add, (uint16_t*)out, topk, H);
-  else launch_k(moe_combine_kernel<false>, dim3(T), dim3(256), 0, s, 0, (const uint16_t*)ys, pos, w, (const uint16_t*)add, (uint16_t*)out, topk, H);
+  if (dtype == 1)
+    launch_k(moe_combine_kernel<true>, dim3(T), dim3(256), 0, s, 0, (const uint16_t*)ys, pos, w, (const uint16_t*)add, add_gate, ld_gate, (uint16_t*)out, topk, H);
+  else
+    launch_k(moe_combine_kernel<false>, dim3(T), dim3(256), 0, s, 0, (const uint16_t*)ys, pos, w, (const uint16_t*)add, add_gate, ld_gate, (uint16_t*)out, topk, H);
   return (int)cudaGetLastError();
+}
+
+extern "C" int fb_moe_combine(const void* ys, const int* pos, const float* w, const void* add, void* out, int T, int topk, int H,
+                              int dtype, void* stream) {
+  return fb_moe_combine_gated(ys, pos, w, add, nullptr, 0, out, T, topk, H, dtype, stream);
 }
 
 extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out, const void* bias, const int* counts, const int* offsets,

@@ -139,6 +139,7 @@ class MLPWeights:
         # MoE
         self.router = None          # fp32 [E, H]
         self.router_16 = None       # 16-bit copy for the tensor-core router GEMM
+        self.router_gate_16 = None  # the same with the shared expert's gate as row E, padded with zero rows
         self.router_bias = None     # fp32 [E]   selection-only correction bias (DeepSeek-V3)
         self.router_scale = None    # fp32 [E]   learned per-expert output scale (Pangu Pro MoE)
         self.router_logit_bias = None   # fp32 [E] bias of the router projection itself (gpt-oss)
@@ -557,7 +558,8 @@ class DecoderModel:
             return w(x, residual=residual)
         return self.tp.comm.row_linear(w, x, residual)
 
-    def _norm(self, h, ln_w):
+    def _norm(self, h, ln_w, residual=None):
+        """``residual`` (RMS norms of 16-bit rows on CUDA): ``residual += h`` in place, then its norm."""
         if self.cfg.residual_f32:
             return S.rmsnorm32(h, ln_w, self.cfg.rms_eps) if ln_w is not None else h.to(self.dtype)
         if self.cfg.norm_kind == "layernorm":
@@ -570,7 +572,7 @@ class DecoderModel:
                 from ..ops import quant_gemm
 
                 qm = quant_gemm.act_quant_mode(cons, h.shape[0])
-        return B.rmsnorm(h, ln_w, self.cfg.rms_eps, unit_offset=self.cfg.norm_unit_offset, quant_mode=qm)
+        return B.rmsnorm(h, ln_w, self.cfg.rms_eps, residual=residual, unit_offset=self.cfg.norm_unit_offset, quant_mode=qm)
 
     def _norm_consumers(self) -> dict:
         """Norm weight -> the single quantised projection that reads that norm's output (its quantiser is fused into the norm)."""
@@ -628,6 +630,9 @@ class DecoderModel:
         c = self.cfg
         if needs_reduce and self._fused_active:
             return self.tp.comm.fused.ar_norm(partial, next_ln, c.rms_eps, c.norm_unit_offset, True)
+        if not needs_reduce and not self._fused_active and partial.is_cuda and partial.dim() == 2 and c.norm_kind == "rms" and not c.residual_f32 \
+                and partial.dtype == h.dtype and h.is_contiguous() and partial.dtype in (torch.float16, torch.bfloat16) and next_ln is not None:
+            return h, self._norm(partial, next_ln, residual=h)          # residual add and norm are one launch, in place
         if needs_reduce:
             h = self.tp.all_reduce(partial, h)
         elif self._fused_active:
@@ -823,6 +828,12 @@ class DecoderModel:
         if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and lw.router.shape[0] % 8 == 0:
             if lw.router_16 is None:
                 lw.router_16 = lw.router.to(x.dtype).contiguous()
+            if lw.shared_gate is not None and lw.shared_gate.dtype == x.dtype:
+                # the shared expert's gate is one more row of the product (padded to the large-batch kernel's tiling): column E of the logits
+                if lw.router_gate_16 is None:
+                    rows = torch.cat([lw.router_16, lw.shared_gate.reshape(1, -1)])
+                    lw.router_gate_16 = torch.cat([rows, rows.new_zeros((-rows.shape[0] % 32, rows.shape[1]))]).contiguous()
+                return B.linear(x, lw.router_gate_16, out_f32=True)
             return B.linear(x, lw.router_16, out_f32=True)
         return torch.matmul(x.float(), lw.router.t())
 
@@ -890,7 +901,7 @@ class DecoderModel:
                 act = self._glu(lw.gate_up(x), c.hidden_act, lw.gate_up.interleaved)
             return self._row_parallel_norm(lw.down, act, residual, next_ln, lw.post_ln, consumer)
         # ---- mixture of experts ----
-        fused_route = False
+        fused_route, gate_logit = False, None
         if x.is_cuda and lw.router_logit_bias is None and not c.route_group_top1 and x.dtype in (torch.float16, torch.bfloat16):
             if lw.router_16 is None and lw.router.shape[0] % 8 == 0:
                 lw.router_16 = lw.router.to(x.dtype).contiguous()
@@ -901,6 +912,9 @@ class DecoderModel:
                                        0 if c.scoring_func == "softmax" else 1, c.norm_topk_prob, c.routed_scaling_factor)
         else:
             logits = self._router_logits(lw, x)
+            E = lw.router.shape[0]
+            if logits.shape[1] > E:
+                logits, gate_logit = logits[:, :E], logits[:, E]
             if lw.router_logit_bias is not None:
                 logits = logits + lw.router_logit_bias
             if c.route_group_top1:
@@ -919,7 +933,9 @@ class DecoderModel:
                 shared = lw.shared_down(lw.shared_gate_up(x, swiglu=True))
             if self._beta != 1.0:
                 shared = shared * self._beta
-            if lw.shared_gate is not None:
+            if lw.shared_gate is not None and gate_logit is not None and self._fused_active:
+                shared, gate_logit = shared * torch.sigmoid(gate_logit)[:, None].to(shared.dtype), None
+            elif lw.shared_gate is not None and gate_logit is None:
                 shared = shared * torch.sigmoid(torch.matmul(x.float(), lw.shared_gate.float().t())).to(shared.dtype)
         if self._fused_active and lw.experts.stacked is not None and not self.tp.comm.fused._big(x.shape[0]):
             # expert-parallel combine fused with the cross-rank reduction + residual + norm (one kernel)
@@ -931,9 +947,7 @@ class DecoderModel:
                 r = self.tp.comm.fused.moe_combine_ar_norm(ys, pos, w32, shared, next_ln, c.rms_eps, c.norm_unit_offset, True)
                 if r is not None:
                     return r
-        y = MOE.moe_forward(x, idx, wts, lw.experts, self.ep)
-        if shared is not None:
-            y = y + shared
+        y = MOE.moe_forward(x, idx, wts, lw.experts, self.ep, shared, gate_logit if shared is not None else None)
         return self._reduce_norm(y, residual, next_ln, self.tp.size > 1)
 
     # -----------------------------------------------------------------------------------------------

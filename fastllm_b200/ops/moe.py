@@ -221,19 +221,24 @@ def output_is_complete(ep) -> bool:
     return bool(ep is not None and getattr(ep, "combines", False))
 
 
-def moe_forward(x, idx, wts, experts: ExpertWeights, ep=None):
+def moe_forward(x, idx, wts, experts: ExpertWeights, ep=None, add=None, add_gate=None):
     """``y[t] = sum_k wts[t,k] * down_e(silu(gate_e x) * up_e x)`` over the experts this rank owns (``scale_input``: each
-    expert reads ``wts[t,k] * x`` and its result is added as it is).
+    expert reads ``wts[t,k] * x`` and its result is added as it is), plus ``add`` ``[T, H]`` (a shared expert's rows; ``add_gate``: fp32
+    logits ``[T]``, times their sigmoid).
 
     Tokens are grouped by expert; each non-empty local expert runs the two GEMMs on its token group.
     With expert parallelism the result is this rank's partial sum (the caller all-reduces it).
     """
+    if add is not None and (experts.host or experts.stacked is None or not x.is_cuda or experts.act not in ("swiglu", "gelu") or experts.scale_input
+                            or x.dtype not in (torch.float16, torch.bfloat16)):
+        y = moe_forward(x, idx, wts, experts, ep)
+        return y + (add if add_gate is None else (add * torch.sigmoid(add_gate)[:, None].to(add.dtype)))
     if experts.host and experts.act == "swiglu":
         return _moe_forward_host(x, idx, wts, experts)
     if experts.stacked is not None and x.is_cuda and experts.act in ("swiglu", "gelu") and not experts.scale_input:
         from . import moe_grouped
 
-        y = moe_grouped.forward(x, idx, wts, experts)
+        y = moe_grouped.forward(x, idx, wts, experts, add=add, add_gate=add_gate)
         if y is not None:
             return y
     T, H = x.shape

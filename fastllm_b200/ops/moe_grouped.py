@@ -24,6 +24,7 @@ _lib.register_sigs({
     "fb_moe_plan_table": [P, I, P, I, P, P, P, P, I, I, I, P],
     "fb_moe_gather": [P, P, P, I, I, I, P],
     "fb_moe_combine": [P, P, P, P, P, I, I, I, I, P],
+    "fb_moe_combine_gated": [P, P, P, P, P, I, P, I, I, I, I, P],
     "fb_moe_grouped_gemm": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P],
     "fb_moe_grouped_gemm_act": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, ctypes.c_float, ctypes.c_float, P],
     "fb_moe_grouped_gemm_quant": [P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P],
@@ -177,8 +178,9 @@ def _forward32(x, st, plan, experts, wts, rows32):
 
 
 def forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, experts, add: torch.Tensor | None = None, combine: bool = True, plan=None,
-            rows32: torch.Tensor | None = None):
-    """``combine=False`` stops before the weighted sum and returns ``(ys, pos, wts)`` for a fused combine.  ``plan``: the routing
+            rows32: torch.Tensor | None = None, add_gate: torch.Tensor | None = None):
+    """``add`` ``[T, H]``: a shared expert's rows, added in the combine; ``add_gate``: fp32 ``[T]`` (any stride), they count times its sigmoid.
+    ``combine=False`` stops before the weighted sum and returns ``(ys, pos, wts)`` for a fused combine.  ``plan``: the routing
     plan (counts, offsets, pos, total) where it is known already (``ops.moe.TableRouter``).  ``rows32``: the experts' inputs are these
     fp32 rows times the pair's weight, in place of ``x``."""
     st = experts.stacked
@@ -278,5 +280,8 @@ def forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, experts, add:
     if not combine:
         return ys, pos, wts
     out = torch.empty((T, H), device=dev, dtype=x.dtype)
-    _lib.check(lib.fb_moe_combine(_ptr(ys), _ptr(pos), _ptr(wts), _ptr(add), _ptr(out), T, topk, H, dt, s), "fb_moe_combine")
+    if add is not None and not (add.is_contiguous() and add.dtype == x.dtype):
+        add = add.to(x.dtype).contiguous()
+    _lib.check(lib.fb_moe_combine_gated(_ptr(ys), _ptr(pos), _ptr(wts), _ptr(add), _ptr(add_gate), add_gate.stride(0) if add_gate is not None else 0, _ptr(out), T,
+                                        topk, H, dt, s), "fb_moe_combine")
     return out

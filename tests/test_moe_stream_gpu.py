@@ -1,0 +1,112 @@
+"""Grouped dense expert GEMM in one persistent launch, routing plan on many blocks, combine with a gated shared expert: edges of tiles and of row chunks."""
+import pytest
+import torch
+
+from fastllm_b200.ops import _lib, basic as B
+from fastllm_b200.ops import moe_grouped as MG
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+# rows per expert around the tile widths 16 .. 256, unequal chunks, experts without rows (first, last and in between)
+COUNTS = [[1], [0, 16, 17, 0, 15], [33, 0, 31, 64, 65, 1], [127, 129, 0, 200], [257, 0, 256, 511, 1, 0, 300]]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["plain", "swiglu", "clamp", "gelu"])
+@pytest.mark.parametrize("counts,hint", [(c, h) for c in COUNTS for h in (1, 20, 40, 100, 256) if h <= max(16, 2 * max(c))])
+def test_grouped_gemm(counts, hint, form, dtype):
+    E, N, K = len(counts), 384, 200                                     # a k tail of 8, three weight tiles
+    g = torch.Generator(device=DEV).manual_seed(sum(counts) + hint)
+    offsets, at = [], 0
+    for c in counts:
+        offsets.append(at)
+        at += (c + MG.PAD - 1) // MG.PAD * MG.PAD
+    cap = at + 128
+    x = torch.randn(cap, K, device=DEV, generator=g).to(dtype)
+    w = (torch.randn(E, N, K, device=DEV, generator=g) * (0.3 if form == "clamp" else 0.1)).to(dtype)
+    half = form in ("swiglu", "clamp")
+    stacked = torch.stack([B.interleave_gate_up(w[e, :N // 2], w[e, N // 2:]) for e in range(E)]).contiguous() if half else w
+    cols = N // 2 if half else N
+    out = torch.full((cap, cols), 7.0, device=DEV, dtype=dtype)
+    cd, od = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in (counts, offsets))
+    flags = {"plain": 0, "swiglu": B.GEMM_SWIGLU, "clamp": B.GEMM_SWIGLU | B.GEMM_GLU_CLAMP, "gelu": B.GEMM_GELU}[form]
+    rc = _lib.kernels().fb_moe_grouped_gemm_act(x.data_ptr(), stacked.data_ptr(), out.data_ptr(), None, cd.data_ptr(), od.data_ptr(), cap, E, N, K, cols,
+                                                max(counts) | (hint << 16), 1 if dtype == torch.bfloat16 else 0, flags, sum(counts), 2.0, 1.7, _stream())
+    assert rc == 0
+    torch.cuda.synchronize()
+    _lib.check_device_errors()
+    u = torch.finfo(dtype).eps / 2
+    for e, (o, n) in enumerate(zip(offsets, counts)):
+        xs = x[o:o + n].double()
+        y = xs @ w[e].double().t()
+        # the products are exact; each of the sum's K steps may cut off one unit of fp32 of the largest partial sum
+        err = K * 2.0 ** -23 * (xs.abs() @ w[e].double().abs().t())
+        if form == "gelu":
+            y, err = torch.nn.functional.gelu(y), 1.13 * err            # |gelu'| < 1.13
+        elif half:
+            a, b, ea, eb = y[:, :cols], y[:, cols:], err[:, :cols], err[:, cols:]
+            if form == "clamp":
+                a, b = a.clamp(max=2.0), b.clamp(-2.0, 2.0) + 1.0
+                y, slope = a * torch.sigmoid(1.7 * a), 1.1              # |d/da a sigmoid(c a)| < 1.1 for every c
+            else:
+                y, slope = torch.nn.functional.silu(a), 1.1
+            y, err = y * b, slope * ea * b.abs() + y.abs() * eb
+        # the activations in fp32 with fast exponentials (2^-20), then one rounding
+        tol = err + y.abs() * (u + 2.0 ** -20) + 2.0 ** -22
+        if dtype == torch.float16:
+            tol = tol + 2.0 ** -25
+        assert bool(((out[o:o + n].double() - y).abs() <= tol).all()), (e, n, ((out[o:o + n].double() - y).abs() / tol).max().item())
+        assert bool((out[o + n:offsets[e + 1] if e + 1 < E else cap] == 7.0).all())          # rows between the segments stay as they are
+
+
+@pytest.mark.parametrize("T,topk,E,first,n_local", [(513, 8, 8, 0, 8), (700, 6, 1024, 0, 1024), (4001, 10, 512, 0, 512), (2049, 2, 16, 9, 7), (34, 31, 512, 128, 256)])
+def test_plan_on_many_blocks(T, topk, E, first, n_local):
+    g = torch.Generator().manual_seed(T)
+    idx = torch.rand(T, E, generator=g).topk(topk, dim=1).indices.int()
+    idx[:T // 2, 0] = first                                               # a busy expert; a token may name it twice
+    flat = idx.flatten().long() - first
+    mine = (flat >= 0) & (flat < n_local)
+    onehot = torch.zeros(T * topk, n_local, dtype=torch.int32)
+    onehot[mine, flat[mine]] = 1
+    cnt = onehot.sum(0)
+    padded = (cnt + 15) // 16 * 16
+    off = padded.cumsum(0) - padded
+    rank = onehot.cumsum(0) - 1
+    want = torch.full((T * topk,), -1, dtype=torch.long)
+    want[mine] = off[flat[mine]] + rank[mine, flat[mine]]
+    plan = [torch.full((n,), -7, dtype=torch.int32, device=DEV) for n in (n_local, n_local, T * topk, 1)]
+    d = idx.to(DEV)
+    rc = _lib.kernels().fb_moe_plan(d.data_ptr(), T, topk, first, n_local, *(t.data_ptr() for t in plan), 16, _stream())
+    assert rc == 0
+    for got, w in zip(plan, (cnt, off, want, padded.sum().reshape(1))):
+        assert torch.equal(got.cpu().long(), w.long())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,H,topk,ld", [(1, 8, 1, 1), (37, 264, 8, 13), (300, 4096, 3, 544)])
+def test_combine_with_gated_rows(T, H, topk, ld, dtype):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    ys, add = torch.randn(T * topk + 5, H, device=DEV, generator=g).to(dtype), torch.randn(T, H, device=DEV, generator=g).to(dtype)
+    pos = torch.randperm(T * topk + 5, device=DEV, generator=g)[:T * topk].int()
+    pos[::7] = -1                                                         # experts of another rank
+    w = torch.rand(T, topk, device=DEV, generator=g)
+    gate = (4 * torch.randn(T, ld, device=DEV, generator=g))[:, ld // 2]
+    out = torch.empty(T, H, device=DEV, dtype=dtype)
+    picked = (ys.double()[pos.clamp(min=0).long()] * (pos >= 0)[:, None]).view(T, topk, H) * w.double()[:, :, None]
+    for a, gt in ((None, None), (add, None), (add, gate)):
+        rc = _lib.kernels().fb_moe_combine_gated(ys.data_ptr(), pos.data_ptr(), w.data_ptr(), a.data_ptr() if a is not None else None,
+                                                 gt.data_ptr() if gt is not None else None, gt.stride(0) if gt is not None else 0, out.data_ptr(), T, topk, H,
+                                                 1 if dtype == torch.bfloat16 else 0, _stream())
+        assert rc == 0
+        extra = 0.0 if a is None else add.double() * (1.0 if gt is None else torch.sigmoid(gate.double())[:, None])
+        ref = picked.sum(1) + extra
+        size = picked.abs().sum(1) + (extra.abs() if a is not None else 0.0)
+        # topk + 1 sums in fp32 and a fast sigmoid (2^-20), then one rounding
+        tol = ref.abs() * torch.finfo(dtype).eps / 2 + size * ((topk + 1) * 2.0 ** -23 + 2.0 ** -20) + 2.0 ** -25
+        assert bool(((out.double() - ref).abs() <= tol).all())
