@@ -4,7 +4,7 @@
 // runs these as one-CTA-per-output-row GEMV for < 8 tokens and convert + cublasGemmEx otherwise
 // (reference: src/devices/cuda/linear/fastllm-linear-fp16.cu:561-650, fastllm-linear-bf16.cu:332-648).
 //
-// Two kernels, both tcgen05 (UMMA) with fp32 accumulators in TMEM, operands staged by TMA into
+// Three kernels, all tcgen05 (UMMA) with fp32 accumulators in TMEM, operands staged by TMA into
 // 128-byte-swizzled shared memory through an mbarrier ring:
 //
 //  * small-M ("decode") kernel: swap-AB.  The weight tile [128 out-features x 64 k] is the UMMA A operand,
@@ -14,6 +14,7 @@
 //    and writing a slice of the tile with the epilogue applied.  No global scratch.
 //  * large-M ("prefill") kernel: 128 tokens x 256 out-features tile per CTA, K pipelined, epilogue straight
 //    from TMEM to global.
+//  * the same on CTA pairs: 256 x 256 tiles, each SM brings half of the operands that it used to.
 //
 // SwiGLU epilogue expects the gate/up weight rows interleaved per 128-row tile: rows [0,64) of tile t are
 // gate rows 64t..64t+63 and rows [64,128) are the matching up rows; output column = 64t + i.
@@ -25,6 +26,7 @@ FB_DEFINE_ERROR_API(gemm)
 
 #include "gemm_smallm.cuh"
 #include "gemm_largem.cuh"
+#include "gemm_pair.cuh"
 
 namespace fb {
 
@@ -69,6 +71,12 @@ __global__ void __launch_bounds__(192, 1)
 gemm_largem_extra_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const GemmParams p,
                          int tiles_m, int tiles_n, const GemmExtra ex) {
   gemm_largem_device<BN, BF16, LargeMPlainHook, true>(tmX, tmW, p, tiles_m, tiles_n, LargeMPlainHook{}, ex);
+}
+
+template <bool BF16, bool EXTRA>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const GemmParams p, int tiles_m, int tiles_n, const GemmExtra ex) {
+  gemm_pair_device<BF16, LargeMPlainHook, EXTRA>(tmX, tmW, p, tiles_m, tiles_n, LargeMPlainHook{}, ex);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -263,7 +271,35 @@ static cudaError_t launch_largem(const CUtensorMap& tmX, const CUtensorMap& tmW,
   return cudaGetLastError();
 }
 
+template <bool BF16>
+static cudaError_t launch_pair(const CUtensorMap& tmX, const CUtensorMap& tmW, const GemmParams& p, cudaStream_t stream, const GemmExtra* ex, int sms) {
+  auto kern = gemm_pair_kernel<BF16, false>;
+  auto kern_extra = gemm_pair_kernel<BF16, true>;
+  static DeviceOnce configured;
+  if (configured.need()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern_extra, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+  }
+  const int tiles_n = (p.N + 255) / 256, tiles_m = (p.M + 255) / 256;
+  const long long tiles = (long long)tiles_n * tiles_m;
+  const int grid = 2 * (int)(tiles < sms / 2 ? tiles : sms / 2);
+  if (ex != nullptr) kern_extra<<<grid, 192, PairCfg::SMEM_BYTES, stream>>>(tmX, tmW, p, tiles_m, tiles_n, *ex);
+  else kern<<<grid, 192, PairCfg::SMEM_BYTES, stream>>>(tmX, tmW, p, tiles_m, tiles_n, GemmExtra());
+  return cudaGetLastError();
+}
+
 }  // namespace fb
+
+// CTA pairs (256 x 256 tiles) or one CTA a tile (128 x bn): rounds of tiles over the SMs times the time of a round.  With 4096 of k a round of pairs takes
+// 26 us, of 128 x 256 tiles 34, of 128 x 128 tiles 18 to 20 (counted as 4, 5 and 3).  Both sides in us, one CTA -> pairs: 8190 x 6144 x 4096 322 -> 277,
+// 1000 x 4096 x 14336 121 -> 91, 4095 x 5120 x 2048 82 -> 72, 600 x 4096 x 4096 48 -> 42; 333 x 28672 x 4096 (3 rounds against 4) 102 -> 105 and
+// 333 x 6144 x 4096 30 -> 37 stay with one CTA.
+static bool pair_is_faster(int M, int N, int bn, int sms) {
+  const long long one = (long long)((N + bn - 1) / bn) * ((M + 127) / 128), two = (long long)((N + 255) / 256) * ((M + 255) / 256);
+  const long long rounds_one = (one + sms - 1) / sms, rounds_two = (two + sms / 2 - 1) / (sms / 2);
+  return 4 * rounds_two < (bn == 256 ? 5 : 3) * rounds_one;
+}
 
 // Heuristic used by the launcher: how many cluster ranks split K so that about one CTA lands on each SM.
 extern "C" int fb_gemm_pick_split(int M, int N, int K, int slots) {
@@ -386,14 +422,21 @@ static int gemm_16bit_impl(const void* X, const void* W, void* out, const void* 
   }
   if (N % 32 != 0) return -1;
   p.kb_per_split = p.kb_total;
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int bn = (N >= 256 && N % 256 == 0) || N > 2048 ? 256 : 128;
   {
     // too few 128 x 256 tiles to occupy the SMs (a few hundred tokens): halve the tile width to double the CTA count
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long t256 = (long long)((N + 255) / 256) * ((M + 127) / 128);
     if (bn == 256 && t256 < sms && !(flags & GEMM_SWIGLU && N % 256 != 0)) bn = 128;
+  }
+  if (pair_is_faster(M, N, bn, sms)) {
+    p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 256, 256);
+    CUtensorMap tmW, tmX;
+    if (!make_tmap_2d(&tmX, X, M, K, ldx, 128, 64, 2, 3)) return -2;
+    if (!make_tmap_2d(&tmW, W, N, K, ldw, 128, 64, 2, 3)) return -2;
+    return (int)(bf16 ? launch_pair<true>(tmX, tmW, p, stream, ex, sms) : launch_pair<false>(tmX, tmW, p, stream, ex, sms));
   }
   p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, bn);
   CUtensorMap tmW, tmX;
@@ -586,6 +629,15 @@ extern "C" int fb_gemm_16bit_blocks(const void* X, const void* W, float* out, in
   p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, bn);
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   CUtensorMap tmW, tmX;
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (bn == 256 && pair_is_faster(M, p.N, bn, sms)) {            // (a 256-row weight tile lies within one block)
+    p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 256, 256);
+    if (!make_tmap_2d(&tmX, X, M, (uint64_t)batch * K, ldx, 128, 64, 2, 3)) return -2;
+    if (!make_tmap_2d(&tmW, W, (uint64_t)batch * N, K, K, 128, 64, 2, 3)) return -2;
+    return (int)(bf16 ? launch_pair<true>(tmX, tmW, p, stream, nullptr, sms) : launch_pair<false>(tmX, tmW, p, stream, nullptr, sms));
+  }
   if (!make_tmap_2d(&tmX, X, M, (uint64_t)batch * K, ldx, 128, 64, 2, 3)) return -2;
   if (!make_tmap_2d(&tmW, W, (uint64_t)batch * N, K, K, bn, 64, 2, 3)) return -2;
   if (bn == 256)
