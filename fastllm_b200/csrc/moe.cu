@@ -251,8 +251,8 @@ moe_plan_table_kernel(const long long* __restrict__ meta, const int* __restrict_
 // an expert's projections (512 to 2048: 8 to 32 stages) does not pay a pipeline fill, a TMEM set-up and a drain per tile, and two
 // accumulators let the epilogue of a tile run under the products of the next.  Chunks of one expert are neighbours in the list: the
 // second reads the weights from L2.  The product is as wide as the chunk has rows (multiples of 16), whatever the tile is laid out for.
-// Per layer of width 2048 (gate/up + down; us; one CTA per tile before): 128 experts x 768 at 4095 x 8 rows 948 -> 600, 512 x 512 at 4001 x 10
-// rows 1597 -> 640, at 32 x 10 rows 657 -> 263, 128 x 768 at 32 x 8 rows 237 -> 179.
+// Per layer of width 2048 (gate/up + down; us; one CTA per tile before): 128 experts x 768 at 4095 x 8 rows 948 -> 372, 512 x 512 at 4001 x 10
+// rows 1597 -> 592, at 32 x 10 rows 657 -> 263, 128 x 768 at 32 x 8 rows 237 -> 179.
 struct MoeStreamInfo {
   const int* counts;       // [n_local] routed rows per expert
   const int* offsets;      // [n_local] first row of the expert's segment in the sorted buffer
@@ -265,8 +265,8 @@ struct MoeStreamCfg {
   static constexpr int A_BYTES = 128 * 128;
   static constexpr int BOX = MPAD < 64 ? MPAD : 64;                 // token rows per load
   static constexpr int STAGE_BYTES = A_BYTES + MPAD * 128;
-  static constexpr int X_BYTES = 2 * 32 * 64 * 4;                   // up sums on their way to the gate's warps, two buffers of 32 tokens
-  static constexpr int TAIL_BYTES = X_BYTES + (MS_MAX_EXPERTS + 1) * 4 + 28 + 512;
+  static constexpr int X_BYTES = 2 * (MPAD < 32 ? MPAD : 32) * 64 * 4;      // sums that gate and up warps exchange, two buffers of 32 tokens
+  static constexpr int TAIL_BYTES = X_BYTES + 3 * MS_MAX_EXPERTS * 4 + 32 + 512;
   static constexpr int MAX_STAGES = (226 * 1024 - TAIL_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = MAX_STAGES > 12 ? 12 : MAX_STAGES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + TAIL_BYTES + 1024;
@@ -274,16 +274,16 @@ struct MoeStreamCfg {
 };
 
 struct MoeTile { int e, n_tile, row0, rows; };
-// tile t of the list; first[e] = chunks of the experts before e
+// tile t of the list; first[e] = chunks of the experts before e, counts[e] = rows
 template <int MPAD>
-__device__ __forceinline__ MoeTile moe_tile(const MoeStreamInfo& gi, const int* first, int t) {
+__device__ __forceinline__ MoeTile moe_tile(const MoeStreamInfo& gi, const int* first, const int* counts, int t) {
   int lo = 0, hi = gi.n_local - 1;                     // the last expert whose first tile is at or before t
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (first[mid] * gi.n_tiles <= t) lo = mid; else hi = mid - 1;
   }
   MoeTile r;
-  const int ch = first[lo + 1] - first[lo], at = t - first[lo] * gi.n_tiles, cnt = gi.counts[lo];
+  const int ch = first[lo + 1] - first[lo], at = t - first[lo] * gi.n_tiles, cnt = counts[lo];
   const int per = ((cnt + ch - 1) / ch + 15) & ~15;    // rows of a chunk: equal shares, at most MPAD
   const int chunk = at % ch;
   r.e = lo;
@@ -291,6 +291,22 @@ __device__ __forceinline__ MoeTile moe_tile(const MoeStreamInfo& gi, const int* 
   r.row0 = chunk * per;
   r.rows = min(per, cnt - r.row0);
   return r;
+}
+
+// One output column of the first cnt of N tokens, ld apart.  One epilogue warp sits on each sub-core, so its instructions are a chain: with an
+// address from scratch and two conditions per element (21 instructions) the epilogue took longer than the tile's products.
+template <int N, bool BF16>
+__device__ __forceinline__ void store_column(uint16_t* out, int ld, const float (&v)[N], int cnt) {
+  if (cnt >= N) {
+#pragma unroll
+    for (int j = 0; j < N; ++j, out += ld) *out = (uint16_t)(pack_16<BF16>(v[j], 0.f) & 0xFFFFu);
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j, out += ld) {
+      if (j >= cnt) break;
+      *out = (uint16_t)(pack_16<BF16>(v[j], 0.f) & 0xFFFFu);
+    }
+  }
 }
 
 template <int MPAD, bool BF16, bool EXTRA>
@@ -302,7 +318,9 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* X = reinterpret_cast<float*>(smem + Cfg::STAGES * Cfg::STAGE_BYTES);
   int* first = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(X) + Cfg::X_BYTES);              // [n_local + 1]
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(first + MS_MAX_EXPERTS + 8);
+  int* counts = first + MS_MAX_EXPERTS + 8;            // copies of the plan's tables: a tile is looked up by three roles
+  int* offsets = counts + MS_MAX_EXPERTS;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(offsets + MS_MAX_EXPERTS);
   uint64_t* empty_bar = full_bar + Cfg::STAGES;
   uint64_t* acc_full = empty_bar + Cfg::STAGES;        // [2]
   uint64_t* acc_empty = acc_full + 2;                  // [2]
@@ -322,7 +340,13 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   {
     const int each = (gi.n_local + 191) / 192, e0 = tid * each;
     int sum = 0;
-    for (int i = 0; i < each; ++i) sum += e0 + i < gi.n_local ? (gi.counts[e0 + i] + MPAD - 1) / MPAD : 0;
+    for (int i = 0; i < each; ++i) {
+      if (e0 + i >= gi.n_local) break;
+      const int c = gi.counts[e0 + i];
+      counts[e0 + i] = c;
+      offsets[e0 + i] = gi.offsets[e0 + i];
+      sum += (c + MPAD - 1) / MPAD;
+    }
     int incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
@@ -333,7 +357,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     for (int i = 0; i < each; ++i) {
       if (e0 + i >= gi.n_local) break;
       first[e0 + i] = run;
-      run += (gi.counts[e0 + i] + MPAD - 1) / MPAD;
+      run += (counts[e0 + i] + MPAD - 1) / MPAD;
       if (e0 + i == gi.n_local - 1) first[gi.n_local] = run;
     }
   }
@@ -349,9 +373,9 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const uint64_t pol_x = l2_policy_evict_last();
       int it = 0;
       for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
-        const MoeTile m = moe_tile<MPAD>(gi, first, t);
+        const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
         if (m.rows <= 0) continue;
-        const int w_row = (m.e * gi.n_tiles + m.n_tile) * 128, x_row = gi.offsets[m.e] + m.row0, boxes = (m.rows + Cfg::BOX - 1) / Cfg::BOX;
+        const int w_row = (m.e * gi.n_tiles + m.n_tile) * 128, x_row = offsets[m.e] + m.row0, boxes = (m.rows + Cfg::BOX - 1) / Cfg::BOX;
         for (int i = 0; i < kb_cnt; ++i, ++it) {
           const int s = it % Cfg::STAGES;
           if (!mbar_wait(&empty_bar[s], ((uint32_t)(it / Cfg::STAGES) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 1)) break;
@@ -368,7 +392,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     if (elect_one()) {
       int it = 0, u = 0;
       for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
-        const MoeTile m = moe_tile<MPAD>(gi, first, t);
+        const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
         if (m.rows <= 0) continue;
         const int buf = u & 1;
         if (!mbar_wait(&acc_empty[buf], ((uint32_t)(u >> 1) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 4)) break;
@@ -397,7 +421,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
     int u = 0, ci = 0;                                 // tiles and 32-token pieces done
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
-      const MoeTile m = moe_tile<MPAD>(gi, first, t);
+      const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
       if (m.rows <= 0) continue;
       const int buf = u & 1;
       mbar_wait(&acc_full[buf], (uint32_t)(u >> 1) & 1u, dead, KID_MOE_GROUPED, 3);
@@ -405,7 +429,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       __syncwarp();
       tc_fence_after_sync();
       const uint32_t acc = tmem_base + (uint32_t)(buf * MPAD) + ((uint32_t)(q * 32) << 16);
-      uint16_t* orow = outp + (size_t)(gi.offsets[m.e] + m.row0) * p.ld_out;
+      uint16_t* orow = outp + (size_t)(offsets[m.e] + m.row0) * p.ld_out;
       constexpr int CH = MPAD < 32 ? MPAD : 32;
       for (int c0 = 0; c0 < m.rows; c0 += CH, ++ci) {
         uint32_t r[32];
@@ -414,43 +438,46 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
         tmem_ld_wait();
         const int cnt = min(CH, m.rows - c0);
         if (swiglu) {
-          // rows 0..63 of a tile are gate rows, 64..127 the up rows of the same columns: barrier 1 + b "buffer b holds up sums", 3 + b "buffer b has been read"
-          const int b = ci & 1;
-          float* xb = X + b * 32 * 64;
-          if (q >= 2) {
-            if (ci >= 2) asm volatile("bar.sync %0, 128;\n" ::"r"(3 + b) : "memory");
+          // rows 0..63 of a tile are gate rows, 64..127 the up rows of the same columns.  The gate's warps do the first half of the tokens and take the
+          // up sums from shared memory, the up warps do the second half and take the gate sums; two buffers, so one barrier a piece is enough
+          constexpr int HALF = CH / 2;
+          const int col = n_local & 63, first_tok = q < 2 ? 0 : HALF;
+          float* xb = X + (ci & 1) * CH * 64 + col;
+          float v[HALF], o[HALF];
+          if (q < 2) {
 #pragma unroll
-            for (int j = 0; j < CH; ++j) xb[j * 64 + n_local - 64] = __uint_as_float(r[j]);
-            asm volatile("bar.arrive %0, 128;\n" ::"r"(1 + b) : "memory");
+            for (int j = 0; j < HALF; ++j) { v[j] = __uint_as_float(r[j]); xb[(HALF + j) * 64] = __uint_as_float(r[HALF + j]); }
           } else {
-            asm volatile("bar.sync %0, 128;\n" ::"r"(1 + b) : "memory");
-            const int n = m.n_tile * 64 + n_local;
-            const bool live = !dead && n < (p.N >> 1);
 #pragma unroll
-            for (int j = 0; j < CH; ++j) {
-              const float g = __uint_as_float(r[j]), up = xb[j * 64 + n_local];
-              const float v = (p.flags & GEMM_GLU_CLAMP) ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : silu_f(g) * up;
-              if (live && j < cnt) orow[(size_t)(c0 + j) * p.ld_out + n] = (uint16_t)(pack_16<BF16>(v, 0.f) & 0xFFFFu);
-            }
-            asm volatile("bar.arrive %0, 128;\n" ::"r"(3 + b) : "memory");
+            for (int j = 0; j < HALF; ++j) { v[j] = __uint_as_float(r[HALF + j]); xb[j * 64] = __uint_as_float(r[j]); }
           }
+          asm volatile("bar.sync 1, 128;\n" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < HALF; ++j) o[j] = xb[(first_tok + j) * 64];
+          const bool clamp = (p.flags & GEMM_GLU_CLAMP) != 0;
+#pragma unroll
+          for (int j = 0; j < HALF; ++j) {
+            const float g = q < 2 ? v[j] : o[j], up = q < 2 ? o[j] : v[j];
+            v[j] = clamp ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : silu_f(g) * up;
+          }
+          const int n = m.n_tile * 64 + col;
+          if (!dead && n < (p.N >> 1)) store_column<HALF, BF16>(orow + (size_t)(c0 + first_tok) * p.ld_out + n, p.ld_out, v, cnt - first_tok);
         } else {
           const int n = m.n_tile * 128 + n_local;
-          const bool live = !dead && n < p.N;
+          float v[CH];
 #pragma unroll
-          for (int j = 0; j < CH; ++j) {
-            float v = __uint_as_float(r[j]);
-            if (EXTRA && (p.flags & GEMM_GELU)) v = gelu_erf_f(v);
-            if (live && j < cnt) orow[(size_t)(c0 + j) * p.ld_out + n] = (uint16_t)(pack_16<BF16>(v, 0.f) & 0xFFFFu);
+          for (int j = 0; j < CH; ++j) v[j] = __uint_as_float(r[j]);
+          if (EXTRA && (p.flags & GEMM_GELU)) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) v[j] = gelu_erf_f(v[j]);
           }
+          if (!dead && n < p.N) store_column<CH, BF16>(orow + (size_t)c0 * p.ld_out + n, p.ld_out, v, cnt);
         }
       }
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
-    if (swiglu && q >= 2)                              // the last two buffers' arrivals are taken, too
-      for (int k = ci > 2 ? ci - 2 : 0; k < ci; ++k) asm volatile("bar.sync %0, 128;\n" ::"r"(3 + (k & 1)) : "memory");
   }
   tc_fence_before_sync();
   __syncthreads();
