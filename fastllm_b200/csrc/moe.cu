@@ -251,20 +251,25 @@ moe_plan_table_kernel(const long long* __restrict__ meta, const int* __restrict_
 // an expert's projections (512 to 2048: 8 to 32 stages) does not pay a pipeline fill, a TMEM set-up and a drain per tile, and two
 // accumulators let the epilogue of a tile run under the products of the next.  Chunks of one expert are neighbours in the list: the
 // second reads the weights from L2.  The product is as wide as the chunk has rows (multiples of 16), whatever the tile is laid out for.
-// Per layer of width 2048 (gate/up + down; us; one CTA per tile before): 128 experts x 768 at 4095 x 8 rows 948 -> 372, 512 x 512 at 4001 x 10
+// Per layer of width 2048 (gate/up + down; us; one CTA per tile before): 128 experts x 768 at 4095 x 8 rows 948 -> 326, 512 x 512 at 4001 x 10
 // rows 1597 -> 592, at 32 x 10 rows 657 -> 263, 128 x 768 at 32 x 8 rows 237 -> 179.
 struct MoeStreamInfo {
   const int* counts;       // [n_local] routed rows per expert
   const int* offsets;      // [n_local] first row of the expert's segment in the sorted buffer
-  int n_local, n_tiles;    // weight tiles per expert
+  int n_local, n_tiles;    // tiles of a chunk: 128 weight rows, 256 for a pair
+  int w_tiles;             // 128-row weight tiles per expert
 };
 
 constexpr int MS_MAX_EXPERTS = 1024;
-template <int MPAD>
+// Tiles laid out for this many rows or more are done by CTA pairs: 128 experts, 4095 x 8 rows 238 + 133 -> 206 + 120 us; with tiles of 128 rows
+// (512 experts, 4001 x 10 rows) pairs take 378 + 233 us, one CTA a tile 380 + 212.
+constexpr int MS_PAIR_FROM = 256;
+template <int MPAD, bool PAIR>
 struct MoeStreamCfg {
   static constexpr int A_BYTES = 128 * 128;
-  static constexpr int BOX = MPAD < 64 ? MPAD : 64;                 // token rows per load
-  static constexpr int STAGE_BYTES = A_BYTES + MPAD * 128;
+  static constexpr int X_ROWS = PAIR ? MPAD / 2 : MPAD;             // token rows that one CTA holds
+  static constexpr int BOX = X_ROWS < 64 ? X_ROWS : 64;             // token rows per load
+  static constexpr int STAGE_BYTES = A_BYTES + X_ROWS * 128;
   static constexpr int X_BYTES = 2 * (MPAD < 32 ? MPAD : 32) * 64 * 4;      // sums that gate and up warps exchange, two buffers of 32 tokens
   static constexpr int TAIL_BYTES = X_BYTES + 3 * MS_MAX_EXPERTS * 4 + 32 + 512;
   static constexpr int MAX_STAGES = (226 * 1024 - TAIL_BYTES) / STAGE_BYTES;
@@ -309,10 +314,10 @@ __device__ __forceinline__ void store_column(uint16_t* out, int ld, const float 
   }
 }
 
-template <int MPAD, bool BF16, bool EXTRA>
+template <int MPAD, bool BF16, bool EXTRA, bool PAIR>
 __global__ void __launch_bounds__(192, 1)
 moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmParams p, const MoeStreamInfo gi) {
-  using Cfg = MoeStreamCfg<MPAD>;
+  using Cfg = MoeStreamCfg<MPAD, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ int wsum[6];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -326,16 +331,21 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   uint64_t* acc_empty = acc_full + 2;                  // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = PAIR ? (int)cluster_ctarank() : 0;
+  const int unit = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, units = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   bool dead = false;
   pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < Cfg::STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 4); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], PAIR ? 8 : 4); }
     mbar_init_fence();
     tma_prefetch_desc(&tmW);
     tma_prefetch_desc(&tmX);
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
+  if (warp == 1) {
+    if (PAIR) { tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish_pair(); }
+    else { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
+  }
   pdl_wait();                                          // counts and offsets come from the plan kernel
   {
     const int each = (gi.n_local + 191) / 192, e0 = tid * each;
@@ -363,6 +373,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (PAIR) cluster_sync_all();                        // the other CTA's barriers exist, too
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   const int total = first[gi.n_local] * gi.n_tiles, kb_cnt = p.kb_total;
@@ -372,44 +383,62 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       const uint64_t pol_w = l2_policy_evict_first();
       const uint64_t pol_x = l2_policy_evict_last();
       int it = 0;
-      for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
+      for (int t = unit; t < total && !dead; t += units) {
         const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
         if (m.rows <= 0) continue;
-        const int w_row = (m.e * gi.n_tiles + m.n_tile) * 128, x_row = offsets[m.e] + m.row0, boxes = (m.rows + Cfg::BOX - 1) / Cfg::BOX;
+        const int share = PAIR ? ((m.rows + 31) & ~31) >> 1 : m.rows;              // token rows of this CTA
+        const int w_row = (m.e * gi.w_tiles + (PAIR ? 2 * m.n_tile + rank : m.n_tile)) * 128, x_row = offsets[m.e] + m.row0 + rank * share;
+        const int boxes = (share + Cfg::BOX - 1) / Cfg::BOX;
         for (int i = 0; i < kb_cnt; ++i, ++it) {
           const int s = it % Cfg::STAGES;
           if (!mbar_wait(&empty_bar[s], ((uint32_t)(it / Cfg::STAGES) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 1)) break;
           uint8_t* a = smem + s * Cfg::STAGE_BYTES;
+          if (PAIR) {
+            const uint32_t bar = mapa_u32(smem_u32(&full_bar[s]), 0);
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (Cfg::A_BYTES + boxes * Cfg::BOX * 128));
+            tma_load_2d_pair(a, &tmW, bar, i * 64, w_row);
+            for (int b = 0; b < boxes; ++b) tma_load_2d_pair(a + Cfg::A_BYTES + b * Cfg::BOX * 128, &tmX, bar, i * 64, x_row + b * Cfg::BOX);
+            continue;
+          }
           mbar_expect_tx(&full_bar[s], Cfg::A_BYTES + boxes * Cfg::BOX * 128);
           if (MPAD <= 64) tma_load_2d_hint(a, &tmW, &full_bar[s], i * 64, w_row, pol_w);
           else tma_load_2d(a, &tmW, &full_bar[s], i * 64, w_row);                 // (the expert's next chunk reads them again)
           for (int b = 0; b < boxes; ++b) tma_load_2d_hint(a + Cfg::A_BYTES + b * Cfg::BOX * 128, &tmX, &full_bar[s], i * 64, x_row + b * Cfg::BOX, pol_x);
         }
       }
+      // a pair: the last products' commits have reached this CTA before it may leave
+      for (int k = !PAIR ? it : it > Cfg::STAGES ? it - Cfg::STAGES : 0; k < it; ++k)
+        if (!mbar_wait(&empty_bar[k % Cfg::STAGES], (uint32_t)(k / Cfg::STAGES) & 1u, dead, KID_MOE_GROUPED, 5)) break;
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (elect_one()) {
+    if (rank == 0 && elect_one()) {
       int it = 0, u = 0;
-      for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
+      for (int t = unit; t < total && !dead; t += units) {
         const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
         if (m.rows <= 0) continue;
         const int buf = u & 1;
-        if (!mbar_wait(&acc_empty[buf], ((uint32_t)(u >> 1) & 1u) ^ 1u, dead, KID_MOE_GROUPED, 4)) break;
+        const uint32_t use = ((uint32_t)(u >> 1) & 1u) ^ 1u;
+        if (!(PAIR ? mbar_wait_cluster(&acc_empty[buf], use, dead, KID_MOE_GROUPED, 4) : mbar_wait(&acc_empty[buf], use, dead, KID_MOE_GROUPED, 4))) break;
         tc_fence_after_sync();
-        const uint32_t acc = tmem_base + (uint32_t)(buf * MPAD), idesc = p.idesc | ((uint32_t)((m.rows + 15) >> 4) << 18);      // N = rows in multiples of 16
+        // N = rows in multiples of 16 (a pair: of 16 a CTA)
+        const uint32_t acc = tmem_base + (uint32_t)(buf * MPAD), idesc = p.idesc | ((PAIR ? (uint32_t)((m.rows + 31) >> 5) << 1 : (uint32_t)((m.rows + 15) >> 4)) << 18);
         for (int i = 0; i < kb_cnt; ++i, ++it) {
           const int s = it % Cfg::STAGES;
-          if (!mbar_wait(&full_bar[s], (uint32_t)(it / Cfg::STAGES) & 1u, dead, KID_MOE_GROUPED, 2)) break;
+          const uint32_t ph = (uint32_t)(it / Cfg::STAGES) & 1u;
+          if (!(PAIR ? mbar_wait_cluster(&full_bar[s], ph, dead, KID_MOE_GROUPED, 2) : mbar_wait(&full_bar[s], ph, dead, KID_MOE_GROUPED, 2))) break;
           tc_fence_after_sync();
           const uint32_t a_addr = smem_u32(smem + s * Cfg::STAGE_BYTES);
           const uint64_t da = make_smem_desc(a_addr, 16, 1024, SWZ_128B), db = make_smem_desc(a_addr + Cfg::A_BYTES, 16, 1024, SWZ_128B);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16(acc, da + 2 * k, db + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
-          umma_commit(&empty_bar[s]);
+          for (int k = 0; k < 4; ++k) {
+            if (PAIR) umma_f16_pair(acc, da + 2 * k, db + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+            else umma_f16(acc, da + 2 * k, db + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+          }
+          if (PAIR) umma_commit_pair(&empty_bar[s]); else umma_commit(&empty_bar[s]);
         }
         if (dead) break;
-        umma_commit(&acc_full[buf]);
+        if (PAIR) umma_commit_pair(&acc_full[buf]); else umma_commit(&acc_full[buf]);
         ++u;
       }
     }
@@ -420,11 +449,13 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
     const bool swiglu = (p.flags & GEMM_SWIGLU) != 0;
     uint16_t* outp = reinterpret_cast<uint16_t*>(p.out);
     int u = 0, ci = 0;                                 // tiles and 32-token pieces done
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-      const MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
+    for (int t = unit; t < total; t += units) {
+      MoeTile m = moe_tile<MPAD>(gi, first, counts, t);
       if (m.rows <= 0) continue;
+      if (PAIR) m.n_tile = 2 * m.n_tile + rank;        // this CTA's weight rows
       const int buf = u & 1;
-      mbar_wait(&acc_full[buf], (uint32_t)(u >> 1) & 1u, dead, KID_MOE_GROUPED, 3);
+      if (PAIR) mbar_wait_cluster(&acc_full[buf], (uint32_t)(u >> 1) & 1u, dead, KID_MOE_GROUPED, 3);
+      else mbar_wait(&acc_full[buf], (uint32_t)(u >> 1) & 1u, dead, KID_MOE_GROUPED, 3);
       ++u;
       __syncwarp();
       tc_fence_after_sync();
@@ -476,19 +507,27 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
       }
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[buf]), 0)); else mbar_arrive(&acc_empty[buf]);
+      }
     }
   }
+  __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  if (PAIR) cluster_sync_all();                        // neither CTA's barriers or operands are in use any more
+  if (warp == 1) {
+    if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS); else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+  }
+  __syncwarp();
+  if (PAIR) cluster_sync_all();
 }
 
-template <int MPAD, bool BF16>
+template <int MPAD, bool BF16, bool PAIR>
 static cudaError_t launch_stream(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, const MoeStreamInfo& gi, int grid, cudaStream_t stream) {
-  using Cfg = MoeStreamCfg<MPAD>;
-  auto plain = moe_stream_kernel<MPAD, BF16, false>;
-  auto extra = moe_stream_kernel<MPAD, BF16, true>;
+  using Cfg = MoeStreamCfg<MPAD, PAIR>;
+  auto plain = moe_stream_kernel<MPAD, BF16, false, PAIR>;
+  auto extra = moe_stream_kernel<MPAD, BF16, true, PAIR>;
   static DeviceOnce configured;
   if (configured.need()) {
     cudaError_t e = cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
@@ -500,8 +539,13 @@ static cudaError_t launch_stream(const CUtensorMap& tmW, const CUtensorMap& tmX,
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, 0);
+  cudaLaunchAttribute attr[2];
+  if (PAIR) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  }
+  cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, PAIR ? 1 : 0);
   return cudaLaunchKernelEx(&cfg, (p.flags & GEMM_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
 }
 
@@ -588,9 +632,10 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
   GemmParams p = {};
   p.out = out; p.N = N; p.K = K; p.ld_out = ld_out; p.kb_total = (K + 63) / 64; p.flags = flags;
   p.act_limit = act_limit; p.act_alpha = act_alpha;
-  p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, 0);
+  const bool pair = mpad >= MS_PAIR_FROM;
+  p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, pair ? 256 : 128, 0);
   MoeStreamInfo gi;
-  gi.counts = counts; gi.offsets = offsets; gi.n_local = E_local; gi.n_tiles = n_tiles;
+  gi.counts = counts; gi.offsets = offsets; gi.n_local = E_local; gi.n_tiles = pair ? (n_tiles + 1) / 2 : n_tiles; gi.w_tiles = n_tiles;
   CUtensorMap tmW, tmX;
   if (!make_tmap_2d(&tmW, W, (uint64_t)E_local * n_tiles * 128, K, K, 128, 64, 2, 3)) return -2;
   if (!make_tmap_2d(&tmX, Xs, rows_cap, K, K, mpad < 64 ? mpad : 64, 64, 2, 3)) return -2;
@@ -603,8 +648,10 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
   // no more CTAs than tiles can exist: every routed row touches an expert, every expert's last chunk may be short
   long long bound = (long long)E_local * ((most + mpad - 1) / mpad);
   if (total_rows > 0 && bound > (long long)total_rows) bound = total_rows;
-  const int grid = (int)(bound * n_tiles < sms ? bound * n_tiles : sms);
-#define FB_MG(MP) return (int)(bf16 ? launch_stream<MP, true>(tmW, tmX, p, gi, grid, stream) : launch_stream<MP, false>(tmW, tmX, p, gi, grid, stream));
+  const int units = pair ? sms / 2 : sms;
+  const int grid = (int)(bound * gi.n_tiles < units ? bound * gi.n_tiles : units) * (pair ? 2 : 1);
+#define FB_MG(MP) \
+  return (int)(bf16 ? launch_stream<MP, true, (MP >= MS_PAIR_FROM)>(tmW, tmX, p, gi, grid, stream) : launch_stream<MP, false, (MP >= MS_PAIR_FROM)>(tmW, tmX, p, gi, grid, stream));
   switch (mpad) {
     case 16: FB_MG(16)
     case 32: FB_MG(32)
