@@ -740,7 +740,8 @@ __global__ void argmax_kernel(const void* __restrict__ logits, int* __restrict__
 // ------------------------------------------------------------------------------------------------
 // Router: scores = softmax / sigmoid / identity of logits [M, E] (fp32), optional bias added for selection
 // only, optional group-limited selection (n_group groups, keep topk_group groups ranked by the sum of their
-// two best biased scores), top-k, optional renormalisation, times route_scale.  One warp per token, E <= 512.
+// two best biased scores), top-k, optional renormalisation, times route_scale.  One warp per token, E <= 512.  PER: scores a lane holds,
+// in registers: as arrays walked by a run-time count they lay in local memory (512 experts, 10 picked, with the launch: 32 tokens 20.6 -> 11.1 us, 4001 tokens 50 -> 25.3).
 // ------------------------------------------------------------------------------------------------
 struct RouteParams {
   const float* logits; const float* bias; int* out_idx; float* out_w;
@@ -748,26 +749,31 @@ struct RouteParams {
   float route_scale;
   int ld, group_max;         // row stride of the logits; a group's score is its largest score instead of the sum of its two largest
 };
-__global__ void route_topk_kernel(const RouteParams p) {
+template <int PER>
+__global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
   pdl_launch_dependents();
   pdl_wait();
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (gw >= p.M) return;
   const float* lg = p.logits + (size_t)gw * p.ld;
-  float sc[16], sel[16];
-  const int per = (p.E + 31) >> 5;
+  float sc[PER], sel[PER];
   float mx = -INFINITY;
-  for (int s = 0; s < per; ++s) { const int e = lane + 32 * s; sc[s] = e < p.E ? lg[e] : -INFINITY; mx = fmaxf(mx, sc[s]); }
+#pragma unroll
+  for (int s = 0; s < PER; ++s) { const int e = lane + 32 * s; sc[s] = e < p.E ? lg[e] : -INFINITY; mx = fmaxf(mx, sc[s]); }
   if (p.score_mode == 0) {
     mx = warp_max(mx);
     float sum = 0.f;
-    for (int s = 0; s < per; ++s) { const int e = lane + 32 * s; sc[s] = e < p.E ? __expf(sc[s] - mx) : 0.f; sum += sc[s]; }
+#pragma unroll
+    for (int s = 0; s < PER; ++s) { const int e = lane + 32 * s; sc[s] = e < p.E ? __expf(sc[s] - mx) : 0.f; sum += sc[s]; }
     sum = warp_sum(sum);
-    for (int s = 0; s < per; ++s) sc[s] /= sum;
+#pragma unroll
+    for (int s = 0; s < PER; ++s) sc[s] /= sum;
   } else if (p.score_mode == 1) {
-    for (int s = 0; s < per; ++s) sc[s] = 1.f / (1.f + __expf(-sc[s]));
+#pragma unroll
+    for (int s = 0; s < PER; ++s) sc[s] = 1.f / (1.f + __expf(-sc[s]));
   }
-  for (int s = 0; s < per; ++s) {
+#pragma unroll
+  for (int s = 0; s < PER; ++s) {
     const int e = lane + 32 * s;
     sel[s] = e < p.E ? sc[s] + (p.bias ? p.bias[e] : 0.f) : -INFINITY;
   }
@@ -777,7 +783,8 @@ __global__ void route_topk_kernel(const RouteParams p) {
     float gscore[32];
     for (int g = 0; g < p.n_group; ++g) {
       float m1 = -INFINITY, m2 = -INFINITY;
-      for (int s = 0; s < per; ++s) {
+#pragma unroll
+      for (int s = 0; s < PER; ++s) {
         const int e = lane + 32 * s;
         if (e < p.E && e / gs == g) { const float x = sel[s]; if (x > m1) { m2 = m1; m1 = x; } else if (x > m2) m2 = x; }
       }
@@ -799,7 +806,8 @@ __global__ void route_topk_kernel(const RouteParams p) {
         if (!((keep >> g) & 1u) && (bg < 0 || gscore[g] > bv)) { bg = g; bv = gscore[g]; }
       keep |= 1u << bg;
     }
-    for (int s = 0; s < per; ++s) {
+#pragma unroll
+    for (int s = 0; s < PER; ++s) {
       const int e = lane + 32 * s;
       if (e < p.E && !((keep >> (e / gs)) & 1u)) sel[s] = -INFINITY;
     }
@@ -808,7 +816,8 @@ __global__ void route_topk_kernel(const RouteParams p) {
   float my_w = 0.f; int my_i = 0;
   for (int k = 0; k < p.topk; ++k) {
     float bv = -INFINITY; int bi = 0x7fffffff; float bs = 0.f;
-    for (int s = 0; s < per; ++s) {
+#pragma unroll
+    for (int s = 0; s < PER; ++s) {
       const int e = lane + 32 * s;
       if (e < p.E && (sel[s] > bv || (sel[s] == bv && e < bi))) { bv = sel[s]; bi = e; bs = sc[s]; }
     }
@@ -819,7 +828,8 @@ __global__ void route_topk_kernel(const RouteParams p) {
       const float os = __shfl_xor_sync(0xffffffffu, bs, o);
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; bs = os; }
     }
-    if ((bi & 31) == lane) sel[bi >> 5] = -INFINITY;   // remove from further rounds
+#pragma unroll
+    for (int s = 0; s < PER; ++s) sel[s] = bi == lane + 32 * s ? -INFINITY : sel[s];   // remove from further rounds
     wsum += bs;
     if (lane == k) { my_w = bs; my_i = bi; }
   }
@@ -1016,7 +1026,13 @@ extern "C" int fb_route_topk(const float* logits, const float* bias, int* out_id
   if (ld < E || topk > E || E > 512 || topk > 32 || n_group > 32 || (n_group > 1 && E % n_group != 0)) return -1;
   RouteParams p{logits, bias, out_idx, out_w, M, E, topk, score_mode, renorm, n_group, topk_group, route_scale, ld, group_max};
   const int wpb = 4;
-  launch_k(route_topk_kernel, dim3((M + wpb - 1) / wpb), dim3(wpb * 32), 0, reinterpret_cast<cudaStream_t>(stream), 0, p);
+  const dim3 grid((M + wpb - 1) / wpb), block(wpb * 32);
+  auto st = reinterpret_cast<cudaStream_t>(stream);
+  if (E <= 32) launch_k(route_topk_kernel<1>, grid, block, 0, st, 0, p);
+  else if (E <= 64) launch_k(route_topk_kernel<2>, grid, block, 0, st, 0, p);
+  else if (E <= 128) launch_k(route_topk_kernel<4>, grid, block, 0, st, 0, p);
+  else if (E <= 256) launch_k(route_topk_kernel<8>, grid, block, 0, st, 0, p);
+  else launch_k(route_topk_kernel<16>, grid, block, 0, st, 0, p);
   return (int)cudaGetLastError();
 }
 

@@ -110,3 +110,21 @@ def test_combine_with_gated_rows(T, H, topk, ld, dtype):
         # topk + 1 sums in fp32 and a fast sigmoid (2^-20), then one rounding
         tol = ref.abs() * torch.finfo(dtype).eps / 2 + size * ((topk + 1) * 2.0 ** -23 + 2.0 ** -20) + 2.0 ** -25
         assert bool(((out.double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("mode,bias,groups", [(0, False, (1, 1)), (1, True, (1, 1)), (1, True, (4, 2)), (2, False, (1, 1))])
+@pytest.mark.parametrize("E", [1, 31, 32, 33, 64, 65, 128, 129, 256, 257, 511, 512])
+def test_route_at_every_width(E, mode, bias, groups):
+    from fastllm_b200.ops import moe as MOE
+
+    n_group, keep = groups if E % 4 == 0 else (1, 1)
+    g = torch.Generator(device=DEV).manual_seed(E)
+    wide = torch.randn(67, E + 3, device=DEV, generator=g)
+    b = 0.1 * torch.randn(E, device=DEV, generator=g) if bias else None
+    topk = min(10, E // n_group * keep)
+    for logits in (wide[:, :E].contiguous(), wide[:, 3:]):
+        idx, w = MOE.route_topk(logits, b, topk, mode, mode != 2, n_group, keep, 2.5)
+        ri, rw = MOE.route_topk_ref(logits.double(), b.double() if bias else None, topk, mode, mode != 2, n_group, keep, 2.5)
+        # picked in order of their scores; a score is an fp32 exponential (2^-20) over a sum, the weights are renormalised: no near-tie at this seed
+        assert torch.equal(idx.long(), ri.long())
+        torch.testing.assert_close(w.double(), rw.double(), rtol=2.0 ** -18, atol=1e-7)
