@@ -193,6 +193,17 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         *reinterpret_cast<uint4*>(prow + AX_PT + ((g ^ (r & 7)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
       }
       l_run = fmaf(l_run, alpha, l_add);
+      if (n == n_steps - 1 && pos0 + rows < kv0 + AX_KV) {
+        // keys behind the block's last row have no weight, but what stands there may be no number: their values count as zeros.  (The
+        // product of step n - 2, which had this buffer before, was issued ahead of this step's scores: the wait is for this step's values.)
+        mbar_wait(&full_v[n & 1], (uint32_t)(n >> 1) & 1u, dead, KID_ATTN_WIDE, 10);
+        if ((r & 63) >= pos0 + rows - kv0) {
+          uint4* vrow = reinterpret_cast<uint4*>(v_smem + (n & 1) * vt * AX_KT + (r & 63) * 128);
+          for (int j = r >> 6; j < vt; j += 2)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) vrow[j * (AX_KT / 16) + e] = make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(p_ready);

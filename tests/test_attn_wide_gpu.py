@@ -78,3 +78,22 @@ def test_large_scores_and_empty_rows():
     ln[1] = 0
     out = A.attn_decode(q[:2].contiguous(), kp, vp, pt, ln, D ** -0.5, Hq, Hkv, D)
     assert torch.isfinite(out).all() and (out[1] == 0).all()
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 2), (72, 3, 3), (256, 20, 1)])
+@pytest.mark.parametrize("lens,news", [([1, 63, 64, 130, 700], [1, 63, 40, 130, 300])])
+def test_values_behind_a_request_stay_out(lens, news, D, Hq, Hkv, value):
+    """A page's slots behind its request's end hold whatever an earlier owner left there (``news`` None: decoded tokens)."""
+    scale = D ** -0.5
+    q, gate, kp, vp, pt, ln, cu = _setup(torch.float16, D, Hq, Hkv, lens, news or [1] * len(lens), D + 2)
+
+    def run():
+        return (A.attn_prefill(q, kp, vp, pt, ln, cu, scale, Hq, Hkv, D, gate=gate) if news else A.attn_decode(q, kp, vp, pt, ln, scale, Hq, Hkv, D, gate=gate))
+
+    want = run()
+    assert torch.isfinite(want).all()
+    for b, n in enumerate(lens):
+        last = pt[b, (n - 1) // PAGE]
+        kp[last, (n - 1) % PAGE + 1:], vp[last, (n - 1) % PAGE + 1:] = value, value
+    assert torch.equal(run(), want)
