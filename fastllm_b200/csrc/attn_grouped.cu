@@ -12,7 +12,7 @@
 // denominator and applies o * sigmoid(gate).  Sigmoid weights need no maximum and no denominator: partials are added up.  Kept first tokens are pages of their own in the work list, before the window's.
 //
 // Every row is its own request (its own page-table row and length), so decoded tokens and short portions of prompts share a launch.
-// Page pools must hold finite values everywhere: unused keys of a page are multiplied by P = 0.
+// Values behind a request's end are cleared in shared memory before the product (P = 0 alone would pass NaN and infinity on).
 #include "ptx.cuh"
 #include "launch.h"
 #include "tmap.h"
@@ -277,6 +277,16 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           }
           if (h < GP || it == 0) *reinterpret_cast<uint16_t*>(pb + (h >> 3) * 128 + (h & 7) * 16) = bits;      // unused rows: zeroed once
           if (TERMS == 2 && h >= GP && it == 0) *reinterpret_cast<uint16_t*>(pb + AG_P_BYTES + (h >> 3) * 128 + (h & 7) * 16) = 0;
+        }
+      }
+      if ((pg + 1) * AG_PAGE > n) {
+        // slots behind the request's end have no weight, but what an earlier owner left there may be no number: their values count as zeros
+        mbar_wait(full_v, ph, dead, KID_ATTN_GROUPED, 9);
+        if (key >= n) {
+          uint4* vrow = reinterpret_cast<uint4*>(v_smem + t * 128);
+          for (int j = 0; j < vt; ++j)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) vrow[j * (AG_TILE / 16) + e] = make_uint4(0u, 0u, 0u, 0u);
         }
       }
       fence_proxy_async_smem();

@@ -82,7 +82,7 @@ def test_large_scores_and_empty_rows():
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 2), (72, 3, 3), (256, 20, 1)])
-@pytest.mark.parametrize("lens,news", [([1, 63, 64, 130, 700], [1, 63, 40, 130, 300])])
+@pytest.mark.parametrize("lens,news", [([1, 63, 64, 130, 700], [1, 63, 40, 130, 300]), ([1, 63, 128, 130, 700], None)])
 def test_values_behind_a_request_stay_out(lens, news, D, Hq, Hkv, value):
     """A page's slots behind its request's end hold whatever an earlier owner left there (``news`` None: decoded tokens)."""
     scale = D ** -0.5
