@@ -89,7 +89,8 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* s_full = bars + 13;       // [2]
   uint64_t* p_ready = bars + 15;      // [2]
   uint64_t* o_full = bars + 17;       // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* v_clean = bars + 19;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x, kv_head = head / p.group;
@@ -116,11 +117,15 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
   auto takes = [&](int b, int it) { return (EXT && it < kb[b]) || (it >= f[b] && it < e[b]); };
   auto order = [&](int b, int it) { return EXT ? (it < kb[b] ? it : kb[b] + it - f[b]) : it - f[b]; };
+  // Keys of the last step behind the last row have no weight, but what stands there (the next request's first keys, or what a page's earlier
+  // owner left) may be no number: the loading warp clears their values in shared memory before the product
+  const int last_keys = hi - step_key(n_steps - 1);
   bool dead = false;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { mbar_init(&full_k[s], 1); mbar_init(&full_v[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(q_full, 1);
+    mbar_init(v_clean, 1);
     for (int b = 0; b < 2; ++b) { mbar_init(&s_full[b], 1); mbar_init(&p_ready[b], 128); mbar_init(&o_full[b], 1); }
     mbar_init_fence();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
@@ -161,6 +166,16 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
     __syncwarp();
+    if (last_keys < AW_KV) {
+      const int s = (n_steps - 1) % stages;
+      mbar_wait(&full_v[s], (uint32_t)((n_steps - 1) / stages) & 1u, dead, KID_ATTN_WINDOW, 11);
+      uint4* v = reinterpret_cast<uint4*>(kv_smem + s * stage_bytes + dt * AW_KT);
+      for (int i = last_keys * 8 + lane; i < AW_KV * 8; i += 32)
+        for (int j = 0; j < vt; ++j) v[j * (AW_KT / 16) + i] = make_uint4(0u, 0u, 0u, 0u);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(v_clean);
+    }
   } else if (warp == 1) {
     if (elect_one()) {
       const uint32_t qb = smem_u32(q_smem), pb = smem_u32(p_smem);
@@ -190,6 +205,7 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           if (takes(b, it)) {
             if (!mbar_wait(&p_ready[b], (uint32_t)order(b, it) & 1u, dead, KID_ATTN_WINDOW, 4)) { ok = false; break; }
             if (!have_v && !mbar_wait(&full_v[s], ph, dead, KID_ATTN_WINDOW, 5)) { ok = false; break; }
+            if (!have_v && it == n_steps - 1 && last_keys < AW_KV && !mbar_wait(v_clean, 0, dead, KID_ATTN_WINDOW, 12)) { ok = false; break; }
             have_v = true;
             tc_fence_after_sync();
             // O_b += P_b * V : A = P_b (K-major, 64 keys), B = V step MN-major (16 keys per MMA)

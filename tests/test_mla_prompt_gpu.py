@@ -57,3 +57,33 @@ def test_mla_prompt(dtype, mode, H, lens, news):
     rel = lambda x: ((x.double() - want).norm() / want.norm()).item()
     # both ways round four times to 16 bits between the projections
     assert rel(got) <= 1.05 * rel(old), (rel(got), rel(old))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_neighbours_stay_out(value):
+    """Requests are expanded side by side: the first keys of one must not reach the rows of the one before."""
+    H, nope, rope, lora, vd, dtype = 5, 128, 64, 512, 128, torch.float16
+    lens, g = [700, 300, 250], torch.Generator(device="cuda").manual_seed(1)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    T, counts = sum(lens), [(n + PAGE - 1) // PAGE for n in lens]
+    table = torch.zeros(len(lens), max(counts), dtype=torch.int32, device="cuda")
+    for b, c in enumerate(counts):
+        table[b, :c] = torch.arange(sum(counts[:b]), sum(counts[:b]) + c)
+    pool = rnd(sum(counts), PAGE, 1, lora + rope).to(dtype)
+    w_uk, w_uv = ((lora ** -0.5 * rnd(H, n, lora)).to(dtype) for n in (nope, vd))
+    q = rnd(T, H * (nope + rope)).to(dtype)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    pos = [j for n in lens for j in range(n)]
+    tables = A.build_rope_tables(rope, 1024, 1e4, None, "cuda")
+    la = LA.from_absorbed(H, nope, rope, lora, vd, w_uk, w_uk.transpose(1, 2).contiguous(), w_uv, (nope + rope) ** -0.5, True)
+
+    def run():
+        fb = ForwardBatch(ids=i32([0] * T), positions=i32(pos), slots=i32([-1] * T), page_table=table, kv_lens=i32(lens), cu_q=i32(cu), cu_q_host=cu, kv_lens_host=lens)
+        qc = q.clone()
+        return LA.attention(la, qc, pool, fb, qc, None, tables)
+
+    want = run()
+    pool[counts[0]] = value
+    got = run()
+    assert torch.equal(got[:cu[1]], want[:cu[1]]) and torch.equal(got[cu[2]:], want[cu[2]:])
