@@ -118,7 +118,8 @@ __device__ __forceinline__ bool ag_item(const AttnGroupedParams& p, int w, int& 
 }
 
 // TERMS 2: probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder), for models whose decode kept
-// them in fp32; the product is made twice, which the page stream hides.
+// them in fp32; the product is made twice, which the page stream hides.  fp16 terms are scaled by 2^15, which the sum shares: what they leave out is
+// 2^-40 of the page's largest weight (unscaled, weights below 2^-14 were losing digits of the first term, and the second was gone).
 template <bool BF16, int GP, int MODE, int TERMS>
 __global__ void __launch_bounds__(192, 3)
 attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -261,7 +262,7 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           uint16_t bits = 0;
           if (h < GP) {
             const float mx = fmaxf(fmaxf(red_max[h], red_max[16 + h]), fmaxf(red_max[32 + h], red_max[48 + h]));
-            const float pv = (h < nh && valid) ? exp2f(sv[h < GP ? h : 0] - mx) : 0.f;
+            const float pv = (h < nh && valid) ? exp2f(sv[h < GP ? h : 0] - mx + (TERMS == 2 && !BF16 ? 15.f : 0.f)) : 0.f;
             bits = BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(pv)) : __half_as_ushort(__float2half_rn(pv));
             // the sum of what the tensor core will see
             float pr = BF16 ? __bfloat162float(__ushort_as_bfloat16(bits)) : __half2float(__ushort_as_half(bits));

@@ -5,9 +5,9 @@
 // Two score buffers: the tensor core makes the scores of step i + 1 while the softmax warps, a thread a query row, work on step i.  Keys and
 // values have rings of their own (two steps each; a key step is free as soon as its scores exist).  At 256 x 256 the queries take 64 KB,
 // the rings 128 KB, P 32 KB, and O 256 of the 512 TMEM columns, so that one CTA fills an SM; K and V of a group's heads meet in the L2.
-// Probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder): they keep 16 bits and more, as the
-// evaluation in fp32 that this kernel replaces kept them beyond what the 16-bit result shows.  O is rescaled only when a row's maximum has
-// grown by more than 2^8, which changes no rounding of P and keeps fp16 terms finite.
+// Probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder): 16 bits of them in bf16.  In fp16 the terms are
+// scaled by 2^13, which the sum shares, so that what they leave out is 2^-38 of the largest weight.  O is rescaled only when a row's maximum has grown
+// by more than 2^8 (fp16: 2^2), which changes no rounding of P and keeps fp16 terms finite (up to 2^15).
 // Bound: the softmax thread's 64 exponentials and term splits of a step (about 1200 cycles) above the products' 768.
 // 4001 tokens x 16 heads x 256: 252 us (PyTorch, gathered fp32 keys and values and fp32 scores in memory: 7.0 ms).
 #include "ptx.cuh"
@@ -157,8 +157,8 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // (the first key is in step 0: from there on the maximum is finite)
       float alpha = 1.f;
-      if ((m_new - m_run) * p.scale_log2 > 8.f) { alpha = exp2f((m_run - m_new) * p.scale_log2); m_run = m_new; }
-      const float m_use = m_run * p.scale_log2;
+      if ((m_new - m_run) * p.scale_log2 > (BF16 ? 8.f : 2.f)) { alpha = exp2f((m_run - m_new) * p.scale_log2); m_run = m_new; }
+      const float m_use = m_run * p.scale_log2 - (BF16 ? 0.f : 13.f);
       if (n > 0) {
         mbar_wait(o_full, (uint32_t)(n - 1) & 1u, dead, KID_ATTN_WIDE, 8);      // P may be overwritten, O rescaled
         __syncwarp();

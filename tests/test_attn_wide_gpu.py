@@ -97,3 +97,28 @@ def test_values_behind_a_request_stay_out(lens, news, D, Hq, Hkv, value):
         last = pt[b, (n - 1) // PAGE]
         kp[last, (n - 1) % PAGE + 1:], vp[last, (n - 1) % PAGE + 1:] = value, value
     assert torch.equal(run(), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("D", [64, 256])
+def test_small_weights_keep_their_digits(D, dtype):
+    """One key takes nearly all of the weight and has no value: what comes out is the 2^-20 of the weight that another one gets."""
+    T, L = 150, 200
+    q = torch.zeros(T, D, device="cuda")
+    q[:, 0] = torch.linspace(1.0, 1.1, T, device="cuda")
+    k, v = torch.zeros(2, PAGE, 1, D, device="cuda"), torch.randn(2, PAGE, 1, D, device="cuda")
+    k[..., 0] = -300.0
+    k[0, 0, 0, 0], k[0, 1, 0, 0] = 0.0, -13.0
+    v[0, 0], v[0, 1] = 0.0, 1000.0
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    i32 = lambda t: torch.tensor(t, dtype=torch.int32, device="cuda")
+    p = torch.exp(q[:, 0].double() * k[0, 1, 0, 0].double())
+    want = (p / (1 + p) * v[0, 1, 0, 0].double())[:, None].expand(T, D)
+    # One rounding to 16 bits.  The weight in two terms: 2^-17 of it in bf16; in fp16 what the scaled second term leaves, 2^-38 of the largest
+    # weight and 2^-17.3 of this one (above 2^-20.7).  Its exponent has three roundings to fp32 (the scale, the product, the difference):
+    # 21 ln 2 * 3 * 2^-24 < 2^-18.4; exponential, sum and quotient add less than 2^-21.
+    bound = torch.finfo(dtype).eps / 2 + 2.0 ** -16
+    got = A.attn_prefill(q, k, v, i32([[0, 1]]), i32([L]), i32([0, T]), 1.0, 1, 1, D)
+    assert ((got.double() - want).abs() <= bound * want).all()
+    got = A.attn_decode(q, k, v, i32([[0, 1]] * T), i32([L] * T), 1.0, 1, 1, D)
+    assert ((got.double() - want).abs() <= bound * want).all()
