@@ -382,8 +382,22 @@ def wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim) -> bool:
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
 
 
+def _wide_operands_ok(q, k_pool, v_pool, lists, page_table, out, gate) -> bool:
+    """What the kernels of ``wide_ok`` take as it is, beside the queries: pages like the queries' heads, 32-bit lists on the device (``lists``:
+    lengths and offsets) and rows of 16 bytes; other operands run the PyTorch evaluation."""
+    rows = lambda t: t is None or (t.shape == q.shape and t.dtype == q.dtype and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0)
+    return bool(q.dim() == 2 and v_pool.shape == k_pool.shape and v_pool.dtype == k_pool.dtype and rows(out) and rows(gate)
+                and all(p.is_contiguous() and p.data_ptr() % 16 == 0 and p.device == q.device for p in (k_pool, v_pool))
+                and all(t.dtype == torch.int32 and t.device == q.device and t.is_contiguous() for t in lists)
+                and page_table.dtype == torch.int32 and page_table.device == q.device and page_table.stride(1) == 1)
+
+
 def _gate_args(gate):
     return _ptr(gate), gate.stride(0) if gate is not None else 0
+
+
+def _gated(o, gate):
+    return o if gate is None else (o.float() * torch.sigmoid(gate.float())).to(o.dtype)
 
 
 KV8_KERNEL = True          # e4m3 page pools run the decode kernel's KV8 mode (tests switch it off to compare with the PyTorch path)
@@ -397,7 +411,7 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
                 window: int = 0, softcap: float = 0.0, sinks=None, q8_ready: bool = False, gate=None):
     """One new token per request. q: ``[B, Hq*D]`` -> ``[B, Hq*D]``.
 
-    ``gate`` (head widths of ``wide_ok`` only): 16-bit logits ``[B, Hq*D]``, contiguous rows; the output is multiplied by their sigmoid.
+    ``gate``: 16-bit logits ``[B, Hq*D]``; the output is multiplied by their sigmoid (in the kernel at head widths of ``wide_ok``).
 
     ``window`` > 0: sliding-window attention; ``softcap`` > 0: tanh soft-capping of the logits; ``sinks``: fp32 ``[Hq]`` per-head
     sink logits in the softmax denominator.  All three run inside the same kernels.
@@ -406,6 +420,11 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
     k block of the output projection -- and the result carries it as ``out.fb_quant`` (see ``ops.basic.rmsnorm``)."""
     B = q.shape[0]
     variant = bool(window or softcap or sinks is not None)
+    wide = (not variant and B <= 1024 and wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim)
+            and _wide_operands_ok(q, k_pool, v_pool, (seq_lens,), page_table, out, gate))
+    if gate is not None and not wide:
+        return _gated(attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num_kv_heads, head_dim, ws, out, planned, grid_ctas, 0, window,
+                                  softcap, sinks, q8_ready), gate)
     if not q.is_cuda:
         cu = torch.arange(B + 1, dtype=torch.int32)
         if variant:
@@ -417,12 +436,11 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
     G = num_q_heads // num_kv_heads
     kv8 = (k_pool.dtype == torch.float8_e4m3fn and v_pool.dtype == torch.float8_e4m3fn and KV8_KERNEL
            and q.dtype in (torch.float16, torch.bfloat16))
-    if not variant and wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim):
+    if wide:
         P_ = page_table.shape[1]
-        if ws is None or ws.part_o.numel() < B * num_q_heads * ws.max_pages * head_dim:
+        if (ws is None or B > ws.max_batch or P_ > ws.max_pages or ws.part_o.numel() < B * num_q_heads * ws.max_pages * head_dim
+                or ws.part_ml.numel() < B * num_q_heads * ws.max_pages * 2):
             ws, planned = DecodeWorkspace(B, num_kv_heads, G, P_, q.device, head_dim), False
-        if B > ws.max_batch or P_ > ws.max_pages:
-            raise ValueError("decode workspace too small for this batch / page table")
         if not planned:
             ws.plan(seq_lens)
         out = torch.empty_like(q) if out is None else out
@@ -529,6 +547,9 @@ def attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_head
                  cu_q_host=None, gate=None, plans: dict | None = None):
     """Packed causal prefill (also chunked prefill / prefix-cache continuation). q: ``[T, Hq*D]``; ``gate`` as in ``attn_decode``;
     ``plans``: a dict that lives as long as the batch does, for what the layers of a pass share."""
+    wide = wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim) and _wide_operands_ok(q, k_pool, v_pool, (kv_lens, cu_q), page_table, out, gate)
+    if gate is not None and not wide:
+        return _gated(attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim, out, cu_q_host, plans=plans), gate)
     if cpu_native(q) and k_pool.dtype == torch.float32:
         return cpu.attention_paged(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim)
     if (q.is_cuda and k_pool.dtype == torch.float8_e4m3fn and head_dim == 128 and k_pool.shape[1] == PAGE_LEN
@@ -545,7 +566,7 @@ def attn_prefill(q, k_pool, v_pool, page_table, kv_lens, cu_q, scale, num_q_head
         kt = k_pool.index_select(0, used).to(q.dtype)
         vt = v_pool.index_select(0, used).to(q.dtype)
         return attn_prefill(q, kt, vt, pt, kv_lens, cu_q, scale, num_q_heads, num_kv_heads, head_dim, out, cu_q_host, plans=plans)
-    if wide_ok(q, k_pool, num_q_heads, num_kv_heads, head_dim):
+    if wide:
         blk, n_blocks = _query_blocks(cu_q, cu_q_host, q.device, plans)
         out = torch.empty_like(q) if out is None else out
         if not n_blocks:

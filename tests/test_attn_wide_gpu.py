@@ -122,3 +122,38 @@ def test_small_weights_keep_their_digits(D, dtype):
     assert ((got.double() - want).abs() <= bound * want).all()
     got = A.attn_decode(q, k, v, i32([[0, 1]] * T), i32([L] * T), 1.0, 1, 1, D)
     assert ((got.double() - want).abs() <= bound * want).all()
+
+
+@pytest.mark.parametrize("form", ["int64 lists", "lists on the host", "pools with gaps", "values of another type"])
+def test_other_operands_take_the_general_evaluation(form):
+    """What the kernels cannot read as it is gives what it gave before there were kernels."""
+    D, Hq, Hkv, scale = 64, 4, 2, 0.125
+    q, gate, kp, vp, pt, ln, cu = _setup(torch.bfloat16, D, Hq, Hkv, [300, 5, 129], [40, 5, 129], 11)
+    assert A.wide_ok(q, kp, Hq, Hkv, D)
+    ref = lambda q, cu: A.paged_attention_ref(q, kp, vp, pt, ln.cpu(), cu.cpu(), scale, Hq, Hkv, D)
+    want, one = ref(q, cu), ref(q[:3], torch.arange(4))
+    k, v, t, n, c = kp, vp, pt, ln, cu
+    if form == "int64 lists":
+        t, n, c = pt.long(), ln.long(), cu.long()
+    elif form == "lists on the host":
+        n, c = ln.cpu(), cu.cpu()
+    elif form == "pools with gaps":
+        k, v = (torch.stack([x, x], dim=1)[:, 0] for x in (kp, vp))
+    else:
+        v = vp.float()
+    assert torch.equal(A.attn_prefill(q, k, v, t, n, c, scale, Hq, Hkv, D), want)
+    assert torch.equal(A.attn_decode(q[:3], k, v, t, n, scale, Hq, Hkv, D), one)
+    assert torch.equal(A.attn_prefill(q, k, v, t, n, c, scale, Hq, Hkv, D, gate=gate), (want.float() * torch.sigmoid(gate.float())).to(q.dtype))
+    assert torch.equal(A.attn_decode(q[:3], k, v, t, n, scale, Hq, Hkv, D, gate=gate[:3]), (one.float() * torch.sigmoid(gate[:3].float())).to(q.dtype))
+
+
+@pytest.mark.parametrize("n,made_for", [(3, (2, 8)), (3, (8, 1)), (1030, (8, 8))])
+def test_decode_beyond_a_workspace(n, made_for):
+    """More rows or pages than the workspace was made for, and more rows than a plan takes."""
+    D, Hq, Hkv, scale = 64, 4, 2, 0.125
+    lens = [300, 5, 129] + [1] * (n - 3)
+    q, _, kp, vp, pt, ln, cu = _setup(torch.bfloat16, D, Hq, Hkv, lens, [1] * n, n)
+    ws = A.DecodeWorkspace(made_for[0], Hkv, Hq // Hkv, made_for[1], q.device, D)
+    got = A.attn_decode(q, kp, vp, pt, ln, scale, Hq, Hkv, D, ws=ws)
+    want = _exact(q, None, kp, vp, pt, ln, cu, scale, Hq, Hkv, D)
+    assert rel(got, want) <= 1.05 * rel(A.paged_attention_ref(q, kp, vp, pt, ln.cpu(), cu.cpu(), scale, Hq, Hkv, D), want)
