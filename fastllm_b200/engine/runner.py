@@ -135,9 +135,9 @@ class ModelRunner:
             return False        # these paths evaluate attention with host-synchronising PyTorch ops
         if len({int(lw.attn.window) for lw in self.model.layers if lw.attn.window}) > 1 or (c.rope_local_theta and any(lw.attn.window for lw in self.model.layers)):
             return False        # several window lengths / a second RoPE base for local layers: PyTorch evaluation
-        if not c.use_mla and c.head_dim != 128 and not (c.head_dim % 8 == 0 and c.head_dim <= 256 and self.model.dtype in (torch.float16, torch.bfloat16)
+        if not c.use_mla and c.head_dim != 128 and not (c.head_dim % 8 == 0 and c.head_dim <= 256 and self.cfg.max_batch <= 1024 and self.model.dtype in (torch.float16, torch.bfloat16)
                                                         and not c.attn_softcap and not any(lw.attn.window or lw.attn.sinks is not None for lw in self.model.layers)):
-            return False        # head widths other than 128: plain causal attention only; the rest runs the PyTorch evaluation
+            return False        # head widths other than 128: plain causal attention of up to 1024 rows; the rest runs the PyTorch evaluation
         if c.has_linear_attn and not (c.lin_kind == "gdn" and c.lin_k_dim == 128 and c.lin_v_dim == 128
                                       and self.model.dtype in (torch.float16, torch.bfloat16)):
             return False        # delta-rule state shapes outside the recurrent kernel run the PyTorch evaluation
