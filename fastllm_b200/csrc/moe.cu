@@ -261,6 +261,7 @@ struct MoeStreamInfo {
 };
 
 constexpr int MS_MAX_EXPERTS = 1024;
+constexpr int MS_EXTRA_FLAGS = GEMM_EXTRA_FLAGS | GEMM_BIAS | GEMM_RELU2;       // done by the EXTRA kernels alone
 // Tiles laid out for this many rows or more are done by CTA pairs: 128 experts, 4095 x 8 rows 238 + 133 -> 206 + 120 us; with tiles of 128 rows
 // (512 experts, 4001 x 10 rows) pairs take 378 + 233 us, one CTA a tile 380 + 212.
 constexpr int MS_PAIR_FROM = 256;
@@ -486,21 +487,34 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
 #pragma unroll
           for (int j = 0; j < HALF; ++j) o[j] = xb[(first_tok + j) * 64];
           const bool clamp = (p.flags & GEMM_GLU_CLAMP) != 0;
+          const int n = m.n_tile * 64 + col;
+          float bg = 0.f, bu = 0.f;
+          if (EXTRA && (p.flags & GEMM_BIAS) && n < (p.N >> 1)) {
+            const uint16_t* b = reinterpret_cast<const uint16_t*>(p.bias) + (size_t)m.e * p.N + m.n_tile * 128 + col;
+            bg = unpack_16<BF16>(b[0]).x;
+            bu = unpack_16<BF16>(b[64]).x;
+          }
 #pragma unroll
           for (int j = 0; j < HALF; ++j) {
-            const float g = q < 2 ? v[j] : o[j], up = q < 2 ? o[j] : v[j];
-            v[j] = clamp ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : silu_f(g) * up;
+            const float g = (q < 2 ? v[j] : o[j]) + bg, up = (q < 2 ? o[j] : v[j]) + bu;
+            v[j] = clamp ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : EXTRA && (p.flags & GEMM_GEGLU) ? gelu_tanh_f(g) * up : silu_f(g) * up;
+            if (EXTRA && (p.flags & GEMM_RELU2)) v[j] = relu2_f(v[j]);
           }
-          const int n = m.n_tile * 64 + col;
           if (!dead && n < (p.N >> 1)) store_column<HALF, BF16>(orow + (size_t)(c0 + first_tok) * p.ld_out + n, p.ld_out, v, cnt - first_tok);
         } else {
           const int n = m.n_tile * 128 + n_local;
           float v[CH];
 #pragma unroll
           for (int j = 0; j < CH; ++j) v[j] = __uint_as_float(r[j]);
-          if (EXTRA && (p.flags & GEMM_GELU)) {
+          if (EXTRA) {
+            const float bias = (p.flags & GEMM_BIAS) && n < p.N ? unpack_16<BF16>(reinterpret_cast<const uint16_t*>(p.bias)[(size_t)m.e * p.N + n]).x : 0.f;
 #pragma unroll
-            for (int j = 0; j < CH; ++j) v[j] = gelu_erf_f(v[j]);
+            for (int j = 0; j < CH; ++j) {
+              v[j] += bias;
+              if (p.flags & GEMM_RELU2) v[j] = relu2_f(v[j]);
+              if (p.flags & GEMM_GELU) v[j] = gelu_erf_f(v[j]);
+              if (p.flags & GEMM_GELU_TANH) v[j] = gelu_tanh_f(v[j]);
+            }
           }
           if (!dead && n < p.N) store_column<CH, BF16>(orow + (size_t)c0 * p.ld_out + n, p.ld_out, v, cnt);
         }
@@ -546,7 +560,7 @@ static cudaError_t launch_stream(const CUtensorMap& tmW, const CUtensorMap& tmX,
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   }
   cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, PAIR ? 1 : 0);
-  return cudaLaunchKernelEx(&cfg, (p.flags & GEMM_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
+  return cudaLaunchKernelEx(&cfg, (p.flags & MS_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
 }
 
 }  // namespace fb
@@ -607,8 +621,9 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
                                        int total_rows, float act_limit, float act_alpha, void* stream_);
 
 // Grouped Y_e = X_e W_e^T over the sorted buffer.  Xs: [rows_cap, K] sorted rows; W: stacked [E_local * N, K] with every
-// expert's rows padded to a multiple of 128; out: [rows_cap, N or N/2].
-// max_rows_per_expert bounds the chunk count (T for decode: every token could pick the same expert).
+// expert's rows padded to a multiple of 128; out: [rows_cap, N or N/2]; bias (with GEMM_BIAS): 16-bit [E_local, N], added before the activation.
+// max_rows_per_expert: low 16 bits the most rows an expert can get (T for decode: every token could pick the same one), above them the rows of a
+// typical busy expert, for which the tiles are laid out (0: the most).
 extern "C" int fb_moe_grouped_gemm(const void* Xs, const void* W, void* out, const void* bias, const int* counts, const int* offsets,
                                    int rows_cap, int E_local, int N, int K, int ld_out, int max_rows_per_expert, int dtype, int flags,
                                    int total_rows, void* stream_) {
@@ -622,15 +637,16 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
                                        int total_rows, float act_limit, float act_alpha, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (E_local <= 0 || rows_cap <= 0) return 0;
-  if (K % 8 != 0 || N % 8 != 0 || ((flags & GEMM_SWIGLU) && N % 128 != 0) || (dtype != 0 && dtype != 1) || bias != nullptr || E_local > MS_MAX_EXPERTS) return -1;
+  if (K % 8 != 0 || N % 8 != 0 || ((flags & GEMM_SWIGLU) && N % 128 != 0) || (dtype != 0 && dtype != 1) || E_local > MS_MAX_EXPERTS ||
+      ((flags & GEMM_BIAS) && bias == nullptr) || (flags & ~(MS_EXTRA_FLAGS | GEMM_SWIGLU | GEMM_GLU_CLAMP)))
+    return -1;
   const int n_tiles = (N + 127) / 128;
   const bool bf16 = dtype == 1;
-  // rows the tile is laid out for: low 16 bits of max_rows_per_expert = most rows an expert can get, the rest = rows of a typical busy expert (0: the most)
   const int hint = max_rows_per_expert >> 16, most = max_rows_per_expert & 0xFFFF, want = hint > 0 && hint < most ? hint : most;
   int mpad = 16;
   while (mpad < want && mpad < 256) mpad <<= 1;
   GemmParams p = {};
-  p.out = out; p.N = N; p.K = K; p.ld_out = ld_out; p.kb_total = (K + 63) / 64; p.flags = flags;
+  p.out = out; p.bias = bias; p.N = N; p.K = K; p.ld_out = ld_out; p.kb_total = (K + 63) / 64; p.flags = flags;
   p.act_limit = act_limit; p.act_alpha = act_alpha;
   const bool pair = mpad >= MS_PAIR_FROM;
   p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, pair ? 256 : 128, 0);

@@ -128,3 +128,53 @@ def test_route_at_every_width(E, mode, bias, groups):
         # picked in order of their scores; a score is an fp32 exponential (2^-20) over a sum, the weights are renormalised: no near-tie at this seed
         assert torch.equal(idx.long(), ri.long())
         torch.testing.assert_close(w.double(), rw.double(), rtol=2.0 ** -18, atol=1e-7)
+
+
+@pytest.mark.parametrize("counts,hint", [([33, 0, 31, 64, 65, 1], 20), ([257, 0, 300], 256)])
+@pytest.mark.parametrize("form", ["bias", "swiglu+bias", "clamp+bias", "geglu", "relu2", "gelu tanh+bias"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_grouped_gemm_epilogues(counts, hint, form, dtype):
+    """A bias per expert and the less common activations: what the entry took before the tiles went through one launch."""
+    E, N, K = len(counts), 384, 200
+    g = torch.Generator(device=DEV).manual_seed(sum(counts))
+    offsets, at = [], 0
+    for c in counts:
+        offsets.append(at)
+        at += (c + MG.PAD - 1) // MG.PAD * MG.PAD
+    x, bias = torch.randn(at + 128, K, device=DEV, generator=g).to(dtype), torch.randn(E, N, device=DEV, generator=g).to(dtype)
+    w = (torch.randn(E, N, K, device=DEV, generator=g) * 0.1).to(dtype)
+    half = form.split("+")[0] in ("swiglu", "clamp", "geglu")
+    mix = lambda t: torch.stack([B.interleave_gate_up(t[e, :N // 2], t[e, N // 2:]) for e in range(E)]).contiguous()
+    wk, bk = (mix(w), mix(bias[..., None])[..., 0].contiguous()) if half else (w, bias)
+    cols = N // 2 if half else N
+    out = torch.empty(at + 128, cols, device=DEV, dtype=dtype)
+    cd, od = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in (counts, offsets))
+    flags = {"bias": 0, "swiglu": B.GEMM_SWIGLU, "clamp": B.GEMM_SWIGLU | B.GEMM_GLU_CLAMP, "geglu": B.GEMM_SWIGLU | B.GEMM_GEGLU, "relu2": B.GEMM_RELU2,
+             "gelu tanh": B.GEMM_GELU_TANH}[form.split("+")[0]] | (B.GEMM_BIAS if "bias" in form else 0)
+    call = lambda b, f: _lib.kernels().fb_moe_grouped_gemm_act(x.data_ptr(), wk.data_ptr(), out.data_ptr(), b, cd.data_ptr(), od.data_ptr(), at + 128, E, N, K, cols,
+                                                               max(counts) | (hint << 16), 1 if dtype == torch.bfloat16 else 0, f, sum(counts), 2.0, 1.7, _stream())
+    assert call(bk.data_ptr(), flags) == 0
+    _lib.check_device_errors()
+    for e, (o, n) in enumerate(zip(offsets, counts)):
+        xs = x[o:o + n].double()
+        y = xs @ w[e].double().t()
+        err = K * 2.0 ** -23 * (xs.abs() @ w[e].double().abs().t())            # as above
+        if "bias" in form:
+            y, err = y + bias[e].double(), err + 2.0 ** -23 * (y.abs() + bias[e].double().abs())
+        if form == "relu2":
+            y, err = y.relu().square(), 2.0 * y.abs() * err + err * err
+        elif form.startswith("gelu"):
+            y, err = torch.nn.functional.gelu(y, approximate="tanh"), 1.13 * err
+        elif half:
+            a, b, ea, eb = y[:, :cols], y[:, cols:], err[:, :cols], err[:, cols:]
+            if form.startswith("clamp"):
+                a, b = a.clamp(max=2.0), b.clamp(-2.0, 2.0) + 1.0
+                y = a * torch.sigmoid(1.7 * a)
+            else:
+                y = torch.nn.functional.silu(a) if form.startswith("swiglu") else torch.nn.functional.gelu(a, approximate="tanh")
+            y, err = y * b, 1.13 * ea * b.abs() + y.abs() * eb
+        tol = err + y.abs() * (torch.finfo(dtype).eps / 2 + 2.0 ** -19) + 2.0 ** -22 + (2.0 ** -25 if dtype == torch.float16 else 0.0)
+        assert bool(((out[o:o + n].double() - y).abs() <= tol).all()), (e, ((out[o:o + n].double() - y).abs() / tol).max().item())
+    # a bias that the flags do not ask for is not looked at; a bias, residual or 32-bit result that the entry cannot give is refused
+    assert call(bk.data_ptr(), flags & ~B.GEMM_BIAS) == 0
+    assert call(None, flags | B.GEMM_BIAS) == -1 and call(None, B.GEMM_RESIDUAL) == -1 and call(None, B.GEMM_OUT_F32) == -1
