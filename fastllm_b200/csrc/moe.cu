@@ -563,6 +563,59 @@ static cudaError_t launch_stream(const CUtensorMap& tmW, const CUtensorMap& tmX,
   return cudaLaunchKernelEx(&cfg, (p.flags & MS_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
 }
 
+// The same for few tiles: a cluster splits a tile's k among its CTAs and adds the parts up through distributed shared memory, in rank order; a CTA
+// group per (expert, chunk, 128 weight rows).  With 32 tiles (one expert of 4096 outputs) the persistent launch leaves four fifths of the SMs idle.
+// One expert, 4096 x 14336: 52 -> 31 us at 1 to 32 rows, 70 -> 35 at 128; 4096 x 7168, gated: 31 -> 22.
+struct MoeSplitInfo {
+  const int* counts;       // [n_local] routed rows per expert
+  const int* offsets;      // [n_local] first row of the expert's segment in the sorted buffer
+  int n_local, rows_per_chunk, n_rows_w;      // experts, MPAD, weight rows per expert in the stacked matrix
+};
+
+template <int MPAD, bool BF16, class Epi>
+__global__ void __launch_bounds__(192, 1)
+moe_split_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const GemmParams base, const MoeSplitInfo gi) {
+  pdl_launch_dependents();
+  pdl_wait();                                        // counts and offsets come from the plan kernel
+  int e = 0, chunk = 0;
+  if (!moe_find_item(gi.counts, gi.n_local, gi.rows_per_chunk, (int)blockIdx.z, e, chunk)) return;      // uniform over the cluster
+  GemmParams p = base;
+  const int row0 = chunk * gi.rows_per_chunk, seg = gi.offsets[e] + row0;
+  p.M = min(gi.counts[e] - row0, gi.rows_per_chunk);
+  p.x_row0 = seg;
+  p.w_row0 = e * gi.n_rows_w;
+  p.out = reinterpret_cast<uint16_t*>(base.out) + (size_t)seg * base.ld_out;
+  if (base.bias != nullptr) p.bias = reinterpret_cast<const uint16_t*>(base.bias) + (size_t)e * base.N;
+  uint32_t tmem_base;
+  gemm_smallm_device<MPAD, BF16, 1, Epi>(tmW, tmX, p, tmem_base, KID_MOE_GROUPED, Epi());
+  if ((threadIdx.x >> 5) == 1) tmem_dealloc(tmem_base, SmallMCfg<MPAD, 1>::TMEM_COLS);
+}
+
+template <int MPAD, bool BF16>
+static cudaError_t launch_split(const CUtensorMap& tmW, const CUtensorMap& tmX, const GemmParams& p, const MoeSplitInfo& gi, int nsplit, int n_tiles, int chunks,
+                                cudaStream_t stream) {
+  using Cfg = SmallMCfg<MPAD, 1>;
+  auto plain = moe_split_kernel<MPAD, BF16, StoreEpilogue<BF16>>;
+  auto extra = moe_split_kernel<MPAD, BF16, ExtraEpilogue<BF16>>;
+  static DeviceOnce configured;
+  if (configured.need()) {
+    cudaError_t e = cudaFuncSetAttribute(plain, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(extra, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nsplit, n_tiles, chunks);
+  cfg.blockDim = dim3(192);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = nsplit;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = add_pdl_attr(attr, 1);
+  return cudaLaunchKernelEx(&cfg, (p.flags & GEMM_EXTRA_FLAGS) ? extra : plain, tmW, tmX, p, gi);
+}
+
 }  // namespace fb
 
 using namespace fb;
@@ -664,6 +717,28 @@ extern "C" int fb_moe_grouped_gemm_act(const void* Xs, const void* W, void* out,
   // no more CTAs than tiles can exist: every routed row touches an expert, every expert's last chunk may be short
   long long bound = (long long)E_local * ((most + mpad - 1) / mpad);
   if (total_rows > 0 && bound > (long long)total_rows) bound = total_rows;
+  // Few tiles: four or two CTAs a tile, where that many fit and k is long enough to pay for adding the parts up.  Both sides in us, one CTA a tile ->
+  // split: 4 ways, 2048 of k, 12 tiles 14.4 -> 13.3 (128 rows 19.5 -> 16.4); 1408 of k, 16 tiles, 128 rows 14.3 -> 18.4 stays whole; 2 ways, 7168 of k, 64
+  // tiles 31.7 -> 29.8 (128 rows 46 -> 33); 2048 of k, 56 tiles, 128 rows 18.5 -> 22.5 stays whole.
+  const long long most_tiles = bound * n_tiles;
+  const int nsplit = 4 * most_tiles <= sms && p.kb_total >= 32 ? 4 : 2 * most_tiles <= sms && p.kb_total >= 64 ? 2 : 1;
+  if (nsplit > 1 && mpad <= 128) {
+    p.kb_per_split = (p.kb_total + nsplit - 1) / nsplit;
+    p.idesc = make_idesc(bf16 ? 1 : 0, bf16 ? 1 : 0, 0, 0, 128, mpad);
+    p.scatter_rows = 1;
+    if (!make_tmap_2d(&tmX, Xs, rows_cap, K, K, mpad, 64, 2, 3)) return -2;
+    MoeSplitInfo si;
+    si.counts = counts; si.offsets = offsets; si.n_local = E_local; si.rows_per_chunk = mpad; si.n_rows_w = n_tiles * 128;
+#define FB_MS(MP) \
+  return (int)(bf16 ? launch_split<MP, true>(tmW, tmX, p, si, nsplit, n_tiles, (int)bound, stream) : launch_split<MP, false>(tmW, tmX, p, si, nsplit, n_tiles, (int)bound, stream));
+    switch (mpad) {
+      case 16: FB_MS(16)
+      case 32: FB_MS(32)
+      case 64: FB_MS(64)
+      default: FB_MS(128)
+    }
+#undef FB_MS
+  }
   const int units = pair ? sms / 2 : sms;
   const int grid = (int)(bound * gi.n_tiles < units ? bound * gi.n_tiles : units) * (pair ? 2 : 1);
 #define FB_MG(MP) \

@@ -178,3 +178,47 @@ def test_grouped_gemm_epilogues(counts, hint, form, dtype):
     # a bias that the flags do not ask for is not looked at; a bias, residual or 32-bit result that the entry cannot give is refused
     assert call(bk.data_ptr(), flags & ~B.GEMM_BIAS) == 0
     assert call(None, flags | B.GEMM_BIAS) == -1 and call(None, B.GEMM_RESIDUAL) == -1 and call(None, B.GEMM_OUT_F32) == -1
+
+
+@pytest.mark.parametrize("counts", [[1], [16], [40], [128], [0, 17, 0, 3], [5, 0]])
+@pytest.mark.parametrize("N,K,form", [(1536, 2048, "swiglu+bias"), (520, 4104, "plain"), (2048, 4160, "gelu"), (4096, 4096, "swiglu"), (4096, 14336, "plain")])
+def test_few_tiles_share_out_their_k(counts, N, K, form):
+    """Two and four CTAs a tile (k blocks that do not divide, a last tile of 8 rows, experts without rows) against 64 bits, and the same bits again."""
+    E, dtype = len(counts), torch.bfloat16
+    g = torch.Generator(device=DEV).manual_seed(N + sum(counts))
+    offsets, at = [], 0
+    for c in counts:
+        offsets.append(at)
+        at += (c + MG.PAD - 1) // MG.PAD * MG.PAD
+    x = torch.randn(at + 128, K, device=DEV, generator=g).to(dtype)
+    w = (torch.randn(E, (N + 127) // 128 * 128, K, device=DEV, generator=g) * K ** -0.5).to(dtype)
+    bias = torch.randn(E, N, device=DEV, generator=g).to(dtype)
+    half = form.startswith("swiglu")
+    cols = N // 2 if half else N
+    flags = {"plain": 0, "gelu": B.GEMM_GELU, "swiglu": B.GEMM_SWIGLU, "swiglu+bias": B.GEMM_SWIGLU | B.GEMM_BIAS}[form]
+    cd, od = (torch.tensor(t, dtype=torch.int32, device=DEV) for t in (counts, offsets))
+    outs = []
+    for _ in range(3):
+        out = torch.full((at + 128, cols), 7.0, device=DEV, dtype=dtype)
+        rc = _lib.kernels().fb_moe_grouped_gemm_act(x.data_ptr(), w.data_ptr(), out.data_ptr(), bias.data_ptr(), cd.data_ptr(), od.data_ptr(), at + 128, E, N, K, cols,
+                                                    max(counts), 1, flags, sum(counts), 0.0, 1.0, _stream())
+        assert rc == 0
+        outs.append(out)
+    _lib.check_device_errors()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    for e, (o, n) in enumerate(zip(offsets, counts)):
+        xs, wd = x[o:o + n].double(), w[e, :N].double()
+        y, err = xs @ wd.t(), K * 2.0 ** -23 * (xs.abs() @ wd.abs().t())
+        if form == "gelu":
+            y, err = torch.nn.functional.gelu(y), 1.13 * err
+        elif half:
+            if "bias" in form:
+                y, err = y + bias[e].double(), err + 2.0 ** -23 * (y.abs() + bias[e].double().abs())
+            t = torch.arange(cols, device=DEV)
+            gate = t // 64 * 128 + t % 64                                   # rows of a 128-row tile: 64 of the gate, 64 of the other factor
+            a, b, ea, eb = y[:, gate], y[:, gate + 64], err[:, gate], err[:, gate + 64]
+            y = torch.nn.functional.silu(a)
+            y, err = y * b, 1.1 * ea * b.abs() + y.abs() * eb
+        tol = err + y.abs() * (torch.finfo(dtype).eps / 2 + 2.0 ** -20) + 2.0 ** -22
+        assert bool(((outs[0][o:o + n].double() - y).abs() <= tol).all()), (e, n)
+        assert bool((outs[0][o + n:offsets[e + 1] if e + 1 < E else None] == 7.0).all())
