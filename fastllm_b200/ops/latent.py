@@ -2,12 +2,14 @@
 key part that all heads share is cached behind the latent (``[latent | 0 | rotated part]``); the queries may come through a latent of
 their own, and the output gate is one per element or one per head.
 
-Two evaluations of the same mixer, chosen per request of a batch:
+Evaluations of the same mixer, chosen per request of a batch:
 
 * *absorbed* (decoded tokens, short portions): queries are multiplied into the latent space, every row attends to the cached
   latents themselves (``csrc/attn_mla.cu``), the result is multiplied by the value projection with the output gate in its epilogue;
 * *expanded* (prompt chunks): the latents the chunk's queries see are gathered once, one GEMM expands them to keys and values, and
-  the windowed prefill kernel (``csrc/attn_window.cu``) runs on plain heads, output gate in its epilogue.
+  the windowed prefill kernel (``csrc/attn_window.cu``) runs on plain heads, output gate in its epilogue;
+* *folded* (layers of ``from_absorbed``: some tens of rows behind a long history): absorbed queries of all heads as the rows of two
+  GEMMs over the latents, with the softmax between them in memory.
 
 Other element types or widths (float32; latents beyond the decode kernel) run every row through ``csrc/full32.cu``.  CPU tensors
 evaluate the PyTorch definition.
@@ -15,6 +17,7 @@ evaluate the PyTorch definition.
 from __future__ import annotations
 
 import ctypes
+import math
 
 import numpy as np
 import torch
@@ -33,7 +36,7 @@ _lib.register_sigs({
 }, ["full32", "attn_window"])
 
 ABSORB_ROWS = 16                 # requests that bring at most this many tokens attend in the latent space
-EXPAND_BYTES = 2 << 30           # scratch keys and values of one expanded group of requests
+EXPAND_BYTES = 1 << 30           # scratch of one evaluation: gathered latents, keys and values of an expanded group of requests; scores of folded rows
 _MAX_MLA_ROWS = 1024             # requests per call of the latent decode kernel
 
 
@@ -68,6 +71,7 @@ class LatentWeights:
         self.w_uv = None         # [heads, vdim, lv]  latent space -> values
         self.gate = "elem"       # "elem": one per element, "head": one per head, "": none
         self.more_col = 0        # first of the further rows
+        self.by_cost = False     # the form of a prompt is chosen by ``prompt_form`` (else by ABSORB_ROWS)
 
     @property
     def hd(self) -> int:
@@ -158,7 +162,7 @@ def from_absorbed(heads: int, nope: int, rope: int, lora: int, vdim: int, w_uk, 
     w = LatentWeights()
     w.heads, w.dim, w.vdim, w.rank, w.lv, w.rot, w.rd = heads, nope, vdim, lora, lora, rope, rope
     w.ld, w.scale, w.neox, w.gate = lora + rope, float(scale), neox, ""
-    w.w_uk, w.w_uk_t, w.w_uv = w_uk.reshape(heads * nope, lora), w_uk_t, w_uv
+    w.w_uk, w.w_uk_t, w.w_uv, w.by_cost = w_uk.reshape(heads * nope, lora), w_uk_t, w_uv, True
     return w
 
 
@@ -189,6 +193,7 @@ class LatentPlan:
         self.n_rows = 0
         self.page_table = None       # [n_rows, P] and [n_rows]: every absorbed row is a request of its own
         self.kv_lens = None
+        self.folds: list[tuple] = []           # (first row, row behind the last, keys, slots of the keys and of a padding to whole 64s)
         self.groups: list[_Group] = []
 
 
@@ -199,36 +204,74 @@ def _row_plan(fb, reqs, cu, dev):
     return torch.from_numpy(owner).to(dev, non_blocking=True), torch.from_numpy(rows).to(dev, non_blocking=True)
 
 
-def build_plan(fb, window: int, page_len: int, expand: bool, key_bytes: int) -> LatentPlan:
+def _key_bytes(lw) -> int:
+    return 2 * (lw.heads * (lw.dim + lw.vdim) + lw.ld)
+
+
+def prompt_form(lw, n: int, keys: int, n_req: int = 1, sms: int = 148) -> str:
+    """Cheapest form for a request that brings ``n`` of ``keys`` tokens in a batch of ``n_req``: estimates in microseconds.
+
+    Absorbed rows read the latents once per row and 32 heads; expanding costs by the key and head, then by the step of the longest CTA
+    (a head and 256 rows) or of all CTAs over the SMs, and once more for every slice of heads that the scratch allows; folded rows
+    cost by the row, key and head, after passes over the latents and more launches.  Fitted to 233 measured calls (128 + 64 wide
+    keys, 512-wide latents, 16 to 128 heads, 8 to 1000 rows behind 0 to 100000 tokens, 1 to 16 requests): the choice takes at most 1.3 times
+    the best form's time, 1.2 times where that is above 130 us and beside the folded form alone (the only one before).  17 rows behind
+    32768 tokens, 16 heads: absorbed 239, expanded 1047, folded 333 us; 128 rows: 1121, 1075, 614; 1000 rows: 7749, 1370, 3030."""
+    H, wide = lw.heads, (lw.lv + lw.ld) / 1088
+    absorbed = 50 / n_req + n * keys * -(-H // 32) * (0.25 + 0.2 * min(H, 32) / 32) * 1e-3 * wide
+    fits = EXPAND_BYTES / (keys * _key_bytes(lw))                                       # requests of this length that are expanded at a time
+    chain = 1 / max(1.0, min(n_req, fits)) if fits >= 1 else -(-1 // fits)
+    steps = keys / 64 * (1.9 if n <= 128 else 2.6) * (lw.dim + lw.rd + lw.vdim) / 320
+    expanded = max(64 / n_req, 30 / n_req + keys * H * 0.26e-3 * lw.lv * (lw.dim + lw.vdim) / 131072 + steps * max(H * -(-n // 256) / sms, chain))
+    scores = n * keys * H * 5.3e-6 * wide * min(1.65, max(1.0, keys / 60000))            # (from there on the latents outgrow the L2)
+    folded = max(230.0, 90 + keys * 5e-3 + scores) if lw.ld % 64 == 0 and not lw.window else math.inf
+    return min((absorbed, "absorbed"), (expanded, "expanded"), (folded, "folded"))[1]
+
+
+def build_plan(fb, lw, page_len: int, expand: bool) -> LatentPlan:
     pl = LatentPlan()
     if fb.is_decode:
         pl.page_table, pl.kv_lens, pl.n_rows = fb.page_table, fb.kv_lens, fb.page_table.shape[0]
         return pl
-    dev = fb.page_table.device
+    dev, window, key_bytes = fb.page_table.device, lw.window, _key_bytes(lw)
     cu = fb.cu_q_host if fb.cu_q_host is not None else fb.cu_q.tolist()
     lens = fb.kv_lens_host if fb.kv_lens_host is not None else fb.kv_lens.tolist()
     reqs = [b for b in range(len(cu) - 1) if cu[b + 1] > cu[b]]
-    long = [b for b in reqs if expand and cu[b + 1] - cu[b] > ABSORB_ROWS]
-    short = [b for b in reqs if b not in set(long)]
+    if not expand:
+        form = dict.fromkeys(reqs, "absorbed")
+    elif lw.by_cost:
+        sms = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 148
+        form = {b: prompt_form(lw, cu[b + 1] - cu[b], lens[b], len(reqs), sms) for b in reqs}
+    else:
+        form = {b: "expanded" if cu[b + 1] - cu[b] > ABSORB_ROWS else "absorbed" for b in reqs}
+    short, long = ([b for b in reqs if form[b] == f] for f in ("absorbed", "expanded"))
     if short:
         owner, rows = _row_plan(fb, short, cu, dev)
         pl.n_rows = rows.shape[0]
         pl.page_table = fb.page_table.index_select(0, owner)
         seen = fb.positions + 1
-        pl.kv_lens = seen.to(torch.int32) if not long else seen.index_select(0, rows).to(torch.int32)
-        pl.rows = rows if long else None
+        pl.rows = rows if len(short) < len(reqs) else None
+        pl.kv_lens = (seen if pl.rows is None else seen.index_select(0, rows)).to(torch.int32)
+
+    def slots(spans):
+        """Cache slots of the keys [k, k + n) of requests b, for (b, k, n) in ``spans``."""
+        owner = np.concatenate([np.full(n, b, dtype=np.int64) for b, _, n in spans])
+        pos = np.concatenate([np.arange(k, k + n, dtype=np.int64) for _, k, n in spans])
+        meta = torch.from_numpy(np.stack([owner, pos])).to(dev, non_blocking=True)
+        pages = fb.page_table[meta[0], torch.div(meta[1], page_len, rounding_mode="floor")].long()
+        return pages * page_len + meta[1] % page_len
+
+    for b in reqs:
+        if form[b] == "folded":                        # whole 64s of keys: what lies behind the last one is cleared after the gather
+            pl.folds.append((cu[b], cu[b + 1], lens[b], torch.nn.functional.pad(slots([(b, 0, lens[b])]), (0, -lens[b] % 64))))
     group, base = [], 0
     pending: list = []
 
     def flush():
         if not pending:
             return
-        owner = np.concatenate([np.full(n, b, dtype=np.int64) for b, _, n in pending])
-        pos = np.concatenate([np.arange(k, k + n, dtype=np.int64) for _, k, n in pending])
-        meta = torch.from_numpy(np.stack([owner, pos])).to(dev, non_blocking=True)
-        pages = fb.page_table[meta[0], torch.div(meta[1], page_len, rounding_mode="floor")].long()
         blocks = sorted(group, key=lambda t: -(min(t[1] + t[2] - t[4], (window or 1 << 30) + t[2])))      # most keys first
-        pl.groups.append(_Group(pages * page_len + meta[1] % page_len, torch.tensor(blocks, dtype=torch.int32).to(dev, non_blocking=True), len(blocks)))
+        pl.groups.append(_Group(slots(pending), torch.tensor(blocks, dtype=torch.int32).to(dev, non_blocking=True), len(blocks)))
 
     for b in long:
         n, start = cu[b + 1] - cu[b], lens[b] - (cu[b + 1] - cu[b])
@@ -245,11 +288,10 @@ def build_plan(fb, window: int, page_len: int, expand: bool, key_bytes: int) -> 
 
 
 def _plan(fb, lw, page_len: int, expand: bool) -> LatentPlan:
-    key_bytes = lw.heads * (lw.dim + lw.vdim) * 2
-    key = (lw.window, expand, key_bytes)
+    key = (lw.window, expand, lw.by_cost, lw.heads, lw.dim, lw.vdim, lw.ld)
     cache = fb.__dict__.setdefault("_latent_plans", {})
     if key not in cache:
-        cache[key] = build_plan(fb, lw.window, page_len, expand, key_bytes)
+        cache[key] = build_plan(fb, lw, page_len, expand)
     return cache[key]
 
 
@@ -276,13 +318,20 @@ def post(lw, proj, fb, pool, rope, eps: float):
     return (lw.q_up(cq) if cq is not None else proj)[:, :lw.heads * lw.hd], gates
 
 
-def _absorbed(lw, q, gate, head_gate, pool, page_table, kv_lens, out, positions, rope):
-    """Rows ``q`` [n, heads * hd] (row stride free) against their own page-table rows; the gated values go to ``out`` [n, heads * vdim]."""
+def _latent_queries(lw, q, positions, rope):
+    """Queries [n, heads * hd] -> [n, heads, ld]: multiplied into the latent space, rotated parts turned."""
     n, H = q.shape[0], lw.heads
     q_lat = torch.empty((n, H, lw.ld), device=q.device, dtype=q.dtype)
     B.linear_batched(q, lw.w_uk_t, H, lw.hd, q_lat.view(n, H * lw.ld), lw.ld)
     if lw.rd:
         S.rope_heads(q[:, lw.dim:], lw.hd, q_lat.view(n, H * lw.ld)[:, lw.lv:], lw.ld, H, lw.rot, lw.rd, positions, *rope, lw.neox)
+    return q_lat
+
+
+def _absorbed(lw, q, gate, head_gate, pool, page_table, kv_lens, out, positions, rope):
+    """Rows ``q`` [n, heads * hd] (row stride free) against their own page-table rows; the gated values go to ``out`` [n, heads * vdim]."""
+    n, H = q.shape[0], lw.heads
+    q_lat = _latent_queries(lw, q, positions, rope)
     if decode_kernel_ok(lw, q.dtype, pool.shape[1]):
         part = lambda i, j: mla_decode(q_lat[i:j], pool, page_table[i:j], kv_lens[i:j], lw.scale, lora=lw.lv, window=lw.window,
                                        head_gate=head_gate[i:j] if head_gate is not None else None)
@@ -295,19 +344,48 @@ def _absorbed(lw, q, gate, head_gate, pool, page_table, kv_lens, out, positions,
     B.linear_batched(o_lat.view(n, H * lw.lv), lw.w_uv, H, lw.lv, out, lw.vdim, gate=gate)
 
 
-def expand(lw, rows):
-    """Latent rows [n, lv] -> (keys [n, >= heads * dim], values [n, >= heads * vdim])"""
+def _folded(lw, q, pool, keys: int, slots, out, positions, rope):
+    """Rows ``q`` [n, heads * hd] of one request that end at its last of ``keys`` tokens (an ungated layer, no window)."""
+    n, H, lib, dt = q.shape[0], lw.heads, _lib.kernels(), dtype_code(q.dtype)
+    rows = S.gather_rows(pool.view(-1, lw.ld), slots)
+    cols = rows.shape[0]
+    rows[keys:] = 0
+    values = rows[:, :lw.lv].t().contiguous()
+    step = max(1, EXPAND_BYTES // (6 * H * cols))
+    for i in range(0, n, step):
+        m = min(n, i + step) - i
+        q_lat = _latent_queries(lw, q[i:i + m], positions[i:i + m], rope)
+        s = B.linear(q_lat.view(m * H, lw.ld), rows, out_f32=True)
+        p = torch.empty((m * H, cols), device=q.device, dtype=q.dtype)
+        rc = lib.fb_softmax_causal_rows(_ptr(s), cols, _ptr(p), cols, m * H, cols, H, keys - n + i, lw.scale, dt, _stream())
+        _lib.check(rc, "fb_softmax_causal_rows")
+        B.linear_batched(B.linear(p, values).view(m, H * lw.lv), lw.w_uv, H, lw.lv, out[i:i + m], lw.vdim)
+
+
+def expand(lw, rows, h0: int, h1: int):
+    """Latent rows [n, lv] -> (keys [n, >= heads * dim], values [n, >= heads * vdim]) of the heads [h0, h1)"""
+    H, D, V = lw.heads, lw.dim, lw.vdim
     if lw.w_ukv is None:
-        return B.linear(rows, lw.w_uk), B.linear(rows, lw.w_uv.view(-1, lw.lv))
+        return B.linear(rows, lw.w_uk[h0 * D:h1 * D]), B.linear(rows, lw.w_uv.view(-1, lw.lv)[h0 * V:h1 * V])
+    if h1 - h0 < H:
+        return B.linear(rows, lw.w_ukv[h0 * D:h1 * D]), B.linear(rows, lw.w_ukv[H * D + h0 * V:H * D + h1 * V])
     kv = B.linear(rows, lw.w_ukv)
-    return kv[:, :lw.heads * lw.dim], kv[:, lw.heads * lw.dim:]
+    return kv[:, :H * D], kv[:, H * D:]
 
 
 def window_attention(lw, grp, q, gate, kv, out, head_gate=None, shared=None):
-    """Prefill kernel over one group's expanded keys and values ``kv``: [n_keys, >= heads * (dim + vdim)], or a pair of matrices; ``shared``:
-    [n_keys, rd] rotated key parts."""
+    """Prefill kernel over one group's expanded keys and values ``kv``: [n_keys, >= heads * (dim + vdim)]; ``shared``: [n_keys, rd] rotated
+    key parts."""
     H = lw.heads
-    k, v = kv if isinstance(kv, tuple) else (kv[:, :H * lw.dim], kv[:, H * lw.dim:])
+    _window_heads(lw, grp, q, gate, (kv[:, :H * lw.dim], kv[:, H * lw.dim:]), out, head_gate, shared, 0, H)
+
+
+def _window_heads(lw, grp, q, gate, kv, out, head_gate, shared, h0: int, h1: int):
+    """The same for the heads [h0, h1), whose keys and values are the pair ``kv``."""
+    H, (k, v) = h1 - h0, kv
+    q, out = q[:, h0 * lw.hd:], out[:, h0 * lw.vdim:]
+    gate = gate[:, h0 * lw.vdim:] if gate is not None else None
+    head_gate = head_gate[:, h0:] if head_gate is not None else None
     st = lambda t: t.stride(0) if t is not None else 0
     rc = _lib.kernels().fb_attn_window(_ptr(q), q.stride(0), lw.hd, q.shape[0], _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(shared), st(shared), k.shape[0],
                                        _ptr(out), out.stride(0), _ptr(gate), st(gate), _ptr(head_gate), st(head_gate), _ptr(grp.blocks), grp.n_blocks,
@@ -332,12 +410,18 @@ def attention(lw, proj, pool, fb, q=None, head_gate=None, rope=None):
         pick = lambda t: t.index_select(0, pl.rows) if t is not None else None
         _absorbed(lw, pick(q), pick(gate), pick(head_gate), pool, pl.page_table, pl.kv_lens, part, pick(fb.positions), rope)
         out.index_copy_(0, pl.rows, part)
+    for r0, r1, keys, slots in pl.folds:
+        _folded(lw, q[r0:r1], pool, keys, slots, out[r0:r1], fb.positions[r0:r1], rope)
     if pl.groups and lw.rd:
         qr = q[:, lw.dim:]
         S.rope_heads(qr, lw.hd, qr, lw.hd, H, lw.rot, lw.rd, fb.positions, *rope, lw.neox)
     for grp in pl.groups:
         rows = S.gather_rows(pool.view(-1, lw.ld), grp.key_idx)
-        window_attention(lw, grp, q, gate, expand(lw, rows[:, :lw.lv]), out, head_gate, rows[:, lw.lv:] if lw.rd else None)
+        # one long request alone may be too much: some of its heads at a time
+        slices = min(H, -(-2 * rows.shape[0] * H * (lw.dim + lw.vdim) // max(1, EXPAND_BYTES - rows.numel() * rows.element_size())))
+        for i in range(slices):
+            h0, h1 = i * H // slices, (i + 1) * H // slices
+            _window_heads(lw, grp, q, gate, expand(lw, rows[:, :lw.lv], h0, h1), out, head_gate, rows[:, lw.lv:] if lw.rd else None, h0, h1)
     return out
 
 

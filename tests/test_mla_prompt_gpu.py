@@ -59,8 +59,16 @@ def test_mla_prompt(dtype, mode, H, lens, news):
     assert rel(got) <= 1.05 * rel(old), (rel(got), rel(old))
 
 
+@pytest.mark.parametrize("form", ["absorbed", "expanded", "folded", "mixed"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_form(dtype, form, monkeypatch):
+    picks = iter(["folded", "expanded", "absorbed"])
+    monkeypatch.setattr(LA, "prompt_form", lambda *a: next(picks) if form == "mixed" else form)
+    test_mla_prompt(dtype, A.ROPE_INTERLEAVED, 16, [700, 300, 90], [700, 44, 1])
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
-def test_neighbours_stay_out(value):
+def test_neighbours_stay_out(value, monkeypatch):
     """Requests are expanded side by side: the first keys of one must not reach the rows of the one before."""
     H, nope, rope, lora, vd, dtype = 5, 128, 64, 512, 128, torch.float16
     lens, g = [700, 300, 250], torch.Generator(device="cuda").manual_seed(1)
@@ -78,6 +86,8 @@ def test_neighbours_stay_out(value):
     tables = A.build_rope_tables(rope, 1024, 1e4, None, "cuda")
     la = LA.from_absorbed(H, nope, rope, lora, vd, w_uk, w_uk.transpose(1, 2).contiguous(), w_uv, (nope + rope) ** -0.5, True)
 
+    monkeypatch.setattr(LA, "prompt_form", lambda *a: "expanded")
+
     def run():
         fb = ForwardBatch(ids=i32([0] * T), positions=i32(pos), slots=i32([-1] * T), page_table=table, kv_lens=i32(lens), cu_q=i32(cu), cu_q_host=cu, kv_lens_host=lens)
         qc = q.clone()
@@ -87,3 +97,37 @@ def test_neighbours_stay_out(value):
     pool[counts[0]] = value
     got = run()
     assert torch.equal(got[:cu[1]], want[:cu[1]]) and torch.equal(got[cu[2]:], want[cu[2]:])
+
+
+@pytest.mark.parametrize("form", ["expanded", "folded"])
+def test_scratch_is_bounded(form, monkeypatch):
+    """One request behind a long history alone may need more than the limit: slices of heads, or of rows."""
+    H, nope, rope, lora, vd, dtype, keys, n, limit = 12, 128, 64, 512, 128, torch.bfloat16, 4000, 70, 16 << 20
+    g = torch.Generator(device="cuda").manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    pages = (keys + PAGE - 1) // PAGE
+    pool, q = rnd(pages, PAGE, 1, lora + rope), rnd(n, H * (nope + rope))
+    w_uk, w_uv = (lora ** -0.5 * rnd(H, d, lora) for d in (nope, vd))
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    tables = A.build_rope_tables(rope, 4096, 1e4, None, "cuda")
+    la = LA.from_absorbed(H, nope, rope, lora, vd, w_uk, w_uk.transpose(1, 2).contiguous(), w_uv, (nope + rope) ** -0.5, True)
+    monkeypatch.setattr(LA, "prompt_form", lambda *a: form)
+
+    def run():
+        fb = ForwardBatch(ids=i32([0] * n), positions=i32(list(range(keys - n, keys))), slots=i32([-1] * n), page_table=i32([list(range(pages))]), kv_lens=i32([keys]),
+                          cu_q=i32([0, n]), cu_q_host=[0, n], kv_lens_host=[keys])
+        qc = q.clone()
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out = LA.attention(la, qc, pool, fb, qc, None, tables)
+        return out, torch.cuda.max_memory_allocated() - before
+
+    monkeypatch.setattr(LA, "EXPAND_BYTES", 1 << 30)
+    want, free = run()
+    monkeypatch.setattr(LA, "EXPAND_BYTES", limit)
+    got, bounded = run()
+    # heads by themselves: the same sums; rows in other portions: sums over k in another order before two roundings to bf16
+    assert torch.equal(got, want) if form == "expanded" else (got.double() - want.double()).norm() <= 2.0 ** -8 * want.double().norm()
+    # folded: the gathered latents (4.6 MB) and their values beside the scores; both: plan, queries and result (below 2 MB)
+    assert free > 1.5 * limit and bounded < limit + (12 << 20)
