@@ -219,6 +219,8 @@ def prompt_form(lw, n: int, keys: int, n_req: int = 1, sms: int = 148) -> str:
     32768 tokens, 16 heads: absorbed 239, expanded 1047, folded 333 us; 128 rows: 1121, 1075, 614; 1000 rows: 7749, 1370, 3030."""
     H, wide = lw.heads, (lw.lv + lw.ld) / 1088
     absorbed = 50 / n_req + n * keys * -(-H // 32) * (0.25 + 0.2 * min(H, 32) / 32) * 1e-3 * wide
+    if lw.lv > 512 or lw.ld > 576:                     # beyond the latent decode kernel
+        absorbed = math.inf
     fits = EXPAND_BYTES / (keys * _key_bytes(lw))                                       # requests of this length that are expanded at a time
     chain = 1 / max(1.0, min(n_req, fits)) if fits >= 1 else -(-1 // fits)
     steps = keys / 64 * (1.9 if n <= 128 else 2.6) * (lw.dim + lw.rd + lw.vdim) / 320

@@ -23,3 +23,9 @@ def test_choice_of_the_form(H, n, keys, n_req, want, monkeypatch):
     la = LA.LatentWeights()
     la.heads, la.dim, la.vdim, la.rank, la.lv, la.rot, la.rd, la.ld = H, 128, 128, 512, 512, 64, 64, 576
     assert LA.prompt_form(la, n, keys, n_req) == want
+
+
+def test_latents_beyond_the_decode_kernel_are_not_absorbed():
+    la = LA.LatentWeights()
+    la.heads, la.dim, la.vdim, la.rank, la.lv, la.rot, la.rd, la.ld = 16, 128, 128, 1024, 1024, 64, 64, 1088
+    assert LA.prompt_form(la, 4, 32000) == "folded" and LA.prompt_form(la, 4000, 4000) == "expanded"
