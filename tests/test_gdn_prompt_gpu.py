@@ -88,3 +88,18 @@ def test_prompt_matches_the_rule(dtype, lens, decay, monkeypatch):
         assert rel(got, want) <= 1.02 * rel(old, want) + 2.0 ** -21
         untouched = [s for s in range(5) if s not in slots]
         assert torch.equal(rec[untouched], first[1][untouched]) and torch.equal(conv[untouched], first[0][untouched])
+
+
+def test_convolution_rounds_as_often_wrongly_as_fp32():
+    """SiLU in full precision: results that are not the nearest fp16 value are as rare as with the fp32 operators (1700 of 16 million, spread 2.5 %)."""
+    T, C, dev, dtype = 4000, 4096, "cuda", torch.float16
+    gen = torch.Generator(device=dev).manual_seed(8)
+    x, w = torch.randn(T, C, device=dev, generator=gen).to(dtype), (0.5 * torch.randn(C, 4, device=dev, generator=gen)).to(dtype)
+    state = torch.zeros(1, C, 3, device=dev, dtype=dtype)
+    plan, y = L._PromptPlan([0, T], [0], dev), torch.empty(T, C, device=dev, dtype=dtype)
+    rc = _lib.kernels().fb_gdn_conv_prompt(x.data_ptr(), C, w.data_ptr(), state.clone().data_ptr(), plan.chunks.data_ptr(), plan.n_chunks, plan.reqs.data_ptr(),
+                                           plan.n_reqs, y.data_ptr(), C, 0, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    want = _conv64(x, w, state.clone(), [0, T], [0], C).to(dtype)
+    off = lambda t: (t != want).double().mean().item()
+    assert off(y) <= 1.1 * off(L.causal_conv1d(x, w, state.clone(), [0, T], [0])), (off(y), off(L.causal_conv1d(x, w, state.clone(), [0, T], [0])))
