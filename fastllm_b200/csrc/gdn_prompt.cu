@@ -11,11 +11,14 @@
 //                              S^T stays in registers as accumulator fragments, which are operand fragments of the next product as they
 //                              are (the k index of both operands is permuted alike); the chunk's keys and T are fetched a chunk ahead.
 //  * gdn_chunk_out_kernel      outputs of every (chunk, head), in parallel, with the norm over the head and the gate in the epilogue.
-// Products run on tf32 operands with fp32 accumulation.  Queries, keys and values are 16-bit numbers and exact there (their norms are
-// factors of rows, applied in fp32); every fp32 operand enters as two terms, the rounded value and the rounded remainder, so that products
-// carry 22 bits of it.  Decays, norms, gates, T and the state are fp32.
+// Products have fp32 accumulators.  Queries, keys and values are 16-bit numbers and exact (their norms are factors of rows, applied in
+// fp32); an fp32 operand of the chain over bf16 keys enters as three bf16 terms, all 24 bits, elsewhere as two tf32 terms (22 bits; fp16 V' three).
+// Decays, norms, gates, T and the state are fp32.  The tensor core cuts its sums off instead of rounding them, which adds up where a state forgets
+// slowly: in the chain every product of 8 or 16 terms is summed by itself, smallest terms first, and added in fp32.  Error of the states against
+// 64 bits over 28 calls of 30 tokens and more: 0.12 to 1.12 of that of fp32 operators, 0.53 in the mean (two tf32 terms and running sums: 2.1 times where
+// little is forgotten).
 //
-// 4001 tokens x 32 heads: 0.54 ms a layer (convolution 41 us, T 62, chain 270, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
+// 4001 tokens x 32 heads, bf16: 0.56 ms a layer (convolution 62 us, T 62, chain CHAIN, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
 #include "ptx.cuh"
 #include "launch.h"
 
@@ -68,6 +71,16 @@ __device__ __forceinline__ void gp_mma_16(float* c, const uint32_t* a, uint32_t 
   else
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void gp_add4(float* c, const float* t) { c[0] += t[0]; c[1] += t[1]; c[2] += t[2]; c[3] += t[3]; }
+// Two fp32 numbers as three bf16 terms each: all 24 bits.
+__device__ __forceinline__ void gp_split_bf16(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_16<true>(x, y);
+  const float2 f = unpack_16<true>(hi);
+  x -= f.x; y -= f.y;
+  mid = pack_16<true>(x, y);
+  const float2 g = unpack_16<true>(mid);
+  lo = pack_16<true>(x - g.x, y - g.y);
 }
 __device__ __forceinline__ void gp_ldsm4(uint32_t* r, const uint16_t* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)) : "memory");
@@ -262,8 +275,11 @@ __global__ void __launch_bounds__(128) gdn_chunk_inverse_kernel(const GdnPromptP
         for (int kk = 0; kk < 8; kk += 2) {
           uint32_t b[4];
           gp_ldsm4(b, ks + (nt * 8 + (lane & 7)) * GP_LDK + kk * 16 + (lane >> 3) * 8);
-          gp_mma_16<BF16>(acc, a[kk], b[0], b[1]);
-          gp_mma_16<BF16>(acc, a[kk + 1], b[2], b[3]);
+          float t[4] = {0.f, 0.f, 0.f, 0.f}, v[4] = {0.f, 0.f, 0.f, 0.f};
+          gp_mma_16<BF16>(t, a[kk], b[0], b[1]);
+          gp_mma_16<BF16>(v, a[kk + 1], b[2], b[3]);
+          gp_add4(t, v);
+          gp_add4(acc, t);
         }
       }
 #pragma unroll
@@ -297,8 +313,8 @@ __global__ void __launch_bounds__(128) gdn_chunk_inverse_kernel(const GdnPromptP
 // ------------------------------------------------------------------------------------------------
 // the chain over a request's chunks: a CTA of four warps takes 32 columns of a head's state, two warps 16 of them: each carries 64 of the 128 key
 // channels.  They add up K S, share out the columns of T's product (equal parts of its triangle) and exchange V', twice a chunk
-// through shared memory.  Bound by the issue of tf32 products (310 a warp and chunk at about 16 cycles; with one warp for all 128
-// channels 620, on half of the tensor cores): 270 us a layer at 4001 tokens x 32 heads, 375 us before.
+// through shared memory.  Bound by the issue of products (bf16: 192 of 16 terms and 54 tf32 ones a warp and chunk, and the fp32 additions between
+// them).  4001 tokens x 32 heads with the kernels before and behind it: 496 us; two tf32 terms and running sums 507, tf32 with separate sums 578.
 // ------------------------------------------------------------------------------------------------
 constexpr int GS_THREADS = 128;
 constexpr int GS_LDV = 40;
@@ -373,18 +389,42 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
     float r[8][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) r[j][0] = r[j][1] = r[j][2] = r[j][3] = 0.f;
+    if (BF16) {
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      float hi[4], lo[4];
-      gp_split(s[kk][0], hi[0], lo[0]); gp_split(s[kk][2], hi[1], lo[1]); gp_split(s[kk][1], hi[2], lo[2]); gp_split(s[kk][3], hi[3], lo[3]);
-      uint32_t b[8];
-      gp_ldsm4(b, ks + lane * GP_LDK + kk * 8);
-      gp_ldsm4(b + 4, ks + (32 + lane) * GP_LDK + kk * 8);
+      for (int kk = 0; kk < 4; ++kk) {
+        uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float2 f = unpack_16<BF16>(b[j]);
-        gp_mma_tf32(r[j], hi, f.x, f.y);
-        gp_mma_tf32(r[j], lo, f.x, f.y);
+        for (int i = 0; i < 4; ++i) gp_split_bf16(s[2 * kk + (i >> 1)][2 * (i & 1)], s[2 * kk + (i >> 1)][2 * (i & 1) + 1], hi[i], mid[i], lo[i]);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          uint32_t b[4];
+          gp_ldsm4(b, ks + (8 * (j + (lane >> 4)) + (lane & 7)) * GP_LDK + kk * 16 + ((lane >> 3) & 1) * 8);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+            gp_mma_16<true>(t, lo, b[2 * e], b[2 * e + 1]);
+            gp_mma_16<true>(t, mid, b[2 * e], b[2 * e + 1]);
+            gp_mma_16<true>(t, hi, b[2 * e], b[2 * e + 1]);
+            gp_add4(r[j + e], t);
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk) {
+        float hi[4], lo[4];
+        gp_split(s[kk][0], hi[0], lo[0]); gp_split(s[kk][2], hi[1], lo[1]); gp_split(s[kk][1], hi[2], lo[2]); gp_split(s[kk][3], hi[3], lo[3]);
+        uint32_t b[8];
+        gp_ldsm4(b, ks + lane * GP_LDK + kk * 8);
+        gp_ldsm4(b + 4, ks + (32 + lane) * GP_LDK + kk * 8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 f = unpack_16<BF16>(b[j]);
+          float t[4] = {0.f, 0.f, 0.f, 0.f};
+          gp_mma_tf32(t, lo, f.x, f.y);
+          gp_mma_tf32(t, hi, f.x, f.y);
+          gp_add4(r[j], t);
+        }
       }
     }
 #pragma unroll
@@ -402,9 +442,9 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
       r[j][3] = fmaf(-cb.y, r[j][3] + o.w, be.y * gp_ld<BF16>(vp[GS_LDV + 8]));
     }
     // V'^T = (right-hand side)^T T^T: token tiles 0, 3, 4, 7 or 1, 2, 5, 6, 18 products of the triangle each
-    float w[4][4];
+    float w[4][4], wl[4][4];                      // products of first terms, the others'
 #pragma unroll
-    for (int x = 0; x < 4; ++x) w[x][0] = w[x][1] = w[x][2] = w[x][3] = 0.f;
+    for (int x = 0; x < 4; ++x) w[x][0] = w[x][1] = w[x][2] = w[x][3] = wl[x][0] = wl[x][1] = wl[x][2] = wl[x][3] = 0.f;
     auto tile = [&](int x) { return 2 * x + ((x & 1) ^ half); };
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
@@ -417,42 +457,77 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
         float bh0, bl0, bh1, bl1;
         gp_split(tv.x, bh0, bl0);
         gp_split(tv.y, bh1, bl1);
-        gp_mma_tf32(w[x], hi, bh0, bh1);
-        gp_mma_tf32(w[x], lo, bh0, bh1);
-        gp_mma_tf32(w[x], hi, bl0, bl1);
+        float t[4] = {0.f, 0.f, 0.f, 0.f};
+        gp_mma_tf32(t, hi, bh0, bh1);
+        gp_add4(w[x], t);
+        gp_mma_tf32(wl[x], lo, bh0, bh1);
+        gp_mma_tf32(wl[x], hi, bl0, bl1);
       }
     }
     float* vn = p.vnew + (unit * GP_D + vr) * GP_T + 2 * q;
 #pragma unroll
     for (int x = 0; x < 4; ++x) {
+      gp_add4(w[x], wl[x]);
       new_own[32 * x] = make_float4(w[x][0], w[x][1], w[x][2], w[x][3]);
       *reinterpret_cast<float2*>(vn + 8 * tile(x)) = make_float2(w[x][0], w[x][1]);
       *reinterpret_cast<float2*>(vn + 8 * GP_T + 8 * tile(x)) = make_float2(w[x][2], w[x][3]);
     }
     meet();
-    // S^T <- e^(G_last) S^T + (decayed V')^T K.  The chunk's sum is made by itself: the tensor core's sums are cut off, not rounded, which would
-    // add up in a state that forgets slowly
+    // S^T <- e^(G_last) S^T + (decayed V')^T K
     float u[8][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) u[j][0] = u[j][1] = u[j][2] = u[j][3] = 0.f;
+    if (BF16) {
 #pragma unroll
-    for (int y = 0; y < 8; ++y) {
-      const bool mine = y < 4;
-      const int x = y & 3, kk = 2 * x + ((x & 1) ^ (mine ? half : half ^ 1));
-      const float4 wv = mine ? make_float4(w[x][0], w[x][1], w[x][2], w[x][3]) : new_other[32 * x];
-      const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 8 * kk + 2 * q);
-      float hi[4], lo[4];
-      gp_split(wv.x * cd.x, hi[0], lo[0]); gp_split(wv.z * cd.x, hi[1], lo[1]);
-      gp_split(wv.y * cd.y, hi[2], lo[2]); gp_split(wv.w * cd.y, hi[3], lo[3]);
+      for (int c = 0; c < 4; ++c) {               // 16 tokens: a tile of this warp's and one of the other's
+        const bool own_first = ((c & 1) ^ half) == 0;
+        const float4 own = make_float4(w[c][0], w[c][1], w[c][2], w[c][3]), other = new_other[32 * c];
+        uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
-      for (int j = 0; j < 8; j += 4) {
-        uint32_t b[4];
-        gp_ldsm4_t(b, ks + (8 * kk + (lane & 7)) * GP_LDK + (j + (lane >> 3)) * 8);
+        for (int i = 0; i < 2; ++i) {
+          const float4 wv = own_first == (i == 0) ? own : other;
+          const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 16 * c + 8 * i + 2 * q);
+          gp_split_bf16(wv.x * cd.x, wv.y * cd.y, hi[2 * i], mid[2 * i], lo[2 * i]);
+          gp_split_bf16(wv.z * cd.x, wv.w * cd.y, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
+        }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 f = unpack_16<BF16>(b[e]);
-          gp_mma_tf32(u[j + e], hi, f.x, f.y);
-          gp_mma_tf32(u[j + e], lo, f.x, f.y);
+        for (int j = 0; j < 8; j += 2) {
+          uint32_t b[4];
+          gp_ldsm4_t(b, ks + (16 * c + (lane & 15)) * GP_LDK + (j + (lane >> 4)) * 8);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+            gp_mma_16<true>(t, lo, b[2 * e], b[2 * e + 1]);
+            gp_mma_16<true>(t, mid, b[2 * e], b[2 * e + 1]);
+            gp_mma_16<true>(t, hi, b[2 * e], b[2 * e + 1]);
+            gp_add4(u[j + e], t);
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int y = 0; y < 8; ++y) {
+        const bool mine = y < 4;
+        const int x = y & 3, kk = 2 * x + ((x & 1) ^ (mine ? half : half ^ 1));
+        const float4 wv = mine ? make_float4(w[x][0], w[x][1], w[x][2], w[x][3]) : new_other[32 * x];
+        const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 8 * kk + 2 * q);
+        float hi[4], mid[4], lo[4];
+        const float wd[4] = {wv.x * cd.x, wv.z * cd.x, wv.y * cd.y, wv.w * cd.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { gp_split(wd[i], hi[i], mid[i]); lo[i] = gp_tf32((wd[i] - hi[i]) - mid[i]); }
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          uint32_t b[4];
+          gp_ldsm4_t(b, ks + (8 * kk + (lane & 7)) * GP_LDK + (j + (lane >> 3)) * 8);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = unpack_16<BF16>(b[e]);
+            float t[4] = {0.f, 0.f, 0.f, 0.f};
+            gp_mma_tf32(t, lo, f.x, f.y);
+            gp_mma_tf32(t, mid, f.x, f.y);
+            gp_mma_tf32(t, hi, f.x, f.y);
+            gp_add4(u[j + e], t);
+          }
         }
       }
     }

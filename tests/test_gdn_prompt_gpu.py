@@ -103,3 +103,34 @@ def test_convolution_rounds_as_often_wrongly_as_fp32():
     want = _conv64(x, w, state.clone(), [0, T], [0], C).to(dtype)
     off = lambda t: (t != want).double().mean().item()
     assert off(y) <= 1.1 * off(L.causal_conv1d(x, w, state.clone(), [0, T], [0])), (off(y), off(L.causal_conv1d(x, w, state.clone(), [0, T], [0])))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("lens,decay,Hk,Hv", [([30, 64], 0.0, 2, 4), ([63, 130], 3.0, 2, 4), ([65, 127, 200], -2.0, 2, 4), ([700], -6.0, 3, 3), ([1500], -8.0, 2, 4),
+                                              ([900], 1.0, 8, 16), ([333], -2.0, 8, 16)])
+@pytest.mark.parametrize("fresh", [False, True])
+def test_states_keep_fp32(dtype, lens, decay, Hk, Hv, fresh):
+    """The states' error against 64 bits is that of the operators in fp32."""
+    dev, kd, vd, T = "cuda", Hk * 128, Hv * 128, sum(lens)
+    gen = torch.Generator(device=dev).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=gen)
+    C, width = 2 * kd + vd, (2 * kd + 2 * vd + 2 * Hv + 7) // 8 * 8
+    proj, conv_w, norm_w = rnd(T, width).to(dtype), (0.5 * rnd(C, 4)).to(dtype), (1 + 0.1 * rnd(128)).to(dtype)
+    A_log, dt_bias = torch.log(0.3 + rnd(Hv).abs()), rnd(Hv) + decay
+    slots, cu = list(range(len(lens))), [sum(lens[:i]) for i in range(len(lens) + 1)]
+    conv, first = rnd(len(lens), C, 3).to(dtype), (0.0 if fresh else 0.2) * rnd(len(lens), Hv, 128, 128)
+    plan, rec, rec32, rec64 = L._PromptPlan(cu, slots, dev), first.clone(), first.clone(), first.double()
+    y = _conv64(proj, conv_w, conv.clone(), cu, slots, C).to(dtype)
+    _rule64(y, proj, A_log, dt_bias, norm_w, 1e-6, rec64, cu, slots, Hk, Hv)
+    b, a = proj[:, C + vd:C + vd + Hv], proj[:, C + vd + Hv:C + vd + 2 * Hv]
+    L.gated_delta_rule(y[:, :kd].reshape(T, Hk, 128), y[:, kd:2 * kd].reshape(T, Hk, 128), y[:, 2 * kd:].reshape(T, Hv, 128), a, b, A_log, dt_bias, rec32, cu, slots,
+                       Hv // Hk)
+    scratch = [torch.empty(plan.n_chunks * Hv * k, device=dev) for k in (64 * 64, 9 * 64, 128 * 64, 128 * 128)]
+    out, p = torch.empty(T, vd, device=dev, dtype=dtype), lambda t: t.data_ptr()
+    rc = _lib.kernels().fb_gdn_prompt(p(y), C, p(a), p(b), width, p(proj[:, C:]), width, p(A_log), p(dt_bias), p(norm_w), p(rec), p(out), p(plan.chunks), plan.n_chunks,
+                                      p(plan.reqs), plan.n_reqs, *map(p, scratch), Hk, Hv, 0, Hv, 1e-6, 1 if dtype == torch.bfloat16 else 0,
+                                      torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    rel = lambda x: ((x.double() - rec64).norm() / rec64.norm()).item()
+    # 2^-25: half a unit in the last place of the states themselves, whichever way their last addition rounds
+    assert rel(rec) <= rel(rec32) + 2.0 ** -25, (rel(rec), rel(rec32))
