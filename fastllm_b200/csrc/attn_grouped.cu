@@ -287,7 +287,7 @@ attn_grouped_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           uint4* vrow = reinterpret_cast<uint4*>(v_smem + t * 128);
           for (int j = 0; j < vt; ++j)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) vrow[j * (AG_TILE / 16) + e] = make_uint4(0u, 0u, 0u, 0u);
+            for (int e = 0; e < 8; ++e) vrow[j * (AG_TILE / 16) + ((e + t) & 7)] = make_uint4(0u, 0u, 0u, 0u);      // (a warp's rows share banks)
         }
       }
       fence_proxy_async_smem();

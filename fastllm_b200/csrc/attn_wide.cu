@@ -201,7 +201,7 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           uint4* vrow = reinterpret_cast<uint4*>(v_smem + (n & 1) * vt * AX_KT + (r & 63) * 128);
           for (int j = r >> 6; j < vt; j += 2)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) vrow[j * (AX_KT / 16) + e] = make_uint4(0u, 0u, 0u, 0u);
+            for (int e = 0; e < 8; ++e) vrow[j * (AX_KT / 16) + ((e + r) & 7)] = make_uint4(0u, 0u, 0u, 0u);      // (a warp's rows share banks)
         }
       }
       fence_proxy_async_smem();
