@@ -18,7 +18,7 @@
 // 64 bits over 28 calls of 30 tokens and more: 0.12 to 1.12 of that of fp32 operators, 0.53 in the mean (two tf32 terms and running sums: 2.1 times where
 // little is forgotten).
 //
-// 4001 tokens x 32 heads, bf16: 0.56 ms a layer (convolution 62 us, T 62, chain CHAIN, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
+// 4001 tokens x 32 heads, bf16: 0.54 ms a layer (convolution 56 us, T 61, chain 258, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
 #include "ptx.cuh"
 #include "launch.h"
 
