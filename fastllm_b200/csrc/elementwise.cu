@@ -845,12 +845,21 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
 
 using namespace fb;
 
+static int device_sms() {
+  static int count[64] = {};
+  int d = 0;
+  cudaGetDevice(&d);
+  int& n = count[d & 63];
+  if (n == 0) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d);
+  return n;
+}
+
 // Two waves of one CTA an SM or fewer: a vector a thread; more rows: four a thread, two where that leaves no full warp group.
 template <bool BF16, int QMODE>
 static void launch_rmsnorm(const void* x, const void* w, void* y, void* residual, int M, int H, int ldx, int ldy, float eps, float unit_offset, const NormQuantOut& qo,
                            cudaStream_t s) {
   const int vecs = H / 8;
-  const int nv = vecs > 1024 ? 4 : M <= 296 ? 1 : vecs > 256 ? 4 : vecs > 128 ? 2 : 1;
+  const int nv = vecs > 1024 ? 4 : M <= 2 * device_sms() ? 1 : vecs > 256 ? 4 : vecs > 128 ? 2 : 1;
   const int threads = ((vecs + nv - 1) / nv + 31) / 32 * 32;
 #define FB_NORM(NV)                                                                                                                             \
   launch_k(rmsnorm_kernel<BF16, QMODE, NV>, dim3(M), dim3(threads), 0, s, 0, (const uint16_t*)x, (const uint16_t*)w, (uint16_t*)y, (uint16_t*)residual, H, ldx, ldy, \

@@ -72,3 +72,40 @@ def test_qkv_rows(T, D, rot, mode, norm, Hq, Hkv):
     unused = torch.ones(3 * 128, dtype=torch.bool)
     unused[at] = False
     assert not kp.view(3 * 128, -1).cpu()[unused].any() and not vp.view(3 * 128, -1).cpu()[unused].any()
+
+
+# rows behind two waves of the SMs (four and two vectors a thread), a last round that half a warp or one warp has part in, more than 1024 vectors
+@pytest.mark.parametrize("M,H", [(1, 8320), (64, 1152), (64, 8320), (297, 1152), (297, 1920), (297, 2944), (297, 8320), (330, 4096)])
+@pytest.mark.parametrize("mode", [1, 2, 3, 4])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_rmsnorm_with_8_bit_rows(M, H, mode, dtype):
+    """The quantised rows beside the norm, or the norm rounded to their grid: the separate launches' bits."""
+    from fastllm_b200.ops import quant_gemm as QG
+
+    if mode < 3 and M > 128:
+        pytest.skip("8-bit rows are made for up to 128")
+    g = torch.Generator(device=DEV).manual_seed(M + H)
+    x, res = torch.randn(M, H, device=DEV, generator=g).to(dtype), torch.randn(M, H, device=DEV, generator=g).to(dtype)
+    w = (1 + 0.1 * torch.randn(H, device=DEV, generator=g)).to(dtype)
+    for residual in (None, res):
+        r0, r1 = (t.clone() if t is not None else None for t in (residual, residual))
+        plain, y = B.rmsnorm(x, w, 1e-5, residual=r0), B.rmsnorm(x, w, 1e-5, residual=r1, quant_mode=mode)
+        assert y.fb_quant[0] == mode and (residual is None or torch.equal(r0, r1))
+        if mode >= 3:
+            assert torch.equal(y, QG.round_act(plain, mode - 3))
+            continue
+        _, xq, scales, sums, _ = y.fb_quant
+        want = QG.quant_act_i8(plain) if mode == 1 else QG.quant_act_fp8(plain)
+        assert torch.equal(y, plain) and torch.equal(xq, want[0]) and torch.equal(scales[:, :M], want[1][:, :M])
+        assert mode == 2 or torch.equal(sums[:, :M], want[2][:, :M])
+
+
+def test_norm_rule_follows_the_device():
+    """Rows on either side of the count from which a thread takes more vectors (two rows an SM)."""
+    n = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator(device=DEV).manual_seed(n)
+    x, w = torch.randn(n + 1, 4096, device=DEV, generator=g).bfloat16(), (1 + 0.1 * torch.randn(4096, device=DEV, generator=g)).bfloat16()
+    many, few = B.rmsnorm(x, w, 1e-6), B.rmsnorm(x[:n], w, 1e-6)
+    ref = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    for y in (many[:n], few):
+        assert bool(((y.double() - ref[:n]).abs() <= ref[:n].abs() * (torch.finfo(y.dtype).eps / 2 + 2.0 ** -20) + 2.0 ** -24).all())
