@@ -29,3 +29,31 @@ def test_stages_are_not_refilled_under_their_readers(kind, rows):
     want = want @ w.dequant(torch.bfloat16).double().t()
     err = (first.double() - want).norm(dim=1) / want.norm(dim=1)
     assert err.max() < 3 * 2.0 ** -8, err
+
+
+@pytest.mark.parametrize("kind", ["fp8", "int8", "int4g128"])
+@pytest.mark.parametrize("rows", [8, 40, 100])
+def test_grouped_stages_are_not_refilled_under_their_readers(kind, rows):
+    """The same of the grouped products: a few experts, every one with rows, 32 k blocks; the dequantised weights' products per expert."""
+    from fastllm_b200.ops import basic as B
+    from fastllm_b200.ops import moe as MOE
+    from fastllm_b200.ops import moe_grouped
+
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    E, topk, H, inter, dt = 3, 2, 4096, 1024, torch.bfloat16
+    load = lambda w, **k: LinearWeight.from_dense((0.02 * w).to(dt), kind, act_dtype=dt, **k)
+    gu = [load(B.interleave_gate_up(rnd(inter, H), rnd(inter, H)), interleaved=True) for _ in range(E)]
+    experts = MOE.ExpertWeights(E, 0, gu, [load(rnd(H, inter)) for _ in range(E)])
+    experts.stacked = moe_grouped.stack_experts(experts)
+    assert experts.stacked is not None and experts.stacked.kind != "dense"
+    scale = torch.exp2(torch.randint(-6, 7, (rows, H // 128, 1), device="cuda", generator=g).float()).expand(-1, -1, 128).reshape(rows, H)
+    x = (rnd(rows, H) * scale * 0.05).to(dt)
+    idx, wts = MOE.route_topk(rnd(rows, E), None, topk, 0, True)
+    first = moe_grouped.forward(x, idx, wts, experts)
+    for _ in range(20):
+        assert torch.equal(moe_grouped.forward(x, idx, wts, experts), first)
+    # rows by themselves: each row's factors are its own whatever stands beside it (the products' sums and roundings are the same)
+    for t in (0, rows // 2, rows - 1):
+        one = moe_grouped.forward(x[t:t + 1].contiguous(), idx[t:t + 1].contiguous(), wts[t:t + 1].contiguous(), experts)
+        assert ((one - first[t:t + 1]).double().norm() <= 2.0 ** -6 * one.double().norm())

@@ -59,3 +59,20 @@ def test_block_diagonal(M, N, K, blocks):
     xd, wd = x.double().view(M, blocks, K), w.double().view(blocks, N, K)
     ref, size = torch.einsum("mbk,bnk->mbn", xd, wd), torch.einsum("mbk,bnk->mbn", xd.abs(), wd.abs())
     assert bool(((out.double().view(M, blocks, N) - ref).abs() <= K * 2.0 ** -23 * size).all())
+
+
+@pytest.mark.parametrize("M,N,K", [(1025, 4352, 136), (4001, 3072, 512), (1000, 4096, 14336)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["plain", "bias+residual", "f32", "swiglu"])
+def test_pairs_give_the_bits_of_one_cta(M, N, K, dtype, form):
+    """Every output is the same sum in the same order whichever kernel makes it: portions of rows that stay with one CTA a tile against the whole."""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, w = torch.randn(M, K, device=DEV, generator=g).to(dtype), (torch.randn(N, K, device=DEV, generator=g) * 0.1).to(dtype)
+    b, r = torch.randn(N, device=DEV, generator=g).to(dtype), torch.randn(M, N, device=DEV, generator=g).to(dtype)
+    call = {"plain": lambda s: B.linear(x[s], w), "bias+residual": lambda s: B.linear(x[s], w, bias=b, residual=r[s]), "f32": lambda s: B.linear(x[s], w, out_f32=True),
+            "swiglu": lambda s: B.linear(x[s], w, swiglu=True)}[form]
+    got = call(slice(None))
+    for lo in range(0, M - 257, 333):                          # 333 rows: three row tiles of one CTA, never pairs at these widths
+        s = slice(lo, min(lo + 333, M))
+        if s.stop - s.start > 256:
+            assert torch.equal(call(s), got[s])
