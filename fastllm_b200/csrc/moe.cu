@@ -496,7 +496,8 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant
           }
 #pragma unroll
           for (int j = 0; j < HALF; ++j) {
-            const float g = (q < 2 ? v[j] : o[j]) + bg, up = (q < 2 ? o[j] : v[j]) + bu;
+            float g = q < 2 ? v[j] : o[j], up = q < 2 ? o[j] : v[j];
+            if (EXTRA) { g += bg; up += bu; }
             v[j] = clamp ? glu_clamp_f(g, up, p.act_limit, p.act_alpha) : EXTRA && (p.flags & GEMM_GEGLU) ? gelu_tanh_f(g) * up : silu_f(g) * up;
             if (EXTRA && (p.flags & GEMM_RELU2)) v[j] = relu2_f(v[j]);
           }
