@@ -4,11 +4,13 @@
 //     S[128 q x 64 k] = Q * K^T        O[128 q x V] += P * V
 // Two score buffers: the tensor core makes the scores of step i + 1 while the softmax warps, a thread a query row, work on step i.  Keys and
 // values have rings of their own (two steps each; a key step is free as soon as its scores exist).  At 256 x 256 the queries take 64 KB,
-// the rings 128 KB, P 32 KB, and O 256 of the 512 TMEM columns, so that one CTA fills an SM; K and V of a group's heads meet in the L2.
+// the rings 128 KB, P 32 KB, and O 256 of the 512 TMEM columns, so that one CTA fills an SM; K and V of a group's heads meet in the L2.  (Narrower
+// heads leave shared memory for a second CTA, but all columns are taken whatever V is: it waits for them.)
 // Probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder): 16 bits of them in bf16.  In fp16 the terms are
 // scaled by 2^13, which the sum shares, so that what they leave out is 2^-38 of the largest weight.  O is rescaled only when a row's maximum has grown
 // by more than 2^8 (fp16: 2^2), which changes no rounding of P and keeps fp16 terms finite (up to 2^15).
-// Bound: the softmax thread's 64 exponentials and term splits of a step (about 1200 cycles) above the products' 768.
+// Bound: latency of the one softmax warp on each sub-core, step after step (2000 tokens x 16 heads x 256: tensor pipe 42 % busy, special-function
+// unit 14 %, issue slots 21 %).
 // 4001 tokens x 16 heads x 256: 252 us (PyTorch, gathered fp32 keys and values and fp32 scores in memory: 7.0 ms).
 #include "ptx.cuh"
 #include "launch.h"
