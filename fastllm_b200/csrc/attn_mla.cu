@@ -4,7 +4,8 @@
 // Query per head: q_nope already multiplied by W_UK, followed by the rotated q_pe where the model has one.
 //     S^T[128 tokens x N heads] = Lat_page[128 x dq] * Q^T              column tiles of 64, K-major, SW128 (DeepSeek: 9)
 //     O^T[dv dims    x N heads] = Lat_page[:, :dv]^T * P^T              row blocks of 128 dims, A read MN-major (DeepSeek: 4)
-// With a sliding window the plan lists the pages the window touches and the softmax masks the keys before it.
+// With a sliding window the plan lists the pages the window touches and the softmax masks the keys before it.  Values behind a request's
+// end are cleared in shared memory before the second product (P = 0 alone would pass NaN and infinity on).
 // The latent page is both K and V: it is loaded ONCE into 16 KB tiles, each with its own full/empty barrier, so the
 // next page streams in tile by tile while the current page's softmax and PV products still run (one CTA per SM, 144 KB of
 // page + 36 KB of queries).  A work item is a run of consecutive pages of one request and one group of <= 32 heads; the
@@ -304,6 +305,17 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap tmLat, const __grid_consta
         if (GP < ML_N) {
 #pragma unroll
           for (int h = GP; h < ML_N; ++h) *reinterpret_cast<uint16_t*>(pb + (h >> 3) * 128 + (h & 7) * 16) = 0;
+        }
+        if (key >= seq) {
+          // slots behind the request's end have no weight, but what an earlier owner left there may be no number: their values count as zeros.
+          // (The page's scores are made, so every tile has landed, and none is refilled before its product below.)
+#pragma unroll 1
+          for (int j = 0; j < p.vtiles; ++j) {
+            mbar_wait(&full[j], ph, dead, KID_MLA, 10);
+            uint4* vrow = reinterpret_cast<uint4*>(lat + j * ML_TILE_BYTES + t * 128);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) vrow[(e + t) & 7] = make_uint4(0u, 0u, 0u, 0u);      // (a warp's rows share banks)
+          }
         }
         fence_proxy_async_smem();
         tc_fence_before_sync();

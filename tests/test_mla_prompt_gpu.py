@@ -99,6 +99,35 @@ def test_neighbours_stay_out(value, monkeypatch):
     assert torch.equal(got[:cu[1]], want[:cu[1]]) and torch.equal(got[cu[2]:], want[cu[2]:])
 
 
+@pytest.mark.parametrize("form", ["absorbed", "expanded", "folded"])
+@pytest.mark.parametrize("H", [5, 40])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_earlier_owners_stay_out(value, H, form, monkeypatch):
+    """What stands in a request's last page behind its end, left by the page's earlier owner, must not reach its rows."""
+    nope, rope, lora, vd, dtype, lens, n = 128, 64, 512, 128, torch.float16, [300, 129, 256], 3
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    pages = (max(lens) + PAGE - 1) // PAGE
+    table = torch.arange(len(lens) * pages, device="cuda", dtype=torch.int32).view(len(lens), pages)
+    pool = rnd(len(lens) * pages, PAGE, 1, lora + rope).to(dtype)
+    w_uk, w_uv = ((lora ** -0.5 * rnd(H, d, lora)).to(dtype) for d in (nope, vd))
+    q = rnd(n * len(lens), H * (nope + rope)).to(dtype)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    cu, pos = [n * i for i in range(len(lens) + 1)], [j for L in lens for j in range(L - n, L)]
+    tables = A.build_rope_tables(rope, 1024, 1e4, None, "cuda")
+    la = LA.from_absorbed(H, nope, rope, lora, vd, w_uk, w_uk.transpose(1, 2).contiguous(), w_uv, (nope + rope) ** -0.5, True)
+    monkeypatch.setattr(LA, "prompt_form", lambda *a: form)
+    outs = []
+    for fill in (0.0, value):
+        for b, L in enumerate(lens):
+            pool[b * pages:(b + 1) * pages].view(-1, lora + rope)[L:] = fill
+        fb = ForwardBatch(ids=i32([0] * len(pos)), positions=i32(pos), slots=i32([-1] * len(pos)), page_table=table, kv_lens=i32(lens), cu_q=i32(cu), cu_q_host=cu,
+                          kv_lens_host=lens)
+        qc = q.clone()
+        outs.append(LA.attention(la, qc, pool, fb, qc, None, tables))
+    assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("form", ["expanded", "folded"])
 def test_scratch_is_bounded(form, monkeypatch):
     """One request behind a long history alone may need more than the limit: slices of heads, or of rows."""
