@@ -102,7 +102,6 @@ def test_prompts_and_steps(name):
         _lib.check_device_errors()
     # a step captured for four rows runs the same kernels on the same rows
     assert torch.equal(got, eager)
-    err = lambda x: ((x - want).norm(dim=-1) / want.norm(dim=-1))
     # the CPU's bf16 operators round as often; a near tie of the experts at one token moves single rows of the 15
     err = lambda x: ((x - want).norm(dim=-1) / want.norm(dim=-1))
     assert err(got).median() <= 1.5 * err(low).median() and (err(got) > 3 * err(low).median()).sum() <= 2, (err(got), err(low))
