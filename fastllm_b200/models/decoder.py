@@ -672,7 +672,7 @@ class DecoderModel:
                 o = LA.attention(la, q, lat_pool, fb, q, None, (cos, sin))
                 return self._row_parallel_norm(lw.o, o, residual, next_ln, consumer=consumer)
         # latent norm + rope of the shared key into the cache entry, rope of the heads' rotary query parts: one launch
-        q_full = torch.empty((T, H, lora + rope), device=x.device, dtype=x.dtype)
+        q_full = x.new_empty((T, H, lora + rope))
         A.mla_post(ckv, q, q_full, lat_pool, fb.positions, fb.slots, lw.kv_a_norm, cos, sin, H, nope, rope, lora, self.rope_mode,
                    c.latent_norm_eps or c.rms_eps)
         # absorb: q_lat[h] = q_nope[h] @ W_UK[h] -> attention in latent space with a single shared "KV head"; one batched
@@ -695,7 +695,7 @@ class DecoderModel:
                 wi = torch.matmul(x.float(), lw.idx_weights.t()) * (Hi ** -0.5)
                 sel = MOE.dsa_select(qi, wi, idx_pool, fb, c.index_topk)
         o_lat = MOE.mla_paged_attention(q_full, lat_pool, fb, self.attn_scale, lora, sel)   # [T, H, lora]
-        o = torch.empty((T, H * vd), device=x.device, dtype=x.dtype)
+        o = x.new_empty((T, H * vd))
         B.linear_batched(o_lat.reshape(T, H * lora), lw.w_uv_c, H, lora, o, vd)
         return self._row_parallel_norm(lw.o, o, residual, next_ln, consumer=consumer)
 

@@ -172,7 +172,7 @@ def qkv_post(qkv, positions, slots, k_pool, v_pool, num_q_heads, num_kv_heads, h
         vp[slots[valid].long()] = v[valid].to(vp.dtype)
         return q.reshape(T, Hq * D)
     if q_out is None:
-        q_out = torch.empty((T, Hq * D), device=qkv.device, dtype=qkv.dtype)
+        q_out = qkv.new_empty((T, Hq * D))
     if k_pool.dtype == torch.float8_e4m3fn:
         rc = _lib.kernels().fb_qkv_post_kv8(_ptr(qkv), qkv.stride(0), _ptr(q_out), q_out.stride(0), _ptr(k_pool), _ptr(v_pool),
                                             _ptr(positions), _ptr(slots), _ptr(q_norm_w), _ptr(k_norm_w), _ptr(cos), _ptr(sin), T, Hq,
@@ -232,7 +232,7 @@ def qkv_proj_post(x, w, positions, slots, k_pool, v_pool, num_q_heads, num_kv_he
             or rot % 8 != 0 or rot > D or w.n // 128 > 148 or k_pool.dtype != x.dtype or x.stride(-1) != 1
             or (x.data_ptr() & 15) or (x.stride(0) * 2) % 16):
         return None
-    q_out = torch.empty((T, Hq * D), device=x.device, dtype=x.dtype)
+    q_out = x.new_empty((T, Hq * D))
     pend = _take_pending_wait()
     P = ctypes.c_void_p
     rc = _lib.kernels().fb_gemm_qkv_post(_ptr(x), _ptr(w.w), _ptr(w.bias), T, w.n, w.k, x.stride(0), w.w.stride(0), dtype_code(x.dtype),
@@ -501,9 +501,9 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_lens, scale, num_q_heads, num
     if quant_mode in (1, 2) and not _FUSED_COMBINE and B <= 128:
         K = num_q_heads * head_dim
         ld_a = (B + 128 + 3) // 4 * 4
-        xq = torch.empty((B, K), device=q.device, dtype=torch.int8 if quant_mode == 1 else torch.uint8)
-        sa = torch.empty((num_q_heads, ld_a), device=q.device, dtype=torch.float32)
-        xs = torch.empty((num_q_heads, ld_a), device=q.device, dtype=torch.float32) if quant_mode == 1 else None
+        xq = q.new_empty((B, K), dtype=torch.int8 if quant_mode == 1 else torch.uint8)
+        sa = q.new_empty((num_q_heads, ld_a), dtype=torch.float32)
+        xs = q.new_empty((num_q_heads, ld_a), dtype=torch.float32) if quant_mode == 1 else None
     else:
         quant_mode = 0
     if variant:
@@ -636,7 +636,7 @@ def mla_decode(q_full, lat_pool, page_table, seq_lens, scale, ws: MlaWorkspace |
         if ws is None:
             ws = _MLA_WS[key] = MlaWorkspace(cap, H, q_full.device, lora)
     q_full = q_full.contiguous()
-    out = torch.empty((B, H, lora), device=q_full.device, dtype=q_full.dtype)
+    out = q_full.new_empty((B, H, lora))
     num_slots = lat_pool.shape[0] * lat_pool.shape[1]
     rc = _lib.kernels().fb_mla_decode(_ptr(q_full), _ptr(lat_pool), _ptr(out), _ptr(page_table), _ptr(seq_lens), _ptr(ws.work),
                                       _ptr(ws.n_work), _ptr(ws.item_range), _ptr(ws.part_o), _ptr(ws.part_ml), B, H, dq, lora, num_slots,

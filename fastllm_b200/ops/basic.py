@@ -18,12 +18,14 @@ from . import _lib, cpu
 GEMM_BIAS, GEMM_RESIDUAL, GEMM_SWIGLU, GEMM_OUT_F32, GEMM_RELU2, GEMM_GLU_CLAMP, GEMM_GEGLU, GEMM_GELU, GEMM_GELU_TANH = 1, 2, 4, 8, 32, 64, 128, 512, 1024
 
 
+# What every launch asks for, as plain integers (the launchers' signatures turn them into pointers): a ``torch.cuda.Stream`` object costs 10 us on the host,
+# its handle 0.2, and short prompts are bound by the host (60 tokens through 8 dense layers: 1.8 ms of host work for 1.1 ms on the device).
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else ctypes.c_void_p(0)
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def dtype_code(dt: torch.dtype) -> int:
@@ -224,7 +226,7 @@ def linear_act(x, w, act: str, out=None, row_gate=None, mul=None, mul_rows=None)
     ``mul`` [rows, >= N]; all in the GEMM's epilogue."""
     M, (N, K) = x.shape[0], w.shape
     if out is None:
-        out = torch.empty((M, N), device=x.device, dtype=x.dtype)
+        out = x.new_empty((M, N))
     if not x.is_cuda:
         flush_pending_wait()
         y = act_ref(x.float() @ w.float().t(), act)
@@ -263,7 +265,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, swiglu: b
             return cpu_linear_epilogue(cpu.linear(x, w, bias), residual, swiglu, interleaved)
         return linear_ref(x, w, bias, residual, swiglu, interleaved, torch.float32 if out_f32 else None)
     lead = x.shape[:-1]
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
     M, K = x2.shape
@@ -298,15 +300,20 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, swiglu: b
         raise ValueError("CUDA SwiGLU epilogue needs tile-interleaved gate/up weights (interleave_gate_up)")
     n_out = N // 2 if swiglu else N
     if out is None:
-        out = torch.empty((M, n_out), device=x.device, dtype=torch.float32 if out_f32 else x.dtype)
+        out = x.new_empty((M, n_out), dtype=torch.float32 if out_f32 else x.dtype)
     flags = (GEMM_BIAS if bias is not None else 0) | (GEMM_RESIDUAL if residual is not None else 0) | \
             (GEMM_SWIGLU | (GEMM_GEGLU if geglu else 0) if swiglu else 0) | (GEMM_OUT_F32 if out_f32 else 0) | (GEMM_RELU2 if relu2 else 0)
-    res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
+    res2 = residual if residual is None or residual.dim() == 2 else residual.reshape(-1, residual.shape[-1])
     lib = _lib.kernels()
     dt = dtype_code(x.dtype)
     if M <= 256 or N % 32 != 0:
         step = 256
         pend = _take_pending_wait()
+        if M <= step and pend is None:
+            rc = lib.fb_gemm_16bit(_ptr(x2), _ptr(w), _ptr(out), _ptr(bias), _ptr(res2), M, N, K, x2.stride(0), w.stride(0), out.stride(0),
+                                   res2.stride(0) if res2 is not None else 0, dt, flags, nsplit, _stream())
+            _lib.check(rc, "fb_gemm_16bit")
+            M = 0
         for m0 in range(0, M, step):
             m1 = min(M, m0 + step)
             if pend is not None:
@@ -327,7 +334,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, swiglu: b
         rc = lib.fb_gemm_16bit(_ptr(x2), _ptr(w), _ptr(out), _ptr(bias), _ptr(res2), M, N, K, x2.stride(0), w.stride(0),
                                out.stride(0), res2.stride(0) if res2 is not None else 0, dt, flags, nsplit, _stream())
         _lib.check(rc, "fb_gemm_16bit")
-    return out.reshape(*lead, n_out)
+    return out if x.dim() == 2 and out.dim() == 2 else out.reshape(*lead, n_out)
 
 
 def linear_batched(x: torch.Tensor, w: torch.Tensor, batch: int, x_cols: int, out: torch.Tensor, out_cols: int, gate=None) -> torch.Tensor:
@@ -368,7 +375,7 @@ def linear_blocks(x, w):
     flush_pending_wait()
     if not x.is_cuda:
         return torch.einsum("mzk,znk->mzn", x.reshape(M, batch, K).float(), w.float()).reshape(M, batch * N)
-    out = torch.empty((M, batch * N), device=x.device, dtype=torch.float32)
+    out = x.new_empty((M, batch * N), dtype=torch.float32)
     if not tc_operands_ok(x, w.view(batch * N, K)) or N % 8:
         return linear_full32(x, w, out=out, batch=batch, x_cols=K, out_cols=N)
     rc = _lib.kernels().fb_gemm_16bit_blocks(_ptr(x), _ptr(w), _ptr(out), M, N, K, batch, x.stride(0), out.stride(0), dtype_code(x.dtype), _stream())
@@ -405,10 +412,10 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor
         if residual is not None:
             residual.copy_(new_res)
         return y
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     M, H = x2.shape
     if out is None:
-        out = torch.empty((M, H), device=x.device, dtype=x.dtype)
+        out = x.new_empty((M, H))
     if residual is not None and not residual.is_contiguous():
         raise ValueError("residual must be contiguous")
     if quant_mode in (3, 4) and H % 128 == 0 and x.dtype in (torch.float16, torch.bfloat16):
@@ -422,9 +429,9 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor
         return y
     if quant_mode in (1, 2) and H % 128 == 0 and M <= 128 and x.dtype in (torch.float16, torch.bfloat16):
         ld_a = (M + 128 + 3) // 4 * 4
-        xq = torch.empty((M, H), device=x.device, dtype=torch.int8 if quant_mode == 1 else torch.uint8)
-        sa = torch.empty((H // 128, ld_a), device=x.device, dtype=torch.float32)
-        xs = torch.empty((H // 128, ld_a), device=x.device, dtype=torch.float32) if quant_mode == 1 else None
+        xq = x.new_empty((M, H), dtype=torch.int8 if quant_mode == 1 else torch.uint8)
+        sa = x.new_empty((H // 128, ld_a), dtype=torch.float32)
+        xs = x.new_empty((H // 128, ld_a), dtype=torch.float32) if quant_mode == 1 else None
         rc = _lib.kernels().fb_rmsnorm_quant(_ptr(x2), _ptr(w), _ptr(out), _ptr(residual), M, H, x2.stride(0), out.stride(0), float(eps),
                                              float(unit_offset), dtype_code(x.dtype), quant_mode, _ptr(xq), H, _ptr(sa), _ptr(xs), ld_a,
                                              _stream())
@@ -435,7 +442,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, residual: torch.Tensor
     rc = _lib.kernels().fb_rmsnorm(_ptr(x2), _ptr(w), _ptr(out), _ptr(residual), M, H, x2.stride(0), out.stride(0), float(eps),
                                    float(unit_offset), dtype_code(x.dtype), _stream())
     _lib.check(rc, "fb_rmsnorm")
-    return out.reshape(x.shape)
+    return out if x.dim() == 2 and out.dim() == 2 else out.reshape(x.shape)
 
 
 # ---------------------------------------------------------------------------------------------------
@@ -450,7 +457,7 @@ def silu_mul(x: torch.Tensor) -> torch.Tensor:
         g, u = x.float().chunk(2, dim=-1)
         return (F.silu(g) * u).to(x.dtype)
     x2 = x.reshape(-1, x.shape[-1])
-    out = torch.empty((x2.shape[0], inter), device=x.device, dtype=x.dtype)
+    out = x.new_empty((x2.shape[0], inter))
     rc = _lib.kernels().fb_silu_mul(_ptr(x2), _ptr(out), x2.shape[0], inter, x2.stride(0), out.stride(0), dtype_code(x.dtype),
                                     _stream())
     _lib.check(rc, "fb_silu_mul")
@@ -485,7 +492,7 @@ def glu_act(x: torch.Tensor, act: str, interleaved: bool = False) -> torch.Tenso
     x2 = x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1:
         x2 = x2.contiguous()
-    out = torch.empty((x2.shape[0], inter), device=x.device, dtype=x.dtype)
+    out = x.new_empty((x2.shape[0], inter))
     rc = _lib.kernels().fb_glu_act(_ptr(x2), _ptr(out), x2.shape[0], inter, x2.stride(0), out.stride(0), GLU_ACTS[act],
                                    1 if interleaved else 0, dtype_code(x.dtype), _stream())
     _lib.check(rc, "fb_glu_act")
@@ -498,7 +505,7 @@ def embedding(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor | None =
     ids32 = ids.reshape(-1).to(torch.int32)
     M, H = ids32.numel(), table.shape[1]
     if out is None:
-        out = torch.empty((M, H), device=table.device, dtype=table.dtype)
+        out = table.new_empty((M, H))
     rc = _lib.kernels().fb_embedding(_ptr(ids32), _ptr(table), _ptr(out), M, H, table.shape[0], _stream())
     _lib.check(rc, "fb_embedding")
     return out.reshape(*ids.shape, H)
@@ -515,8 +522,8 @@ def argmax(logits: torch.Tensor, id_offset: int = 0, want_values: bool = False, 
         return (i, v) if want_values else i
     l2 = logits.reshape(-1, logits.shape[-1])
     M, V = l2.shape
-    ids = out if out is not None else torch.empty((M,), device=logits.device, dtype=torch.int32)
-    vals = torch.empty((M,), device=logits.device, dtype=torch.float32) if want_values else None
+    ids = out if out is not None else logits.new_empty((M,), dtype=torch.int32)
+    vals = logits.new_empty((M,), dtype=torch.float32) if want_values else None
     kind = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[logits.dtype]
     rc = _lib.kernels().fb_argmax(_ptr(l2), _ptr(ids), _ptr(vals), M, V, l2.stride(0), id_offset, kind, _stream())
     _lib.check(rc, "fb_argmax")

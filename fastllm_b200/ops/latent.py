@@ -323,7 +323,7 @@ def post(lw, proj, fb, pool, rope, eps: float):
 def _latent_queries(lw, q, positions, rope):
     """Queries [n, heads * hd] -> [n, heads, ld]: multiplied into the latent space, rotated parts turned."""
     n, H = q.shape[0], lw.heads
-    q_lat = torch.empty((n, H, lw.ld), device=q.device, dtype=q.dtype)
+    q_lat = q.new_empty((n, H, lw.ld))
     B.linear_batched(q, lw.w_uk_t, H, lw.hd, q_lat.view(n, H * lw.ld), lw.ld)
     if lw.rd:
         S.rope_heads(q[:, lw.dim:], lw.hd, q_lat.view(n, H * lw.ld)[:, lw.lv:], lw.ld, H, lw.rot, lw.rd, positions, *rope, lw.neox)
@@ -339,7 +339,7 @@ def _absorbed(lw, q, gate, head_gate, pool, page_table, kv_lens, out, positions,
                                        head_gate=head_gate[i:j] if head_gate is not None else None)
         o_lat = part(0, n) if n <= _MAX_MLA_ROWS else torch.cat([part(i, i + _MAX_MLA_ROWS) for i in range(0, n, _MAX_MLA_ROWS)])
     else:
-        o_lat = torch.empty((n, H, lw.lv), device=q.device, dtype=q.dtype)
+        o_lat = q.new_empty((n, H, lw.lv))
         rc = _lib.kernels().fb_latent_attn32(_ptr(q_lat), _ptr(pool), _ptr(o_lat), _ptr(page_table), _ptr(kv_lens), n, H, lw.ld, lw.lv, lw.ld,
                                              page_table.stride(0), pool.shape[1], lw.window, lw.scale, _ptr(head_gate), S.act_code(q.dtype), _stream())
         _lib.check(rc, "fb_latent_attn32")
@@ -358,7 +358,7 @@ def _folded(lw, q, pool, keys: int, slots, out, positions, rope):
         m = min(n, i + step) - i
         q_lat = _latent_queries(lw, q[i:i + m], positions[i:i + m], rope)
         s = B.linear(q_lat.view(m * H, lw.ld), rows, out_f32=True)
-        p = torch.empty((m * H, cols), device=q.device, dtype=q.dtype)
+        p = q.new_empty((m * H, cols))
         rc = lib.fb_softmax_causal_rows(_ptr(s), cols, _ptr(p), cols, m * H, cols, H, keys - n + i, lw.scale, dt, _stream())
         _lib.check(rc, "fb_softmax_causal_rows")
         B.linear_batched(B.linear(p, values).view(m, H * lw.lv), lw.w_uv, H, lw.lv, out[i:i + m], lw.vdim)
@@ -403,12 +403,12 @@ def attention(lw, proj, pool, fb, q=None, head_gate=None, rope=None):
     gate = proj[:, lw.gate_col:lw.gate_col + H * lw.vdim] if lw.gate == "elem" else None
     if not proj.is_cuda:
         return attention_ref(lw, q, gate, pool, fb, head_gate, rope)
-    out = torch.empty((T, H * lw.vdim), device=proj.device, dtype=proj.dtype)
+    out = proj.new_empty((T, H * lw.vdim))
     pl = _plan(fb, lw, pool.shape[1], expand_ok(lw, proj.dtype) and not fb.is_decode)
     if pl.n_rows and pl.rows is None:
         _absorbed(lw, q, gate, head_gate, pool, pl.page_table, pl.kv_lens, out, fb.positions, rope)
     elif pl.n_rows:
-        part = torch.empty((pl.n_rows, H * lw.vdim), device=proj.device, dtype=proj.dtype)
+        part = proj.new_empty((pl.n_rows, H * lw.vdim))
         pick = lambda t: t.index_select(0, pl.rows) if t is not None else None
         _absorbed(lw, pick(q), pick(gate), pick(head_gate), pool, pl.page_table, pl.kv_lens, part, pick(fb.positions), rope)
         out.index_copy_(0, pl.rows, part)

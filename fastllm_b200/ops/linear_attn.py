@@ -231,7 +231,7 @@ def gated_delta_decode(mixed, a, b, z, A_log, dt_bias, norm_w, eps, rec_state, s
     B = mixed.shape[0]
     if (mixed.is_cuda and mixed.dtype in (torch.float16, torch.bfloat16) and Dk == 128 and Dv == 128 and Hv % Hk == 0
             and rec_state.dtype == torch.float32 and a.dtype == mixed.dtype and z.dtype == mixed.dtype):
-        out = torch.empty((B, Hv * Dv), device=mixed.device, dtype=mixed.dtype)
+        out = mixed.new_empty((B, Hv * Dv))
         rc = _lib.kernels().fb_gdn_recurrent(_ptr(mixed), mixed.stride(0), _ptr(a), a.stride(0), _ptr(b), _ptr(z), _ptr(A_log),
                                              _ptr(dt_bias), _ptr(norm_w), _ptr(rec_state), _ptr(slots_dev), _ptr(out), B, Hk, Hv, Dk, Dv,
                                              z.stride(0), float(eps), dtype_code(mixed.dtype), _stream())

@@ -55,8 +55,8 @@ def route_topk(logits, bias, topk, score_mode, renorm, n_group=1, topk_group=1, 
     lg = logits.float()
     lg = lg if lg.stride(1) == 1 else lg.contiguous()
     M, E = lg.shape
-    idx = torch.empty((M, topk), device=lg.device, dtype=torch.int32)
-    w = torch.empty((M, topk), device=lg.device, dtype=torch.float32)
+    idx = lg.new_empty((M, topk), dtype=torch.int32)
+    w = lg.new_empty((M, topk), dtype=torch.float32)
     b = bias.float().contiguous() if bias is not None else None
     rc = _lib.kernels().fb_route_topk(_ptr(lg), _ptr(b), _ptr(idx), _ptr(w), M, E, topk, score_mode, 1 if renorm else 0,
                                       n_group, topk_group, float(route_scale), lg.stride(0), 1 if group_max else 0, _stream())
@@ -83,8 +83,8 @@ def route_fused(x, router_16, bias, topk, score_mode, renorm, route_scale=1.0):
     """``route_topk(x @ router^T, ...)`` as one kernel: (expert index int32 ``[M, topk]``, weight fp32 ``[M, topk]``)."""
     M, K = x.shape
     E = router_16.shape[0]
-    idx = torch.empty((M, topk), device=x.device, dtype=torch.int32)
-    w = torch.empty((M, topk), device=x.device, dtype=torch.float32)
+    idx = x.new_empty((M, topk), dtype=torch.int32)
+    w = x.new_empty((M, topk), dtype=torch.float32)
     b = bias.float().contiguous() if bias is not None else None
     rc = _lib.kernels().fb_gemm_route(_ptr(x), _ptr(router_16), M, E, K, x.stride(0), K, 1 if x.dtype == torch.bfloat16 else 0, _ptr(b),
                                       _ptr(idx), _ptr(w), topk, score_mode, 1 if renorm else 0, float(route_scale), _stream())
@@ -394,7 +394,7 @@ def mla_paged_attention(q_full, lat_pool, fb, scale, lora, select=None):
             Lp = (L + 63) // 64 * 64
             latp = lat16[:Lp] if lat16.shape[0] >= Lp else torch.cat([lat16, lat16.new_zeros(Lp - lat16.shape[0], Dq)])
             s = B.linear(q_full[q0:q1].reshape(nq * H, Dq), latp.contiguous(), out_f32=True).view(nq, H, Lp)
-            p = torch.empty((nq * H, Lp), device=s.device, dtype=q_full.dtype)
+            p = s.new_empty((nq * H, Lp), dtype=q_full.dtype)
             rc = _lib.kernels().fb_softmax_causal_rows(_ptr(s), Lp, _ptr(p), Lp, nq * H, Lp, H, L - nq, float(scale),
                                                        B.dtype_code(q_full.dtype), _stream())
             _lib.check(rc, "fb_softmax_causal_rows")

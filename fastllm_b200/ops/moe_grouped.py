@@ -149,9 +149,8 @@ def prepare_model(m) -> None:
 def _make_plan(idx, experts):
     """(counts, offsets, pos, total) of the pairs ``idx`` [T, top] (``fb_moe_plan``)."""
     T, topk = idx.shape
-    dev, E = idx.device, experts.stacked.n_local
-    counts, offsets = torch.empty(E, device=dev, dtype=torch.int32), torch.empty(E, device=dev, dtype=torch.int32)
-    pos, total = torch.empty((T, topk), device=dev, dtype=torch.int32), torch.empty(1, device=dev, dtype=torch.int32)
+    E = experts.stacked.n_local
+    counts, offsets, pos, total = (idx.new_empty(shape, dtype=torch.int32) for shape in (E, E, (T, topk), 1))
     idx = idx.contiguous()
     _lib.check(_lib.kernels().fb_moe_plan(_ptr(idx), T, topk, experts.first, E, _ptr(counts), _ptr(offsets), _ptr(pos), _ptr(total), PAD, _stream()), "fb_moe_plan")
     return counts, offsets, pos, total
@@ -164,7 +163,7 @@ def _forward32(x, st, plan, experts, wts, rows32):
     counts, offsets, pos, _ = plan
     T, H = x.shape
     topk = pos.shape[1]
-    xs = torch.empty((T * topk + st.n_local * PAD + 128, H), device=x.device, dtype=x.dtype)
+    xs = x.new_empty((T * topk + st.n_local * PAD + 128, H))
     if rows32 is not None:
         moe_gather_scaled(rows32, pos, wts, xs)
     else:
@@ -213,23 +212,23 @@ def forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, experts, add:
     int_a8 = QG.INT_A8 and (st.kind == "int8" or (st.kind == "int4g" and st.group == 128)) and H % 128 == 0 and st.inter % 128 == 0
     if int_a8 and st.a8 is None:
         _prepare_a8(st, experts)
-    act = torch.empty((rows_cap, st.inter), device=dev, dtype=x.dtype)
-    ys = torch.empty((rows_cap, H), device=dev, dtype=x.dtype)
+    act = x.new_empty((rows_cap, st.inter))
+    ys = x.new_empty((rows_cap, H))
     if fp8_native:
         # gather fused with the e4m3 quantisation of the rows (the 16-bit sorted copy is never materialised)
         ld_a = (rows_cap + 128 + 3) // 4 * 4
-        xq = torch.empty((rows_cap, H), device=dev, dtype=torch.uint8)
-        sa = torch.empty((H // 128, ld_a), device=dev, dtype=torch.float32)
+        xq = x.new_empty((rows_cap, H), dtype=torch.uint8)
+        sa = x.new_empty((H // 128, ld_a), dtype=torch.float32)
         _lib.check(lib.fb_moe_gather_quant_fp8(_ptr(x.contiguous()), _ptr(pos), _ptr(xq), _ptr(sa), ld_a, T, topk, H, dt, s),
                    "fb_moe_gather_quant_fp8")
     elif int_a8:
         # gather fused with the int8 quantisation of the rows
         xq, sa, sx, ld_a = QG.quant_act_i8(x.contiguous(), pos=pos, topk=topk, rows_cap=rows_cap)
     elif rows32 is not None:
-        xs = torch.empty((rows_cap, H), device=dev, dtype=x.dtype)
+        xs = x.new_empty((rows_cap, H))
         moe_gather_scaled(rows32, pos, wts, xs)
     else:
-        xs = torch.empty((rows_cap, H), device=dev, dtype=x.dtype)
+        xs = x.new_empty((rows_cap, H))
         _lib.check(lib.fb_moe_gather(_ptr(x.contiguous()), _ptr(pos), _ptr(xs), T, topk, H, s), "fb_moe_gather")
     if st.kind == "dense":
         clamp, plain = experts.act == "gptoss", experts.act == "gelu"
@@ -279,7 +278,7 @@ def forward(x: torch.Tensor, idx: torch.Tensor, wts: torch.Tensor, experts, add:
                    "fb_moe_grouped_gemm_quant(down)")
     if not combine:
         return ys, pos, wts
-    out = torch.empty((T, H), device=dev, dtype=x.dtype)
+    out = x.new_empty((T, H))
     if add is not None and not (add.is_contiguous() and add.dtype == x.dtype):
         add = add.to(x.dtype).contiguous()
     _lib.check(lib.fb_moe_combine_gated(_ptr(ys), _ptr(pos), _ptr(wts), _ptr(add), _ptr(add_gate), add_gate.stride(0) if add_gate is not None else 0, _ptr(out), T,

@@ -56,9 +56,9 @@ def quant_act_i8(x2: torch.Tensor, rows_used=None, pos=None, topk: int = 1, rows
     M, K = x2.shape
     rows = rows_cap if rows_cap is not None else M
     ld_a = (rows + 128 + 3) // 4 * 4
-    xq = torch.empty((rows, K), device=x2.device, dtype=torch.int8)
-    sa = torch.empty((K // 128, ld_a), device=x2.device, dtype=torch.float32)
-    xs = torch.empty((K // 128, ld_a), device=x2.device, dtype=torch.float32)
+    xq = x2.new_empty((rows, K), dtype=torch.int8)
+    sa = x2.new_empty((K // 128, ld_a), dtype=torch.float32)
+    xs = x2.new_empty((K // 128, ld_a), dtype=torch.float32)
     n = M * topk if pos is not None else M
     rc = _lib.kernels().fb_quant_act_i8(_ptr(x2), x2.stride(0), _ptr(xq), K, _ptr(sa), _ptr(xs), ld_a, n, K, dtype_code(x2.dtype),
                                         _ptr(rows_used), _ptr(pos), topk, _stream())
@@ -71,7 +71,7 @@ def round_act(x: torch.Tensor, mode: int) -> torch.Tensor:
     x2 = x.reshape(-1, x.shape[-1])
     if x2.stride(-1) != 1 or x2.stride(0) % 4 != 0:
         x2 = x2.contiguous()
-    out = torch.empty((x2.shape[0], x2.shape[1]), device=x.device, dtype=x.dtype)
+    out = x.new_empty((x2.shape[0], x2.shape[1]))
     rc = _lib.kernels().fb_round_act(_ptr(x2), x2.stride(0), _ptr(out), out.stride(0), x2.shape[0], x2.shape[1], dtype_code(x.dtype), mode,
                                      _stream())
     _lib.check(rc, "fb_round_act")
@@ -142,8 +142,8 @@ def quant_act_fp8(x2: torch.Tensor, rows_used: torch.Tensor | None = None):
     """x ``[M, K]`` 16-bit -> (e4m3 ``[M, K]``, scales fp32 ``[K / 128, ld_a]`` with ``ld_a >= M + 128``, multiple of 4)."""
     M, K = x2.shape
     ld_a = (M + 128 + 3) // 4 * 4
-    xq = torch.empty((M, K), device=x2.device, dtype=torch.uint8)
-    sa = torch.empty((K // 128, ld_a), device=x2.device, dtype=torch.float32)
+    xq = x2.new_empty((M, K), dtype=torch.uint8)
+    sa = x2.new_empty((K // 128, ld_a), dtype=torch.float32)
     rc = _lib.kernels().fb_quant_act_fp8(_ptr(x2), x2.stride(0), _ptr(xq), K, _ptr(sa), ld_a, M, K, dtype_code(x2.dtype), _ptr(rows_used),
                                          _stream())
     _lib.check(rc, "fb_quant_act_fp8")
@@ -206,7 +206,7 @@ def linear_quant(x, lw, residual=None, swiglu=False, out_f32=False):
     a8 = uses_int_a8(lw) and M <= INT_A8_MAX_M[lw.kind] and x2.stride(0) % 4 == 0
     scale, zero = (None, None) if a8 else _kernel_tensors(lw)[:2]
     n_out = N // 2 if swiglu else N
-    out = torch.empty((M, n_out), device=x.device, dtype=torch.float32 if out_f32 else x.dtype)
+    out = x.new_empty((M, n_out), dtype=torch.float32 if out_f32 else x.dtype)
     res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
     flags = (GEMM_BIAS if lw.bias is not None else 0) | (GEMM_RESIDUAL if residual is not None else 0) | \
             (GEMM_SWIGLU if swiglu else 0) | (GEMM_OUT_F32 if out_f32 else 0)
