@@ -27,6 +27,10 @@ FB_DEFINE_ERROR_API(gemm)
 #include "gemm_smallm.cuh"
 #include "gemm_largem.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_mid.cuh"
+
+#include <algorithm>
+#include <atomic>
 
 namespace fb {
 
@@ -77,6 +81,13 @@ template <bool BF16, bool EXTRA>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const GemmParams p, int tiles_m, int tiles_n, const GemmExtra ex) {
   gemm_pair_device<BF16, LargeMPlainHook, EXTRA>(tmX, tmW, p, tiles_m, tiles_n, LargeMPlainHook{}, ex);
+}
+
+template <bool BF16>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MidCfg::THREADS, 1)
+gemm_mid_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2, const GemmParams p,
+                const MidPlan pl) {
+  gemm_mid_device<BF16>(tmW, tmX1, tmX2, p, pl);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -445,6 +456,128 @@ static int gemm_16bit_impl(const void* X, const void* W, void* out, const void* 
   if (bn == 256)
     return (int)(bf16 ? launch_largem<256, true>(tmX, tmW, p, stream, ex) : launch_largem<256, false>(tmX, tmW, p, stream, ex));
   return (int)(bf16 ? launch_largem<128, true>(tmX, tmW, p, stream, ex) : launch_largem<128, false>(tmX, tmW, p, stream, ex));
+}
+
+// Split of a product of M rows over `tok_tiles` token tiles and the pairs of `sms` SMs; false where the kernel does not take it.
+static bool mid_plan(int M, int N, int K, int tok_tiles, int sms, fb::MidPlan& pl) {
+  if (M <= 0 || N <= 0 || K % 8 != 0 || N % 8 != 0 || tok_tiles <= 0) return false;
+  const int kb = (K + 63) / 64, pairs = sms / 2;
+  const int nt = ((M + tok_tiles - 1) / tok_tiles + 31) / 32 * 32;
+  if (nt > 512 || kb <= 0 || pairs <= 0) return false;
+  pl.nt1 = nt <= 256 ? nt : (nt / 2 + 31) / 32 * 32;
+  pl.nt2 = nt - pl.nt1;
+  pl.tok_tiles = (M + nt - 1) / nt;
+  pl.row_tiles = (N + 255) / 256;
+  const long long tiles = (long long)pl.tok_tiles * pl.row_tiles;
+  if (tiles > (1 << 20)) return false;
+  pl.rest = (int)(tiles % pairs);
+  pl.full = (int)tiles - pl.rest;
+  pl.splits = pl.rest ? std::min(std::min(pairs / pl.rest, 8), kb / 8) : 1;      // at least 8 k blocks a split
+  if (pl.splits <= 1) { pl.full = (int)tiles; pl.rest = 0; pl.splits = 1; }
+  pl.stages = std::min((int)fb::MidCfg::MAX_STAGES, (int)fb::MidCfg::PIPE_BYTES / (fb::MidCfg::A_BYTES + nt * 64));
+  return true;
+}
+
+static int sm_count_of_device() {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Bytes of workspace that fb_gemm_16bit_mid needs (16-byte aligned; its contents are of no matter), -1 where it does not take the product.
+extern "C" int fb_gemm_mid_workspace(int M, int N, int K, int tok_tiles, int sms) {
+  fb::MidPlan pl;
+  if (!mid_plan(M, N, K, tok_tiles, sms > 0 ? sms : sm_count_of_device(), pl)) return -1;
+  const long long nt = pl.nt1 + pl.nt2;
+  return (int)((long long)pl.rest * pl.splits * 2 * nt * 128 * 4 + (long long)pl.rest * 2 * pl.splits * pl.splits * 8);      // (40 MB at most)
+}
+
+// Token tiles with which fb_gemm_16bit_mid is the fastest kernel for a product of M rows; 0: another one is.  Both sides' times in us, fitted to
+// measurements of 12 weight shapes (2048 .. 28672 features, k of 2048 .. 14336) at 48 .. 2000 rows on 148 SMs (rms 7 %; 10 % for the other kernels).  Up to 64
+// rows the small-M kernel streams weights as fast and starts sooner (28672 x 4096 at 48 rows: 43 against 47 us).  Measured, other kernel -> this one:
+// 28672 x 4096 at 140 / 256 / 333 rows 71 / 79 / 87 -> 51 / 60 / 74; 16384 x 2048 at 140 / 333 rows 24 / 29 -> 19 / 26; 4096 x 14336 at 170 rows
+// 34.5 -> 31.6; 2048 x 8192 at 96 / 256 rows 23 / 35 -> 17 / 20; 4096 x 4096 at 200 rows stays (18.6 against 19.9).
+extern "C" int fb_gemm_mid_pick(int M, int N, int K, int sms) {
+  if (M <= 64 || M > 2048 || N < 2048 || K <= 0) return 0;      // (what was measured)
+  if (sms <= 0) sms = sm_count_of_device();
+  if (sms < 2) return 0;
+  const int kb = (K + 63) / 64;
+  double other;
+  if (M <= 256) {
+    const int tiles = (N + 127) / 128, occ = M <= 128 && tiles > sms ? 2 : 1, s = fb_gemm_pick_split(M, N, K, sms * occ);
+    const double kbs = occ == 2 ? std::max(1.0, (double)tiles * s / (2 * sms)) * kb / s * 2 : (double)((tiles * s + sms - 1) / sms) * kb / s;
+    other = M <= 128 ? 6.7 + 0.372 * kbs + (s == 8 ? 9.4 : 0.0) : 9.0 + 0.528 * kbs + (s == 8 ? 12.8 : 0.0);
+    if (M <= 128 && s < 8) return 0;             // nearly the same weight stream; eight splits cost the small-M kernel more than its loads
+  } else {
+    int bn = (N >= 256 && N % 256 == 0) || N > 2048 ? 256 : 128;
+    if (bn == 256 && (long long)((N + 255) / 256) * ((M + 127) / 128) < sms) bn = 128;
+    const long long one = (long long)((N + bn - 1) / bn) * ((M + 127) / 128), two = (long long)((N + 255) / 256) * ((M + 255) / 256);
+    if (pair_is_faster(M, N, bn, sms)) other = 8.7 + 0.338 * kb * ((two + sms / 2 - 1) / (sms / 2));
+    else other = 6.0 + (bn == 256 ? 0.425 : 0.228) * kb * ((one + sms - 1) / sms);
+  }
+  int best = 0;
+  double best_us = other / 1.05;
+  for (int tt = 1; tt <= 4; ++tt) {
+    fb::MidPlan pl;
+    if (!mid_plan(M, N, K, tt, sms, pl)) continue;
+    if (M > 256 && pl.rest) continue;            // more than 256 rows: one sum in one order whatever the batch, as the other kernels give it
+    const int nt = pl.nt1 + pl.nt2, rounds = (pl.full + sms / 2 - 1) / (sms / 2);
+    const double kbs = (double)rounds * kb + (pl.rest ? (double)kb / pl.splits : 0.0);
+    const double us = 5.3 + kbs * std::max(0.287, 0.161 + 0.001 * nt) + 0.0143 * nt * (nt > 256 ? rounds : std::min(rounds, 1)) + (pl.rest ? 2.8 + 0.0227 * nt : 0.0);
+    if (us < best_us) { best = tt; best_us = us; }
+  }
+  return best;
+}
+
+// Y = X W^T for a few hundred rows (gemm_mid.cuh): `tok_tiles` tiles of at most 512 rows each.  Flags as for fb_gemm_16bit but for the less common epilogues.
+extern "C" int fb_gemm_16bit_mid(const void* X, const void* W, void* out, const void* bias, const void* residual, int M, int N, int K, int ldx, int ldw,
+                                 int ld_out, int ld_res, int dtype, int flags, int tok_tiles, void* workspace, long long ws_bytes, void* stream_) {
+  using namespace fb;
+  if (M <= 0 || N <= 0) return 0;
+  if ((dtype != 0 && dtype != 1) || (flags & GEMM_EXTRA_FLAGS) || ((flags & GEMM_SWIGLU) && (N % 128 != 0))) return -1;
+  MidPlan pl;
+  const int sms = sm_count_of_device();
+  if (!mid_plan(M, N, K, tok_tiles, sms, pl)) return -1;
+  const long long need = fb_gemm_mid_workspace(M, N, K, tok_tiles, sms);
+  if (need > 0 && (workspace == nullptr || ws_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15))) return -1;
+  pl.part = reinterpret_cast<float*>(workspace);
+  const int used = pl.rest * pl.splits;
+  pl.flags = reinterpret_cast<unsigned long long*>(pl.part + (size_t)used * 2 * (pl.nt1 + pl.nt2) * 128);
+  // an odd multiple of a large odd number: differs in every launch of a process, and memory that held something else does not hold it by chance
+  static std::atomic<unsigned long long> launches{0};
+  pl.tag = (2 * launches.fetch_add(1, std::memory_order_relaxed) + 1) * 0x9E3779B97F4A7C15ull;
+  GemmParams p;
+  p.out = out; p.bias = bias; p.residual = residual;
+  p.M = M; p.N = N; p.K = K; p.ld_out = ld_out; p.ld_res = ld_res;
+  p.kb_total = (K + 63) / 64; p.kb_per_split = p.kb_total;
+  p.flags = flags;
+  p.scatter_tp = 0; p.scatter_rows = 1; p.scatter_rank = 0; p.w_row0 = 0; p.x_row0 = 0;
+  for (int i = 0; i < 8; ++i) p.scatter_out[i] = nullptr;
+  const uint32_t f = dtype == 1 ? 1u : 0u;
+  pl.idesc1 = make_idesc(f, f, 0, 0, 256, pl.nt1);
+  pl.idesc2 = pl.nt2 ? make_idesc(f, f, 0, 0, 256, pl.nt2) : 0u;
+  CUtensorMap tmW, tmX1, tmX2;
+  if (!make_tmap_2d(&tmW, W, N, K, ldw, 128, 64, 2, 3)) return -2;
+  if (!make_tmap_2d(&tmX1, X, M, K, ldx, pl.nt1 / 2, 64, 2, 3)) return -2;
+  tmX2 = tmX1;
+  if (pl.nt2 && !make_tmap_2d(&tmX2, X, M, K, ldx, pl.nt2 / 2, 64, 2, 3)) return -2;
+  auto kern = dtype == 1 ? gemm_mid_kernel<true> : gemm_mid_kernel<false>;
+  static DeviceOnce configured[2];
+  if (configured[dtype].need()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MidCfg::SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+  }
+  cudaLaunchConfig_t cfg = {};
+  const int pairs = pl.full >= sms / 2 ? sms / 2 : std::max(pl.full, pl.rest ? used : 0);
+  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.blockDim = dim3(MidCfg::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = MidCfg::SMEM_BYTES;
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream_);
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = add_pdl_attr(attr, 0);
+  return (int)cudaLaunchKernelEx(&cfg, kern, tmW, tmX1, tmX2, p, pl);
 }
 
 // Same, for activations that a fused collective broadcast without waiting for its peers (small-M path only): the kernel

@@ -123,102 +123,108 @@ struct SmallMCfg {
   static constexpr int TMEM_COLS = MPAD < 32 ? 32 : MPAD;
 };
 
+// Epilogue of four neighbouring columns c.. of the 128-wide tile n_tile, row j: bias -> activation -> factors -> residual -> store / scatter.
+// SwiGLU and its kin: `acc` holds gate columns (c < 64), `acc2` the up columns that belong to them.
+template <bool BF16, bool EXTRA = false>
+__device__ __forceinline__ void smallm_finish(const GemmParams& p, int j, int n_tile, int c, float4 acc, float4 acc2, const GemmExtra& ex = GemmExtra()) {
+  const bool swiglu = (p.flags & GEMM_SWIGLU) != 0;
+  int n_out;
+  if (swiglu) {
+    n_out = n_tile * 64 + c;
+    if (p.flags & GEMM_BIAS) {
+      const uint32_t* bg = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.bias) + n_tile * 128 + c);
+      float2 b0 = unpack_16<BF16>(bg[0]), b1 = unpack_16<BF16>(bg[1]);
+      float2 u0 = unpack_16<BF16>(bg[32]), u1 = unpack_16<BF16>(bg[33]);
+      acc.x += b0.x; acc.y += b0.y; acc.z += b1.x; acc.w += b1.y;
+      acc2.x += u0.x; acc2.y += u0.y; acc2.z += u1.x; acc2.w += u1.y;
+    }
+    if (p.flags & GEMM_GLU_CLAMP) {
+      acc.x = glu_clamp_f(acc.x, acc2.x, p.act_limit, p.act_alpha); acc.y = glu_clamp_f(acc.y, acc2.y, p.act_limit, p.act_alpha);
+      acc.z = glu_clamp_f(acc.z, acc2.z, p.act_limit, p.act_alpha); acc.w = glu_clamp_f(acc.w, acc2.w, p.act_limit, p.act_alpha);
+    } else if (EXTRA && (p.flags & GEMM_GEGLU)) {
+      acc.x = gelu_tanh_f(acc.x) * acc2.x; acc.y = gelu_tanh_f(acc.y) * acc2.y;
+      acc.z = gelu_tanh_f(acc.z) * acc2.z; acc.w = gelu_tanh_f(acc.w) * acc2.w;
+    } else {
+      acc.x = silu_f(acc.x) * acc2.x; acc.y = silu_f(acc.y) * acc2.y;
+      acc.z = silu_f(acc.z) * acc2.z; acc.w = silu_f(acc.w) * acc2.w;
+    }
+    if (n_out >= (p.N >> 1)) return;
+  } else {
+    n_out = n_tile * 128 + c;
+    if (n_out >= p.N) return;
+    if (p.flags & GEMM_BIAS) {
+      const uint32_t* bp = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.bias) + n_out);
+      float2 b0 = unpack_16<BF16>(bp[0]), b1 = unpack_16<BF16>(bp[1]);
+      acc.x += b0.x; acc.y += b0.y; acc.z += b1.x; acc.w += b1.y;
+    }
+  }
+  if (p.flags & GEMM_RELU2) { acc.x = relu2_f(acc.x); acc.y = relu2_f(acc.y); acc.z = relu2_f(acc.z); acc.w = relu2_f(acc.w); }
+  if (EXTRA && (p.flags & GEMM_GELU)) { acc.x = gelu_erf_f(acc.x); acc.y = gelu_erf_f(acc.y); acc.z = gelu_erf_f(acc.z); acc.w = gelu_erf_f(acc.w); }
+  if (EXTRA && (p.flags & GEMM_GELU_TANH)) { acc.x = gelu_tanh_f(acc.x); acc.y = gelu_tanh_f(acc.y); acc.z = gelu_tanh_f(acc.z); acc.w = gelu_tanh_f(acc.w); }
+  if (EXTRA && ex.row_gate != nullptr) {
+    const float g = sigmoid_f(ex.row_gate[(size_t)j * ex.ld_row_gate]);
+    acc.x *= g; acc.y *= g; acc.z *= g; acc.w *= g;
+  }
+  if (EXTRA && ex.mul != nullptr) {
+    const uint2 mv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(ex.mul) + (size_t)clamp_row(ex.mul_rows[j], ex.mul_count) * ex.ld_mul + n_out);
+    const float2 m0 = unpack_16<BF16>(mv.x), m1 = unpack_16<BF16>(mv.y);
+    acc.x *= m0.x; acc.y *= m0.y; acc.z *= m1.x; acc.w *= m1.y;
+  }
+  if (p.gate != nullptr) {
+    const uint2 gv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.gate) + (size_t)j * p.ld_gate +
+                                                     (size_t)blockIdx.z * (size_t)p.batch_out_cols + n_out);
+    const float2 g0 = unpack_16<BF16>(gv.x), g1 = unpack_16<BF16>(gv.y);
+    acc.x *= sigmoid_f(g0.x); acc.y *= sigmoid_f(g0.y); acc.z *= sigmoid_f(g1.x); acc.w *= sigmoid_f(g1.y);
+  }
+  if ((p.flags & GEMM_RESIDUAL) && (p.flags & GEMM_RES_F32)) {
+    const float4 rv = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.residual) + (size_t)j * p.ld_res + n_out);
+    acc.x = rv.x + p.alpha * acc.x; acc.y = rv.y + p.alpha * acc.y; acc.z = rv.z + p.alpha * acc.z; acc.w = rv.w + p.alpha * acc.w;
+  } else if (p.flags & GEMM_RESIDUAL) {
+    const uint2 rv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.residual) + (size_t)j * p.ld_res + n_out);
+    float2 r0 = unpack_16<BF16>(rv.x), r1 = unpack_16<BF16>(rv.y);
+    acc.x += r0.x; acc.y += r0.y; acc.z += r1.x; acc.w += r1.y;
+  }
+  const size_t zo = (size_t)blockIdx.z * (size_t)p.batch_out_cols;
+  if (p.scatter_tp > 0) {
+    float* dst = p.scatter_out[j / p.scatter_rows] + ((size_t)p.scatter_rank * p.M + j) * p.ld_out + n_out;
+    *reinterpret_cast<float4*>(dst) = acc;
+  } else if (p.flags & GEMM_OUT_F32) {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)j * p.ld_out + zo + n_out) = acc;
+    if (EXTRA && ex.out16 != nullptr)
+      *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(ex.out16) + (size_t)j * ex.ld_out16 + n_out) =
+          make_uint2(pack_16<BF16>(acc.x, acc.y), pack_16<BF16>(acc.z, acc.w));
+  } else {
+    uint2 o;
+    o.x = pack_16<BF16>(acc.x, acc.y);
+    o.y = pack_16<BF16>(acc.z, acc.w);
+    *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)j * p.ld_out + zo + n_out) = o;
+  }
+}
+
 // Cross-CTA reduction over the k splits + epilogue.  Every CTA of the cluster holds its fp32 partial tile P[token][n]
-// at `smem`; this CTA reduces and stores its own column slice (bias -> SwiGLU -> residual -> store / scatter).
+// at `smem`; this CTA reduces and stores its own column slice.
 template <bool BF16, bool EXTRA = false>
 __device__ __forceinline__ void smallm_reduce_store(const GemmParams& p, uint8_t* smem, int split, int nsplit, int n_tile, const GemmExtra& ex = GemmExtra()) {
-  {
-    const bool swiglu = (p.flags & GEMM_SWIGLU) != 0;
-    const int outw = swiglu ? 64 : 128;
-    const int per = outw / nsplit;           // columns owned by this CTA (>= 8)
-    const int vec_per_row = per >> 2;
-    const int items = p.M * vec_per_row;
-    const uint32_t P_addr = smem_u32(smem);
-    for (int it = threadIdx.x; it < items; it += blockDim.x) {
-      const int j = it / vec_per_row;
-      const int c = split * per + (it - j * vec_per_row) * 4;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = acc;
-      for (int s = 0; s < nsplit; ++s) {
-        const uint32_t ra = mapa_u32(P_addr + (uint32_t)(j * 128 + c) * 4u, (uint32_t)s);
-        float4 v = ld_dsmem_f4(ra);
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        if (swiglu) {
-          float4 u = ld_dsmem_f4(ra + 64 * 4);
-          acc2.x += u.x; acc2.y += u.y; acc2.z += u.z; acc2.w += u.w;
-        }
-      }
-      int n_out;
+  const bool swiglu = (p.flags & GEMM_SWIGLU) != 0;
+  const int outw = swiglu ? 64 : 128;
+  const int per = outw / nsplit;           // columns owned by this CTA (>= 8)
+  const int vec_per_row = per >> 2;
+  const int items = p.M * vec_per_row;
+  const uint32_t P_addr = smem_u32(smem);
+  for (int it = threadIdx.x; it < items; it += blockDim.x) {
+    const int j = it / vec_per_row;
+    const int c = split * per + (it - j * vec_per_row) * 4;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), acc2 = acc;
+    for (int s = 0; s < nsplit; ++s) {
+      const uint32_t ra = mapa_u32(P_addr + (uint32_t)(j * 128 + c) * 4u, (uint32_t)s);
+      float4 v = ld_dsmem_f4(ra);
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
       if (swiglu) {
-        n_out = n_tile * 64 + c;
-        if (p.flags & GEMM_BIAS) {
-          const uint32_t* bg = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.bias) + n_tile * 128 + c);
-          float2 b0 = unpack_16<BF16>(bg[0]), b1 = unpack_16<BF16>(bg[1]);
-          float2 u0 = unpack_16<BF16>(bg[32]), u1 = unpack_16<BF16>(bg[33]);
-          acc.x += b0.x; acc.y += b0.y; acc.z += b1.x; acc.w += b1.y;
-          acc2.x += u0.x; acc2.y += u0.y; acc2.z += u1.x; acc2.w += u1.y;
-        }
-        if (p.flags & GEMM_GLU_CLAMP) {
-          acc.x = glu_clamp_f(acc.x, acc2.x, p.act_limit, p.act_alpha); acc.y = glu_clamp_f(acc.y, acc2.y, p.act_limit, p.act_alpha);
-          acc.z = glu_clamp_f(acc.z, acc2.z, p.act_limit, p.act_alpha); acc.w = glu_clamp_f(acc.w, acc2.w, p.act_limit, p.act_alpha);
-        } else if (EXTRA && (p.flags & GEMM_GEGLU)) {
-          acc.x = gelu_tanh_f(acc.x) * acc2.x; acc.y = gelu_tanh_f(acc.y) * acc2.y;
-          acc.z = gelu_tanh_f(acc.z) * acc2.z; acc.w = gelu_tanh_f(acc.w) * acc2.w;
-        } else {
-          acc.x = silu_f(acc.x) * acc2.x; acc.y = silu_f(acc.y) * acc2.y;
-          acc.z = silu_f(acc.z) * acc2.z; acc.w = silu_f(acc.w) * acc2.w;
-        }
-        if (n_out >= (p.N >> 1)) continue;
-      } else {
-        n_out = n_tile * 128 + c;
-        if (n_out >= p.N) continue;
-        if (p.flags & GEMM_BIAS) {
-          const uint32_t* bp = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(p.bias) + n_out);
-          float2 b0 = unpack_16<BF16>(bp[0]), b1 = unpack_16<BF16>(bp[1]);
-          acc.x += b0.x; acc.y += b0.y; acc.z += b1.x; acc.w += b1.y;
-        }
-      }
-      if (p.flags & GEMM_RELU2) { acc.x = relu2_f(acc.x); acc.y = relu2_f(acc.y); acc.z = relu2_f(acc.z); acc.w = relu2_f(acc.w); }
-      if (EXTRA && (p.flags & GEMM_GELU)) { acc.x = gelu_erf_f(acc.x); acc.y = gelu_erf_f(acc.y); acc.z = gelu_erf_f(acc.z); acc.w = gelu_erf_f(acc.w); }
-      if (EXTRA && (p.flags & GEMM_GELU_TANH)) { acc.x = gelu_tanh_f(acc.x); acc.y = gelu_tanh_f(acc.y); acc.z = gelu_tanh_f(acc.z); acc.w = gelu_tanh_f(acc.w); }
-      if (EXTRA && ex.row_gate != nullptr) {
-        const float g = sigmoid_f(ex.row_gate[(size_t)j * ex.ld_row_gate]);
-        acc.x *= g; acc.y *= g; acc.z *= g; acc.w *= g;
-      }
-      if (EXTRA && ex.mul != nullptr) {
-        const uint2 mv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(ex.mul) + (size_t)clamp_row(ex.mul_rows[j], ex.mul_count) * ex.ld_mul + n_out);
-        const float2 m0 = unpack_16<BF16>(mv.x), m1 = unpack_16<BF16>(mv.y);
-        acc.x *= m0.x; acc.y *= m0.y; acc.z *= m1.x; acc.w *= m1.y;
-      }
-      if (p.gate != nullptr) {
-        const uint2 gv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.gate) + (size_t)j * p.ld_gate +
-                                                         (size_t)blockIdx.z * (size_t)p.batch_out_cols + n_out);
-        const float2 g0 = unpack_16<BF16>(gv.x), g1 = unpack_16<BF16>(gv.y);
-        acc.x *= sigmoid_f(g0.x); acc.y *= sigmoid_f(g0.y); acc.z *= sigmoid_f(g1.x); acc.w *= sigmoid_f(g1.y);
-      }
-      if ((p.flags & GEMM_RESIDUAL) && (p.flags & GEMM_RES_F32)) {
-        const float4 rv = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.residual) + (size_t)j * p.ld_res + n_out);
-        acc.x = rv.x + p.alpha * acc.x; acc.y = rv.y + p.alpha * acc.y; acc.z = rv.z + p.alpha * acc.z; acc.w = rv.w + p.alpha * acc.w;
-      } else if (p.flags & GEMM_RESIDUAL) {
-        const uint2 rv = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(p.residual) + (size_t)j * p.ld_res + n_out);
-        float2 r0 = unpack_16<BF16>(rv.x), r1 = unpack_16<BF16>(rv.y);
-        acc.x += r0.x; acc.y += r0.y; acc.z += r1.x; acc.w += r1.y;
-      }
-      const size_t zo = (size_t)blockIdx.z * (size_t)p.batch_out_cols;
-      if (p.scatter_tp > 0) {
-        float* dst = p.scatter_out[j / p.scatter_rows] + ((size_t)p.scatter_rank * p.M + j) * p.ld_out + n_out;
-        *reinterpret_cast<float4*>(dst) = acc;
-      } else if (p.flags & GEMM_OUT_F32) {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + (size_t)j * p.ld_out + zo + n_out) = acc;
-        if (EXTRA && ex.out16 != nullptr)
-          *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(ex.out16) + (size_t)j * ex.ld_out16 + n_out) =
-              make_uint2(pack_16<BF16>(acc.x, acc.y), pack_16<BF16>(acc.z, acc.w));
-      } else {
-        uint2 o;
-        o.x = pack_16<BF16>(acc.x, acc.y);
-        o.y = pack_16<BF16>(acc.z, acc.w);
-        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(p.out) + (size_t)j * p.ld_out + zo + n_out) = o;
+        float4 u = ld_dsmem_f4(ra + 64 * 4);
+        acc2.x += u.x; acc2.y += u.y; acc2.z += u.z; acc2.w += u.w;
       }
     }
+    smallm_finish<BF16, EXTRA>(p, j, n_tile, c, acc, acc2, ex);
   }
 }
 

@@ -26,6 +26,9 @@ LL = c_longlong
 _KERNEL_SIGS = {
     "fb_gemm_16bit": [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P],
     "fb_gemm_16bit_wait": [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, P, P],
+    "fb_gemm_16bit_mid": [P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, P, LL, P],
+    "fb_gemm_mid_workspace": [I, I, I, I, I],
+    "fb_gemm_mid_pick": [I, I, I, I],
     "fb_gemm_qkv_post": [P, P, P, I, I, I, I, I, I, P, P, P, I, P, P, P, P, P, P, P, P, I, I, I, I, F, F, P],
     "fb_gemm_route": [P, P, I, I, I, I, I, I, P, P, P, I, I, I, F, P],
     "fb_gemm_16bit_batched": [P, P, P, I, I, I, I, I, I, I, I, I, I, P],
@@ -143,7 +146,7 @@ class _KernelProxy:
         if c is not None:
             return c
         fn = getattr(self._lib, name)
-        if not name.startswith("fb_") or name.endswith("_read_error") or name == "fb_gemm_pick_split":
+        if not name.startswith("fb_") or name.endswith("_read_error") or name in ("fb_gemm_pick_split", "fb_gemm_mid_pick", "fb_gemm_mid_workspace"):
             self._cache[name] = fn
             return fn
         n = _LAUNCHES_PER_CALL.get(name, 1)

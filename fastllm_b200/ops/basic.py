@@ -8,6 +8,7 @@ b[k]) -> y[n,k]`` with weights stored ``[out, in]`` row-major.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -247,6 +248,15 @@ def linear_act(x, w, act: str, out=None, row_gate=None, mul=None, mul_rows=None)
     return out
 
 
+@functools.lru_cache(maxsize=8192)
+def _mid_plan(M: int, N: int, K: int, device: int):
+    """(token tiles, workspace bytes) of the kernel for a few hundred rows; (0, 0) where another one is faster."""
+    lib = _lib.kernels()
+    tiles = lib.fb_gemm_mid_pick(M, N, K, 0)
+    need = lib.fb_gemm_mid_workspace(M, N, K, tiles, 0) if tiles > 0 else -1
+    return (tiles, need) if need >= 0 else (0, 0)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, swiglu: bool = False, interleaved: bool = True,
            out_f32: bool = False, out: torch.Tensor | None = None, nsplit: int = 0, relu2: bool = False, geglu: bool = False) -> torch.Tensor:
     """``y = x @ w.T`` with optional fused bias, SwiGLU (``w`` = gate/up stacked; ``geglu``: tanh-form GELU in place of SiLU, 16-bit CUDA
@@ -306,7 +316,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias=None, residual=None, swiglu: b
     res2 = residual if residual is None or residual.dim() == 2 else residual.reshape(-1, residual.shape[-1])
     lib = _lib.kernels()
     dt = dtype_code(x.dtype)
-    if M <= 256 or N % 32 != 0:
+    tiles, need = _mid_plan(M, N, K, x.device.index) if 64 < M <= 2048 and nsplit == 0 and not geglu and _pending_wait is None else (0, 0)
+    if tiles:
+        ws = torch.empty((need,), device=x.device, dtype=torch.uint8) if need else None
+        rc = lib.fb_gemm_16bit_mid(_ptr(x2), _ptr(w), _ptr(out), _ptr(bias), _ptr(res2), M, N, K, x2.stride(0), w.stride(0), out.stride(0),
+                                   res2.stride(0) if res2 is not None else 0, dt, flags, tiles, _ptr(ws), need, _stream())
+        _lib.check(rc, "fb_gemm_16bit_mid")
+    elif M <= 256 or N % 32 != 0:
         step = 256
         pend = _take_pending_wait()
         if M <= step and pend is None:
