@@ -26,8 +26,9 @@ _lib.register_sigs({
     "fb_moe_gather_quant_fp8": [P, P, P, P, I, I, I, I, I, P],
     "fb_quant_act_i8": [P, I, P, I, P, P, I, I, I, I, P, P, I, P],
     "fb_gemm_i8": [P, I, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, P, P, I, I, I, P],
+    "fb_gemm_i4_rows": [P, I, P, P, I, P, P, P, P, P, I, I, I, I, I, I, I, P],
     "fb_gemv_i4": [P, I, P, P, I, P, P, P, I, I, I, I, I, I, P, P, I, P],
-}, ["gemm_fp8", "gemm_i8"])
+}, ["gemm_fp8", "gemm_i8", "gemm_i4_rows"])
 
 _QMODE = {"int8": 1, "int4g": 2, "fp8": 3, "fp4": 4}
 # FP8 weights run as W8A8 (activations quantised per token and 128-wide k block, e4m3 x e4m3 on the tensor core) for decode-sized
@@ -96,8 +97,8 @@ def prepare(lw) -> None:
         _a8_tensors(lw)
 
 
-I4_GEMV = os.environ.get("FB_I4_GEMV", "1") != "0"      # int4-group weights at one to four rows: dp4a kernel (csrc/gemv_i4.cu)
-I4_GEMV_MAX_M = 4
+I4_GEMV = os.environ.get("FB_I4_GEMV", "1") != "0"      # int4-group weights at about one row a matrix: dp4a kernel (csrc/gemv_i4.cu)
+I4_ROWS_MAX_M = 32
 
 
 def _a8_tensors(lw):
@@ -122,13 +123,20 @@ def _linear_i8(x2, lw, out, bias, res2, flags, pre=None):
         _, xq, sa, xs, ld_a = pre              # quantised by the kernel that produced x (fused RMSNorm)
     else:
         xq, sa, xs, ld_a = quant_act_i8(x2)
-    if (kind == 2 and M <= I4_GEMV_MAX_M and I4_GEMV and bias is None and res2 is None and (flags & ~GEMM_SWIGLU) == 0
+    if (kind == 2 and M == 1 and lw.n >= 16384 and I4_GEMV and bias is None and res2 is None and (flags & ~GEMM_SWIGLU) == 0
             and lw.n % 128 == 0 and K <= 16384 and lw.group == 128 and out.dtype == x2.dtype):
-        # one to four rows: the CUDA-core dp4a kernel streams the packed rows directly (no unpack / MMA / promotion pipeline)
+        # one row and many weight rows: the CUDA-core dp4a kernel (28672 x 4096 14.1 us against 15.3 below; 2 rows 16.3 against 15.3, 6144 x 4096 10.6 against 4.7)
         rc = _lib.kernels().fb_gemv_i4(_ptr(xq), K, _ptr(sa), _ptr(xs), ld_a, _ptr(w), _ptr(sc), _ptr(out), M, lw.n, K, out.stride(0),
                                        dtype_code(x2.dtype), flags, _ptr(None), _ptr(None), 1, _stream())
         _lib.check(rc, "fb_gemv_i4")
         return
+    if kind == 2 and M <= I4_ROWS_MAX_M:
+        # few rows: warp-level products on weights in registers; -1 where the tcgen05 route is faster or alone fits
+        rc = _lib.kernels().fb_gemm_i4_rows(_ptr(xq), K, _ptr(sa), _ptr(xs), ld_a, _ptr(w), _ptr(sc), _ptr(out), _ptr(bias), _ptr(res2), M, lw.n, K, out.stride(0),
+                                            res2.stride(0) if res2 is not None else 0, dtype_code(x2.dtype), flags, _stream())
+        if rc != -1:
+            _lib.check(rc, "fb_gemm_i4_rows")
+            return
     for m0 in range(0, M, 128):           # the kernel takes up to 128 rows; the weights of later chunks come from L2
         m1 = min(M, m0 + 128)
         rc = _lib.kernels().fb_gemm_i8(_ptr(xq[m0:m1]), K, _ptr(sa[:, m0:]), _ptr(xs[:, m0:]), ld_a, _ptr(w), _ptr(sc), _ptr(zr),
