@@ -254,13 +254,18 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 // Second-generation kernel: two query heads of one KV head per CTA, half-page (64-token) KV steps.
 //
 // Both heads read the same K / V tiles (loaded once), and their softmax runs on two separate warp groups, so the tensor
-// core alternates between the heads: while head B's probabilities are being formed it computes P_A * V and the next
-// Q_A * K^T, and vice versa.  TMEM holds S_A, S_B (64 columns each) and O_A, O_B (128 each).  A softmax thread owns one
-// query row and keeps the step's 64 logits in registers (one TMEM read per step).
-//   shared memory: Q_A, Q_B 64 KB | 3-stage ring of (K, V) half pages 96 KB | P_A, P_B 32 KB
+// core alternates between the heads.  TMEM holds two S tiles a head (64 columns each) and O_A, O_B (128 each): the logits of a
+// step are there when the softmax of the step before ends, so that a softmax group waits for no product.  A softmax thread owns
+// one query row and keeps the step's 64 logits in registers (one TMEM read per step).
+//   shared memory: Q_A, Q_B 64 KB | 4-stage ring of (K, V) half pages 128 KB | P_A, P_B 32 KB
+//
+// Bound: the softmax warps (64 exponentials a row and step are 1024 cycles of the special-function unit for both heads; the products of a step
+// take 1024, too).  The accumulator is rescaled only when a row's maximum has grown by more than 8 (a factor 256) since it was last rescaled: the
+// exponentials are then at most 256, which keeps their relative precision, and the sum carries the same factor.
 // ---------------------------------------------------------------------------------------------------
 constexpr int AP2_KV = 64;
-constexpr int AP2_STAGES = 3;
+constexpr int AP2_STAGES = 4;
+constexpr float AP2_GROWTH = 8.f;                 // log2 of the factor that the exponentials may exceed 1 by
 constexpr int AP2_KT = AP2_KV * 128 * 2;          // 16 KB: 64 rows x 128 values, two 8 KB halves (64 dims each)
 constexpr int AP2_PT = 128 * AP2_KV * 2;          // 16 KB: 128 query rows x 64 probabilities
 constexpr int AP2_SMEM_BYTES = 2 * AP_TILE + AP2_STAGES * 2 * AP2_KT + 2 * AP2_PT + 256 + 1024;
@@ -279,10 +284,10 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   uint64_t* full_v = bars + AP2_STAGES;
   uint64_t* empty = bars + 2 * AP2_STAGES;
   uint64_t* q_full = bars + 3 * AP2_STAGES;
-  uint64_t* s_full = q_full + 1;      // [2]
-  uint64_t* p_ready = q_full + 3;     // [2]
-  uint64_t* o_full = q_full + 5;      // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 7);
+  uint64_t* s_full = q_full + 1;      // [2 heads][2 tiles]
+  uint64_t* p_ready = q_full + 5;     // [2]
+  uint64_t* o_full = q_full + 7;      // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_full + 9);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // grid: x = head pair (fast), y = query block; the host lists the blocks longest-first, so CTAs are handed out heaviest
@@ -301,7 +306,7 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < AP2_STAGES; ++s) { mbar_init(&full_k[s], 1); mbar_init(&full_v[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(q_full, 1);
-    for (int h = 0; h < 2; ++h) { mbar_init(&s_full[h], 1); mbar_init(&p_ready[h], 128); mbar_init(&o_full[h], 1); }
+    for (int h = 0; h < 2; ++h) { mbar_init(&s_full[2 * h], 1); mbar_init(&s_full[2 * h + 1], 1); mbar_init(&p_ready[h], 128); mbar_init(&o_full[h], 1); }
     mbar_init_fence();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -310,7 +315,7 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem0 = *tmem_slot;
-  // columns: S_A [0,64) S_B [64,128) O_A [128,256) O_B [256,384)
+  // columns: S_A [0,64) [64,128), S_B [128,192) [192,256), O_A [256,384), O_B [384,512)
 
   if (warp == 0) {
     if (elect_one()) {
@@ -340,28 +345,29 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     if (elect_one()) {
       bool ok = n_steps > 0 && mbar_wait(q_full, 0, dead, KID_ATTN_PREFILL, 12);
       const uint32_t qb = smem_u32(q_smem), pb = smem_u32(p_smem);
-      auto issue_s = [&](int h, uint32_t kb) {
+      auto issue_s = [&](int h, int it) {
+        const uint32_t kb = smem_u32(kv_smem + (it % AP2_STAGES) * 2 * AP2_KT);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint64_t da = make_smem_desc(qb + h * AP_TILE + (k >> 2) * (AP_TILE / 2) + (k & 3) * 32, 16, 1024, SWZ_128B);
           const uint64_t db = make_smem_desc(kb + (k >> 2) * (AP2_KT / 2) + (k & 3) * 32, 16, 1024, SWZ_128B);
-          umma_f16(tmem0 + (uint32_t)(h * 64), da, db, p.idesc_s, k != 0 ? 1u : 0u);
+          umma_f16(tmem0 + (uint32_t)(h * 128 + (it & 1) * 64), da, db, p.idesc_s, k != 0 ? 1u : 0u);
         }
-        umma_commit(&s_full[h]);
+        umma_commit(&s_full[2 * h + (it & 1)]);
       };
-      if (ok) ok = mbar_wait(&full_k[0], 0, dead, KID_ATTN_PREFILL, 13);
-      if (ok) {
+      for (int it = 0; ok && it < 2 && it < n_steps; ++it) {
+        ok = mbar_wait(&full_k[it], 0, dead, KID_ATTN_PREFILL, 13);
+        if (!ok) break;
         tc_fence_after_sync();
-        issue_s(0, smem_u32(kv_smem));
-        issue_s(1, smem_u32(kv_smem));
+        issue_s(0, it);
+        issue_s(1, it);
       }
       for (int it = 0; ok && it < n_steps; ++it) {
-        const int s = it % AP2_STAGES, s1 = (it + 1) % AP2_STAGES;
-        const uint32_t ph = (uint32_t)(it / AP2_STAGES) & 1u, ph1 = (uint32_t)((it + 1) / AP2_STAGES) & 1u;
+        const int s = it % AP2_STAGES, s2 = (it + 2) % AP2_STAGES;
+        const uint32_t ph = (uint32_t)(it / AP2_STAGES) & 1u, ph2 = (uint32_t)((it + 2) / AP2_STAGES) & 1u;
         const uint32_t iph = (uint32_t)it & 1u;
         const uint32_t vb = smem_u32(kv_smem + s * 2 * AP2_KT) + AP2_KT;
-        const uint32_t kb1 = smem_u32(kv_smem + s1 * 2 * AP2_KT);
-        const bool more = it + 1 < n_steps;
+        const bool more = it + 2 < n_steps;
         for (int h = 0; h < 2; ++h) {
           if (!mbar_wait(&p_ready[h], iph, dead, KID_ATTN_PREFILL, 14)) { ok = false; break; }
           if (h == 0 && !mbar_wait(&full_v[s], ph, dead, KID_ATTN_PREFILL, 15)) { ok = false; break; }
@@ -371,13 +377,14 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int k = 0; k < 4; ++k) {
             const uint64_t da = make_smem_desc(pb + h * AP2_PT + k * 32, 16, 1024, SWZ_128B);
             const uint64_t db = make_smem_desc(vb + k * 2048, AP2_KT / 2, 1024, SWZ_128B);
-            umma_f16(tmem0 + 128u + (uint32_t)(h * 128), da, db, p.idesc_o, (it | k) != 0 ? 1u : 0u);
+            umma_f16(tmem0 + 256u + (uint32_t)(h * 128), da, db, p.idesc_o, (it | k) != 0 ? 1u : 0u);
           }
           umma_commit(&o_full[h]);
           if (more) {
-            if (h == 0 && !mbar_wait(&full_k[s1], ph1, dead, KID_ATTN_PREFILL, 16)) { ok = false; break; }
+            // (this head's softmax has read the tile that is overwritten: it arrived at p_ready)
+            if (h == 0 && !mbar_wait(&full_k[s2], ph2, dead, KID_ATTN_PREFILL, 16)) { ok = false; break; }
             tc_fence_after_sync();
-            issue_s(h, kb1);
+            issue_s(h, it + 2);
           }
         }
         if (ok) umma_commit(&empty[s]);
@@ -390,12 +397,13 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int r = q * 32 + lane;
     const int pos = pos0 + r;
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    const uint32_t tmem_s = tmem0 + (uint32_t)(h * 64), tmem_o = tmem0 + 128u + (uint32_t)(h * 128);
+    const uint32_t tmem_o = tmem0 + 256u + (uint32_t)(h * 128);
     uint8_t* prow = p_smem + h * AP2_PT + r * 128;
     float m_run = -INFINITY, l_run = 0.f;
     for (int it = 0; it < n_steps; ++it) {
       const uint32_t iph = (uint32_t)it & 1u;
-      mbar_wait(&s_full[h], iph, dead, KID_ATTN_PREFILL, 17);
+      const uint32_t tmem_s = tmem0 + (uint32_t)(h * 128 + (it & 1) * 64);
+      mbar_wait(&s_full[2 * h + (it & 1)], (uint32_t)(it >> 1) & 1u, dead, KID_ATTN_PREFILL, 17);
       tc_fence_after_sync();
       const int kv0 = it * AP2_KV;
       uint32_t sreg[64];
@@ -406,27 +414,29 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // causal diagonal of this block (or the end of the cache) pay for the mask; kv0 + 63 <= pos0 means every row of
       // the block sees the whole step.
       const bool full_step = kv0 + AP2_KV - 1 <= pos0 && kv0 + AP2_KV <= kv_len;
-      float m_raw = -INFINITY;
+      float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};      // four chains: a single one of 64 would be waited for
       if (full_step) {
 #pragma unroll
-        for (int j = 0; j < 64; ++j) m_raw = fmaxf(m_raw, __uint_as_float(sreg[j]));
+        for (int j = 0; j < 64; ++j) m4[j & 3] = fmaxf(m4[j & 3], __uint_as_float(sreg[j]));
       } else {
 #pragma unroll
         for (int j = 0; j < 64; ++j) {
           const int kv = kv0 + j;
           const float sv = (kv <= pos && kv < kv_len) ? __uint_as_float(sreg[j]) : -INFINITY;
           sreg[j] = __float_as_uint(sv);
-          m_raw = fmaxf(m_raw, sv);
+          m4[j & 3] = fmaxf(m4[j & 3], sv);
         }
       }
+      const float m_raw = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       const float m_new = fmaxf(m_run, m_raw * p.scale_log2);          // scale > 0: the maximum commutes with it
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      const float alpha = exp2f(m_run - m_use);
       if (it > 0) {
         // the previous P * V of this head must be complete before P is overwritten or O is rescaled
         mbar_wait(&o_full[h], iph ^ 1u, dead, KID_ATTN_PREFILL, 18);
         tc_fence_after_sync();
-        if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+      }
+      if (__any_sync(0xffffffffu, !(m_new <= m_run + AP2_GROWTH))) {
+        const float alpha = exp2f(m_run - (m_new == -INFINITY ? 0.f : m_new));
+        if (it > 0) {
 #pragma unroll 1
           for (int c0 = 0; c0 < 128; c0 += 32) {
             uint32_t oreg[32];
@@ -438,22 +448,29 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
           tmem_st_wait();
         }
+        l_run *= alpha;
+        m_run = m_new;
       }
-      float l_add = 0.f;
+      const float m_use = m_run == -INFINITY ? 0.f : m_run;
+      const uint64_t sc2 = pack_f32x2(p.scale_log2, p.scale_log2), m2 = pack_f32x2(-m_use, -m_use);
+      uint64_t l2[4] = {0ull, 0ull, 0ull, 0ull};
 #pragma unroll
       for (int g = 0; g < 8; ++g) {
         uint32_t pk[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sreg[8 * g + 2 * j]), p.scale_log2, -m_use));
-          const float p1 = exp2f(fmaf(__uint_as_float(sreg[8 * g + 2 * j + 1]), p.scale_log2, -m_use));
+          float p0, p1;
+          unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sreg[8 * g + 2 * j]), __uint_as_float(sreg[8 * g + 2 * j + 1])), sc2, m2), p0, p1);
+          p0 = exp2f(p0);
+          p1 = exp2f(p1);
           pk[j] = pack_16<BF16>(p0, p1);
-          l_add += p0 + p1;
+          l2[j] = add_f32x2(l2[j], pack_f32x2(p0, p1));
         }
         *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
-      l_run = l_run * alpha + l_add;
-      m_run = m_new;
+      float l_a, l_b;
+      unpack_f32x2(add_f32x2(add_f32x2(l2[0], l2[1]), add_f32x2(l2[2], l2[3])), l_a, l_b);
+      l_run += l_a + l_b;
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(&p_ready[h]);

@@ -395,6 +395,7 @@ __device__ __forceinline__ uint32_t pack_f16(float a, float b) {
 __device__ __forceinline__ uint64_t pack_f32x2(float a, float b) { uint64_t v; asm("mov.b64 %0, {%1, %2};\n" : "=l"(v) : "f"(a), "f"(b)); return v; }
 __device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(a), "=f"(b) : "l"(v)); }
 __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) { uint64_t v; asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(v) : "l"(a), "l"(b)); return v; }
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) { uint64_t v; asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(v) : "l"(a), "l"(b)); return v; }
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t v;
   asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(v) : "l"(a), "l"(b), "l"(c));
