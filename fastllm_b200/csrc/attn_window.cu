@@ -84,13 +84,18 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* bars = reinterpret_cast<uint64_t*>(p_smem + 2 * AW_PT);
   uint64_t* full_k = bars;                                  // [4]
   uint64_t* full_v = bars + 4;
-  uint64_t* empty = bars + 8;
-  uint64_t* q_full = bars + 12;
-  uint64_t* s_full = bars + 13;       // [2]
-  uint64_t* p_ready = bars + 15;      // [2]
-  uint64_t* o_full = bars + 17;       // [2]
-  uint64_t* v_clean = bars + 19;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t* empty_k = bars + 8;
+  uint64_t* empty_v = bars + 12;
+  uint64_t* q_full = bars + 16;
+  uint64_t* s_full = bars + 17;       // [2 blocks][2 tiles]
+  uint64_t* p_ready = bars + 21;      // [2]
+  uint64_t* o_full = bars + 23;       // [2]
+  uint64_t* v_clean = bars + 25;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
+  // Plain softmax and values of at most 128: tensor memory holds two score tiles a block, and the scores of a step are there when the softmax of the step
+  // before ends (1 x 4000 latent prompt, see launch_window).
+  const bool two_s = !EXT && vt <= 2;
+  const int ahead = two_s ? 2 : 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x, kv_head = head / p.group;
@@ -123,10 +128,10 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   bool dead = false;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) { mbar_init(&full_k[s], 1); mbar_init(&full_v[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < stages; ++s) { mbar_init(&full_k[s], 1); mbar_init(&full_v[s], 1); mbar_init(&empty_k[s], 1); mbar_init(&empty_v[s], 1); }
     mbar_init(q_full, 1);
     mbar_init(v_clean, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(&s_full[b], 1); mbar_init(&p_ready[b], 128); mbar_init(&o_full[b], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&s_full[2 * b], 1); mbar_init(&s_full[2 * b + 1], 1); mbar_init(&p_ready[b], 128); mbar_init(&o_full[b], 1); }
     mbar_init_fence();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -135,8 +140,11 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem0 = *tmem_slot;
-  // columns: S_0 [0,64) S_1 [64,128) O_0 [128, 128 + 64 vt) O_1 behind it
-  const uint32_t o_cols = (uint32_t)(vt * 64);
+  // columns: S_0, S_1 (one tile of 64 or two each), then O_0 and O_1 of 64 vt
+  const uint32_t o_cols = (uint32_t)(vt * 64), tmem_o0 = tmem0 + (two_s ? 256u : 128u);
+  auto s_tile = [&](int b, int n) { return tmem0 + (uint32_t)(two_s ? b * 128 + (n & 1) * 64 : b * 64); };      // scores of block b's n-th step,
+  auto s_bar = [&](int b, int n) { return &s_full[2 * b + (two_s ? n & 1 : 0)]; };                              // their barrier and its phase
+  auto s_phase = [&](int n) { return (uint32_t)(two_s ? n >> 1 : n) & 1u; };
 
   if (warp == 0) {
     if (elect_one()) {
@@ -145,24 +153,32 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int b = 0; b < nb; ++b)
         for (int j = 0; j < dt; ++j)
           tma_load_3d(q_smem + (b * dt + j) * AW_QT, j < own ? &tmQ : &tmQr, q_full, (j < own ? j : j - own) * 64, head, q_row0 + b * 128);
-      for (int it = 0; it < n_steps; ++it) {
-        const int s = it % stages;
-        const uint32_t ph = (uint32_t)(it / stages) & 1u;
-        if (!mbar_wait(&empty[s], ph ^ 1u, dead, KID_ATTN_WINDOW, 1)) break;
+      auto row_of = [&](int it) {
         const int key = step_key(it);
-        int row = key_row0 + (key - key0);
-        if (p.page_table != nullptr) {
-          int page = (key >> 7) < p.max_pages ? p.page_table[(size_t)blk[5] * p.max_pages + (key >> 7)] : 0;
-          if ((unsigned)page >= (unsigned)p.num_pages) { report_error(ERR_BAD_ARG, KID_ATTN_WINDOW, 20); page = 0; }
-          row = page * 128 + (key & 127);
-        }
+        if (p.page_table == nullptr) return key_row0 + (key - key0);
+        int page = (key >> 7) < p.max_pages ? p.page_table[(size_t)blk[5] * p.max_pages + (key >> 7)] : 0;
+        if ((unsigned)page >= (unsigned)p.num_pages) { report_error(ERR_BAD_ARG, KID_ATTN_WINDOW, 20); page = 0; }
+        return page * 128 + (key & 127);
+      };
+      auto load_k = [&](int it) {
+        const int s = it % stages, row = row_of(it);
+        if (!mbar_wait(&empty_k[s], ((uint32_t)(it / stages) & 1u) ^ 1u, dead, KID_ATTN_WINDOW, 1)) return;
         uint8_t* ks = kv_smem + s * stage_bytes;
-        uint8_t* vb = ks + dt * AW_KT;
         mbar_expect_tx(&full_k[s], dt * AW_KT);
         for (int j = 0; j < own; ++j) tma_load_3d(ks + j * AW_KT, &tmK, &full_k[s], j * 64, kv_head, row);
         for (int j = own; j < dt; ++j) tma_load_3d(ks + j * AW_KT, &tmKr, &full_k[s], (j - own) * 64, 0, row);
+      };
+      auto load_v = [&](int it) {
+        const int s = it % stages, row = row_of(it);
+        if (!mbar_wait(&empty_v[s], ((uint32_t)(it / stages) & 1u) ^ 1u, dead, KID_ATTN_WINDOW, 13)) return;
         mbar_expect_tx(&full_v[s], vt * AW_KT);
-        for (int j = 0; j < vt; ++j) tma_load_3d(vb + j * AW_KT, &tmV, &full_v[s], j * 64, kv_head, row);
+        for (int j = 0; j < vt; ++j) tma_load_3d(kv_smem + s * stage_bytes + (dt + j) * AW_KT, &tmV, &full_v[s], j * 64, kv_head, row);
+      };
+      // keys are needed a step before values and their slots are free earlier
+      if (n_steps > 0) load_k(0);
+      for (int it = 0; it < n_steps && !dead; ++it) {
+        if (it + 1 < n_steps) load_k(it + 1);
+        load_v(it);
       }
     }
     __syncwarp();
@@ -180,26 +196,29 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (elect_one()) {
       const uint32_t qb = smem_u32(q_smem), pb = smem_u32(p_smem);
       const int ks = (p.D + 15) / 16, kr = 4 * own, kre = kr + (p.R + 15) / 16;       // 16-wide k steps of the S product: [0, ks) and [kr, kre)
-      auto issue_s = [&](int b, uint32_t kb) {
+      auto issue_s = [&](int b, int it) {
+        const uint32_t kb = smem_u32(kv_smem + (it % stages) * stage_bytes);
+        const int n = order(b, it);
         for (int k = 0; k < kre; k = k + 1 == ks ? kr : k + 1) {
           const uint64_t da = make_smem_desc(qb + (b * dt + (k >> 2)) * AW_QT + (k & 3) * 32, 16, 1024, SWZ_128B);
           const uint64_t db = make_smem_desc(kb + (k >> 2) * AW_KT + (k & 3) * 32, 16, 1024, SWZ_128B);
-          umma_f16(tmem0 + (uint32_t)(b * 64), da, db, p.idesc_s, k != 0 ? 1u : 0u);
+          umma_f16(s_tile(b, n), da, db, p.idesc_s, k != 0 ? 1u : 0u);
         }
-        umma_commit(&s_full[b]);
+        umma_commit(s_bar(b, n));
       };
       bool ok = mbar_wait(q_full, 0, dead, KID_ATTN_WINDOW, 2);
-      if (ok) ok = mbar_wait(&full_k[0], 0, dead, KID_ATTN_WINDOW, 3);
-      if (ok) {
+      for (int it = 0; ok && it < ahead && it < n_steps; ++it) {
+        ok = mbar_wait(&full_k[it], 0, dead, KID_ATTN_WINDOW, 3);
+        if (!ok) break;
         tc_fence_after_sync();
         for (int b = 0; b < 2; ++b)
-          if (takes(b, 0)) issue_s(b, smem_u32(kv_smem));
+          if (takes(b, it)) issue_s(b, it);
+        umma_commit(&empty_k[it]);
       }
       for (int it = 0; ok && it < n_steps; ++it) {
-        const int s = it % stages, s1 = (it + 1) % stages;
-        const uint32_t ph = (uint32_t)(it / stages) & 1u, ph1 = (uint32_t)((it + 1) / stages) & 1u;
+        const int s = it % stages, s1 = (it + ahead) % stages;
+        const uint32_t ph = (uint32_t)(it / stages) & 1u, ph1 = (uint32_t)((it + ahead) / stages) & 1u;
         const uint32_t vb = smem_u32(kv_smem + s * stage_bytes + dt * AW_KT);
-        const uint32_t kb1 = smem_u32(kv_smem + s1 * stage_bytes);
         bool have_v = false, have_k1 = false;
         for (int b = 0; b < 2; ++b) {
           if (takes(b, it)) {
@@ -213,21 +232,26 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             for (int k = 0; k < 4; ++k) {
               const uint64_t da = make_smem_desc(pb + b * AW_PT + k * 32, 16, 1024, SWZ_128B);
               const uint64_t db = make_smem_desc(vb + k * 2048, AW_KT, 1024, SWZ_128B);
-              umma_f16(tmem0 + 128u + (uint32_t)b * o_cols, da, db, p.idesc_o, (order(b, it) != 0 || k != 0) ? 1u : 0u);
+              umma_f16(tmem_o0 + (uint32_t)b * o_cols, da, db, p.idesc_o, (order(b, it) != 0 || k != 0) ? 1u : 0u);
             }
             umma_commit(&o_full[b]);
           }
-          if (takes(b, it + 1)) {
+          // (the tile that is overwritten was read before this block's softmax arrived at p_ready two steps, or one, before)
+          if (it + ahead < n_steps && takes(b, it + ahead)) {
             if (!have_k1 && !mbar_wait(&full_k[s1], ph1, dead, KID_ATTN_WINDOW, 6)) { ok = false; break; }
             have_k1 = true;
             tc_fence_after_sync();
-            issue_s(b, kb1);
+            issue_s(b, it + ahead);
           }
+        }
+        if (ok && it + ahead < n_steps) {
+          if (!have_k1 && !mbar_wait(&full_k[s1], ph1, dead, KID_ATTN_WINDOW, 14)) break;
+          umma_commit(&empty_k[s1]);
         }
         if (ok) {
           // (a step no block used for V has its load outstanding: the slot may only be refilled once it has landed)
           if (!have_v && !mbar_wait(&full_v[s], ph, dead, KID_ATTN_WINDOW, 7)) break;
-          umma_commit(&empty[s]);
+          umma_commit(&empty_v[s]);
         }
       }
     }
@@ -239,14 +263,15 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const int pos_b = pos0 + b * 128, pos = pos_b + r;
     const int first = aw_first(p, pos), first_all = aw_first(p, pos_b + 127);      // of this row; no earlier than any row of the block's
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-    const uint32_t tmem_s = tmem0 + (uint32_t)(b * 64), tmem_o = tmem0 + 128u + (uint32_t)b * o_cols;
+    const uint32_t tmem_o = tmem_o0 + (uint32_t)b * o_cols;
     uint8_t* prow = p_smem + b * AW_PT + r * 128;
     const int cnt = (EXT ? kb[b] : 0) + e[b] - f[b];
     float m_run = -INFINITY, l_run = 0.f;
     const float bias = MODE == 2 ? p.score_bias[head] * 1.4426950408889634f : 0.f;
     for (int n = 0; n < cnt; ++n) {
       const uint32_t iph = (uint32_t)n & 1u;
-      mbar_wait(&s_full[b], iph, dead, KID_ATTN_WINDOW, 8);
+      const uint32_t tmem_s = s_tile(b, n);
+      mbar_wait(s_bar(b, n), s_phase(n), dead, KID_ATTN_WINDOW, 8);
       tc_fence_after_sync();
       const int kv0 = EXT ? step_key(n < kb[b] ? n : f[b] + n - kb[b]) : lo + (f[b] + n) * AW_KV;
       uint32_t sreg[64];
@@ -255,7 +280,6 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tmem_ld_wait();
       // only steps on the causal diagonal or on the window's edge pay for the mask
       const bool full_step = kv0 + AW_KV - 1 <= pos_b && (kv0 >= first_all || (EXT && kv0 + AW_KV <= p.keep));
-      float m_new = m_run;
       const bool cap = EXT && p.cap_in != 0.f;
       if (cap) {
         float am = 0.f;
@@ -312,12 +336,13 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_arrive(&p_ready[b]);
         continue;
       }
+      float m4[4] = {m_run, -INFINITY, -INFINITY, -INFINITY};      // four chains: a single one of 64 would be waited for
       if (full_step) {
 #pragma unroll
         for (int j = 0; j < 64; ++j) {
           const float sv = __uint_as_float(sreg[j]) * sc;
           sreg[j] = __float_as_uint(sv);
-          m_new = fmaxf(m_new, sv);
+          m4[j & 3] = fmaxf(m4[j & 3], sv);
         }
       } else {
 #pragma unroll
@@ -325,16 +350,20 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const int kv = kv0 + j;
           const float sv = (kv <= pos && (kv >= first || (EXT && kv < p.keep))) ? __uint_as_float(sreg[j]) * sc : -INFINITY;
           sreg[j] = __float_as_uint(sv);
-          m_new = fmaxf(m_new, sv);
+          m4[j & 3] = fmaxf(m4[j & 3], sv);
         }
       }
-      const float m_use = m_new == -INFINITY ? 0.f : m_new;
-      const float alpha = exp2f(m_run - m_use);
+      const float m_new = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       if (n > 0) {
         // the previous P * V of this block must be complete before P is overwritten or O is rescaled
         mbar_wait(&o_full[b], iph ^ 1u, dead, KID_ATTN_WINDOW, 9);
         tc_fence_after_sync();
-        if (__any_sync(0xffffffffu, alpha != 1.0f)) {
+      }
+      // Rescaled only where some row's maximum has grown by more than 8 since it last was: exponentials of up to 256 keep their relative precision,
+      // and the sum carries the same factor (some row of 32 has a new maximum in most steps).
+      if (__any_sync(0xffffffffu, !(m_new <= m_run + 8.f))) {
+        const float alpha = exp2f(m_run - (m_new == -INFINITY ? 0.f : m_new));
+        if (n > 0) {
 #pragma unroll 1
           for (int c0 = 0; c0 < (int)o_cols; c0 += 32) {
             uint32_t oreg[32];
@@ -346,8 +375,11 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           }
           tmem_st_wait();
         }
+        l_run *= alpha;
+        m_run = m_new;
       }
-      float l_add = 0.f;
+      const float m_use = m_run == -INFINITY ? 0.f : m_run;
+      float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int g = 0; g < 8; ++g) {
         uint32_t pk[4];
@@ -356,12 +388,11 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const float p0 = exp2f(__uint_as_float(sreg[8 * g + 2 * j]) - m_use);
           const float p1 = exp2f(__uint_as_float(sreg[8 * g + 2 * j + 1]) - m_use);
           pk[j] = pack_16<BF16>(p0, p1);
-          l_add += p0 + p1;
+          l4[j] += p0 + p1;
         }
         *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
-      l_run = l_run * alpha + l_add;
-      m_run = m_new;
+      l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(&p_ready[b]);
