@@ -88,6 +88,20 @@ def test_plan_on_many_blocks(T, topk, E, first, n_local):
         assert torch.equal(got.cpu().long(), w.long())
 
 
+# a CTA a place below 256 tokens, a CTA a token from there; rows narrower and wider than a CTA, places in and beside multiples of 4
+@pytest.mark.parametrize("T,H,topk", [(1, 8, 1), (255, 264, 5), (256, 2056, 3), (300, 2048, 8), (257, 4104, 10)])
+def test_rows_reach_their_places(T, H, topk):
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randint(-32768, 32767, (T, H), device=DEV, generator=g, dtype=torch.int16)
+    pos = torch.randperm(T * topk + 9, device=DEV, generator=g)[:T * topk].int()
+    pos[3::7] = -1                                                        # experts of another rank
+    xs = torch.full((T * topk + 9, H), 7, device=DEV, dtype=torch.int16)
+    want = xs.clone()
+    want[pos[pos >= 0].long()] = x.repeat_interleave(topk, dim=0)[pos >= 0]
+    assert _lib.kernels().fb_moe_gather(x.data_ptr(), pos.data_ptr(), xs.data_ptr(), T, topk, H, _stream()) == 0
+    assert torch.equal(xs, want)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("T,H,topk,ld", [(1, 8, 1, 1), (37, 264, 8, 13), (300, 4096, 3, 544)])
 def test_combine_with_gated_rows(T, H, topk, ld, dtype):
