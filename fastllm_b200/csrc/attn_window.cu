@@ -93,7 +93,7 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* v_clean = bars + 25;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   // Plain softmax and values of at most 128: tensor memory holds two score tiles a block, and the scores of a step are there when the softmax of the step
-  // before ends (1 x 4000 latent prompt, see launch_window).
+  // before ends (latent prompts of 2 x 2000 tokens, 16 heads of 192 + 128: 89 -> 81 us).
   const bool two_s = !EXT && vt <= 2;
   const int ahead = two_s ? 2 : 1;
 

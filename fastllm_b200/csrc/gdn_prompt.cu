@@ -7,7 +7,7 @@
 //     S <- e^(G_last) S + sum_t e^(G_last - G_t) k_t V'_t^T,     o_t = e^(G_t) q_t S + sum_(s <= t) e^(G_t - G_s) (q_t . k_s) V'_s
 //  * gdn_chunk_inverse_kernel  gates, norms and T of every (chunk, head), in parallel: K K^T on the tensor core, the unit lower-triangular
 //                              inverse by forward substitution, a column per thread in registers.
-//  * gdn_chunk_scan_kernel     the chain over the chunks.  Columns of the state never meet: two warps carry 16 of them through all chunks.
+//  * gdn_chunk_scan_kernel     the chain over the chunks.  Columns of the state never meet: four warps carry 16 of them through all chunks.
 //                              S^T stays in registers as accumulator fragments, which are operand fragments of the next product as they
 //                              are (the k index of both operands is permuted alike); the chunk's keys and T are fetched a chunk ahead.
 //  * gdn_chunk_out_kernel      outputs of every (chunk, head), in parallel, with the norm over the head and the gate in the epilogue.
@@ -15,10 +15,10 @@
 // fp32); an fp32 operand of the chain over bf16 keys enters as three bf16 terms, all 24 bits, elsewhere as two tf32 terms (22 bits; fp16 V' three).
 // Decays, norms, gates, T and the state are fp32.  The tensor core cuts its sums off instead of rounding them, which adds up where a state forgets
 // slowly: in the chain every product of 8 or 16 terms is summed by itself, smallest terms first, and added in fp32.  Error of the states against
-// 64 bits over 28 calls of 30 tokens and more: 0.12 to 1.12 of that of fp32 operators, 0.53 in the mean (two tf32 terms and running sums: 2.1 times where
+// 64 bits over 28 calls of 30 tokens and more: 0.11 to 1.12 of that of fp32 operators, 0.67 in the mean (two tf32 terms and running sums: 2.1 times where
 // little is forgotten).
 //
-// 4001 tokens x 32 heads, bf16: 0.54 ms a layer (convolution 56 us, T 61, chain 258, outputs 160); PyTorch operators took about 1500 launches and 12 ms.
+// 4001 tokens x 32 heads, bf16: 0.44 ms a layer (convolution 56 us, T 61, chain 198, outputs 126); PyTorch operators took about 1500 launches and 12 ms.
 #include "ptx.cuh"
 #include "launch.h"
 
@@ -46,8 +46,8 @@ struct GdnPromptParams {
   const int* reqs;                               // [n_reqs][4] = (first chunk, chunks, state slot, rows)
   float* inv;                                    // [units][64][64]; unit = chunk * Hn + head - h0
   float* vecs;                                   // [units][GP_VECS][64]
-  float* vnew;                                   // [units][128 v][64 t]
-  float* s0;                                     // [units][128 v][128 d]
+  float4* vnew;                                  // [units][8 blocks of 16 v][8 tiles of 8 t][32 lanes], as the accumulators hold them: (v, t), (v, t + 1),
+  float4* s0;                                    // (v + 8, t), (v + 8, t + 1) of v = lane / 4, t = 2 (lane % 4); [units][8][16 tiles of 8 d][32]
   int Hk, Hv, h0, Hn;
   float eps;
 };
@@ -58,7 +58,7 @@ __device__ __forceinline__ float gp_ex2(float x) { return exp2f(x); }       // (
 __device__ __forceinline__ float gp_tf32(float x) { uint32_t y; asm("cvt.rna.tf32.f32 %0, %1;\n" : "=r"(y) : "f"(x)); return __uint_as_float(y); }
 __device__ __forceinline__ void gp_split(float x, float& hi, float& lo) { hi = gp_tf32(x); lo = gp_tf32(x - hi); }
 __device__ __forceinline__ void gp_mma_tf32(float* c, const float* a, float b0, float b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
                  "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
@@ -66,13 +66,27 @@ __device__ __forceinline__ void gp_mma_tf32(float* c, const float* a, float b0, 
 template <bool BF16>
 __device__ __forceinline__ void gp_mma_16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   if (BF16)
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   else
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void gp_add4(float* c, const float* t) { c[0] += t[0]; c[1] += t[1]; c[2] += t[2]; c[3] += t[3]; }
+// the same with a sum that starts at zero
+__device__ __forceinline__ void gp_mma0_tf32(float* c, const float* a, float b0, float b1) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+        "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)), "f"(0.f));
+}
+__device__ __forceinline__ void gp_mma0_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void gp_add4(float* c, const float* t) {
+  unpack_f32x2(add_f32x2(pack_f32x2(c[0], c[1]), pack_f32x2(t[0], t[1])), c[0], c[1]);
+  unpack_f32x2(add_f32x2(pack_f32x2(c[2], c[3]), pack_f32x2(t[2], t[3])), c[2], c[3]);
+}
 // Two fp32 numbers as three bf16 terms each: all 24 bits.
 __device__ __forceinline__ void gp_split_bf16(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   hi = pack_16<true>(x, y);
@@ -311,35 +325,39 @@ __global__ void __launch_bounds__(128) gdn_chunk_inverse_kernel(const GdnPromptP
 }
 
 // ------------------------------------------------------------------------------------------------
-// the chain over a request's chunks: a CTA of four warps takes 32 columns of a head's state, two warps 16 of them: each carries 64 of the 128 key
-// channels.  They add up K S, share out the columns of T's product (equal parts of its triangle) and exchange V', twice a chunk
-// through shared memory.  Bound by the issue of products (bf16: 192 of 16 terms and 54 tf32 ones a warp and chunk, and the fp32 additions between
-// them).  4001 tokens x 32 heads with the kernels before and behind it: 496 us; two tf32 terms and running sums 507, tf32 with separate sums 578.
+// the chain over a request's chunks: a CTA of eight warps takes 32 columns of a head's state, four warps 16 of them: each carries 32 of the 128 key
+// channels.  They add up K S, a warp two of the eight token tiles, share out the columns of T's product (token tiles f and 7 - f: equal parts of its
+// triangle) and exchange V', three times a chunk through shared memory.  Bound by the chain of a chunk: a warp issues 150 products of the tensor core and
+// about 1000 instructions a chunk, two warps share a sub-core, and shared memory is busy half of the time.  Chain of 4001 tokens x 32 heads: 261 us with
+// two warps per 16 columns, 229 with four, 207 with eight sums in flight between a product and the next one of its own sum, 198 with the state and V' stored as
+// the accumulators hold them.  8 requests of 1000 tokens: 311 -> 284 us with the last two.
 // ------------------------------------------------------------------------------------------------
-constexpr int GS_THREADS = 128;
+constexpr int GS_THREADS = 256;
 constexpr int GS_LDV = 40;
 constexpr int GS_K = GP_T * GP_LDK * 2, GS_T = GP_T * GP_LDT * 4, GS_V = GP_T * GS_LDV * 2, GS_VEC = 3 * GP_T * 4;
 constexpr int GS_STAGE = GS_K + GS_T + GS_V + GS_VEC;
 constexpr int GS_STAGES = 2;
-constexpr int GS_PART = 8 * 32 * 16, GS_NEW = 4 * 32 * 16;       // bytes of a warp's partial K S and of its columns of V'
-constexpr int GS_SMEM = GS_STAGES * GS_STAGE + 4 * (GS_PART + GS_NEW);
+constexpr int GS_TILE = 32 * 16;                                  // bytes of a 16 x 8 fp32 tile as fragments
+constexpr int GS_PART = 3 * 8 * GS_TILE;                          // of four warps: the partial sums of three others for every tile
+constexpr int GS_SMEM = GS_STAGES * GS_STAGE + 2 * GS_PART;
 
 template <bool BF16>
-__global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPromptParams p) {
+__global__ void __launch_bounds__(GS_THREADS, 2) gdn_chunk_scan_kernel(const GdnPromptParams p) {
   extern __shared__ __align__(16) uint8_t gs_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
-  const int pair = warp >> 1, half = warp & 1, d0 = half * 64;
+  const int four = warp >> 2, f = warp & 3, d0 = f * 32;
   const int hl = blockIdx.y, h = p.h0 + hl, hk = h / (p.Hv / p.Hk), v0 = blockIdx.x * 32;
-  float4* part_own = reinterpret_cast<float4*>(gs_smem + GS_STAGES * GS_STAGE + warp * GS_PART) + lane;
-  const float4* part_other = reinterpret_cast<const float4*>(gs_smem + GS_STAGES * GS_STAGE + (warp ^ 1) * GS_PART) + lane;
-  float4* new_own = reinterpret_cast<float4*>(gs_smem + GS_STAGES * GS_STAGE + 4 * GS_PART + warp * GS_NEW) + lane;
-  const float4* new_other = reinterpret_cast<const float4*>(gs_smem + GS_STAGES * GS_STAGE + 4 * GS_PART + (warp ^ 1) * GS_NEW) + lane;
-  auto meet = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(1 + pair) : "memory"); };
+  // [3][4 warps][2 tiles][32 lanes]: what three other warps have summed for a warp's tiles; once it has read them, the first third takes its rows of the
+  // right-hand side and, after the barrier behind that, the rest takes V'
+  float4* part = reinterpret_cast<float4*>(gs_smem + GS_STAGES * GS_STAGE + four * GS_PART) + lane;
+  float4* vx = part + 8 * 32;
+  auto meet = [&]() { asm volatile("bar.sync %0, 128;\n" ::"r"(1 + four) : "memory"); };
   const int* rq = p.reqs + 4 * blockIdx.z;
   const int c0 = rq[0], nc = rq[1], slot = rq[2];
+  int row0 = p.chunks[3 * c0], n = p.chunks[3 * c0 + 1];           // of the chunk to be fetched next
   auto fetch = [&](int i) {
     uint8_t* st = gs_smem + (i % GS_STAGES) * GS_STAGE;
-    const int c = c0 + i, row0 = p.chunks[3 * c], n = p.chunks[3 * c + 1];
+    const int c = c0 + i;
     const size_t unit = (size_t)c * p.Hn + hl;
     const uint16_t* kp = p.y + (size_t)row0 * p.ld_y + (p.Hk + hk) * GP_D;
     const uint16_t* vp = p.y + (size_t)row0 * p.ld_y + (size_t)2 * p.Hk * GP_D + (size_t)h * GP_D + v0;
@@ -351,26 +369,26 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
       gp_cp16(st + (t * GP_LDK + u * 8) * 2, kp + (size_t)(t < n ? t : 0) * p.ld_y + u * 8, t < n);
       gp_cp16(st + GS_K + (t * GP_LDT + u * 4) * 4, tp + t * GP_T + u * 4, true);
     }
-#pragma unroll
-    for (int j = tid; j < GP_T * 4; j += GS_THREADS) {
-      const int t = j >> 2, u = j & 3;
+    {
+      const int t = tid >> 2, u = tid & 3;
       gp_cp16(st + GS_K + GS_T + (t * GS_LDV + u * 8) * 2, vp + (size_t)(t < n ? t : 0) * p.ld_y + u * 8, t < n);
     }
     if (tid < 48) gp_cp16(st + GS_K + GS_T + GS_V + tid * 16, gp + tid * 4, true);           // beta, cb, cd
+    if (i + 1 < nc) { row0 = p.chunks[3 * c + 3]; n = p.chunks[3 * c + 4]; }
   };
-  float s[8][4];                                  // S^T: rows v = g, g + 8, columns d = d0 + 8 i + 2 q, + 1
-  float* S = p.state + ((size_t)slot * p.Hv + h) * GP_D * GP_D + (size_t)d0 * GP_D + v0 + pair * 16;
+  float s[4][4];                                  // S^T: rows v = g, g + 8, columns d = d0 + 8 i + 2 q, + 1
+  float* S = p.state + ((size_t)slot * p.Hv + h) * GP_D * GP_D + (size_t)d0 * GP_D + v0 + four * 16;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) s[i][e] = S[(size_t)(8 * i + 2 * q + (e & 1)) * GP_D + g + 8 * (e >> 1)];
   fetch(0);
   gp_cp_commit();
   for (int i = 0; i < nc; ++i) {
+    gp_cp_wait<0>();
+    __syncthreads();                              // this chunk is there for all, and the other stage and the exchanged parts are done with
     if (i + 1 < nc) fetch(i + 1);
     gp_cp_commit();
-    gp_cp_wait<1>();
-    __syncthreads();
     const uint8_t* st = gs_smem + (i % GS_STAGES) * GS_STAGE;
     const uint16_t* ks = reinterpret_cast<const uint16_t*>(st) + d0;
     const float* ts = reinterpret_cast<const float*>(st + GS_K);
@@ -378,40 +396,37 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
     const float* vec = reinterpret_cast<const float*>(st + GS_K + GS_T + GS_V);
     const size_t unit = (size_t)(c0 + i) * p.Hn + hl;
     const float last = __ldg(p.vecs + (unit * GP_VECS + GV_LAST) * GP_T);
-    const int vr = v0 + pair * 16 + g;
-    float* s0 = p.s0 + (unit * GP_D + vr) * GP_D + d0 + 2 * q;
+    const int vb = blockIdx.x * 2 + four;
+    float4* s0 = p.s0 + (unit * 128 + vb * 16 + f * 4) * 32 + lane;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      *reinterpret_cast<float2*>(s0 + 8 * j) = make_float2(s[j][0], s[j][1]);
-      *reinterpret_cast<float2*>(s0 + 8 * GP_D + 8 * j) = make_float2(s[j][2], s[j][3]);
-    }
+    for (int j = 0; j < 4; ++j) s0[j * 32] = make_float4(s[j][0], s[j][1], s[j][2], s[j][3]);
     // (K S)^T [16 v x 64 t] over this warp's channels
     float r[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) r[j][0] = r[j][1] = r[j][2] = r[j][3] = 0.f;
     if (BF16) {
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
+      for (int kk = 0; kk < 2; ++kk) {
         uint32_t hi[4], mid[4], lo[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) gp_split_bf16(s[2 * kk + (i >> 1)][2 * (i & 1)], s[2 * kk + (i >> 1)][2 * (i & 1) + 1], hi[i], mid[i], lo[i]);
+        uint32_t b[4][4];
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint32_t b[4];
-          gp_ldsm4(b, ks + (8 * (j + (lane >> 4)) + (lane & 7)) * GP_LDK + kk * 16 + ((lane >> 3) & 1) * 8);
+        for (int j = 0; j < 4; ++j) gp_ldsm4(b[j], ks + (8 * (2 * j + (lane >> 4)) + (lane & 7)) * GP_LDK + kk * 16 + ((lane >> 3) & 1) * 8);
+        float t[8][4];                            // (eight sums at a time: a product waits for the one before it of its own sum)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float t[4] = {0.f, 0.f, 0.f, 0.f};
-            gp_mma_16<true>(t, lo, b[2 * e], b[2 * e + 1]);
-            gp_mma_16<true>(t, mid, b[2 * e], b[2 * e + 1]);
-            gp_mma_16<true>(t, hi, b[2 * e], b[2 * e + 1]);
-            gp_add4(r[j + e], t);
-          }
+        for (int j = 0; j < 8; ++j) gp_mma0_bf16(t[j], lo, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gp_mma_16<true>(t[j], mid, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gp_mma_16<true>(t[j], hi, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          if (kk == 0) { r[j][0] = t[j][0]; r[j][1] = t[j][1]; r[j][2] = t[j][2]; r[j][3] = t[j][3]; }
+          else gp_add4(r[j], t[j]);
         }
       }
     } else {
 #pragma unroll
-      for (int kk = 0; kk < 8; ++kk) {
+      for (int kk = 0; kk < 4; ++kk) {
         float hi[4], lo[4];
         gp_split(s[kk][0], hi[0], lo[0]); gp_split(s[kk][2], hi[1], lo[1]); gp_split(s[kk][1], hi[2], lo[2]); gp_split(s[kk][3], hi[3], lo[3]);
         uint32_t b[8];
@@ -419,136 +434,149 @@ __global__ void __launch_bounds__(GS_THREADS) gdn_chunk_scan_kernel(const GdnPro
         gp_ldsm4(b + 4, ks + (32 + lane) * GP_LDK + kk * 8);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float2 f = unpack_16<BF16>(b[j]);
-          float t[4] = {0.f, 0.f, 0.f, 0.f};
-          gp_mma_tf32(t, lo, f.x, f.y);
-          gp_mma_tf32(t, hi, f.x, f.y);
-          gp_add4(r[j], t);
+          const float2 k2 = unpack_16<BF16>(b[j]);
+          float t[4];
+          gp_mma0_tf32(t, lo, k2.x, k2.y);
+          gp_mma_tf32(t, hi, k2.x, k2.y);
+          if (kk == 0) { r[j][0] = t[0]; r[j][1] = t[1]; r[j][2] = t[2]; r[j][3] = t[3]; }
+          else gp_add4(r[j], t);
         }
       }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) part_own[32 * j] = make_float4(r[j][0], r[j][1], r[j][2], r[j][3]);
-    meet();
+    float own[2][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const int t = 8 * j + 2 * q;
-      const float4 o = part_other[32 * j];
-      const float2 be = *reinterpret_cast<const float2*>(vec + t), cb = *reinterpret_cast<const float2*>(vec + GP_T + t);
-      const uint16_t* vp = vs + t * GS_LDV + pair * 16 + g;
-      r[j][0] = fmaf(-cb.x, r[j][0] + o.x, be.x * gp_ld<BF16>(vp[0]));
-      r[j][1] = fmaf(-cb.y, r[j][1] + o.y, be.y * gp_ld<BF16>(vp[GS_LDV]));
-      r[j][2] = fmaf(-cb.x, r[j][2] + o.z, be.x * gp_ld<BF16>(vp[8]));
-      r[j][3] = fmaf(-cb.y, r[j][3] + o.w, be.y * gp_ld<BF16>(vp[GS_LDV + 8]));
+      const int to = j < 4 ? j : 7 - j, x = j >> 2;
+      if (to == f) { own[x][0] = r[j][0]; own[x][1] = r[j][1]; own[x][2] = r[j][2]; own[x][3] = r[j][3]; }
+      else part[((((f - to - 1) & 3) * 4 + to) * 2 + x) * 32] = make_float4(r[j][0], r[j][1], r[j][2], r[j][3]);
     }
-    // V'^T = (right-hand side)^T T^T: token tiles 0, 3, 4, 7 or 1, 2, 5, 6, 18 products of the triangle each
-    float w[4][4], wl[4][4];                      // products of first terms, the others'
+    meet();
 #pragma unroll
-    for (int x = 0; x < 4; ++x) w[x][0] = w[x][1] = w[x][2] = w[x][3] = wl[x][0] = wl[x][1] = wl[x][2] = wl[x][3] = 0.f;
-    auto tile = [&](int x) { return 2 * x + ((x & 1) ^ half); };
+    for (int x = 0; x < 2; ++x) {
+      const int t = 8 * (x == 0 ? f : 7 - f) + 2 * q;
+      float4* pt = part + (f * 2 + x) * 32;
+      const float4 a = pt[0], b = pt[8 * 32], c = pt[16 * 32];
+      const float2 be = *reinterpret_cast<const float2*>(vec + t), cb = *reinterpret_cast<const float2*>(vec + GP_T + t);
+      const uint16_t* vp = vs + t * GS_LDV + four * 16 + g;
+      float4 o;
+      o.x = fmaf(-cb.x, (own[x][0] + a.x) + (b.x + c.x), be.x * gp_ld<BF16>(vp[0]));
+      o.y = fmaf(-cb.y, (own[x][1] + a.y) + (b.y + c.y), be.y * gp_ld<BF16>(vp[GS_LDV]));
+      o.z = fmaf(-cb.x, (own[x][2] + a.z) + (b.z + c.z), be.x * gp_ld<BF16>(vp[8]));
+      o.w = fmaf(-cb.y, (own[x][3] + a.w) + (b.w + c.w), be.y * gp_ld<BF16>(vp[GS_LDV + 8]));
+      pt[0] = o;
+    }
+    meet();
+    // V'^T = (right-hand side)^T T^T: token tiles f and 7 - f, 9 products of the triangle
+    float w[2][4], wl[2][4], wm[2][4];            // products of first terms, the others'
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) w[x][e] = wl[x][e] = wm[x][e] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
+      if (kk > 7 - f) break;
+      const float4 rv = part[((kk < 4 ? kk : 7 - kk) * 2 + (kk >> 2)) * 32];
       float hi[4], lo[4];
-      gp_split(r[kk][0], hi[0], lo[0]); gp_split(r[kk][2], hi[1], lo[1]); gp_split(r[kk][1], hi[2], lo[2]); gp_split(r[kk][3], hi[3], lo[3]);
+      gp_split(rv.x, hi[0], lo[0]); gp_split(rv.z, hi[1], lo[1]); gp_split(rv.y, hi[2], lo[2]); gp_split(rv.w, hi[3], lo[3]);
 #pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        if (tile(x) < kk) continue;
-        const float2 tv = *reinterpret_cast<const float2*>(ts + (8 * tile(x) + g) * GP_LDT + 8 * kk + 2 * q);
+      for (int x = 0; x < 2; ++x) {
+        if (x == 0 && kk > f) continue;
+        const float2 tv = *reinterpret_cast<const float2*>(ts + (8 * (x == 0 ? f : 7 - f) + g) * GP_LDT + 8 * kk + 2 * q);
         float bh0, bl0, bh1, bl1;
         gp_split(tv.x, bh0, bl0);
         gp_split(tv.y, bh1, bl1);
-        float t[4] = {0.f, 0.f, 0.f, 0.f};
-        gp_mma_tf32(t, hi, bh0, bh1);
+        float t[4];
+        gp_mma0_tf32(t, hi, bh0, bh1);
         gp_add4(w[x], t);
         gp_mma_tf32(wl[x], lo, bh0, bh1);
-        gp_mma_tf32(wl[x], hi, bl0, bl1);
+        gp_mma_tf32(wm[x], hi, bl0, bl1);
       }
     }
-    float* vn = p.vnew + (unit * GP_D + vr) * GP_T + 2 * q;
+    float4* vn = p.vnew + (unit * 64 + vb * 8) * 32 + lane;
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
+    for (int x = 0; x < 2; ++x) {
+      const int tile = x == 0 ? f : 7 - f;
+      gp_add4(wl[x], wm[x]);
       gp_add4(w[x], wl[x]);
-      new_own[32 * x] = make_float4(w[x][0], w[x][1], w[x][2], w[x][3]);
-      *reinterpret_cast<float2*>(vn + 8 * tile(x)) = make_float2(w[x][0], w[x][1]);
-      *reinterpret_cast<float2*>(vn + 8 * GP_T + 8 * tile(x)) = make_float2(w[x][2], w[x][3]);
+      vn[tile * 32] = make_float4(w[x][0], w[x][1], w[x][2], w[x][3]);
+      const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 8 * tile + 2 * q);
+      const float4 wd = make_float4(w[x][0] * cd.x, w[x][1] * cd.y, w[x][2] * cd.x, w[x][3] * cd.y);
+      if (BF16) {                                 // half of a 16-token operand, in its three terms: [4 pairs of tiles][3][32 lanes]
+        uint32_t hi[2], mid[2], lo[2];
+        gp_split_bf16(wd.x, wd.y, hi[0], mid[0], lo[0]);
+        gp_split_bf16(wd.z, wd.w, hi[1], mid[1], lo[1]);
+        uint2* o = reinterpret_cast<uint2*>(vx + (tile >> 1) * 3 * 32) + (tile & 1);
+        o[0] = make_uint2(hi[0], hi[1]); o[64] = make_uint2(mid[0], mid[1]); o[128] = make_uint2(lo[0], lo[1]);
+      } else {
+        vx[tile * 32] = wd;
+      }
     }
     meet();
     // S^T <- e^(G_last) S^T + (decayed V')^T K
-    float u[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) u[j][0] = u[j][1] = u[j][2] = u[j][3] = 0.f;
+    float u[4][4];
     if (BF16) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {               // 16 tokens: a tile of this warp's and one of the other's
-        const bool own_first = ((c & 1) ^ half) == 0;
-        const float4 own = make_float4(w[c][0], w[c][1], w[c][2], w[c][3]), other = new_other[32 * c];
-        uint32_t hi[4], mid[4], lo[4];
+      for (int c = 0; c < 4; ++c) {               // 16 tokens
+        const uint4 h4 = *reinterpret_cast<const uint4*>(vx + c * 96), m4 = *reinterpret_cast<const uint4*>(vx + c * 96 + 32),
+                    l4 = *reinterpret_cast<const uint4*>(vx + c * 96 + 64);
+        const uint32_t hi[4] = {h4.x, h4.y, h4.z, h4.w}, mid[4] = {m4.x, m4.y, m4.z, m4.w}, lo[4] = {l4.x, l4.y, l4.z, l4.w};
+        uint32_t b[2][4];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float4 wv = own_first == (i == 0) ? own : other;
-          const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 16 * c + 8 * i + 2 * q);
-          gp_split_bf16(wv.x * cd.x, wv.y * cd.y, hi[2 * i], mid[2 * i], lo[2 * i]);
-          gp_split_bf16(wv.z * cd.x, wv.w * cd.y, hi[2 * i + 1], mid[2 * i + 1], lo[2 * i + 1]);
-        }
+        for (int j = 0; j < 2; ++j) gp_ldsm4_t(b[j], ks + (16 * c + (lane & 15)) * GP_LDK + (2 * j + (lane >> 4)) * 8);
+        float t[4][4];
 #pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          uint32_t b[4];
-          gp_ldsm4_t(b, ks + (16 * c + (lane & 15)) * GP_LDK + (j + (lane >> 4)) * 8);
+        for (int j = 0; j < 4; ++j) gp_mma0_bf16(t[j], lo, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float t[4] = {0.f, 0.f, 0.f, 0.f};
-            gp_mma_16<true>(t, lo, b[2 * e], b[2 * e + 1]);
-            gp_mma_16<true>(t, mid, b[2 * e], b[2 * e + 1]);
-            gp_mma_16<true>(t, hi, b[2 * e], b[2 * e + 1]);
-            gp_add4(u[j + e], t);
-          }
+        for (int j = 0; j < 4; ++j) gp_mma_16<true>(t[j], mid, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) gp_mma_16<true>(t[j], hi, b[j >> 1][2 * (j & 1)], b[j >> 1][2 * (j & 1) + 1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (c == 0) { u[j][0] = t[j][0]; u[j][1] = t[j][1]; u[j][2] = t[j][2]; u[j][3] = t[j][3]; }
+          else gp_add4(u[j], t[j]);
         }
       }
     } else {
 #pragma unroll
-      for (int y = 0; y < 8; ++y) {
-        const bool mine = y < 4;
-        const int x = y & 3, kk = 2 * x + ((x & 1) ^ (mine ? half : half ^ 1));
-        const float4 wv = mine ? make_float4(w[x][0], w[x][1], w[x][2], w[x][3]) : new_other[32 * x];
-        const float2 cd = *reinterpret_cast<const float2*>(vec + 2 * GP_T + 8 * kk + 2 * q);
+      for (int kk = 0; kk < 8; ++kk) {
+        const float4 wv = vx[kk * 32];
         float hi[4], mid[4], lo[4];
-        const float wd[4] = {wv.x * cd.x, wv.z * cd.x, wv.y * cd.y, wv.w * cd.y};
+        const float wd[4] = {wv.x, wv.z, wv.y, wv.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) { gp_split(wd[i], hi[i], mid[i]); lo[i] = gp_tf32((wd[i] - hi[i]) - mid[i]); }
+        uint32_t b[4];
+        gp_ldsm4_t(b, ks + (8 * kk + (lane & 7)) * GP_LDK + (lane >> 3) * 8);
 #pragma unroll
-        for (int j = 0; j < 8; j += 4) {
-          uint32_t b[4];
-          gp_ldsm4_t(b, ks + (8 * kk + (lane & 7)) * GP_LDK + (j + (lane >> 3)) * 8);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = unpack_16<BF16>(b[e]);
-            float t[4] = {0.f, 0.f, 0.f, 0.f};
-            gp_mma_tf32(t, lo, f.x, f.y);
-            gp_mma_tf32(t, mid, f.x, f.y);
-            gp_mma_tf32(t, hi, f.x, f.y);
-            gp_add4(u[j + e], t);
-          }
+        for (int e = 0; e < 4; ++e) {
+          const float2 k2 = unpack_16<BF16>(b[e]);
+          float t[4];
+          gp_mma0_tf32(t, lo, k2.x, k2.y);
+          gp_mma_tf32(t, mid, k2.x, k2.y);
+          gp_mma_tf32(t, hi, k2.x, k2.y);
+          if (kk == 0) { u[e][0] = t[0]; u[e][1] = t[1]; u[e][2] = t[2]; u[e][3] = t[3]; }
+          else gp_add4(u[e], t);
         }
       }
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[j][e] = fmaf(s[j][e], last, u[j][e]);
-    __syncthreads();                              // the stage is refilled by the next fetch
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int e = 0; e < 4; ++e) S[(size_t)(8 * i + 2 * q + (e & 1)) * GP_D + g + 8 * (e >> 1)] = s[i][e];
 }
 
 // ------------------------------------------------------------------------------------------------
-// outputs of a chunk: warps 2 x 4 over (32 tokens, 32 columns); state halves and V' pass through one buffer, two CTAs share an SM
+// outputs of a chunk: warps 2 x 4 over (32 tokens, 32 columns).  The state comes in quarters of 32 channels and V' in halves of 32 tokens through a ring of
+// three buffers, two ahead of the products; two CTAs share an SM.  Bound by the issue of instructions (splits into tf32 terms, the gate).  4001 tokens x 32 heads:
+// 160 us with one buffer that every step waited for, 147 with the ring, 126 with gates read ahead and without exact exponentials and divisions.
 // ------------------------------------------------------------------------------------------------
 constexpr int GO_THREADS = 256;
-constexpr int GO_QK = GP_T * GP_LDK * 2, GO_P = GP_T * GP_LDT * 4, GO_B = GP_D * GP_LDT * 4;
-constexpr int GO_SMEM = 2 * GO_QK + GO_P + GO_B + GP_T * 4 * 4;
+constexpr int GO_QK = GP_T * GP_LDK * 2, GO_P = GP_T * GP_LDT * 4, GO_B = 8 * 4 * 32 * 16, GO_RING = 3;
+constexpr int GO_SMEM = 2 * GO_QK + GO_P + GO_RING * GO_B + GP_T * 4 * 4;
 
 template <bool BF16>
 __global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnPromptParams p) {
@@ -556,8 +584,8 @@ __global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnP
   uint16_t* qs = reinterpret_cast<uint16_t*>(go_smem);
   uint16_t* ks = reinterpret_cast<uint16_t*>(go_smem + GO_QK);
   float* Ps = reinterpret_cast<float*>(go_smem + 2 * GO_QK);
-  float* Bs = reinterpret_cast<float*>(go_smem + 2 * GO_QK + GO_P);
-  float* red = reinterpret_cast<float*>(go_smem + 2 * GO_QK + GO_P + GO_B);       // [64][4]
+  float4* Bs = reinterpret_cast<float4*>(go_smem + 2 * GO_QK + GO_P);             // [3][8 blocks of 16 v][4 tiles of 8][32 lanes]
+  float* red = reinterpret_cast<float*>(go_smem + 2 * GO_QK + GO_P + GO_RING * GO_B);       // [64][4]
   const int c = blockIdx.x, hl = blockIdx.y, h = p.h0 + hl, hk = h / (p.Hv / p.Hk);
   const int row0 = p.chunks[3 * c], n = p.chunks[3 * c + 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
@@ -571,17 +599,17 @@ __global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnP
     gp_cp16(ks + t * GP_LDK + u * 8, src + p.Hk * GP_D, t < n);
   }
   gp_cp_commit();
-  auto fetch = [&](const float* src, int ld) {    // [128 v][64] into the buffer
+  const float4 *s0 = p.s0 + unit * 128 * 32, *vnew = p.vnew + unit * 64 * 32;
+  auto fetch = [&](int step) {                    // quarters of the state, then halves of V'
+    const float4* src = step < 4 ? s0 + step * 128 : vnew + (step - 4) * 128;
+    const int ld = step < 4 ? 16 * 32 : 8 * 32;
 #pragma unroll
-    for (int j = tid; j < GP_D * 16; j += GO_THREADS) {
-      const int v = j >> 4, u = j & 15;
-      gp_cp16(Bs + v * GP_LDT + u * 4, src + (size_t)v * ld + u * 4, true);
-    }
+    for (int j = tid; j < 8 * 128; j += GO_THREADS) gp_cp16(Bs + (step % GO_RING) * 1024 + j, src + (j >> 7) * ld + (j & 127), true);
     gp_cp_commit();
   };
-  const float* s0 = p.s0 + unit * GP_D * GP_D;
-  fetch(s0, GP_D);
-  gp_cp_wait<1>();
+  fetch(0);
+  fetch(1);
+  gp_cp_wait<2>();
   __syncthreads();
   {                                               // decayed scores, 16 tokens x 32 keys a warp
     const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 4;
@@ -623,68 +651,76 @@ __global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnP
   for (int m = 0; m < 2; ++m)
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[m][j][0] = acc[m][j][1] = acc[m][j][2] = acc[m][j][3] = 0.f;
+  auto terms = [&](const float4* bs, float (*hb)[2], float (*lb)[2]) {            // of 8 rows of B for this warp's 32 columns
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    gp_cp_wait<0>();
-    __syncthreads();
+    for (int j = 0; j < 4; j += 2) {
+      const float4 v = bs[(j >> 1) * 128];
+      gp_split(v.x, hb[j][0], lb[j][0]); gp_split(v.y, hb[j][1], lb[j][1]); gp_split(v.z, hb[j + 1][0], lb[j + 1][0]); gp_split(v.w, hb[j + 1][1], lb[j + 1][1]);
+    }
+  };
+  uint32_t zr[2][2][4];                           // gates of this thread's outputs, asked for ahead of the last products
+  const bool pairs = ((reinterpret_cast<uintptr_t>(p.z) | (uintptr_t)(2 * p.ld_z)) & 3) == 0;
 #pragma unroll
-    for (int kk = 0; kk < 8; kk += 2) {
-      uint32_t a[2][4];                           // rows 0-7 | 8-15 of k step kk, then of kk + 1
+  for (int step = 0; step < 6; ++step) {
+    if (step == 5) gp_cp_wait<0>(); else gp_cp_wait<1>();
+    __syncthreads();                              // this step's operands are there for all, the ones of the step before are done with
+    if (step + 2 < 6) fetch(step + 2);
+    const float4* bs = Bs + (step % GO_RING) * 1024 + vg * 256 + lane;
+    if (step < 4) {
 #pragma unroll
-      for (int m = 0; m < 2; ++m) gp_ldsm4(a[m], qs + (tg * 32 + m * 16 + (lane & 15)) * GP_LDK + half * 64 + (kk + (lane >> 4)) * 8);
+      for (int kk = 0; kk < 4; kk += 2) {
+        uint32_t a[2][4];                         // rows 0-7 | 8-15 of k step kk, then of kk + 1
 #pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        float af[2][4];
+        for (int m = 0; m < 2; ++m) gp_ldsm4(a[m], qs + (tg * 32 + m * 16 + (lane & 15)) * GP_LDK + step * 32 + (kk + (lane >> 4)) * 8);
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-          const float2 f0 = unpack_16<BF16>(a[m][2 * x]), f1 = unpack_16<BF16>(a[m][2 * x + 1]);
-          af[m][0] = f0.x; af[m][1] = f1.x; af[m][2] = f0.y; af[m][3] = f1.y;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 sv = *reinterpret_cast<const float2*>(Bs + (vg * 32 + j * 8 + g) * GP_LDT + (kk + x) * 8 + 2 * q);
-          float h0, l0, h1, l1;
-          gp_split(sv.x, h0, l0);
-          gp_split(sv.y, h1, l1);
+        for (int x = 0; x < 2; ++x) {
+          float af[2][4], hb[4][2], lb[4][2];
 #pragma unroll
           for (int m = 0; m < 2; ++m) {
-            gp_mma_tf32(acc[m][j], af[m], h0, h1);
-            gp_mma_tf32(acc[m][j], af[m], l0, l1);
+            const float2 f0 = unpack_16<BF16>(a[m][2 * x]), f1 = unpack_16<BF16>(a[m][2 * x + 1]);
+            af[m][0] = f0.x; af[m][1] = f1.x; af[m][2] = f0.y; af[m][3] = f1.y;
           }
+          terms(bs + (kk + x) * 32, hb, lb);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) gp_mma_tf32(acc[j & 1][j >> 1], af[j & 1], hb[j >> 1][0], hb[j >> 1][1]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) gp_mma_tf32(acc[j & 1][j >> 1], af[j & 1], lb[j >> 1][0], lb[j >> 1][1]);
         }
       }
-    }
-    __syncthreads();
-    if (half == 0) fetch(s0 + GP_T, GP_D);
-    else fetch(p.vnew + unit * GP_D * GP_T, GP_T);
-  }
+      if (step == 3) {
 #pragma unroll
-  for (int m = 0; m < 2; ++m) {
-    const float e0 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g), e1 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g + 8);
+        for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { acc[m][j][0] *= e0; acc[m][j][1] *= e0; acc[m][j][2] *= e1; acc[m][j][3] *= e1; }
-  }
-  gp_cp_wait<0>();
-  __syncthreads();
-  for (int kk = 0; kk < 4 * (tg + 1); ++kk) {     // (scores behind the diagonal are zeros)
-    float hi[2][4], lo[2][4];
+          for (int e = 0; e < 2; ++e) {
+            const int t = tg * 32 + m * 16 + g + 8 * e;
+            const uint16_t* zp = p.z + (size_t)(row0 + (t < n ? t : 0)) * p.ld_z + (size_t)h * GP_D + vg * 32 + 2 * q;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const float* pp = Ps + (tg * 32 + m * 16 + g) * GP_LDT + kk * 8 + 2 * q;
-      const float2 f0 = *reinterpret_cast<const float2*>(pp), f1 = *reinterpret_cast<const float2*>(pp + 8 * GP_LDT);
-      gp_split(f0.x, hi[m][0], lo[m][0]); gp_split(f1.x, hi[m][1], lo[m][1]); gp_split(f0.y, hi[m][2], lo[m][2]); gp_split(f1.y, hi[m][3], lo[m][3]);
-    }
+            for (int j = 0; j < 4; ++j) zr[m][e][j] = pairs ? *reinterpret_cast<const uint32_t*>(zp + 8 * j) : (uint32_t)zp[8 * j] | (uint32_t)zp[8 * j + 1] << 16;
+          }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 sv = *reinterpret_cast<const float2*>(Bs + (vg * 32 + j * 8 + g) * GP_LDT + kk * 8 + 2 * q);
-      float h0, l0, h1, l1;
-      gp_split(sv.x, h0, l0);
-      gp_split(sv.y, h1, l1);
+        for (int m = 0; m < 2; ++m) {
+          const float e0 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g), e1 = __ldg(vec + GV_EQ * GP_T + tg * 32 + m * 16 + g + 8);
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        gp_mma_tf32(acc[m][j], hi[m], h0, h1);
-        gp_mma_tf32(acc[m][j], lo[m], h0, h1);
-        gp_mma_tf32(acc[m][j], hi[m], l0, l1);
+          for (int j = 0; j < 4; ++j) { acc[m][j][0] *= e0; acc[m][j][1] *= e0; acc[m][j][2] *= e1; acc[m][j][3] *= e1; }
+        }
+      }
+    } else if (step - 4 <= tg) {                  // (scores behind the diagonal are zeros)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        float hi[2][4], lo[2][4], hb[4][2], lb[4][2];
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          const float* pp = Ps + (tg * 32 + m * 16 + g) * GP_LDT + (step - 4) * 32 + kk * 8 + 2 * q;
+          const float2 f0 = *reinterpret_cast<const float2*>(pp), f1 = *reinterpret_cast<const float2*>(pp + 8 * GP_LDT);
+          gp_split(f0.x, hi[m][0], lo[m][0]); gp_split(f1.x, hi[m][1], lo[m][1]); gp_split(f0.y, hi[m][2], lo[m][2]); gp_split(f1.y, hi[m][3], lo[m][3]);
+        }
+        terms(bs + kk * 32, hb, lb);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gp_mma_tf32(acc[j & 1][j >> 1], hi[j & 1], hb[j >> 1][0], hb[j >> 1][1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gp_mma_tf32(acc[j & 1][j >> 1], lo[j & 1], hb[j >> 1][0], hb[j >> 1][1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) gp_mma_tf32(acc[j & 1][j >> 1], hi[j & 1], lb[j >> 1][0], lb[j >> 1][1]);
       }
     }
   }
@@ -723,10 +759,9 @@ __global__ void __launch_bounds__(GO_THREADS, 2) gdn_chunk_out_kernel(const GdnP
         const float2 nw = unpack_16<BF16>(*reinterpret_cast<const uint32_t*>(p.norm_w + v));
         const float2 y1 = unpack_16<BF16>(pack_16<BF16>(o16[m][j][2 * e] * inv, o16[m][j][2 * e + 1] * inv));
         const float2 y2 = unpack_16<BF16>(pack_16<BF16>(nw.x * y1.x, nw.y * y1.y));
-        const uint16_t* zp = p.z + (size_t)(row0 + t) * p.ld_z + (size_t)h * GP_D + v;
-        const float z0 = gp_ld<BF16>(zp[0]), z1 = gp_ld<BF16>(zp[1]);
+        const float2 z = unpack_16<BF16>(zr[m][e][j]);
         *reinterpret_cast<uint32_t*>(p.out + ((size_t)(row0 + t) * p.Hv + h) * GP_D + v) =
-            pack_16<BF16>(y2.x * (z0 / (1.0f + expf(-z0))), y2.y * (z1 / (1.0f + expf(-z1))));
+            pack_16<BF16>(y2.x * gp_silu(z.x), y2.y * gp_silu(z.y));
       }
     }
 }
@@ -761,7 +796,7 @@ extern "C" int fb_gdn_prompt(const void* y, long long ld_y, const void* a, const
   GdnPromptParams p = {};
   p.y = (const uint16_t*)y; p.ld_y = ld_y; p.a = (const uint16_t*)a; p.b = (const uint16_t*)b; p.ld_ab = ld_ab; p.z = (const uint16_t*)z; p.ld_z = ld_z;
   p.A_log = A_log; p.dt_bias = dt_bias; p.norm_w = (const uint16_t*)norm_w; p.state = state; p.out = (uint16_t*)out; p.chunks = chunks; p.reqs = reqs;
-  p.inv = inv; p.vecs = vecs; p.vnew = vnew; p.s0 = s0; p.Hk = Hk; p.Hv = Hv; p.h0 = h0; p.Hn = Hn; p.eps = eps;
+  p.inv = inv; p.vecs = vecs; p.vnew = reinterpret_cast<float4*>(vnew); p.s0 = reinterpret_cast<float4*>(s0); p.Hk = Hk; p.Hv = Hv; p.h0 = h0; p.Hn = Hn; p.eps = eps;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   static DeviceOnce once;
   if (once.need()) {

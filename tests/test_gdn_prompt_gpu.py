@@ -134,3 +134,28 @@ def test_states_keep_fp32(dtype, lens, decay, Hk, Hv, fresh):
     rel = lambda x: ((x.double() - rec64).norm() / rec64.norm()).item()
     # 2^-25: half a unit in the last place of the states themselves, whichever way their last addition rounds
     assert rel(rec) <= rel(rec32) + 2.0 ** -25, (rel(rec), rel(rec32))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [1, 65, 200])
+def test_gates_at_odd_addresses(dtype, T):
+    """Gates are read in pairs where pairs are aligned: the other reads give the same bits."""
+    dev, Hk, Hv = "cuda", 2, 4
+    kd, vd = Hk * 128, Hv * 128
+    gen = torch.Generator(device=dev).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device=dev, generator=gen)
+    y, ab, norm_w = rnd(T, 2 * kd + vd).to(dtype), rnd(T, 2 * Hv).to(dtype), (1 + 0.1 * rnd(128)).to(dtype)
+    A_log, dt_bias, first = torch.log(0.3 + rnd(Hv).abs()), rnd(Hv), 0.2 * rnd(1, Hv, 128, 128)
+    plan, z, p = L._PromptPlan([0, T], [0], dev), rnd(T, vd).to(dtype), lambda t: t.data_ptr()
+    scratch = [torch.empty(plan.n_chunks * Hv * k, device=dev) for k in (64 * 64, 9 * 64, 128 * 64, 128 * 128)]
+    outs = []
+    for pad, at in ((0, 0), (1, 0), (2, 1)):                  # aligned; odd row distance; odd start
+        wide = torch.zeros(T, vd + pad, device=dev, dtype=dtype)
+        wide[:, at:at + vd] = z
+        rec, out = first.clone(), torch.empty(T, vd, device=dev, dtype=dtype)
+        rc = _lib.kernels().fb_gdn_prompt(p(y), 2 * kd + vd, p(ab[:, Hv:]), p(ab), 2 * Hv, p(wide[:, at:]), vd + pad, p(A_log), p(dt_bias), p(norm_w), p(rec), p(out),
+                                          p(plan.chunks), plan.n_chunks, p(plan.reqs), plan.n_reqs, *map(p, scratch), Hk, Hv, 0, Hv, 1e-6,
+                                          1 if dtype == torch.bfloat16 else 0, torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
