@@ -2,16 +2,17 @@
 //
 // One CTA owns one query head and 128 consecutive new tokens of one request and walks the pages in steps of 64 keys:
 //     S[128 q x 64 k] = Q * K^T        O[128 q x V] += P * V
-// Two score buffers: the tensor core makes the scores of step i + 1 while the softmax warps, a thread a query row, work on step i.  Keys and
+// Two score buffers: the tensor core makes the scores of step i + 1 while the softmax warps, two threads a query row, 32 keys each, work on step i.  Keys and
 // values have rings of their own (two steps each; a key step is free as soon as its scores exist).  At 256 x 256 the queries take 64 KB,
 // the rings 128 KB, P 32 KB, and O 256 of the 512 TMEM columns, so that one CTA fills an SM; K and V of a group's heads meet in the L2.  (Narrower
 // heads leave shared memory for a second CTA, but all columns are taken whatever V is: it waits for them.)
 // Probabilities enter the second product as two 16-bit terms (rounded value, rounded remainder): 16 bits of them in bf16.  In fp16 the terms are
 // scaled by 2^13, which the sum shares, so that what they leave out is 2^-38 of the largest weight.  O is rescaled only when a row's maximum has grown
 // by more than 2^8 (fp16: 2^2), which changes no rounding of P and keeps fp16 terms finite (up to 2^15).
-// Bound: latency of the one softmax warp on each sub-core, step after step (2000 tokens x 16 heads x 256: tensor pipe 42 % busy, special-function
-// unit 14 %, issue slots 21 %).
-// 4001 tokens x 16 heads x 256: 252 us (PyTorch, gathered fp32 keys and values and fp32 scores in memory: 7.0 ms).
+// The weights of a step are made in registers under the second product of the step before; only their way into shared memory waits for it.
+// Bound: the chain of a step through the softmax threads (scores, maximum, weights, P), two warps on each sub-core.
+// 4001 tokens x 16 heads x 256: 194 us; 216 with one thread a row, 258 when the weights waited for the product, too (PyTorch, gathered fp32 keys and
+// values and fp32 scores in memory: 7.0 ms).
 #include "ptx.cuh"
 #include "launch.h"
 #include "tmap.h"
@@ -26,7 +27,7 @@ constexpr int AX_KV = 64;                         // keys a step
 constexpr int AX_QT = AX_Q * 128;                 // bytes of a [128 x 64] tile
 constexpr int AX_KT = AX_KV * 128;                // bytes of a [64 x 64] tile
 constexpr int AX_PT = AX_Q * AX_KV * 2;
-constexpr int AX_THREADS = 192;
+constexpr int AX_THREADS = 320;                   // loads, products, two threads a query row
 
 struct AttnWideParams {
   const int* blocks;                              // [n][2] = (request, first new token)
@@ -70,7 +71,7 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) { mbar_init(&full_k[s], 1); mbar_init(&full_v[s], 1); mbar_init(&empty_k[s], 1); mbar_init(&empty_v[s], 1); mbar_init(&s_full[s], 1); }
-    mbar_init(q_full, 1); mbar_init(p_ready, 128); mbar_init(o_full, 1);
+    mbar_init(q_full, 1); mbar_init(p_ready, 256); mbar_init(o_full, 1);
     mbar_init_fence();
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
   }
@@ -133,41 +134,58 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     __syncwarp();
   } else {
-    const int q = warp & 3, r = q * 32 + lane, pos = pos0 + r;
+    const int q = warp & 3, half = (warp - 2) >> 2, r = q * 32 + lane, pos = pos0 + r, b0 = half * (AX_KV / 2);      // keys b0 .. b0 + 31 of a step
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
     uint8_t* prow = p_smem + r * 128;
+    float* rowx = reinterpret_cast<float*>(bars + 16);       // [2][128]
+    auto other = [&](float v) {                              // the number of the row's other thread
+      rowx[half * AX_Q + r] = v;
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + q) : "memory");
+      v = rowx[(half ^ 1) * AX_Q + r];
+      asm volatile("bar.sync %0, 64;\n" ::"r"(1 + q) : "memory");
+      return v;
+    };
     float m_run = -INFINITY, l_run = 0.f;
     for (int n = 0; n < n_steps; ++n) {
       mbar_wait(&s_full[n & 1], (uint32_t)(n >> 1) & 1u, dead, KID_ATTN_WIDE, 7);
       __syncwarp();
       tc_fence_after_sync();
-      uint32_t sr[64];
-      tmem_ld_32x32b_x32(tmem0 + (uint32_t)((n & 1) * AX_KV) + lane_off, sr);
-      tmem_ld_32x32b_x32(tmem0 + (uint32_t)((n & 1) * AX_KV) + lane_off + 32, sr + 32);
+      uint32_t sr[32];
+      tmem_ld_32x32b_x32(tmem0 + (uint32_t)((n & 1) * AX_KV) + lane_off + b0, sr);
       tmem_ld_wait();
       const int kv0 = n * AX_KV;
-      float m_new = m_run;
-      if (kv0 + AX_KV - 1 <= pos0) {                          // every row of the block sees the whole step
+      if (kv0 + AX_KV - 1 > pos0) {                           // a row of the block does not see the whole step
 #pragma unroll
-        for (int j = 0; j < 64; ++j) m_new = fmaxf(m_new, __uint_as_float(sr[j]));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          if (kv0 + j > pos) sr[j] = 0xff800000u;
-          m_new = fmaxf(m_new, __uint_as_float(sr[j]));
-        }
+        for (int j = 0; j < 32; ++j)
+          if (kv0 + b0 + j > pos) sr[j] = 0xff800000u;
       }
+      float mx[4] = {m_run, m_run, m_run, m_run};
+#pragma unroll
+      for (int j = 0; j < 32; ++j) mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(sr[j]));
+      float m_new = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      m_new = fmaxf(m_new, other(m_new));
       // (the first key is in step 0: from there on the maximum is finite)
       float alpha = 1.f;
       if ((m_new - m_run) * p.scale_log2 > (BF16 ? 8.f : 2.f)) { alpha = exp2f((m_run - m_new) * p.scale_log2); m_run = m_new; }
       const float m_use = m_run * p.scale_log2 - (BF16 ? 0.f : 13.f);
+      // P under the product of the step before: two scores give way to the first and the second terms of their weights
+      float la[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float p0 = exp2f(fmaf(__uint_as_float(sr[2 * j]), p.scale_log2, -m_use));
+        const float p1 = exp2f(fmaf(__uint_as_float(sr[2 * j + 1]), p.scale_log2, -m_use));
+        sr[2 * j] = pack_16<BF16>(p0, p1);
+        const float2 f = unpack_16<BF16>(sr[2 * j]);
+        sr[2 * j + 1] = pack_16<BF16>(p0 - f.x, p1 - f.y);
+        la[j & 3] += p0 + p1;
+      }
       if (n > 0) {
         mbar_wait(o_full, (uint32_t)(n - 1) & 1u, dead, KID_ATTN_WIDE, 8);      // P may be overwritten, O rescaled
         __syncwarp();
         tc_fence_after_sync();
         if (__any_sync(0xffffffffu, alpha != 1.f)) {
 #pragma unroll 1
-          for (int c0 = 0; c0 < vt * 64; c0 += 32) {
+          for (int c0 = half * 32; c0 < vt * 64; c0 += 64) {
             uint32_t o[32];
             tmem_ld_32x32b_x32(tmem_o + lane_off + c0, o);
             tmem_ld_wait();
@@ -178,28 +196,18 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           tmem_st_wait();
         }
       }
-      float l_add = 0.f;
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float p0 = exp2f(fmaf(__uint_as_float(sr[8 * g + 2 * j]), p.scale_log2, -m_use));
-          const float p1 = exp2f(fmaf(__uint_as_float(sr[8 * g + 2 * j + 1]), p.scale_log2, -m_use));
-          hi[j] = pack_16<BF16>(p0, p1);
-          const float2 f = unpack_16<BF16>(hi[j]);
-          lo[j] = pack_16<BF16>(p0 - f.x, p1 - f.y);
-          l_add += p0 + p1;
-        }
-        *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(prow + AX_PT + ((g ^ (r & 7)) << 4)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      for (int g = 0; g < 4; ++g) {
+        const int at = ((4 * half + g) ^ (r & 7)) << 4;
+        *reinterpret_cast<uint4*>(prow + at) = make_uint4(sr[8 * g], sr[8 * g + 2], sr[8 * g + 4], sr[8 * g + 6]);
+        *reinterpret_cast<uint4*>(prow + AX_PT + at) = make_uint4(sr[8 * g + 1], sr[8 * g + 3], sr[8 * g + 5], sr[8 * g + 7]);
       }
-      l_run = fmaf(l_run, alpha, l_add);
+      l_run = fmaf(l_run, alpha, (la[0] + la[1]) + (la[2] + la[3]));
       if (n == n_steps - 1 && pos0 + rows < kv0 + AX_KV) {
         // keys behind the block's last row have no weight, but what stands there may be no number: their values count as zeros.  (The
         // product of step n - 2, which had this buffer before, was issued ahead of this step's scores: the wait is for this step's values.)
         mbar_wait(&full_v[n & 1], (uint32_t)(n >> 1) & 1u, dead, KID_ATTN_WIDE, 10);
-        if ((r & 63) >= pos0 + rows - kv0) {
+        if (half == 0 && (r & 63) >= pos0 + rows - kv0) {
           uint4* vrow = reinterpret_cast<uint4*>(v_smem + (n & 1) * vt * AX_KT + (r & 63) * 128);
           for (int j = r >> 6; j < vt; j += 2)
 #pragma unroll
@@ -214,12 +222,13 @@ attn_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_wait(o_full, (uint32_t)(n_steps - 1) & 1u, dead, KID_ATTN_WIDE, 9);
       __syncwarp();
       tc_fence_after_sync();
-      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      const float l_sum = l_run + other(l_run);
+      const float inv = l_sum > 0.f ? 1.f / l_sum : 0.f;
       const bool live = r < rows;
       uint16_t* orow = p.out + (size_t)(row0 + r) * p.ld_out + (size_t)head * p.V;
       const uint16_t* grow = p.gate != nullptr ? p.gate + (size_t)(row0 + r) * p.ld_gate + (size_t)head * p.V : nullptr;
 #pragma unroll 1
-      for (int c0 = 0; c0 < p.V; c0 += 32) {
+      for (int c0 = half * 32; c0 < p.V; c0 += 64) {
         uint32_t o[32];
         __syncwarp();
         tmem_ld_32x32b_x32(tmem_o + lane_off + c0, o);
@@ -276,7 +285,7 @@ extern "C" int fb_attn_wide(const void* q, long long ld_q, int T, const void* k_
   const uint32_t fm = dtype == 1 ? 1u : 0u;
   p.idesc_s = make_idesc(fm, fm, 0, 0, 128, AX_KV);
   p.idesc_o = make_idesc(fm, fm, 0, 1, 128, p.vt * 64);
-  const int smem = p.dt * AX_QT + 2 * (p.dt + p.vt) * AX_KT + 2 * AX_PT + 256 + 1024;
+  const int smem = p.dt * AX_QT + 2 * (p.dt + p.vt) * AX_KT + 2 * AX_PT + 128 + 2 * AX_Q * 4 + 1024;
   static DeviceOnce cfg;
   if (cfg.need()) {
     cudaError_t e = cudaFuncSetAttribute(attn_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
