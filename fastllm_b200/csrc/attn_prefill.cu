@@ -260,11 +260,16 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 //   shared memory: Q_A, Q_B 64 KB | 4-stage ring of (K, V) half pages 128 KB | P_A, P_B 32 KB
 //
 // Bound: the softmax warps (64 exponentials a row and step are 1024 cycles of the special-function unit for both heads; the products of a step
-// take 1024, too).  The accumulator is rescaled only when a row's maximum has grown by more than 8 (a factor 256) since it was last rescaled: the
-// exponentials are then at most 256, which keeps their relative precision, and the sum carries the same factor.
+// take 1024, too).  The accumulator is rescaled where a row's new maximum has at least 1/32 of the row's weight so far, or has grown by a factor of 256:
+// weights above 1 keep their relative precision, but only the maximum's own weight, 1, is not rounded, and that tells where it is a large part of the sum.
+// The sum is that of the rounded weights.  Errors against 64 bits, bf16, standard deviations 0.5, 1, 2, 3 of the logits, 1638 tokens: 2.07, 2.02, 1.84,
+// 1.75e-3 (rescaled at every new maximum, sum of the weights before rounding: 2.09, 2.03, 1.85, 1.76; only at a factor of 256: 2.08, 2.07, 2.01, 1.89).
+// us, unit logits, one S tile a head and a rescaling at every new maximum before: 5 x 1638 tokens, 32 / 8 heads 250 -> 216, 3 x 1365, 32 / 4 124 -> 107,
+// 1 x 4000 247 -> 190, 1 x 8192, 32 / 8 824 -> 599.
 // ---------------------------------------------------------------------------------------------------
 constexpr int AP2_KV = 64;
 constexpr int AP2_STAGES = 4;
+constexpr float AP2_SHARE = 32.f;                 // a new maximum of a smaller part of the sum than 1 / 32 rescales nothing
 constexpr float AP2_GROWTH = 8.f;                 // log2 of the factor that the exponentials may exceed 1 by
 constexpr int AP2_KT = AP2_KV * 128 * 2;          // 16 KB: 64 rows x 128 values, two 8 KB halves (64 dims each)
 constexpr int AP2_PT = 128 * AP2_KV * 2;          // 16 KB: 128 query rows x 64 probabilities
@@ -434,7 +439,7 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         mbar_wait(&o_full[h], iph ^ 1u, dead, KID_ATTN_PREFILL, 18);
         tc_fence_after_sync();
       }
-      if (__any_sync(0xffffffffu, !(m_new <= m_run + AP2_GROWTH))) {
+      if (__any_sync(0xffffffffu, m_new > m_run && !(m_new <= m_run + AP2_GROWTH && exp2f(m_new - m_run) * AP2_SHARE <= l_run))) {
         const float alpha = exp2f(m_run - (m_new == -INFINITY ? 0.f : m_new));
         if (it > 0) {
 #pragma unroll 1
@@ -464,7 +469,8 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           p0 = exp2f(p0);
           p1 = exp2f(p1);
           pk[j] = pack_16<BF16>(p0, p1);
-          l2[j] = add_f32x2(l2[j], pack_f32x2(p0, p1));
+          const float2 back = unpack_16<BF16>(pk[j]);         // (the sum of what the product sees: a row's peak, rounded alike in both, stays exact)
+          l2[j] = add_f32x2(l2[j], pack_f32x2(back.x, back.y));
         }
         *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }

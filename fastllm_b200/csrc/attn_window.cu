@@ -93,7 +93,7 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* v_clean = bars + 25;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   // Plain softmax and values of at most 128: tensor memory holds two score tiles a block, and the scores of a step are there when the softmax of the step
-  // before ends (latent prompts of 2 x 2000 tokens, 16 heads of 192 + 128: 89 -> 81 us).
+  // before ends (latent prompts of 2 x 2000 tokens, 16 heads of 192 + 128: 89 -> 86 us).
   const bool two_s = !EXT && vt <= 2;
   const int ahead = two_s ? 2 : 1;
 
@@ -359,9 +359,9 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         mbar_wait(&o_full[b], iph ^ 1u, dead, KID_ATTN_WINDOW, 9);
         tc_fence_after_sync();
       }
-      // Rescaled only where some row's maximum has grown by more than 8 since it last was: exponentials of up to 256 keep their relative precision,
-      // and the sum carries the same factor (some row of 32 has a new maximum in most steps).
-      if (__any_sync(0xffffffffu, !(m_new <= m_run + 8.f))) {
+      // Rescaled where some row's new maximum has at least 1/32 of the row's weight so far, or has grown by a factor of 256: weights above 1 keep their relative
+      // precision, but only the maximum's own weight, 1, is not rounded.  Errors against 64 bits are not larger than with a rescaling at every new maximum.
+      if (__any_sync(0xffffffffu, m_new > m_run && !(m_new <= m_run + 8.f && exp2f(m_new - m_run) * 32.f <= l_run))) {
         const float alpha = exp2f(m_run - (m_new == -INFINITY ? 0.f : m_new));
         if (n > 0) {
 #pragma unroll 1
@@ -388,7 +388,8 @@ attn_window_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           const float p0 = exp2f(__uint_as_float(sreg[8 * g + 2 * j]) - m_use);
           const float p1 = exp2f(__uint_as_float(sreg[8 * g + 2 * j + 1]) - m_use);
           pk[j] = pack_16<BF16>(p0, p1);
-          l4[j] += p0 + p1;
+          const float2 back = unpack_16<BF16>(pk[j]);         // (the sum of what the product sees: a row's peak, rounded alike in both, stays exact)
+          l4[j] += back.x + back.y;
         }
         *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
