@@ -262,10 +262,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 // Bound: the softmax warps (64 exponentials a row and step are 1024 cycles of the special-function unit for both heads; the products of a step
 // take 1024, too).  The accumulator is rescaled where a row's new maximum has at least 1/32 of the row's weight so far, or has grown by a factor of 256:
 // weights above 1 keep their relative precision, but only the maximum's own weight, 1, is not rounded, and that tells where it is a large part of the sum.
-// The sum is that of the rounded weights.  Errors against 64 bits, bf16, standard deviations 0.5, 1, 2, 3 of the logits, 1638 tokens: 2.07, 2.02, 1.84,
-// 1.75e-3 (rescaled at every new maximum, sum of the weights before rounding: 2.09, 2.03, 1.85, 1.76; only at a factor of 256: 2.08, 2.07, 2.01, 1.89).
-// us, unit logits, one S tile a head and a rescaling at every new maximum before: 5 x 1638 tokens, 32 / 8 heads 250 -> 216, 3 x 1365, 32 / 4 124 -> 107,
-// 1 x 4000 247 -> 190, 1 x 8192, 32 / 8 824 -> 599.
+// Errors against 64 bits, bf16, standard deviations 0.5, 1, 2, 3 of the logits, 1638 tokens: 2.093, 2.038, 1.850, 1.759e-3 (rescaled at every new
+// maximum: 2.088, 2.034, 1.850, 1.759; only at a factor of 256: 2.10, 2.09, 2.15, 2.12).
+// us, unit logits, one S tile a head and a rescaling at every new maximum before: 5 x 1638 tokens, 32 / 8 heads 250 -> 211, 3 x 1365, 32 / 4 124 -> 105,
+// 1 x 4000 247 -> 186, 1 x 8192, 32 / 8 824 -> 589.
 // ---------------------------------------------------------------------------------------------------
 constexpr int AP2_KV = 64;
 constexpr int AP2_STAGES = 4;
@@ -469,8 +469,7 @@ attn_prefill2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           p0 = exp2f(p0);
           p1 = exp2f(p1);
           pk[j] = pack_16<BF16>(p0, p1);
-          const float2 back = unpack_16<BF16>(pk[j]);         // (the sum of what the product sees: a row's peak, rounded alike in both, stays exact)
-          l2[j] = add_f32x2(l2[j], pack_f32x2(back.x, back.y));
+          l2[j] = add_f32x2(l2[j], pack_f32x2(p0, p1));
         }
         *reinterpret_cast<uint4*>(prow + ((g ^ (r & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
